@@ -440,6 +440,31 @@ int bhi_ans_encode(const uint8_t *data, int streams, int n, const uint32_t *freq
     return launch_status("ans_encode launch");
 }
 
+int bhi_split_histogram(const uint16_t *W, int rows, int K, int split_k, uint8_t *A_rem, int M, int row0, uint64_t *histogram,
+                        void *stream) {
+    if (int rc = check_enc(W, rows, K, split_k)) return rc;
+    BHI_REQUIRE(A_rem || histogram, "nothing to write");
+    BHI_REQUIRE(aligned(A_rem, 4) && aligned(histogram, 8), "unaligned output");
+    BHI_REQUIRE(row0 >= 0 && static_cast<int64_t>(row0) + rows <= M, "rows outside the layer");
+    const int64_t groups = (static_cast<int64_t>(rows) * (K >> 7) + kSplitUnroll - 1) / kSplitUnroll;
+    const int64_t need = (groups + kSplitThreads / 32 - 1) / (kSplitThreads / 32);
+    const int64_t cap = static_cast<int64_t>(sm_count()) * 6;       // six blocks of 32 KB fit an SM
+    split_histogram_kernel<<<static_cast<int>(need < cap ? need : cap), kSplitThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const uint32_t *>(W), rows, row0, M, K >> 7, (K / split_k) >> 7, A_rem,
+        reinterpret_cast<unsigned long long *>(histogram));
+    return launch_status("split pass launch");
+}
+
+int bhi_record_offsets(const int32_t *words_per_row, int split_k, int M, int slab_rows, int32_t *offsets, int64_t *total,
+                       void *stream) {
+    BHI_REQUIRE(words_per_row && offsets && total, "null buffer");
+    BHI_REQUIRE(split_k >= 1 && M >= 1 && slab_rows >= 1, "bad shape");
+    BHI_REQUIRE(aligned(words_per_row, 4) && aligned(offsets, 4) && aligned(total, 8), "unaligned buffer");
+    record_offsets_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        words_per_row, static_cast<int64_t>(split_k) * M, M, slab_rows, offsets, total);
+    return launch_status("record offsets launch");
+}
+
 int bhi_huffman_size_pass(const uint16_t *W, int M, int K, int split_k, const uint8_t *code_lengths,
                           int32_t *words_per_row, void *stream) {
     if (int rc = check_enc(W, M, K, split_k)) return rc;
@@ -464,7 +489,7 @@ int bhi_huffman_emit_pass(const uint16_t *W, int M, int K, int split_k, const ui
                           const uint32_t *code_values, const int32_t *offsets,
                           uint8_t *A_rem, uint32_t *A_exp, void *stream) {
     if (int rc = check_enc(W, M, K, split_k)) return rc;
-    BHI_REQUIRE(code_lengths && code_values && offsets && A_rem && A_exp, "null buffer");
+    BHI_REQUIRE(code_lengths && code_values && offsets && A_exp, "null buffer");
     BHI_REQUIRE(aligned(A_rem, 2) && aligned(A_exp, 4), "unaligned output");
     EncGeom g{W, M, K, split_k, K / split_k};
     huffman_emit_kernel<<<enc_blocks(M, split_k), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -476,7 +501,7 @@ int bhi_ans_emit_pass(const uint16_t *W, int M, int K, int split_k, const uint32
                       const uint32_t *cum, const int32_t *offsets, const uint8_t *stream_words,
                       uint8_t *A_rem, uint32_t *A_exp, void *stream) {
     if (int rc = check_enc(W, M, K, split_k)) return rc;
-    BHI_REQUIRE(freq && cum && offsets && stream_words && A_rem && A_exp, "null buffer");
+    BHI_REQUIRE(freq && cum && offsets && stream_words && A_exp, "null buffer");
     BHI_REQUIRE(aligned(A_rem, 2) && aligned(A_exp, 4), "unaligned output");
     EncGeom g{W, M, K, split_k, K / split_k};
     ans_emit_kernel<<<enc_blocks(M, split_k), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(

@@ -393,6 +393,41 @@ EncView enc_of(const Tensor &W, int64_t split_k) {
     return {static_cast<int>(W.size(0)), static_cast<int>(W.size(1)), static_cast<int>(split_k)};
 }
 
+// split_histogram(W, split_k, row0, rem(a!), histogram(b!)) -> ()   (W: rows row0.. of the layer that rem belongs to)
+void boxed_split_histogram(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor W = arg(stack, 0), rem = arg(stack, 3), hist = arg(stack, 4);
+    const int64_t row0 = iarg(stack, 2);
+    EncView v = enc_of(W, iarg(stack, 1));
+    want(rem, ScalarType::Byte, "rem");
+    want(hist, ScalarType::Long, "histogram");
+    same_device(W, rem, "rem");
+    same_device(W, hist, "histogram");
+    STD_TORCH_CHECK(hist.numel() == 256, "histogram must have 256 entries");
+    int64_t M = row0 + v.M;
+    if (rem.numel()) {
+        STD_TORCH_CHECK(rem.numel() % v.K == 0, "rem must be [split_k, M, K/split_k]");
+        M = rem.numel() / v.K;
+    }
+    STD_TORCH_CHECK(row0 >= 0 && row0 + v.M <= M && M < (int64_t{1} << 31), "rows outside the layer");
+    torch::stable::accelerator::DeviceGuard guard(W.get_device_index());
+    check(bhi_split_histogram(ptr<const uint16_t>(W), v.M, v.K, v.S, rem.numel() ? ptr<uint8_t>(rem) : nullptr,
+                              static_cast<int>(M), static_cast<int>(row0), ptr<uint64_t>(hist), stream_of(W)));
+}
+
+// record_offsets(words_per_row, slab_rows, offsets(a!), total(b!)) -> ()
+void boxed_record_offsets(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor rows = arg(stack, 0), off = arg(stack, 2), total = arg(stack, 3);
+    want(rows, ScalarType::Int, "words_per_row", 2);
+    want(off, ScalarType::Int, "offsets", 2);
+    want(total, ScalarType::Long, "total");
+    same_device(rows, off, "offsets");
+    same_device(rows, total, "total");
+    STD_TORCH_CHECK(off.numel() == rows.numel() && total.numel() == 1, "offsets must be [split_k, M] and total [1]");
+    torch::stable::accelerator::DeviceGuard guard(rows.get_device_index());
+    check(bhi_record_offsets(ptr<const int32_t>(rows), static_cast<int>(rows.size(0)), static_cast<int>(rows.size(1)),
+                             static_cast<int>(iarg(stack, 1)), ptr<int32_t>(off), ptr<int64_t>(total), stream_of(rows)));
+}
+
 // huffman_size_pass(W, split_k, code_lengths, words_per_row(a!)) -> ()
 void boxed_huffman_size_pass(StableIValue *stack, uint64_t, uint64_t) {
     Tensor W = arg(stack, 0), len = arg(stack, 2), rows = arg(stack, 3);
@@ -421,10 +456,10 @@ void boxed_huffman_emit_pass(StableIValue *stack, uint64_t, uint64_t) {
     for (const Tensor *t : {&len, &val, &off, &rem, &exp}) same_device(W, *t, "an encoder buffer");
     STD_TORCH_CHECK(len.numel() == 256 && val.numel() == 256, "code tables must have 256 entries");
     STD_TORCH_CHECK(off.numel() == static_cast<int64_t>(v.S) * v.M, "offsets must be [split_k, M]");
-    STD_TORCH_CHECK(rem.numel() == W.numel(), "rem must be [split_k, M, K/split_k]");
+    STD_TORCH_CHECK(rem.numel() == W.numel() || rem.numel() == 0, "rem must be [split_k, M, K/split_k], or empty");
     torch::stable::accelerator::DeviceGuard guard(W.get_device_index());
     check(bhi_huffman_emit_pass(ptr<const uint16_t>(W), v.M, v.K, v.S, ptr<const uint8_t>(len), ptr<const uint32_t>(val),
-                                ptr<const int32_t>(off), ptr<uint8_t>(rem), ptr<uint32_t>(exp), stream_of(W)));
+                                ptr<const int32_t>(off), rem.numel() ? ptr<uint8_t>(rem) : nullptr, ptr<uint32_t>(exp), stream_of(W)));
 }
 
 // ans_size_pass(W, split_k, freq, cum, words_per_row(a!), stream_words(b!)) -> ()
@@ -459,10 +494,10 @@ void boxed_ans_emit_pass(StableIValue *stack, uint64_t, uint64_t) {
     STD_TORCH_CHECK(freq.numel() == 256 && cum.numel() == 256, "freq and cum must have 256 entries");
     STD_TORCH_CHECK(off.numel() == static_cast<int64_t>(v.S) * v.M, "offsets must be [split_k, M]");
     STD_TORCH_CHECK(sw.numel() == static_cast<int64_t>(v.S) * v.M * 64, "stream_words must be [split_k, M, 64]");
-    STD_TORCH_CHECK(rem.numel() == W.numel(), "rem must be [split_k, M, K/split_k]");
+    STD_TORCH_CHECK(rem.numel() == W.numel() || rem.numel() == 0, "rem must be [split_k, M, K/split_k], or empty");
     torch::stable::accelerator::DeviceGuard guard(W.get_device_index());
     check(bhi_ans_emit_pass(ptr<const uint16_t>(W), v.M, v.K, v.S, ptr<const uint32_t>(freq), ptr<const uint32_t>(cum),
-                            ptr<const int32_t>(off), ptr<const uint8_t>(sw), ptr<uint8_t>(rem), ptr<uint32_t>(exp),
+                            ptr<const int32_t>(off), ptr<const uint8_t>(sw), rem.numel() ? ptr<uint8_t>(rem) : nullptr, ptr<uint32_t>(exp),
                             stream_of(W)));
 }
 
@@ -487,6 +522,8 @@ STABLE_TORCH_LIBRARY(BHI_TORCH_NAMESPACE, m) {
     m.def("gemv_bf16_ans_exchange(Tensor A_rem, Tensor A_exp, Tensor X, Tensor offsets, Tensor LUT, Tensor peers, int rank, int row_base, int m_total) -> ()");
     m.def("set_launch_overlap(int on) -> int");
     // whole-layer encoder
+    m.def("split_histogram(Tensor W, int split_k, int row0, Tensor(a!) rem, Tensor(b!) histogram) -> ()");
+    m.def("record_offsets(Tensor words_per_row, int slab_rows, Tensor(a!) offsets, Tensor(b!) total) -> ()");
     m.def("huffman_size_pass(Tensor W, int split_k, Tensor code_lengths, Tensor(a!) words_per_row) -> ()");
     m.def("huffman_emit_pass(Tensor W, int split_k, Tensor code_lengths, Tensor code_values, Tensor offsets, Tensor(a!) rem, Tensor(b!) exp) -> ()");
     m.def("ans_size_pass(Tensor W, int split_k, Tensor freq, Tensor cum, Tensor(a!) words_per_row, Tensor(b!) stream_words) -> ()");
@@ -512,6 +549,8 @@ STABLE_TORCH_LIBRARY_IMPL(BHI_TORCH_NAMESPACE, CUDA, m) {
     m.impl("linear_bf16_ans", &boxed_linear_bf16_ans);
     m.impl("gemv_bf16_huffman_exchange", &boxed_gemv_bf16_huffman_exchange);
     m.impl("gemv_bf16_ans_exchange", &boxed_gemv_bf16_ans_exchange);
+    m.impl("split_histogram", &boxed_split_histogram);
+    m.impl("record_offsets", &boxed_record_offsets);
     m.impl("huffman_size_pass", &boxed_huffman_size_pass);
     m.impl("huffman_emit_pass", &boxed_huffman_emit_pass);
     m.impl("ans_size_pass", &boxed_ans_size_pass);

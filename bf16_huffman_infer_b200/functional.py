@@ -13,16 +13,17 @@ uses for that are still available (``compress_groups``) and produce the same wor
 """
 from __future__ import annotations
 
-from typing import Dict, Optional, Tuple
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import os
 
+import numpy as np
 import torch
 import torch.nn.functional as F
 from torch import Tensor, nn
 from tqdm import tqdm
 
-from . import ops
+from . import ops, transfer
 from .ans import RANSEncoder
 from .huffman import LUTHuffmanEncoder
 from .utils import get_block_size_n, split_bf16
@@ -96,7 +97,12 @@ def _work_device(a: Tensor) -> torch.device:
 
 def _exp_histogram(a: Tensor) -> Tensor:
     """256 exponent counts of a BF16 tensor (int64, on the CPU)."""
-    bits = a.contiguous().view(torch.int16).flatten()
+    a = a.detach().contiguous()
+    if a.is_cuda and a.numel() % 128 == 0 and 0 < a.numel() < 2 ** 38 and a.data_ptr() % 4 == 0:
+        counts = torch.zeros(256, dtype=torch.int64, device=a.device)
+        ops.split_histogram(a.view(-1, 128), 1, 0, torch.empty(0, dtype=torch.uint8, device=a.device), counts)
+        return counts.cpu()
+    bits = a.view(torch.int16).flatten()
     exp = ((bits >> 7) & 0xFF).to(torch.int64)
     return torch.bincount(exp, minlength=256).cpu()
 
@@ -110,16 +116,101 @@ def _record_offsets(words_per_row: Tensor) -> Tuple[Tensor, int]:
     ``:204-231``).
     """
     S, M = words_per_row.shape
+    if words_per_row.is_cuda:
+        offsets, total = _record_offsets_async(words_per_row)
+        return offsets, _checked_total(int(total.item()))
     sizes = words_per_row.to(torch.int64) * 64
     pad = torch.zeros(M, dtype=torch.int64, device=sizes.device)
     pad[SLAB_ROWS - 1::SLAB_ROWS] = 64
     pad[M - 1] = 64
     sizes = (sizes + pad[None, :]).flatten()
     ends = torch.cumsum(sizes, 0)
-    total = int(ends[-1].item())
+    total = _checked_total(int(ends[-1].item()))
+    return (ends - sizes).to(torch.int32).view(S, M), total
+
+
+def _record_offsets_async(words_per_row: Tensor) -> Tuple[Tensor, Tensor]:
+    """Same on the device, without waiting for it: offsets, and the total as an i64 tensor of one value."""
+    offsets = torch.empty_like(words_per_row)
+    total = torch.empty(1, dtype=torch.int64, device=words_per_row.device)
+    ops.record_offsets(words_per_row, SLAB_ROWS, offsets, total)
+    return offsets, total
+
+
+def _checked_total(total: int) -> int:
     if total >= 2 ** 31:
         raise RuntimeError("compressed exponent plane exceeds 2^31 words; split the layer")
-    return (ends - sizes).to(torch.int32).view(S, M), total
+    return total
+
+
+class _Ingested:
+    """A dense layer on the device with what its one pass over the weight yields: the sign/mantissa plane and the
+    exponent counts.  A weight in host memory is passed over slab by slab while the rest is still on its way."""
+
+    def __init__(self, a: Tensor, split_k: int):
+        assert a.dim() == 2 and a.dtype == torch.bfloat16
+        assert a.size(1) % split_k == 0 and (a.size(1) // split_k) % 128 == 0, a.shape
+        a = a.detach()
+        dev = _work_device(a)
+        M, K = a.shape
+        self.split_k = split_k
+        self.rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8, device=dev)
+        counts = torch.zeros(256, dtype=torch.int64, device=dev)
+        if a.is_cuda:
+            self.w = a.contiguous()
+            ops.split_histogram(self.w, split_k, 0, self.rem, counts)
+        else:
+            self.w = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
+            transfer.upload_rows(a, self.w, lambda lo, hi: ops.split_histogram(self.w[lo:hi], split_k, lo, self.rem, counts))
+        self.histogram = counts.cpu()
+
+
+class _Plan:
+    """One coder's measure of a layer: its tables on the device and where every record will lie."""
+
+    def __init__(self, cls, layer: _Ingested, codec):
+        self.cls, self.layer, self.codec = cls, layer, codec
+        self.luts = cls.get_lut_kwargs(codec)
+        self.tables = cls._encoder_tables(codec, layer.w.device)
+        rows = torch.empty(layer.rem.shape[:2], dtype=torch.int32, device=layer.w.device)
+        cls._size_pass(layer, self.tables, rows)
+        self.offsets, self.total = _record_offsets_async(rows)
+
+    def finish(self, total: int, to_cpu: bool) -> "HuffmanWeight":
+        layer, dev = self.layer, self.layer.w.device
+        exp = torch.zeros(_checked_total(total), dtype=torch.int32, device=dev)
+        self.cls._emit_pass(layer, self.tables, self.offsets, exp)
+        if to_cpu:
+            return self.cls(rem=transfer.download(layer.rem), exp=transfer.download(exp),
+                            offsets=transfer.download(self.offsets), **self.luts)
+        luts = _tables_to(self.luts, dev)
+        # the buffers must be complete in memory before a fused kernel with launch overlap reads them
+        torch.cuda.current_stream(dev).synchronize()
+        return self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **luts)
+
+
+def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor]:
+    """Small host tensors on the device, each in memory of its own, through one copy."""
+    raw = [np.ascontiguousarray(t.numpy()).reshape(-1).view(np.uint8) for t in tables.values()]
+    packed = torch.from_numpy(np.concatenate(raw)).to(dev)
+    out, at = {}, 0
+    for (name, t), r in zip(tables.items(), raw):
+        out[name] = packed[at:at + r.size].view(t.dtype).view(t.shape).clone()
+        at += r.size
+    return out
+
+
+def _compress(a: Tensor, split_k: int, coders: Sequence[type], to_cpu: bool) -> "HuffmanWeight":
+    """``a`` by the coder that stores it in the fewest bytes (the first of those that tie).  The sizes are known after
+    the size pass, so only the coder that is kept writes its records."""
+    layer = _Ingested(a, split_k)
+    plans: List[_Plan] = [_Plan(c, layer, c._codec_of(layer.histogram)) for c in coders]
+    totals = torch.cat([p.total for p in plans]).tolist() if len(plans) > 1 else [int(plans[0].total.item())]
+    for t in totals:
+        _checked_total(t)
+    sizes = [4 * t + sum(v.nelement() * v.element_size() for v in p.luts.values()) for p, t in zip(plans, totals)]
+    best = min(range(len(plans)), key=sizes.__getitem__)
+    return plans[best].finish(totals[best], to_cpu)
 
 
 def mv_huffman(
@@ -274,8 +365,12 @@ class HuffmanWeight(nn.Module):
     @classmethod
     def get_codec(cls, a: Tensor) -> LUTHuffmanEncoder:
         """Code tables from the exponent histogram of ``a`` (reference ``functional.py:110-117``)."""
+        return cls._codec_of(_exp_histogram(a.to(_work_device(a))))
+
+    @classmethod
+    def _codec_of(cls, histogram: Tensor) -> LUTHuffmanEncoder:
         codec = LUTHuffmanEncoder()
-        codec.build_lut(_exp_histogram(a.to(_work_device(a))), method=HUFFMAN_TABLES)
+        codec.build_lut(histogram, method=HUFFMAN_TABLES)
         return codec
 
     @classmethod
@@ -313,42 +408,22 @@ class HuffmanWeight(nn.Module):
         return packed.view(torch.int32), row_words.to(torch.int32)
 
     @classmethod
-    def _tables_on(cls, codec, dev) -> Dict[str, Tensor]:
-        return {
-            "code_lengths": torch.from_numpy(codec.code_lengths.copy()).to(dev),
-            "code_values": torch.from_numpy(codec.code_values.view("int32").copy()).to(dev),
-        }
+    def _encoder_tables(cls, codec, dev) -> Dict[str, Tensor]:
+        return _tables_to({"code_values": torch.from_numpy(codec.code_values.view("int32")),
+                           "code_lengths": torch.from_numpy(codec.code_lengths)}, dev)
 
     @classmethod
-    def _encode_layer(cls, w: Tensor, split_k: int, codec) -> Tuple[Tensor, Tensor, Tensor]:
-        """Two-pass device encode of ``w`` (BF16 ``[M, K]`` on a CUDA device)."""
-        dev = w.device
-        M, K = w.shape
-        t = cls._tables_on(codec, dev)
-        rows = torch.empty(split_k, M, dtype=torch.int32, device=dev)
-        ops.huffman_size_pass(w, split_k, t["code_lengths"], rows)
-        offsets, total = _record_offsets(rows)
-        rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8, device=dev)
-        exp = torch.zeros(total, dtype=torch.int32, device=dev)
-        ops.huffman_emit_pass(w, split_k, t["code_lengths"], t["code_values"], offsets, rem, exp)
-        return rem, exp, offsets
+    def _size_pass(cls, layer: _Ingested, t: Dict[str, Tensor], rows: Tensor) -> None:
+        ops.huffman_size_pass(layer.w, layer.split_k, t["code_lengths"], rows)
+
+    @classmethod
+    def _emit_pass(cls, layer: _Ingested, t: Dict[str, Tensor], offsets: Tensor, exp: Tensor) -> None:
+        ops.huffman_emit_pass(layer.w, layer.split_k, t["code_lengths"], t["code_values"], offsets, layer.rem.new_empty(0), exp)
 
     @classmethod
     def compress_split_n(cls, a: Tensor, n: int = 2, to_cpu: bool = True):
         """Encode ``a`` with ``n`` K-chunks (reference ``functional.py:195-238``)."""
-        assert a.dim() == 2 and a.dtype == torch.bfloat16
-        assert a.size(1) % n == 0 and (a.size(1) // n) % 128 == 0, a.shape
-        w = a.detach().to(_work_device(a)).contiguous()
-        codec = cls.get_codec(w)
-        rem, exp, offsets = cls._encode_layer(w, n, codec)
-        # the buffers must be complete in memory before a fused kernel with launch overlap reads them
-        torch.cuda.current_stream(w.device).synchronize()
-        if to_cpu:
-            rem, exp, offsets = rem.cpu(), exp.cpu(), offsets.cpu()
-            luts = cls.get_lut_kwargs(codec)
-        else:
-            luts = {k: v.to(w.device) for k, v in cls.get_lut_kwargs(codec).items()}
-        return cls(rem=rem, exp=exp, offsets=offsets, **luts)
+        return _compress(a, n, (cls,), to_cpu)
 
     @classmethod
     def compress(cls, a: Tensor, to_cpu: bool = True):
@@ -386,14 +461,20 @@ class ANSWeight(HuffmanWeight):
 
     @classmethod
     def get_codec(cls, a: Tensor) -> RANSEncoder:
-        return RANSEncoder(_exp_histogram(a.to(_work_device(a))).tolist(), precision=ANS_PRECISION)
+        return cls._codec_of(_exp_histogram(a.to(_work_device(a))))
+
+    @classmethod
+    def _codec_of(cls, histogram: Tensor) -> RANSEncoder:
+        return RANSEncoder(histogram.tolist(), precision=ANS_PRECISION)
 
     @classmethod
     def get_lut_kwargs(cls, codec: RANSEncoder) -> Dict[str, Tensor]:
         if max(codec.freq) > 0xFFF:
             raise ValueError("one exponent value holds the whole 12-bit model: its frequency does not fit the table word")
-        lut = torch.tensor(codec.decode_lut, dtype=torch.int32)
-        return {"LUT": (lut[:, 0] << 24) | (lut[:, 1] << 12) | lut[:, 2]}
+        freq, cum = np.array(codec.freq), np.array(codec.cum)
+        sym = np.repeat(np.arange(256), freq)
+        words = (sym << 24) | (freq[sym] << 12) | (np.arange(sym.size) - cum[sym])
+        return {"LUT": torch.from_numpy(words.astype(np.uint32).view(np.int32))}
 
     @classmethod
     def compress_groups(cls, x: Tensor, codec: RANSEncoder) -> Tuple[Tensor, Tensor]:
@@ -409,19 +490,18 @@ class ANSWeight(HuffmanWeight):
         return words, counts.view(rows, groups).amax(dim=1)
 
     @classmethod
-    def _encode_layer(cls, w: Tensor, split_k: int, codec) -> Tuple[Tensor, Tensor, Tensor]:
-        dev = w.device
-        M, K = w.shape
-        freq = torch.tensor(codec.freq, dtype=torch.int32, device=dev)
-        cum = torch.tensor(codec.cum, dtype=torch.int32, device=dev)
-        rows = torch.empty(split_k, M, dtype=torch.int32, device=dev)
-        per_stream = torch.empty(split_k, M, 64, dtype=torch.uint8, device=dev)
-        ops.ans_size_pass(w, split_k, freq, cum, rows, per_stream)
-        offsets, total = _record_offsets(rows)
-        rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8, device=dev)
-        exp = torch.zeros(total, dtype=torch.int32, device=dev)
-        ops.ans_emit_pass(w, split_k, freq, cum, offsets, per_stream, rem, exp)
-        return rem, exp, offsets
+    def _encoder_tables(cls, codec, dev) -> Dict[str, Tensor]:
+        return _tables_to({"freq": torch.tensor(codec.freq, dtype=torch.int32),
+                           "cum": torch.tensor(codec.cum, dtype=torch.int32)}, dev)
+
+    @classmethod
+    def _size_pass(cls, layer: _Ingested, t: Dict[str, Tensor], rows: Tensor) -> None:
+        t["stream_words"] = torch.empty(*rows.shape, 64, dtype=torch.uint8, device=rows.device)
+        ops.ans_size_pass(layer.w, layer.split_k, t["freq"], t["cum"], rows, t["stream_words"])
+
+    @classmethod
+    def _emit_pass(cls, layer: _Ingested, t: Dict[str, Tensor], offsets: Tensor, exp: Tensor) -> None:
+        ops.ans_emit_pass(layer.w, layer.split_k, t["freq"], t["cum"], offsets, t["stream_words"], layer.rem.new_empty(0), exp)
 
 
 class CompressedLinear(nn.Module):
@@ -478,37 +558,38 @@ def _buffers_size(w: nn.Module) -> int:
     return sum(b.nelement() * b.element_size() for b in w.buffers())
 
 
+_CODERS = {"huffman": (HuffmanWeight,), "ans": (ANSWeight,), "smallest": (HuffmanWeight, ANSWeight)}
+
+
+def _compress_for(a: Tensor, algo: str) -> HuffmanWeight:
+    """``a`` compressed as ``algo`` says, on the device it is on."""
+    assert algo in _CODERS
+    return _compress(a, get_block_size_n(a)[0], _CODERS[algo], to_cpu=not a.is_cuda)
+
+
 def convert(linear: nn.Linear, name, disable_precision_check: bool = True, algo: str = "huffman"):
     """Compress one ``nn.Linear``; returns a :class:`CompressedLinear`, or ``linear`` itself when
     compression does not pay (ratio >= 1) or, if checking is enabled, when the fused output is off
     by 2 % or more on a random input (reference ``functional.py:323-375``).  The module comes back
     on the device ``linear`` was on."""
-    assert algo in ("huffman", "ans", "smallest")
     home = linear.weight.device
-    if algo == "huffman":
-        weight = HuffmanWeight.compress(linear.weight)
-    elif algo == "ans":
-        weight = ANSWeight.compress(linear.weight)
-    else:
-        weight = min(
-            [HuffmanWeight.compress(linear.weight), ANSWeight.compress(linear.weight)],
-            key=_buffers_size,
-        )
-    module = CompressedLinear(weight=weight, bias=linear.bias)
+    module = CompressedLinear(weight=_compress_for(linear.weight, algo), bias=linear.bias)
 
     ori_size = linear.weight.nelement() * linear.weight.element_size()
     ratio = _buffers_size(module.weight) / ori_size
 
-    work = _work_device(linear.weight)
-    linear.to(work)
-    module.to(work)
-    x = torch.randn(1, linear.in_features, dtype=torch.bfloat16, device=work)
-    with torch.no_grad():
-        y1 = linear(x)
-        y2 = module(x)
-    max_rtol = ((y2 - y1).abs() / y1.abs().clamp(min=1e-4)).max().item()
-    linear.to(home)
-    module.to(home)
+    max_rtol = 0.0
+    if not disable_precision_check:
+        work = _work_device(linear.weight)
+        linear.to(work)
+        module.to(work)
+        x = torch.randn(1, linear.in_features, dtype=torch.bfloat16, device=work)
+        with torch.no_grad():
+            y1 = linear(x)
+            y2 = module(x)
+        max_rtol = ((y2 - y1).abs() / y1.abs().clamp(min=1e-4)).max().item()
+        linear.to(home)
+        module.to(home)
 
     fallback = False
     if ratio >= 1:
@@ -606,12 +687,7 @@ def fuse_sibling_linears(model: nn.Module, groups=SIBLING_GROUPS, algo: str = "h
         home = mods[0].weight.device
         stacked = torch.cat([m.weight.detach() for m in mods], dim=0)
         bias = None if mods[0].bias is None else nn.Parameter(torch.cat([m.bias.detach() for m in mods]), requires_grad=False)
-        if algo == "huffman":
-            weight = HuffmanWeight.compress(stacked)
-        elif algo == "ans":
-            weight = ANSWeight.compress(stacked)
-        else:
-            weight = min([HuffmanWeight.compress(stacked), ANSWeight.compress(stacked)], key=_buffers_size)
+        weight = _compress_for(stacked, algo)
         if _buffers_size(weight) >= stacked.nelement() * stacked.element_size():
             continue                                      # does not pay: leave the layers alone
         bounds, at = [], 0

@@ -108,12 +108,24 @@ def huffman_decode_prepared(A_rem: Tensor, A_exp: Tensor, Y: Tensor, offsets: Te
 
 
 # ---- whole-layer encoder passes --------------------------------------------------------------------
+def split_histogram(W: Tensor, split_k: int, row0: int, rem: Tensor, histogram: Tensor) -> None:
+    """Rows ``row0..`` of a layer: their part of ``rem`` (u8 ``[split_k, M, K/split_k]``, or empty to skip it) is written
+    and their exponents are added to ``histogram`` (i64 ``[256]``)."""
+    _ops.split_histogram.default(W, split_k, row0, rem, histogram)
+
+
+def record_offsets(words_per_row: Tensor, slab_rows: int, offsets: Tensor, total: Tensor) -> None:
+    """Word offset of every record, and the words of the whole exponent plane, from the size pass."""
+    _ops.record_offsets.default(words_per_row, slab_rows, offsets, total)
+
+
 def huffman_size_pass(W: Tensor, split_k: int, code_lengths: Tensor, words_per_row: Tensor) -> None:
     _ops.huffman_size_pass.default(W, split_k, code_lengths, words_per_row)
 
 
 def huffman_emit_pass(W: Tensor, split_k: int, code_lengths: Tensor, code_values: Tensor, offsets: Tensor,
                       rem: Tensor, exp: Tensor) -> None:
+    """``rem`` may be empty: the sign/mantissa plane then comes from :func:`split_histogram`."""
     _ops.huffman_emit_pass.default(W, split_k, code_lengths, code_values, offsets, rem, exp)
 
 

@@ -230,8 +230,20 @@ int bhi_huffman_size_pass(const uint16_t *W, int M, int K, int split_k, const ui
 int bhi_ans_size_pass(const uint16_t *W, int M, int K, int split_k, const uint32_t *freq,
                       const uint32_t *cum, int32_t *words_per_row, uint8_t *stream_words, void *stream);
 
-/* Emit pass: writes A_rem (permuted bytes) and the coded words of every record at its offset.
- * A_exp must be zero-filled by the caller (padding words are never written).
+/* Sign/mantissa plane and exponent histogram of rows [row0, row0 + rows) of a layer of M rows in one pass: W points
+ * at those rows, A_rem at the whole plane u8 [split_k, M, K / split_k]; histogram u64 [256] is added to.  Either output
+ * may be null. */
+int bhi_split_histogram(const uint16_t *W, int rows, int K, int split_k, uint8_t *A_rem, int M, int row0,
+                        uint64_t *histogram, void *stream);
+
+/* offsets i32 [split_k, M] from the size pass: records in storage order, 64 padding words after every slab_rows rows
+ * (the format: 4096) and after the last row of a chunk.  total i64 [1]: words of the exponent plane; offsets are valid
+ * when it is below 2^31. */
+int bhi_record_offsets(const int32_t *words_per_row, int split_k, int M, int slab_rows, int32_t *offsets, int64_t *total,
+                       void *stream);
+
+/* Emit pass: writes A_rem (permuted bytes; null when bhi_split_histogram has written it) and the coded words of every
+ * record at its offset.  A_exp must be zero-filled by the caller (padding words are never written).
  * code_values u32 [256]: code bits with the first path bit in bit 0. */
 int bhi_huffman_emit_pass(const uint16_t *W, int M, int K, int split_k, const uint8_t *code_lengths,
                           const uint32_t *code_values, const int32_t *offsets,
