@@ -74,8 +74,9 @@ static int launch_status(const char *what) {
 
 template <class Codec>
 static int run_gemv(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
-                    uint16_t *Y, int B, cudaStream_t st) {
+                    const uint16_t *bias, uint16_t *Y, int B, cudaStream_t st) {
     BHI_REQUIRE(X && Y, "null activation buffer");
+    BHI_REQUIRE(aligned(bias, 2), "bias must be 2-byte aligned");
     BHI_REQUIRE(B >= 1 && B <= BHI_MAX_BATCH, "batch must be in [1, 8]");
     BHI_REQUIRE(aligned(X, 4) && aligned(Y, 2), "activation buffers must be 4-byte (X) / 2-byte (Y) aligned");
     const int path = g_path.load();
@@ -85,15 +86,15 @@ static int run_gemv(const Layer &L, const typename Codec::Args &targs, const uin
     // rows of X anyway)
     const bool row_first = !(std::is_same<Codec, HuffCodec>::value && complete) && B <= 2;
     if (path == 0 && row_first) {
-        int rc = staged_gemv<Codec>(L, targs, prepared, X, Y, B, st);
+        int rc = staged_gemv<Codec>(L, targs, prepared, X, bias, Y, B, st);
         if (rc != kStagedDeclined) return rc;
     }
     if (path == 0) {
-        int rc = quad_launch<Codec>(L, targs, prepared, X, Y, nullptr, B, complete, st);
+        int rc = quad_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, complete, st);
         if (rc != kStagedDeclined) return rc;
     }
     if (path == 0 || path == 2) {
-        int rc = staged_gemv<Codec>(L, targs, prepared, X, Y, B, st);
+        int rc = staged_gemv<Codec>(L, targs, prepared, X, bias, Y, B, st);
         if (rc != kStagedDeclined) return rc;
     }
     // one warp per row, enough blocks to give every row its own warp up to 8 waves of blocks per SM
@@ -103,7 +104,7 @@ static int run_gemv(const Layer &L, const typename Codec::Args &targs, const uin
     if (blocks > cap) blocks = cap;
 #define BHI_CASE(b)                                                                                  \
     case b:                                                                                          \
-        gemv_generic_kernel<Codec, b><<<blocks, kGenericThreads, 0, st>>>(L, targs, X, Y);           \
+        gemv_generic_kernel<Codec, b><<<blocks, kGenericThreads, 0, st>>>(L, targs, X, bias, Y);           \
         break;
     switch (B) {
         BHI_CASE(1) BHI_CASE(2) BHI_CASE(3) BHI_CASE(4) BHI_CASE(5) BHI_CASE(6) BHI_CASE(7) BHI_CASE(8)
@@ -170,9 +171,9 @@ static int run_exchange(const Layer &L, const typename Codec::Args &targs, const
     int rc = kStagedDeclined;
     const bool complete = pair_complete_hint(prepared);
     const bool row_first = !(std::is_same<Codec, HuffCodec>::value && complete) && B <= 2;
-    if (g_path.load() == 0 && !row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, &peers, B, complete, st);
+    if (g_path.load() == 0 && !row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
     if (rc == kStagedDeclined) rc = staged_exchange<Codec>(L, targs, prepared, X, peers, B, st);
-    if (rc == kStagedDeclined && g_path.load() == 0 && row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, &peers, B, complete, st);
+    if (rc == kStagedDeclined && g_path.load() == 0 && row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
     return rc == kStagedDeclined ? fail(BHI_ERR_ARG, "shape not supported by the exchange kernel") : rc;
 }
 
@@ -260,7 +261,7 @@ int bhi_gemv_bf16_huffman(const uint8_t *A_rem, const uint32_t *A_exp, int64_t e
     BHI_REQUIRE(LUT1 && LUT2 && LUT3 && LUT4 && code_lengths, "null table");
     Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
     HuffArgs t{LUT1, LUT2, LUT3, LUT4, code_lengths};
-    return run_gemv<HuffCodec>(L, t, nullptr, X, Y, batch, static_cast<cudaStream_t>(stream));
+    return run_gemv<HuffCodec>(L, t, nullptr, X, nullptr, Y, batch, static_cast<cudaStream_t>(stream));
 }
 
 int bhi_huffman_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
@@ -291,15 +292,22 @@ int bhi_huffman_prepare(const uint8_t *LUT1, const uint8_t *LUT2, const uint8_t 
 }
 
 // A prepared blob carries the exact tables too, so the five table pointers are not needed here.
-int bhi_gemv_bf16_huffman_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
-                                   const uint16_t *X, uint16_t *Y, const int32_t *offsets,
-                                   const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream) {
+int bhi_gemv_bf16_huffman_prepared_bias(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                                        const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets,
+                                        const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream) {
     if (int rc = check_layer(A_rem, A_exp, exp_words, offsets, split_k, M, Nc)) return rc;
     BHI_REQUIRE(prepared && aligned(prepared, 16), "null or unaligned prepared tables");
     Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
     const uint8_t *ex = prepared + kPairEntries * 4;
     HuffArgs t{ex, ex + 256, ex + 512, ex + 768, ex + 1024};
-    return run_gemv<HuffCodec>(L, t, prepared, X, Y, batch, static_cast<cudaStream_t>(stream));
+    return run_gemv<HuffCodec>(L, t, prepared, X, bias, Y, batch, static_cast<cudaStream_t>(stream));
+}
+
+int bhi_gemv_bf16_huffman_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                                   const uint16_t *X, uint16_t *Y, const int32_t *offsets,
+                                   const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream) {
+    return bhi_gemv_bf16_huffman_prepared_bias(A_rem, A_exp, exp_words, X, nullptr, Y, offsets, prepared, split_k, M, Nc,
+                                               batch, stream);
 }
 
 int bhi_huffman_decode_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
@@ -396,15 +404,22 @@ int bhi_gemv_bf16_ans_exchange(const uint8_t *A_rem, const uint32_t *A_exp, int6
     return run_exchange<AnsCodec>(L, t, nullptr, X, batch, exchange, static_cast<cudaStream_t>(stream));
 }
 
-int bhi_gemv_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
-                      const uint16_t *X, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT, int precision,
-                      int split_k, int M, int Nc, int batch, void *stream) {
+int bhi_gemv_bf16_ans_bias(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                           const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT,
+                           int precision, int split_k, int M, int Nc, int batch, void *stream) {
     if (int rc = check_layer(A_rem, A_exp, exp_words, offsets, split_k, M, Nc)) return rc;
     BHI_REQUIRE(LUT && aligned(LUT, 4), "null or unaligned table");
     BHI_REQUIRE(precision >= BHI_ANS_PRECISION && precision <= BHI_ANS_MAX_PRECISION, "rANS precision must be in [8, 12]");
     Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
     AnsArgs t{LUT, precision};
-    return run_gemv<AnsCodec>(L, t, nullptr, X, Y, batch, static_cast<cudaStream_t>(stream));
+    return run_gemv<AnsCodec>(L, t, nullptr, X, bias, Y, batch, static_cast<cudaStream_t>(stream));
+}
+
+int bhi_gemv_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                      const uint16_t *X, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT, int precision,
+                      int split_k, int M, int Nc, int batch, void *stream) {
+    return bhi_gemv_bf16_ans_bias(A_rem, A_exp, exp_words, X, nullptr, Y, offsets, LUT, precision, split_k, M, Nc, batch,
+                                  stream);
 }
 
 int bhi_ans_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,

@@ -52,6 +52,14 @@ __device__ __forceinline__ uint16_t f32_to_bf16_rn(float f) {
     return h;
 }
 
+// An output value: the 32-bit sum rounded to BF16, then the layer's bias (if it has one) added to that value and the
+// result rounded again - what a separate addition of BF16 tensors gives.
+__device__ __forceinline__ uint16_t finish_value(float v, const uint16_t *bias, int m) {
+    const uint16_t h = f32_to_bf16_rn(v);
+    if (bias == nullptr) return h;
+    return f32_to_bf16_rn(__uint_as_float(static_cast<uint32_t>(h) << 16) + __uint_as_float(static_cast<uint32_t>(__ldg(bias + m)) << 16));
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);

@@ -14,7 +14,8 @@ constexpr int kGenericThreads = 256;
 // order, so the K-split needs no cross-warp combine and the summation order is fixed.
 template <class Codec, int B>
 __global__ void __launch_bounds__(kGenericThreads)
-gemv_generic_kernel(Layer L, typename Codec::Args targs, const uint16_t *__restrict__ X, uint16_t *__restrict__ Y) {
+gemv_generic_kernel(Layer L, typename Codec::Args targs, const uint16_t *__restrict__ X,
+                    const uint16_t *__restrict__ bias, uint16_t *__restrict__ Y) {
     __shared__ typename Codec::Tables tab;
     load_tables(tab, targs, threadIdx.x, blockDim.x);
     __syncthreads();
@@ -62,7 +63,7 @@ gemv_generic_kernel(Layer L, typename Codec::Args targs, const uint16_t *__restr
 #pragma unroll
         for (int b = 0; b < B; b++) {
             const float v = warp_sum(acc[b]);
-            if (lane == 0) Y[static_cast<int64_t>(b) * L.M + m] = f32_to_bf16_rn(v);
+            if (lane == 0) Y[static_cast<int64_t>(b) * L.M + m] = finish_value(v, bias, m);
         }
     }
 }

@@ -222,7 +222,7 @@ struct QuadUnit {
 // PPW = passes per warp: 1 (four warps per group, 32 warps) or 2 (two warps per group, 16 warps of twice the registers).
 template <class Codec, int B, int PPW>
 __global__ void __launch_bounds__(kQuadGroups * (4 / PPW) * 32, 1)
-quad_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const uint32_t *X, uint16_t *Y, PeerSet peers,
+quad_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const uint32_t *X, const uint16_t *bias, uint16_t *Y, PeerSet peers,
             QuadGeom G, Consts kc) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using Tables = typename Codec::Tables;
@@ -540,7 +540,7 @@ quad_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const 
                         const int row = 4 * (q_lo + cur.qi) + t;
                         if (gq < B && row < L.M) {
                             if (exchange) ys[gq * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
-                            else Y[static_cast<int64_t>(gq) * L.M + row] = f32_to_bf16_rn(v);
+                            else Y[static_cast<int64_t>(gq) * L.M + row] = finish_value(v, bias, row);
                         }
                     }
                 }
@@ -624,7 +624,7 @@ static bool quad_plan(const Layer &L, int grid, bool exchange, uint32_t ans_bits
 int quad_passes_per_warp();      // 0 = by table kind, 1 = 32 warps, 2 = 16 warps: see bhi_set_quad_warps
 
 template <class Codec, int B, int PPW>
-static int quad_launch_p(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
+static int quad_launch_p(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
                          const PeerSet *peers, cudaStream_t st) {
     int grid = sm_count();
     const int nquads = (L.M + 3) / 4;
@@ -648,7 +648,7 @@ static int quad_launch_p(const Layer &L, const typename Codec::Args &targs, cons
     cfg.numAttrs = overlap_launches() ? 1 : 0;
     const uint32_t ans_bits = ans_bits_of(targs);
     const Consts k{ans_bits, (1u << ans_bits) - 1u, 1u, 8u, 4u * kCopies, 65536u};
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, reinterpret_cast<const uint32_t *>(X), Y, ps, G, k);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, reinterpret_cast<const uint32_t *>(X), bias, Y, ps, G, k);
     return e == cudaSuccess ? BHI_OK : cuda_fail(e, "quad kernel launch");
 }
 
@@ -658,28 +658,28 @@ static int quad_launch_p(const Layer &L, const typename Codec::Args &targs, cons
 // symbol-by-symbol detour stalls half as many streams.  Only a tuning hint: the kernel itself reads
 // from the table header whether it may skip the per-step test.
 template <class Codec, int B>
-static int quad_launch_b(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
+static int quad_launch_b(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
                          const PeerSet *peers, bool pair_complete, cudaStream_t st) {
     int ppw = quad_passes_per_warp();
     if (ppw == 0) ppw = (pair_complete || !std::is_same<Codec, HuffCodec>::value) ? 2 : 1;
-    if (ppw == 2) return quad_launch_p<Codec, B, 2>(L, targs, prepared, X, Y, peers, st);
-    return quad_launch_p<Codec, B, 1>(L, targs, prepared, X, Y, peers, st);
+    if (ppw == 2) return quad_launch_p<Codec, B, 2>(L, targs, prepared, X, bias, Y, peers, st);
+    return quad_launch_p<Codec, B, 1>(L, targs, prepared, X, bias, Y, peers, st);
 }
 
 template <class Codec>
-static int quad_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
+static int quad_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
                        const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16)) return kStagedDeclined;
     if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31)) return kStagedDeclined;
     switch (B) {
-        case 1: return quad_launch_b<Codec, 1>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 2: return quad_launch_b<Codec, 2>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 3: return quad_launch_b<Codec, 3>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 4: return quad_launch_b<Codec, 4>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 5: return quad_launch_b<Codec, 5>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 6: return quad_launch_b<Codec, 6>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 7: return quad_launch_b<Codec, 7>(L, targs, prepared, X, Y, peers, pair_complete, st);
-        case 8: return quad_launch_b<Codec, 8>(L, targs, prepared, X, Y, peers, pair_complete, st);
+        case 1: return quad_launch_b<Codec, 1>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 2: return quad_launch_b<Codec, 2>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 3: return quad_launch_b<Codec, 3>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 4: return quad_launch_b<Codec, 4>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 5: return quad_launch_b<Codec, 5>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 6: return quad_launch_b<Codec, 6>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 7: return quad_launch_b<Codec, 7>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
+        case 8: return quad_launch_b<Codec, 8>(L, targs, prepared, X, bias, Y, peers, pair_complete, st);
     }
     return kStagedDeclined;
 }

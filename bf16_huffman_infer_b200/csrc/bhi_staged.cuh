@@ -160,6 +160,7 @@ struct GemvSink {
     int64_t row_pairs;      // K / 2
     int row_blocks;         // K / 128
     uint16_t *Y;
+    const uint16_t *bias;   // [M] or null
     int M;
 
     __device__ __forceinline__ void stage(uint8_t *x_region, int tid, int nthreads) {
@@ -236,7 +237,7 @@ struct GemvSink {
 #pragma unroll
         for (int b = 0; b < B; b++) {
             const float v = row_value(b, lane);
-            if (lane == 0) Y[static_cast<int64_t>(b) * M + m] = f32_to_bf16_rn(v);
+            if (lane == 0) Y[static_cast<int64_t>(b) * M + m] = finish_value(v, bias, m);
         }
         clear();
     }
@@ -259,7 +260,7 @@ struct GemvSink {
     __device__ __forceinline__ void combine(const float *part, int row_lo, int rows, int slots, int) {
         for (int i = threadIdx.x; i < B * rows; i += blockDim.x) {
             const int b = i / rows, r = i - b * rows;
-            Y[static_cast<int64_t>(b) * M + row_lo + r] = f32_to_bf16_rn(part_sum(part, i, slots));
+            Y[static_cast<int64_t>(b) * M + row_lo + r] = finish_value(part_sum(part, i, slots), bias, row_lo + r);
         }
     }
 };
@@ -932,7 +933,7 @@ static int staged_launch(const Layer &L, const typename Codec::Args &targs, cons
 
 template <class Codec, int B>
 static int staged_gemv_b(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
-                         uint16_t *Y, cudaStream_t st) {
+                         const uint16_t *bias, uint16_t *Y, cudaStream_t st) {
     constexpr int NW = B <= 4 ? 32 : 16;      // measured: batches 5..8 are faster with 16 warps of twice the registers
     const int64_t K = static_cast<int64_t>(L.S) * L.Nc;
     const int64_t x_need = ((static_cast<int64_t>(B) * K * 2 + 255) / 256) * 256;
@@ -942,6 +943,7 @@ static int staged_gemv_b(const Layer &L, const typename Codec::Args &targs, cons
         sink.row_pairs = K >> 1;
         sink.row_blocks = static_cast<int>(K >> 7);
         sink.Y = Y;
+        sink.bias = bias;
         sink.M = L.M;
         return staged_launch<Codec, GemvSink<B, true>, NW>(L, targs, prepared, sink, static_cast<uint32_t>(x_need), st);
     }
@@ -950,23 +952,24 @@ static int staged_gemv_b(const Layer &L, const typename Codec::Args &targs, cons
     sink.row_pairs = K >> 1;
     sink.row_blocks = static_cast<int>(K >> 7);
     sink.Y = Y;
+    sink.bias = bias;
     sink.M = L.M;
     return staged_launch<Codec, GemvSink<B, false>, NW>(L, targs, prepared, sink, 0u, st);
 }
 
 template <class Codec>
 static int staged_gemv(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
-                       uint16_t *Y, int B, cudaStream_t st) {
+                       const uint16_t *bias, uint16_t *Y, int B, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16)) return kStagedDeclined;
     switch (B) {
-        case 1: return staged_gemv_b<Codec, 1>(L, targs, prepared, X, Y, st);
-        case 2: return staged_gemv_b<Codec, 2>(L, targs, prepared, X, Y, st);
-        case 3: return staged_gemv_b<Codec, 3>(L, targs, prepared, X, Y, st);
-        case 4: return staged_gemv_b<Codec, 4>(L, targs, prepared, X, Y, st);
-        case 5: return staged_gemv_b<Codec, 5>(L, targs, prepared, X, Y, st);
-        case 6: return staged_gemv_b<Codec, 6>(L, targs, prepared, X, Y, st);
-        case 7: return staged_gemv_b<Codec, 7>(L, targs, prepared, X, Y, st);
-        case 8: return staged_gemv_b<Codec, 8>(L, targs, prepared, X, Y, st);
+        case 1: return staged_gemv_b<Codec, 1>(L, targs, prepared, X, bias, Y, st);
+        case 2: return staged_gemv_b<Codec, 2>(L, targs, prepared, X, bias, Y, st);
+        case 3: return staged_gemv_b<Codec, 3>(L, targs, prepared, X, bias, Y, st);
+        case 4: return staged_gemv_b<Codec, 4>(L, targs, prepared, X, bias, Y, st);
+        case 5: return staged_gemv_b<Codec, 5>(L, targs, prepared, X, bias, Y, st);
+        case 6: return staged_gemv_b<Codec, 6>(L, targs, prepared, X, bias, Y, st);
+        case 7: return staged_gemv_b<Codec, 7>(L, targs, prepared, X, bias, Y, st);
+        case 8: return staged_gemv_b<Codec, 8>(L, targs, prepared, X, bias, Y, st);
     }
     return kStagedDeclined;
 }
@@ -982,6 +985,7 @@ static int staged_exchange_b(const Layer &L, const typename Codec::Args &targs, 
         sink.row_pairs = K >> 1;
         sink.row_blocks = static_cast<int>(K >> 7);
         sink.Y = nullptr;
+        sink.bias = nullptr;
         sink.M = L.M;
         sink.peers = peers;
     };

@@ -8,10 +8,13 @@
 #include <torch/csrc/inductor/aoti_torch/c/shim.h>
 #include <torch/csrc/stable/accelerator.h>
 #include <torch/csrc/stable/library.h>
+#include <torch/csrc/stable/ops.h>
 #include <torch/csrc/stable/tensor.h>
 #include <torch/headeronly/core/ScalarType.h>
 
+#include <optional>
 #include <string>
+#include <vector>
 
 #include "../../include/bf16_huffman_b200.h"
 
@@ -170,6 +173,64 @@ void boxed_gemv_bf16_huffman_prepared(StableIValue *stack, uint64_t, uint64_t) {
     check(bhi_gemv_bf16_huffman_prepared(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), v.exp_words,
                                          ptr<const uint16_t>(X), ptr<uint16_t>(Y), ptr<const int32_t>(off),
                                          ptr<const uint8_t>(blob), v.S, v.M, v.Nc, static_cast<int>(B), stream_of(rem)));
+}
+
+// What a layer's forward call needs, in one operator: output allocation, checks and launch.
+struct ForwardCall {
+    LayerView v;
+    Tensor Y;
+    int B;
+    const uint16_t *bias;
+};
+
+ForwardCall forward_of(StableIValue *stack, const Tensor &X, const Tensor &rem, const Tensor &exp, const Tensor &off) {
+    LayerView v = layer_of(rem, exp, off);
+    want(X, ScalarType::BFloat16, "X");
+    same_device(rem, X, "X");
+    const int64_t K = static_cast<int64_t>(v.S) * v.Nc;
+    STD_TORCH_CHECK(X.size(-1) == K, "X must have split_k*Nc columns");
+    const int64_t B = X.numel() / K;
+    STD_TORCH_CHECK(B <= BHI_MAX_BATCH, "batch_size <= 8");
+    std::optional<Tensor> bias = torch::stable::detail::to<std::optional<Tensor>>(stack[5]);
+    const uint16_t *bias_ptr = nullptr;
+    if (bias.has_value()) {
+        want(*bias, ScalarType::BFloat16, "bias");
+        same_device(rem, *bias, "bias");
+        STD_TORCH_CHECK(bias->numel() == v.M, "bias must have M entries");
+        bias_ptr = ptr<const uint16_t>(*bias);
+    }
+    std::vector<int64_t> shape(X.dim());
+    for (int64_t d = 0; d + 1 < X.dim(); d++) shape[d] = X.size(d);
+    shape[X.dim() - 1] = v.M;
+    return {v, torch::stable::new_empty(X, shape), static_cast<int>(B), bias_ptr};
+}
+
+// forward_huffman(X, A_rem, A_exp, offsets, prepared, bias?) -> Y   (up to 8 rows of X, any leading dimensions)
+void boxed_forward_huffman(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor X = arg(stack, 0), rem = arg(stack, 1), exp = arg(stack, 2), off = arg(stack, 3), blob = arg(stack, 4);
+    want(blob, ScalarType::Byte, "prepared");
+    same_device(rem, blob, "prepared");
+    STD_TORCH_CHECK(blob.numel() == bhi_huffman_prepared_bytes(), "prepared has the wrong size");
+    torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
+    ForwardCall f = forward_of(stack, X, rem, exp, off);
+    check(bhi_gemv_bf16_huffman_prepared_bias(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words,
+                                              ptr<const uint16_t>(X), f.bias, ptr<uint16_t>(f.Y), ptr<const int32_t>(off),
+                                              ptr<const uint8_t>(blob), f.v.S, f.v.M, f.v.Nc, f.B, stream_of(rem)));
+    stack[0] = torch::stable::detail::from(f.Y);
+}
+
+// forward_ans(X, A_rem, A_exp, offsets, LUT, bias?) -> Y
+void boxed_forward_ans(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor X = arg(stack, 0), rem = arg(stack, 1), exp = arg(stack, 2), off = arg(stack, 3), lut = arg(stack, 4);
+    want(lut, ScalarType::Int, "LUT");
+    same_device(rem, lut, "LUT");
+    const int precision = ans_precision_of(lut);
+    torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
+    ForwardCall f = forward_of(stack, X, rem, exp, off);
+    check(bhi_gemv_bf16_ans_bias(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X),
+                                 f.bias, ptr<uint16_t>(f.Y), ptr<const int32_t>(off), ptr<const uint32_t>(lut), precision,
+                                 f.v.S, f.v.M, f.v.Nc, f.B, stream_of(rem)));
+    stack[0] = torch::stable::detail::from(f.Y);
 }
 
 // huffman_decode_prepared(A_rem, A_exp, Y(a!), offsets, prepared) -> ()
@@ -520,6 +581,8 @@ STABLE_TORCH_LIBRARY(BHI_TORCH_NAMESPACE, m) {
     m.def("linear_bf16_ans(Tensor A_rem, Tensor A_exp, Tensor X, Tensor(a!) Y, Tensor offsets, Tensor LUT) -> ()");
     m.def("gemv_bf16_huffman_exchange(Tensor A_rem, Tensor A_exp, Tensor X, Tensor offsets, Tensor prepared, Tensor peers, int rank, int row_base, int m_total) -> ()");
     m.def("gemv_bf16_ans_exchange(Tensor A_rem, Tensor A_exp, Tensor X, Tensor offsets, Tensor LUT, Tensor peers, int rank, int row_base, int m_total) -> ()");
+    m.def("forward_huffman(Tensor X, Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor prepared, Tensor? bias) -> Tensor");
+    m.def("forward_ans(Tensor X, Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor LUT, Tensor? bias) -> Tensor");
     m.def("set_launch_overlap(int on) -> int");
     // whole-layer encoder
     m.def("split_histogram(Tensor W, int split_k, int row0, Tensor(a!) rem, Tensor(b!) histogram) -> ()");
@@ -544,6 +607,8 @@ STABLE_TORCH_LIBRARY_IMPL(BHI_TORCH_NAMESPACE, CUDA, m) {
     m.impl("huffman_prepare", &boxed_huffman_prepare);
     m.impl("huffman_table_hint", &boxed_huffman_table_hint);
     m.impl("gemv_bf16_huffman_prepared", &boxed_gemv_bf16_huffman_prepared);
+    m.impl("forward_huffman", &boxed_forward_huffman);
+    m.impl("forward_ans", &boxed_forward_ans);
     m.impl("huffman_decode_prepared", &boxed_huffman_decode_prepared);
     m.impl("linear_bf16_huffman_prepared", &boxed_linear_bf16_huffman_prepared);
     m.impl("linear_bf16_ans", &boxed_linear_bf16_ans);

@@ -342,17 +342,35 @@ class HuffmanWeight(nn.Module):
         """The decode tables folded for the fused kernels (built on first use on each device, so the
         first call has to happen outside CUDA-graph capture; warm-up iterations take care of that).
         Not a buffer: it is derived data and stays out of ``state_dict`` and size accounting."""
-        blob = self.__dict__.get("_prepared")
-        tables = (self.LUT1, self.LUT2, self.LUT3, self.LUT4, self.code_lengths)
-        src = tuple((t.data_ptr(), t._version) for t in tables)      # in-place loads (load_state_dict) bump the version
-        if blob is None or blob.device != self.rem.device or self.__dict__.get("_prepared_src") != src:
+        b = self._buffers
+        t1, t2, t3, t4, cl = b["LUT1"], b["LUT2"], b["LUT3"], b["LUT4"], b["code_lengths"]
+        # in-place loads (load_state_dict) bump the version; a tensor whose data was replaced has another address
+        src = (t1.data_ptr(), t2.data_ptr(), t3.data_ptr(), t4.data_ptr(), cl.data_ptr(),
+               t1._version, t2._version, t3._version, t4._version, cl._version)
+        if self.__dict__.get("_prepared_src") != src:
             blob = torch.empty(ops.PREPARED_BYTES, dtype=torch.uint8, device=self.rem.device)
-            ops.huffman_prepare(*tables, blob)
+            ops.huffman_prepare(t1, t2, t3, t4, cl, blob)
             # codes of at most 6 bits: every 12-bit window holds two whole codes (the kernels pick their warp layout by it)
-            ops.huffman_table_hint(blob, int(self.code_lengths.max().item()) <= 6)
+            ops.huffman_table_hint(blob, int(cl.max().item()) <= 6)
             self.__dict__["_prepared"] = blob
             self.__dict__["_prepared_src"] = src
-        return blob
+        return self.__dict__["_prepared"]
+
+    def _plain(self) -> bool:
+        """The buffers are as the operators take them (``compress`` makes no others)."""
+        b = self._buffers
+        rem, exp, off = b["rem"], b["exp"], b["offsets"]
+        return rem.dim() == 3 and off.dim() == 2 and rem.is_contiguous() and exp.is_contiguous() and off.is_contiguous()
+
+    def _forward(self, x: Tensor, bias: Optional[Tensor]) -> Tensor:
+        b = self._buffers
+        return ops.forward_huffman(x, b["rem"], b["exp"], b["offsets"], self.prepared(), bias)
+
+    def _mv(self, x: Tensor) -> Tensor:
+        return mv_huffman_prepared(self.rem, self.exp, x, self.offsets, self.prepared())
+
+    def _mm(self, x: Tensor) -> Tensor:
+        return mm_huffman_prepared(self.rem, self.exp, x, self.offsets, self.prepared())
 
     def get_weight(self) -> Tensor:
         """Dense BF16 ``[M, K]`` (reference ``functional.py:99-108``)."""
@@ -453,6 +471,16 @@ class ANSWeight(HuffmanWeight):
             return NotImplemented
         return linear_ans(*args, **(kwargs or {}))
 
+    def _forward(self, x: Tensor, bias: Optional[Tensor]) -> Tensor:
+        b = self._buffers
+        return ops.forward_ans(x, b["rem"], b["exp"], b["offsets"], b["LUT"], bias)
+
+    def _mv(self, x: Tensor) -> Tensor:
+        return mv_ans(self.rem, self.exp, x, self.offsets, self.LUT)
+
+    def _mm(self, x: Tensor) -> Tensor:
+        return mm_ans(self.rem, self.exp, x, self.offsets, self.LUT)
+
     def get_weight(self) -> Tensor:
         assert self.rem.device.type == "cuda"
         weight = torch.empty(self.shape, dtype=torch.bfloat16, device=self.rem.device)
@@ -521,15 +549,29 @@ class CompressedLinear(nn.Module):
         return self.weight.shape[1]
 
     def forward(self, input: Tensor) -> Tensor:
-        return F.linear(input, self.weight, self.bias)
+        return _linear_compressed(input, self.weight, self.bias)
 
 
-def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor], fused, tensor) -> Tensor:
+def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> Tensor:
     assert input.dim() >= 2, input
+    rows = input.numel() // max(input.size(-1), 1)
+    if rows <= FUSED_MAX_ROWS and weight._plain():
+        # one operator call; a bias that needs its gradient, or is not a BF16 vector on the layer's device, is added after it
+        assert input.is_cuda and input.dtype == torch.bfloat16
+        if input.requires_grad:
+            input = input.detach()
+        if bias is None:
+            return weight._forward(input.contiguous(), None)
+        if (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
+                and not (bias.requires_grad and torch.is_grad_enabled())):
+            return weight._forward(input.contiguous(), bias)
+        output = weight._forward(input.contiguous(), None)
+        output += bias
+        return output
     shape = input.shape
     input = input.flatten(0, -2)
-    if input.size(0) <= max(FUSED_MAX_ROWS, min(TENSOR_MAX_ROWS, 128)):
-        output = fused(input) if input.size(0) <= FUSED_MAX_ROWS else tensor(input)
+    if rows <= max(FUSED_MAX_ROWS, min(TENSOR_MAX_ROWS, 128)):
+        output = weight._mv(input) if rows <= FUSED_MAX_ROWS else weight._mm(input)
         if bias is not None:
             output += bias[None, :]
     else:
@@ -540,18 +582,12 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
 def linear_huffman(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor] = None) -> Tensor:
     """``F.linear`` on a Huffman-coded weight: fused decode+GEMV up to 8 rows, decode then GEMM beyond
     (reference ``functional.py:390-411``); optionally the fused tensor-core product up to ``TENSOR_MAX_ROWS``."""
-    return _linear_compressed(
-        input, weight, bias,
-        lambda x: mv_huffman_prepared(weight.rem, weight.exp, x, weight.offsets, weight.prepared()),
-        lambda x: mm_huffman_prepared(weight.rem, weight.exp, x, weight.offsets, weight.prepared()))
+    return _linear_compressed(input, weight, bias)
 
 
 def linear_ans(input: Tensor, weight: ANSWeight, bias: Optional[Tensor] = None) -> Tensor:
     """Same for an rANS-coded weight (reference ``functional.py:447-466``)."""
-    return _linear_compressed(
-        input, weight, bias,
-        lambda x: mv_ans(weight.rem, weight.exp, x, weight.offsets, weight.LUT),
-        lambda x: mm_ans(weight.rem, weight.exp, x, weight.offsets, weight.LUT))
+    return _linear_compressed(input, weight, bias)
 
 
 def _buffers_size(w: nn.Module) -> int:

@@ -80,6 +80,13 @@ def gemv_bf16_huffman_prepared(A_rem: Tensor, A_exp: Tensor, X: Tensor, Y: Tenso
     _ops.gemv_bf16_huffman_prepared.default(A_rem, A_exp, X, Y, offsets, prepared)
 
 
+# A layer's forward call as one operator (output allocation, checks, launch, bias): (X, A_rem, A_exp, offsets, prepared or
+# LUT, bias or None) -> Y, up to 8 rows of X with any leading dimensions.  Bound here because a decode step calls them
+# once per layer and the way through Python is most of what a small layer costs.
+forward_huffman = _ops.forward_huffman.default
+forward_ans = _ops.forward_ans.default
+
+
 def linear_bf16_huffman_prepared(A_rem: Tensor, A_exp: Tensor, X: Tensor, Y: Tensor, offsets: Tensor, prepared: Tensor) -> None:
     """Fused decode + tensor-core product for up to 128 rows of ``X`` (no reference counterpart)."""
     _ops.linear_bf16_huffman_prepared.default(A_rem, A_exp, X, Y, offsets, prepared)

@@ -113,6 +113,11 @@ int bhi_huffman_prepare(const uint8_t *LUT1, const uint8_t *LUT2, const uint8_t 
 int bhi_gemv_bf16_huffman_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
                                    const uint16_t *X, uint16_t *Y, const int32_t *offsets,
                                    const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream);
+/* ... with the layer's bias BF16 [M] (may be null): added to the BF16 product and rounded again, as a separate addition of
+ * BF16 tensors would. */
+int bhi_gemv_bf16_huffman_prepared_bias(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                                        const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets,
+                                        const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream);
 int bhi_huffman_decode_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
                                 uint16_t *Y, const int32_t *offsets, const uint8_t *prepared,
                                 int split_k, int M, int Nc, void *stream);
@@ -127,6 +132,9 @@ int bhi_huffman_decode_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int
 int bhi_gemv_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
                       const uint16_t *X, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT, int precision,
                       int split_k, int M, int Nc, int batch, void *stream);
+int bhi_gemv_bf16_ans_bias(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                           const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT,
+                           int precision, int split_k, int M, int Nc, int batch, void *stream);
 int bhi_ans_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
                    uint16_t *Y, const int32_t *offsets, const uint32_t *LUT, int precision,
                    int split_k, int M, int Nc, void *stream);
