@@ -442,3 +442,623 @@ struct GemvDirect : std::conditional<std::is_same<C, HuffCodec>::value, DirectHu
     }
     __device__ __forceinline__ void clamp() {}
 };
+
+// A part of an X row into shared memory: by the calling thread as a bulk copy on `bar`, or (unaligned source) by the whole
+// warp with plain stores.
+__device__ __forceinline__ void copy_x_row(uint32_t dst, const uint16_t *src, uint32_t bytes, uint32_t bar, bool bulk, int lane) {
+    if (bulk) {
+        bulk_copy_g2s(dst, src, bytes, bar);
+    } else {
+        for (uint32_t i = 4u * lane; i < bytes; i += 128u) {
+            const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(src) + (i >> 2));
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + i), "r"(v) : "memory");
+        }
+    }
+}
+
+// NB = groups of eight X rows (0: no product, the dense matrix is written instead).  NG = groups of four warps per CTA.
+// Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
+// X or tables two CTAs could not both hold.  kRing: X passes through a ring that one more warp fills and all groups read in
+// step.  (20 warps of 96 registers instead of 16 gain nothing: it is pipes that are short, not warps.)
+template <class Dec, int NB, int NG, bool kRing>
+__global__ void __launch_bounds__(NG * kGemvWarps * 32 + (kRing ? 32 : 0), NG == 2 ? 2 : 1)
+gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
+            PeerSet peers, GemvGeom G, GemvConsts kc) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    using Codec = typename Dec::Codec;
+    using Tables = typename Codec::Tables;
+    constexpr bool kHuff = std::is_same<Codec, HuffCodec>::value;
+    constexpr int kThreads = NG * kGemvWarps * 32;                     // without the warp that fills the X ring
+    constexpr int kAcc = NB > 0 ? NB : 1;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int group = warp / kGemvWarps, wig = warp % kGemvWarps;      // warp inside the group = its pass
+    const int r = lane >> 3, t = lane & 3, gq = lane >> 2;
+    const uint32_t sigma4 = 4u * (8 * wig + (lane & 7));               // byte offset of the lane's stream inside a word row
+    const bool exchange = NB == 1 && peers.world > 0;
+    const int B = G.batch;
+
+    Tables &tab = *reinterpret_cast<Tables *>(smem + G.exact_off);
+    uint8_t *ctrl = smem + G.exact_off + kExactBytes;
+    const uint32_t smem_base = smem_addr(smem);
+    const uint32_t ctrl_at = smem_addr(ctrl);
+    const uint32_t bar0 = ctrl_at + 16u * group;                       // record copies: two slots per group
+    const uint32_t table_bar = ctrl_at + 80u, x_bar = ctrl_at + 88u;
+    const uint32_t x_full = ctrl_at + 96u, x_empty = x_full + 8u * kXSlotsMax;      // X ring: filled, read by all warps
+    volatile uint32_t *posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256) + 8 * group;     // [slot]{word rows, base, staged}
+    float *part = reinterpret_cast<float *>(smem + G.part_off) + group * (kGemvWarps * 64 * kAcc);
+    uint16_t *ys = reinterpret_cast<uint16_t *>(smem + G.ys_off);
+    const uint32_t xs = smem_base + G.x_off;
+    const uint32_t rem_at = smem_base + G.rem_off + warp * (kRemChunk * 2u);
+    const uint32_t ring = G.ring_off + group * G.ring_bytes;
+
+    GemvCtx ctx;
+    ctx.exact = reinterpret_cast<const HuffTables *>(&tab);
+    ctx.k = kc;
+    ctx.lane_table = kHuff ? 4u * lane : (8u * lane) & (kc.entry - 1u);
+
+    // Quads are dealt to the groups of the grid in equal contiguous ranges; a group takes them two at a time.
+    const int nquads = (L.M + 3) >> 2;
+    auto deal = [&](int g) { return static_cast<int>(static_cast<int64_t>(nquads) * g / (static_cast<int>(gridDim.x) * NG)); };
+    const int quad_lo = deal(blockIdx.x * NG + group), quad_hi = deal(blockIdx.x * NG + group + 1);
+    const int row_lo = 4 * deal(blockIdx.x * NG);                      // rows of the CTA
+    const int rows_cta = min(4 * deal(blockIdx.x * NG + NG), L.M) - row_lo;
+    const int nblk = L.Nc >> 7;
+    const int chunks = (nblk + kRG - 1) / kRG;                         // of a record
+
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (uint32_t i = 0; i < 2u * NG; i++) mbar_init(ctrl_at + 8u * i, 1);
+        mbar_init(table_bar, 1);
+        mbar_init(x_bar, 1);
+        for (uint32_t i = 0; kRing && i < kXSlotsMax; i++) {
+            mbar_init(x_full + 8u * i, 1);
+            mbar_init(x_empty + 8u * i, NG * kGemvWarps);
+        }
+        mbar_fence_init();
+        if (kHuff && prepared != nullptr) {
+            mbar_expect_tx(table_bar, Dec::kTableBytes + kExactBytes);
+            bulk_copy_g2s(smem_base, Dec::source(prepared), Dec::kTableBytes, table_bar);
+            bulk_copy_g2s(smem_base + G.exact_off, prepared + kPairEntries * 4, kExactBytes, table_bar);
+        }
+    }
+    __syncthreads();
+
+    // Segments of X that pass through the ring: every unit reads those of its chunk, in order.
+    int x_total = 0;
+    if (kRing) {
+        for (int g = 0; g < NG; g++) {
+            const int quads = deal(blockIdx.x * NG + g + 1) - deal(blockIdx.x * NG + g);
+            x_total = max(x_total, (quads + G.max_quads - 1) / G.max_quads * L.S * chunks);
+        }
+    }
+    // ---- the warp that fills the X ring.  (With the readers filling it between their chunks, the last reader of a segment
+    // its next one, the refill lay on the slowest warp and cost half as much again as the decoding.)
+    if (kRing && warp == NG * kGemvWarps) {
+        __syncthreads();                                               // the readers' barrier before their loop
+        pdl_wait();
+        const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
+        int slot = 0, k = 0, ch = 0;
+        uint32_t phase = 1u;                                           // nobody has to have read the first lap's places
+        for (int i = 0; i < x_total; i++) {
+            const uint32_t bar = x_full + 8u * slot;
+            if (!mbar_wait_bounded(x_empty + 8u * slot, phase)) {
+                if (lane == 0) atomicExch(&g_staged_status, 3);
+                break;
+            }
+            const uint32_t bytes = 2u * min(kXSegCols, static_cast<uint32_t>(L.Nc) - ch * kXSegCols);
+            const uint16_t *src = X + static_cast<int64_t>(k) * L.Nc + ch * kXSegCols;
+            if (bulk) {
+                if (lane == 0) mbar_expect_tx(bar, bytes * B);
+                __syncwarp();
+            }
+            for (int b = bulk ? lane : 0; b < B; b += bulk ? 32 : 1)
+                copy_x_row(xs + slot * G.x_slot + b * G.x_pitch, src + static_cast<int64_t>(b) * L.S * L.Nc, bytes, bar, bulk, lane);
+            __syncwarp();
+            if (!bulk && lane == 0) mbar_arrive(bar);
+            if (++ch == chunks) {
+                ch = 0;
+                if (++k == L.S) k = 0;
+            }
+            if (++slot == G.x_slots) {
+                slot = 0;
+                phase ^= 1u;
+            }
+        }
+        if (exchange) __syncthreads();                                 // exchange_finish's
+        return;
+    }
+
+    // ---- units ---------------------------------------------------------------------------------------------------------
+    // The quads of the group max_quads by max_quads; for each set, the chunks in order.  The group's first warp knows where
+    // the records of the next unit lie (its lanes 0..7 hold one row each), places them in the ring, starts their copies and
+    // posts {word rows, base, staged} for the others; the offsets it needs are requested one unit ahead of that.
+    struct Place {
+        int quad, k;
+    };
+    auto quads_of = [&](const Place &u) { return min(G.max_quads, quad_hi - u.quad); };
+    auto after = [&](const Place &u) {
+        Place v{u.quad, u.k + 1};
+        if (v.k == L.S) {
+            v.k = 0;
+            v.quad += G.max_quads;
+        }
+        return v;
+    };
+    const uint32_t exp_words = static_cast<uint32_t>(L.exp_words);
+    const bool leader = wig == 0;
+    auto record_of = [&](const Place &u, int row) {                    // row 0..7 of the unit
+        return u.k * L.M + min(4 * u.quad + (row < 4 * quads_of(u) ? row : 0), L.M - 1);
+    };
+    uint32_t off = 0u, end = 0u;                                       // leader, lanes 0..7: first and last exponent word
+    auto request = [&](const Place &u) {
+        if (leader && u.quad < quad_hi) {
+            const int rec = record_of(u, lane & 7);
+            off = static_cast<uint32_t>(__ldg(L.offsets + rec));
+            end = rec + 1 < L.S * L.M ? static_cast<uint32_t>(__ldg(L.offsets + rec + 1)) : exp_words;
+        }
+    };
+    uint32_t words = 0u, at = 0u, foot = 0u, base = 0u;                // leader: the unit being placed
+    bool staged = false;
+    auto place = [&](const Place &u, int slot) {
+        at = off;
+        words = end - off;                                             // in storage order, whole word rows, inside the buffer
+        const bool fits = words - 1u < (1u << 16) && ((words & 63u) | (off & 3u)) == 0u && off < end && end <= exp_words;
+        uint32_t rows = fits ? words >> 6 : 0u;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
+        foot = (4u * quads_of(u) * (rows * 256u + 32u) + 255u) & ~255u;
+        staged = __all_sync(0xFFFFFFFFu, fits) && foot <= G.ring_bytes;
+        base = slot == 0 ? ring : ring + G.ring_bytes - foot;
+        if (lane == 0) {
+            posted[4 * slot] = rows;
+            posted[4 * slot + 1] = base;
+            posted[4 * slot + 2] = staged ? 1u : 0u;
+        }
+    };
+    auto start_copies = [&](const Place &u, int slot) {
+        const uint32_t bar = bar0 + 8u * slot;
+        const int n = quads_of(u);
+        uint32_t total = lane < 4 * n ? words * 4u : 0u, rows = words >> 6;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
+            rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
+        }
+        if (lane == 0) mbar_expect_tx(bar, total);
+        __syncwarp();
+        if (lane < 4 * n) {
+            bulk_copy_g2s(smem_base + base + lane * (rows * 256u + 32u), L.exp + at, words * 4u, bar);
+            prefetch_l2(L.rem + static_cast<int64_t>(record_of(u, lane)) * L.Nc, static_cast<uint32_t>(L.Nc));
+        }
+    };
+
+    // A lane's share of the copies that bring a chunk of its warp's sign/mantissa rows: 16 bytes of block lane / 8 of the
+    // chunk, row (lane / 2) % 4 of each quad.
+    const uint8_t *rem[2];
+    auto rem_rows = [&](const Place &u) {
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            rem[q] = L.rem + static_cast<int64_t>(record_of(u, 4 * q + ((lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 + wig * 32 + (lane & 1) * 16;
+    };
+    uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
+    auto fetch = [&](int n, int blk, uint32_t to) {
+        const uint32_t bytes = blk + (lane >> 3) < nblk ? 16u : 0u, dst = rem_at + to + 16u * lane;
+        cp_async_16(dst, rem[0] + (bytes ? blk * 128 : -(lane >> 3) * 128), bytes);
+        if (n > 1) cp_async_16(dst + 512u, rem[1] + (bytes ? blk * 128 : -(lane >> 3) * 128), bytes);
+    };
+
+    Place cur{quad_lo, 0}, nxt = after(cur);
+    request(cur);
+    if (cur.quad < quad_hi) {
+        rem_rows(cur);
+        fetch(quads_of(cur), 0, 0u);
+        if (leader) {
+            place(cur, 0);
+            if (staged) start_copies(cur, 0);
+        }
+    }
+    request(nxt);
+    uint32_t prev_foot = staged ? foot : 0u;                           // leader: ring bytes of the unit being decoded
+
+    bool usable = smem_base == kTableAt;      // the table's place is a constant in the loads; else records are decoded directly
+    if (kHuff && prepared != nullptr) {
+        if (!mbar_wait_bounded(table_bar, 0u) && tid == 0) atomicExch(&g_staged_status, 2);
+        usable = usable && Dec::usable(*reinterpret_cast<const Tables *>(&tab));
+    } else {
+        load_tables(tab, targs, tid, kThreads);
+        asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
+        Dec::fill(smem, tab, targs, kc, tid, kThreads);
+    }
+
+    // Everything above read weights only.  X (and Y) belong to the previous kernel in the stream.
+    pdl_wait();
+    uint32_t launch_no = 0;
+    if (exchange) {
+        launch_no = *reinterpret_cast<const volatile uint32_t *>(peers.launches) + 1u;
+        if (blockIdx.x == 0 && tid < peers.world) red_release_sys_add(pick(peers.ready, tid), 1u);
+    }
+    if (NB > 0 && !kRing) {
+        const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
+        const uint32_t bytes = static_cast<uint32_t>(L.S) * L.Nc * 2u;
+        if (tid == 0 && bulk) mbar_expect_tx(x_bar, bytes * B);
+        if (bulk) __syncwarp();
+        for (int b = bulk ? tid : warp; b < B; b += bulk ? kThreads : NG * kGemvWarps)
+            copy_x_row(xs + b * G.x_pitch, X + static_cast<int64_t>(b) * L.S * L.Nc, bytes, x_bar, bulk, lane);
+        if (!bulk && tid == 0) mbar_arrive(x_bar);
+    }
+    __syncthreads();
+    if (NB > 0 && !kRing && !mbar_wait_bounded(x_bar, 0u) && tid == 0) atomicExch(&g_staged_status, 3);
+
+    // ---- decode and multiply -------------------------------------------------------------------------------------------
+    float c[2][kAcc][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int g = 0; g < kAcc; g++) c[q][g][0] = c[q][g][1] = c[q][g][2] = c[q][g][3] = 0.f;
+    };
+    clear();
+    // ldmatrix: lane i supplies the address of row i % 8 of matrix i / 8: pairs 8j.., 8j + 4.., 32 + 8j.., 32 + 8j + 4.. of a
+    // block.  Rows past the batch repeat the last one; their products are never read.
+    uint32_t x_row[kAcc];
+#pragma unroll
+    for (int g = 0; g < kAcc; g++)
+        x_row[g] = xs + min(8 * g + (lane & 7), max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 3) & 1) + 128u * (lane >> 4);
+    int x_slot = 0, x_seg = 0;
+    uint32_t x_phase = 0u;
+    auto x_wait = [&]() {
+        if (kRing && !mbar_wait_bounded(x_full + 8u * x_slot, x_phase) && lane == 0) atomicExch(&g_staged_status, 3);
+    };
+    auto x_done = [&]() {
+        if (kRing) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(x_empty + 8u * x_slot);
+            x_seg++;
+            if (++x_slot == G.x_slots) {
+                x_slot = 0;
+                x_phase ^= 1u;
+            }
+        }
+    };
+
+    uint32_t phases = 0u;
+    int slot = 0;
+    while (cur.quad < quad_hi) {
+        const uint32_t rows = posted[4 * slot], ubase = posted[4 * slot + 1];
+        const bool is_staged = posted[4 * slot + 2] != 0u && usable;
+        bool late = false;                    // leader: the next unit's copies have to wait for this one's space
+        if (leader && nxt.quad < quad_hi) {
+            place(nxt, slot ^ 1);
+            late = staged && prev_foot + foot > G.ring_bytes;
+            if (staged && !late) start_copies(nxt, slot ^ 1);
+            prev_foot = staged ? foot : 0u;
+        }
+        const Place nn = after(nxt);
+        request(nn);
+
+        // the unit with n quads, by decoders of type D
+        auto run = [&](auto quads, auto &dec) {
+            constexpr int n = decltype(quads)::value;
+            using D = typename std::remove_reference<decltype(dec[0])>::type;
+            uint32_t *out[2] = {nullptr, nullptr};
+            bool live[2] = {false, false};
+            if (NB == 0) {
+#pragma unroll
+                for (int q = 0; q < n; q++) {
+                    const int m = 4 * (cur.quad + q) + r;
+                    live[q] = m < L.M;
+                    out[q] = reinterpret_cast<uint32_t *>(Y) + (((static_cast<int64_t>(m) * L.S + cur.k) * L.Nc) >> 1) + (sigma4 >> 2);
+                }
+            }
+            uint32_t xo = kRing ? 0u : static_cast<uint32_t>(cur.k * nblk) * 256u;
+            auto pair = [&](auto which, uint32_t rw, uint32_t xa, bool both) {
+                constexpr uint32_t j = decltype(which)::value;          // 0 or 2: block of the chunk
+                uint32_t e[n][2][2];
+                D::step(ctx, dec, e);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    if (i == 0 || both) {
+                        uint32_t w0[n], w1[n];
+#pragma unroll
+                        for (int q = 0; q < n; q++) {
+                            const uint32_t w = q == 0 ? (i == 0 ? lds_now<j * 128u>(rw) : lds_now<j * 128u + 128u>(rw))
+                                                      : (i == 0 ? lds_now<j * 128u + 512u>(rw) : lds_now<j * 128u + 640u>(rw));
+                            w0[q] = bitselect(prmt(w, 0u, 0x1100u), e[q][i][0], kRemMask);
+                            w1[q] = bitselect(prmt(w, 0u, 0x3322u), e[q][i][1], kRemMask);
+                        }
+                        if (NB > 0) {
+#pragma unroll
+                            for (int g = 0; g < kAcc; g++) {
+                                uint32_t f[4];
+                                if (i == 0) ldmatrix_x4<j * 256u>(f, x_row[g] + xa);
+                                else ldmatrix_x4<j * 256u + 256u>(f, x_row[g] + xa);
+#pragma unroll
+                                for (int q = 0; q < n; q++) mma_bf16_16x8x16(c[q][g], f[0], f[1], f[2], f[3], w0[q], w1[q]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < n; q++) {
+                                if (live[q]) {
+                                    out[q][(j + i) * 64u] = w0[q];
+                                    out[q][(j + i) * 64u + 32u] = w1[q];
+                                }
+                            }
+                        }
+                    }
+                }
+            };
+            // Chunks of four blocks.  While one is used the next (the next unit's first, at the end) is copied into the other
+            // half of the warp's buffer.
+#pragma unroll 1
+            for (int blk = 0; blk < nblk; blk += kRG) {
+                cp_async_wait();
+                __syncwarp();                 // the chunk is here for every lane, and the other half is read out
+                if (blk + kRG < nblk) {
+                    fetch(n, blk + kRG, half ^ kRemChunk);
+                } else if (nxt.quad < quad_hi) {
+                    rem_rows(nxt);
+                    fetch(quads_of(nxt), 0, half ^ kRemChunk);
+                }
+                x_wait();
+                const uint32_t rw = rem_at + half + 4u * lane, xa = kRing ? x_slot * G.x_slot : xo;
+                const int left = nblk - blk;
+                using J0 = std::integral_constant<uint32_t, 0>;
+                using J2 = std::integral_constant<uint32_t, 2>;
+                if (left >= kRG) {
+                    pair(J0{}, rw, xa, true);
+                    pair(J2{}, rw, xa, true);
+                } else {
+                    pair(J0{}, rw, xa, left > 1);
+                    if (left > 2) pair(J2{}, rw, xa, false);
+                }
+#pragma unroll
+                for (int q = 0; q < n; q++) {
+                    dec[q].clamp();
+                    if (NB == 0) out[q] += kRG * 64;
+                }
+                half ^= kRemChunk;
+                xo += kRG * 256u;
+                x_done();
+            }
+        };
+        auto dispatch = [&](auto quads) {
+            constexpr int n = decltype(quads)::value;
+            if (is_staged) {
+                const bool arrived = mbar_wait_bounded(bar0 + 8u * slot, (phases >> slot) & 1u);
+                phases ^= 1u << slot;
+                if (!arrived && lane == 0) atomicExch(&g_staged_status, 1);
+                Dec dec[n];
+#pragma unroll
+                for (int q = 0; q < n; q++) dec[q].open(smem_base + ubase + (4 * q + r) * (rows * 256u + 32u) + sigma4, rows);
+                run(quads, dec);
+            } else {
+                if (posted[4 * slot + 2] != 0u) {          // its copies were started all the same
+                    if (!mbar_wait_bounded(bar0 + 8u * slot, (phases >> slot) & 1u) && lane == 0) atomicExch(&g_staged_status, 1);
+                    phases ^= 1u << slot;
+                }
+                GemvDirect<Codec> dec[n];
+#pragma unroll
+                for (int q = 0; q < n; q++) {
+                    const uint32_t first = static_cast<uint32_t>(__ldg(L.offsets + record_of(cur, 4 * q + r)));
+                    dec[q].open(GlobalRecord{L.exp, exp_words, first + (sigma4 >> 2)}, &tab);
+                }
+                run(quads, dec);
+            }
+        };
+        const int n = quads_of(cur);
+        if (n == 2) dispatch(std::integral_constant<int, 2>{});
+        else dispatch(std::integral_constant<int, 1>{});
+
+        const bool set_done = cur.k == L.S - 1;
+        if (NB > 0 && set_done) {
+            gemv_group_barrier(group);        // the previous set's partial sums have been read
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int g = 0; g < kAcc; g++) part[((wig * 2 + q) * kAcc + g) * 32 + lane] = c[q][g][0] + c[q][g][3];
+            clear();
+        }
+        gemv_group_barrier(group);            // the unit's ring space is free; partial sums and the next unit's place are visible
+        if (late) start_copies(nxt, slot ^ 1);
+        if (NB > 0 && set_done) {
+            for (int z = wig; z < n * kAcc; z += kGemvWarps) {          // warp z % 4 finishes (quad, eight X rows) z
+                const int q = z / kAcc, g = z % kAcc;
+                const float *pp = part + (q * kAcc + g) * 32 + lane;
+                float v = pp[0];
+#pragma unroll
+                for (int w = 1; w < kGemvWarps; w++) v += pp[w * 64 * kAcc];
+                const int row = 4 * (cur.quad + q) + t, b = 8 * g + gq;
+                if (b < B && row < L.M) {
+                    if (exchange) ys[b * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
+                    else if (B <= BHI_MAX_BATCH) Y[static_cast<int64_t>(b) * L.M + row] = finish_value(v, bias, row);
+                    else Y[static_cast<int64_t>(b) * L.M + row] =
+                        f32_to_bf16_rn(bias ? v + __uint_as_float(static_cast<uint32_t>(__ldg(bias + row)) << 16) : v);
+                }
+            }
+        }
+        cur = nxt;
+        nxt = nn;
+        slot ^= 1;
+    }
+
+    if (kRing) {                              // groups with fewer units see the segments through, so that the others get theirs
+        while (x_seg < x_total) {
+            x_wait();
+            x_done();
+        }
+    }
+    if (exchange) {
+        // one thread asks whether every peer's buffer may be overwritten (an acquire at system scope); the barrier that
+        // makes the staged results visible hands its answer to the others
+        if (tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
+        asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
+        for (int i = tid; i < B * rows_cta; i += kThreads) {
+            const int b = i / rows_cta, rr = i - b * rows_cta;
+            const uint16_t v = ys[i];
+            const int64_t to = static_cast<int64_t>(b) * peers.m_total + peers.row_base + row_lo + rr;
+#pragma unroll
+            for (int q = 0; q < kMaxPeers; q++)
+                if (q < peers.world) peers.y[q][to] = v;
+        }
+        exchange_finish(peers, launch_no);
+    }
+}
+
+// ---- host side -------------------------------------------------------------------------------------
+int gemv_groups();      // 0 = by the forms below, else 2 or 4 groups only: see bhi_set_quad_warps
+
+enum class GemvX { none, resident, ring };
+
+// One way to lay a launch out: how many groups, how many CTAs share an SM, how many quads a unit has, how many quarters of
+// a unit the record ring holds, where X is.
+struct GemvForm {
+    int groups, per_sm, quads, quarters;
+    GemvX x;
+};
+
+// Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record: the longest of
+// a unit is hardly longer, and a unit that is too long after all starts its copies late or is decoded from global memory.
+static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool exchange,
+                      GemvGeom &G, uint32_t &smem_bytes) {
+    auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
+    const uint32_t cap = f.per_sm == 2 ? kSmemMax / 2 - 512 : kSmemMax;
+    const int64_t per_row = 64 * static_cast<int64_t>(L.S) * L.M;
+    const uint32_t rows = static_cast<uint32_t>((L.exp_words + per_row * 15 / 16) / per_row);
+    const int nq = ((L.M + 3) / 4 * f.groups + grid * f.groups - 1) / (grid * f.groups) + 1;       // most quads of a CTA
+    // table | exact tables, barriers | partial sums | staged results | sign/mantissa chunks | record rings | X (their slack)
+    G.exact_off = up(table_bytes);
+    G.part_off = G.exact_off + kExactBytes + kGemvCtrlBytes;
+    G.ys_off = G.part_off + up(static_cast<uint64_t>(f.groups) * kGemvWarps * 64 * 4 * acc_groups);
+    G.rem_off = G.ys_off + (exchange ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
+    G.ring_off = G.rem_off + f.groups * kGemvWarps * 2u * kRemChunk;
+    G.ring_bytes = up(4ull * f.quads * (rows * 256ull + 32u) * f.quarters / 4u);
+    const uint64_t x_off = static_cast<uint64_t>(G.ring_off) + static_cast<uint64_t>(f.groups) * G.ring_bytes;
+    if (x_off + kSlackBytes > cap) return false;
+    G.x_off = static_cast<uint32_t>(x_off);
+    uint64_t x_bytes = 0;
+    G.x_slots = 0;
+    G.x_pitch = G.x_slot = 0;
+    if (f.x == GemvX::resident) {
+        const uint64_t pitch = static_cast<uint64_t>(L.S) * L.Nc * 2u + kXPad;
+        x_bytes = pitch * B;
+        G.x_pitch = static_cast<uint32_t>(pitch);
+    } else if (f.x == GemvX::ring) {
+        G.x_pitch = 2u * kXSegCols + kXPad;
+        G.x_slot = G.x_pitch * B;
+        G.x_slots = kXSlotsMax;
+        while (G.x_slots > 2 && x_off + static_cast<uint64_t>(G.x_slots) * G.x_slot > cap) G.x_slots--;
+        x_bytes = static_cast<uint64_t>(G.x_slots) * G.x_slot;
+    }
+    if (x_bytes < kSlackBytes) x_bytes = kSlackBytes;
+    if (x_off + x_bytes > cap) return false;
+    smem_bytes = static_cast<uint32_t>(x_off + x_bytes);
+    G.batch = B;
+    G.max_quads = f.quads;
+    return true;
+}
+
+template <class Dec, int NB, int NG, bool kRing>
+static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
+                      cudaStream_t st) {
+    auto kernel = gemv_kernel<Dec, NB, NG, kRing>;
+    if (int rc = staged_prepare(kernel)) return rc;
+    PeerSet ps{};
+    if (peers) ps = *peers;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(NG * kGemvWarps * 32 + (kRing ? 32 : 0));
+    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_launches() ? 1 : 0;
+    const uint32_t bits = ans_bits_of(targs);
+    const GemvConsts k{bits, (1u << bits) - 1u, bits == 12u ? 0xFFFu : (2u << bits) - 1u, 8u, Dec::kTableBytes >> bits};
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, X, bias, Y, ps, G, k);
+    return e == cudaSuccess ? BHI_OK : cuda_fail(e, "gemv kernel launch");
+}
+
+// The first form that fits, best first.  Measured on 12288 x 4096, limit6, in us where each fits with one, four, eight rows:
+//   two CTAs per SM, X resident, two units in the ring   25.8
+//   same, 1.25 units (the next unit's copies wait for this one's space; the other groups work on)   26.2 / 26.7
+//   one CTA of twice the groups (one copy of table and X for all), X resident   27.2 / 27.6; 1.25 units 28.1 / 28.7 / 28.9
+//   same, X through the ring   30.9 / 31.4 / 31.9
+//   units of four rows, for long records   35.7
+template <class Dec, int NB, bool kLast>
+static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                           const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, cudaStream_t st) {
+    constexpr GemvX kFew = NB == 0 ? GemvX::none : GemvX::resident, kMany = NB == 0 ? GemvX::none : GemvX::ring;
+    const GemvForm forms[] = {{2, 2, 2, 8, kFew}, {2, 2, 2, 5, kFew}, {4, 1, 2, 8, kFew}, {4, 1, 2, 5, kFew}, {4, 1, 2, 8, kMany},
+                              {4, 1, 2, 5, kMany}, {4, 1, 1, 8, kMany}, {2, 1, 1, 8, kMany}, {2, 1, 1, 5, kMany}};
+    const int nquads = (L.M + 3) / 4, only = gemv_groups();
+    for (const GemvForm &f : forms) {
+        if (only && f.groups != only) continue;
+        if (!kLast && (f.quads < 2 || f.x == GemvX::ring)) break;
+        if (NB > 1 && (f.x == GemvX::resident || f.groups == 2)) continue;     // more than eight rows hardly ever fit
+        int grid = sm_count() * f.per_sm;
+        if (grid > nquads) grid = nquads;
+        GemvGeom G{};
+        uint32_t smem_bytes = 0;
+        if (!gemv_plan(L, B, Dec::kTableBytes, NB, f, grid, peers != nullptr, G, smem_bytes)) continue;
+        if (f.x == GemvX::ring) {
+            if constexpr (NB > 0 && kLast) {
+                if constexpr (NB == 1) {
+                    if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                }
+                return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+            }
+        } else {
+            if constexpr (NB <= 1) {
+                if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+            }
+        }
+    }
+    return kStagedDeclined;
+}
+
+// kLast: no other decoder is tried after this one, so it takes the less favourable forms too.  kMore: more than eight rows.
+template <class Dec, bool kLast, bool kMore>
+static int gemv_launch_rows(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                            const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, cudaStream_t st) {
+    if (B == 0) return gemv_launch_dec<Dec, 0, kLast>(L, targs, prepared, X, bias, Y, peers, B, st);
+    if (B <= 8) return gemv_launch_dec<Dec, 1, kLast>(L, targs, prepared, X, bias, Y, peers, B, st);
+    if constexpr (kMore) {
+        if (B <= 16) return gemv_launch_dec<Dec, 2, kLast>(L, targs, prepared, X, bias, Y, peers, B, st);
+        if (B <= 24) return gemv_launch_dec<Dec, 3, kLast>(L, targs, prepared, X, bias, Y, peers, B, st);
+        return gemv_launch_dec<Dec, 4, kLast>(L, targs, prepared, X, bias, Y, peers, B, st);
+    }
+    return kStagedDeclined;
+}
+
+// Every eight rows add about 6 us to a 12288 x 4096 layer (limit6: 8 rows 29 us, 16: 35, 24: 40, 32: 47); by way of the
+// dense matrix it is 60 whatever the count, and the accumulators of a fifth eight do not fit the registers.
+constexpr int kGemvMaxRows = 32;
+
+// B rows of X (0: the dense matrix into Y).  pair_complete: the caller knows that no code of the prepared table is longer
+// than 6 bits; only a tuning hint, the kernel reads from the table header whether it is so.
+template <class Codec>
+static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {
+    if (!staged_shape_ok(L) || !aligned(prepared, 16) || B > kGemvMaxRows) return kStagedDeclined;
+    if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31) || L.exp_words >= (1ll << 32)) return kStagedDeclined;
+    if constexpr (std::is_same<Codec, HuffCodec>::value) {
+        if (prepared == nullptr) return gemv_launch_rows<GemvPair<kPairBits>, true, false>(L, targs, prepared, X, bias, Y, peers, B, st);
+        if (pair_complete) return gemv_launch_rows<GemvSingle, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
+        const int rc = gemv_launch_rows<GemvPair<kWidestBits>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
+        if (rc != kStagedDeclined) return rc;
+        return gemv_launch_rows<GemvPair<kWideBits>, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
+    } else {
+        if (targs.bits == 8) {
+            const int rc = gemv_launch_rows<GemvAns<true>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
+            if (rc != kStagedDeclined) return rc;
+        }
+        return gemv_launch_rows<GemvAns<false>, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
+    }
+}
+
+}  // namespace bhi
