@@ -9,7 +9,7 @@
 #include "bhi_encode.cuh"
 #include "bhi_generic.cuh"
 #include "bhi_staged.cuh"
-#include "bhi_quad.cuh"
+#include "bhi_gemv.cuh"
 #include "bhi_tile.cuh"
 #include "bhi_tileq.cuh"
 
@@ -18,9 +18,9 @@ namespace bhi {
 static thread_local std::string g_error;
 static std::atomic<int> g_path{0};
 static std::atomic<int> g_overlap{0};
-static std::atomic<int> g_quad_ppw{0};
+static std::atomic<int> g_gemv_groups{0};
 bool overlap_launches() { return g_overlap.load() != 0; }
-int quad_passes_per_warp() { return g_quad_ppw.load(); }
+int gemv_groups() { return g_gemv_groups.load(); }
 
 // Prepared blobs the caller has declared pair-complete (bhi_huffman_table_hint): device pointer -> true.
 // A tuning hint only; bhi_huffman_prepare forgets the entry of the blob it rewrites.
@@ -81,16 +81,8 @@ static int run_gemv(const Layer &L, const typename Codec::Args &targs, const uin
     BHI_REQUIRE(aligned(X, 4) && aligned(Y, 2), "activation buffers must be 4-byte (X) / 2-byte (Y) aligned");
     const int path = g_path.load();
     const bool complete = pair_complete_hint(prepared);
-    // One or two rows of X with rANS, or with Huffman tables that have unresolved windows: the one-row-per-warp
-    // kernel is the faster one there (its single-symbol detour is cheaper, and its tensor-core tile covers two
-    // rows of X anyway)
-    const bool row_first = !(std::is_same<Codec, HuffCodec>::value && complete) && B <= 2;
-    if (path == 0 && row_first) {
-        int rc = staged_gemv<Codec>(L, targs, prepared, X, bias, Y, B, st);
-        if (rc != kStagedDeclined) return rc;
-    }
     if (path == 0) {
-        int rc = quad_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, complete, st);
+        int rc = gemv_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, complete, st);
         if (rc != kStagedDeclined) return rc;
     }
     if (path == 0 || path == 2) {
@@ -118,6 +110,10 @@ static int run_decode(const Layer &L, const typename Codec::Args &targs, const u
                       cudaStream_t st) {
     BHI_REQUIRE(Y, "null output buffer");
     BHI_REQUIRE(aligned(Y, 4), "output must be 4-byte aligned");
+    if (g_path.load() == 0) {
+        int rc = gemv_launch<Codec>(L, targs, prepared, nullptr, nullptr, Y, nullptr, 0, pair_complete_hint(prepared), st);
+        if (rc != kStagedDeclined) return rc;
+    }
     if (g_path.load() != 1) {
         int rc = staged_decode<Codec>(L, targs, prepared, Y, st);
         if (rc != kStagedDeclined) return rc;
@@ -139,10 +135,23 @@ static int run_linear(const Layer &L, const typename Codec::Args &targs, const u
     BHI_REQUIRE(aligned(X, 16) && aligned(Y, 2), "activation buffers must be 16-byte (X) / 2-byte (Y) aligned");
     BHI_REQUIRE(aligned(L.rem, 16) && aligned(L.exp, 16) && aligned(prepared, 16), "weight buffers must be 16-byte aligned");
     if (g_path.load() != 2) {
-        const int rc = tileq_launch<Codec>(L, targs, prepared, X, Y, B, st);
+        int rc = gemv_launch<Codec>(L, targs, prepared, X, nullptr, Y, nullptr, B, pair_complete_hint(prepared), st);
+        if (rc == kStagedDeclined) rc = tileq_launch<Codec>(L, targs, prepared, X, Y, B, st);
         if (rc != kStagedDeclined) return rc;
     }
     return tile_launch<Codec>(L, targs, prepared, X, Y, B, st);
+}
+
+// up to BHI_MAX_ROWS rows with a bias inside the 32-bit sum; BHI_ERR_LIMIT when only another way serves the layer
+template <class Codec>
+static int run_rows(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias,
+                    uint16_t *Y, int B, cudaStream_t st) {
+    BHI_REQUIRE(X && Y, "null activation buffer");
+    BHI_REQUIRE(B > BHI_MAX_BATCH && B <= BHI_MAX_ROWS, "batch must be in [9, 32]");
+    int rc = kStagedDeclined;
+    if (g_path.load() == 0 && aligned(X, 4) && aligned(Y, 2) && aligned(bias, 2))
+        rc = gemv_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, pair_complete_hint(prepared), st);
+    return rc == kStagedDeclined ? fail(BHI_ERR_LIMIT, "layer or buffers not supported by the fused product of 9 to 32 rows") : rc;
 }
 
 template <class Codec>
@@ -170,10 +179,8 @@ static int run_exchange(const Layer &L, const typename Codec::Args &targs, const
     peers.m_total = ex->M_total;
     int rc = kStagedDeclined;
     const bool complete = pair_complete_hint(prepared);
-    const bool row_first = !(std::is_same<Codec, HuffCodec>::value && complete) && B <= 2;
-    if (g_path.load() == 0 && !row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
+    if (g_path.load() == 0) rc = gemv_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
     if (rc == kStagedDeclined) rc = staged_exchange<Codec>(L, targs, prepared, X, peers, B, st);
-    if (rc == kStagedDeclined && g_path.load() == 0 && row_first) rc = quad_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
     return rc == kStagedDeclined ? fail(BHI_ERR_ARG, "shape not supported by the exchange kernel") : rc;
 }
 
@@ -230,8 +237,8 @@ int bhi_set_kernel_path(int path) { return g_path.exchange(path); }
 int bhi_set_launch_overlap(int on) { return g_overlap.exchange(on ? 1 : 0); }
 int bhi_set_quad_warps(int warps) {
     if (warps != 0 && warps != 16 && warps != 32) return -1;
-    const int prev = g_quad_ppw.exchange(warps == 16 ? 2 : warps == 32 ? 1 : 0);
-    return prev == 2 ? 16 : prev == 1 ? 32 : 0;
+    const int prev = g_gemv_groups.exchange(warps == 16 ? 4 : warps == 32 ? 2 : 0);
+    return prev == 4 ? 16 : prev == 2 ? 32 : 0;
 }
 int bhi_huffman_table_hint(const uint8_t *prepared, int pair_complete) {
     BHI_REQUIRE(prepared, "null prepared tables");
@@ -287,7 +294,7 @@ int bhi_huffman_prepare(const uint8_t *LUT1, const uint8_t *LUT2, const uint8_t 
         std::lock_guard<std::mutex> lock(g_hint_mu);
         g_hints.erase(prepared);
     }
-    huffman_prepare_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(t, prepared);
+    huffman_prepare_kernel<<<17, 1024, 0, static_cast<cudaStream_t>(stream)>>>(t, prepared);
     return launch_status("huffman_prepare launch");
 }
 
@@ -353,6 +360,28 @@ int bhi_linear_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp
     Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
     AnsArgs t{LUT, precision};
     return run_linear<AnsCodec>(L, t, nullptr, X, Y, batch, static_cast<cudaStream_t>(stream));
+}
+
+int bhi_rows_bf16_huffman_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                                   const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets,
+                                   const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream) {
+    if (int rc = check_layer(A_rem, A_exp, exp_words, offsets, split_k, M, Nc)) return rc;
+    BHI_REQUIRE(prepared && aligned(prepared, 16), "null or unaligned prepared tables");
+    Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
+    const uint8_t *ex = prepared + kPairEntries * 4;
+    HuffArgs t{ex, ex + 256, ex + 512, ex + 768, ex + 1024};
+    return run_rows<HuffCodec>(L, t, prepared, X, bias, Y, batch, static_cast<cudaStream_t>(stream));
+}
+
+int bhi_rows_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                      const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT,
+                      int precision, int split_k, int M, int Nc, int batch, void *stream) {
+    if (int rc = check_layer(A_rem, A_exp, exp_words, offsets, split_k, M, Nc)) return rc;
+    BHI_REQUIRE(LUT && aligned(LUT, 4), "null or unaligned table");
+    BHI_REQUIRE(precision >= BHI_ANS_PRECISION && precision <= BHI_ANS_MAX_PRECISION, "rANS precision must be in [8, 12]");
+    Layer L{A_rem, A_exp, exp_words, offsets, split_k, M, Nc};
+    AnsArgs t{LUT, precision};
+    return run_rows<AnsCodec>(L, t, nullptr, X, bias, Y, batch, static_cast<cudaStream_t>(stream));
 }
 
 int bhi_gemv_bf16_huffman_exchange(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,

@@ -202,11 +202,6 @@ template <class Codec> struct QuadOf;
 template <> struct QuadOf<HuffCodec> { using type = QuadHuff; };
 template <> struct QuadOf<AnsCodec> { using type = QuadAns; };
 
-// number of flagged entries of the folded table (0 = every 12-bit window resolves two symbols)
-__device__ __forceinline__ uint32_t prepared_flagged(const uint8_t *exact_region) {
-    return *reinterpret_cast<const uint32_t *>(exact_region + sizeof(HuffTables));
-}
-
 struct QuadUnit {
     int qi, k;              // quad index inside the CTA, chunk
     int rec;                // this lane's row: record index (chunk * M + row)
@@ -279,8 +274,8 @@ quad_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const 
     __syncthreads();
     if (prepared != nullptr && tid == 0) {
         // one copy of the folded table lands at the tail of the table region, the exact tables behind it
-        mbar_expect_tx(table_bar, kPreparedBytes);
-        bulk_copy_g2s(smem_base + G.lut_bytes - kPairEntries * 4, prepared, kPreparedBytes, table_bar);
+        mbar_expect_tx(table_bar, kPreparedSingle);
+        bulk_copy_g2s(smem_base + G.lut_bytes - kPairEntries * 4, prepared, kPreparedSingle, table_bar);
     }
 
     auto describe = [&](int qi, int k, QuadUnit &u) {
@@ -621,7 +616,7 @@ static bool quad_plan(const Layer &L, int grid, bool exchange, uint32_t ans_bits
     return false;
 }
 
-int quad_passes_per_warp();      // 0 = by table kind, 1 = 32 warps, 2 = 16 warps: see bhi_set_quad_warps
+static inline int quad_passes_per_warp() { return 0; }
 
 template <class Codec, int B, int PPW>
 static int quad_launch_p(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,

@@ -84,8 +84,14 @@ struct Consts {
                                              // shift16 = 65536 (a left shift by 16 as a multiply)
 };
 
-// A prepared-table blob (Huffman): one copy of the folded pair table, then the exact tables.
-constexpr int kPreparedBytes = kPairEntries * 4 + kExactBytes;
+// A prepared-table blob (Huffman): one copy of the folded pair table, the exact tables, the single-symbol tables with one
+// copy per lane (codes of at most 6 bits), two pair tables with a wider index.
+constexpr int kSingleBytes = 2 * 64 * 128;
+constexpr int kWideBits = 13, kWidestBits = 14;
+constexpr int kPreparedSingle = kPairEntries * 4 + kExactBytes;
+constexpr int kPreparedWide = kPreparedSingle + kSingleBytes;
+constexpr int kPreparedWidest = kPreparedWide + (4 << kWideBits);
+constexpr int kPreparedBytes = kPreparedWidest + (4 << kWidestBits);
 
 static_assert(sizeof(HuffTables) <= kExactBytes && sizeof(AnsTables) <= kExactBytes, "exact tables do not fit");
 static_assert((4 << kAnsBitsMax) * kCopies <= kLutBytes, "the largest rANS table does not fit the fast-table region");
@@ -110,6 +116,9 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // global -> this CTA's shared memory; both addresses 16-byte aligned, size a multiple of 16
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
@@ -464,11 +473,12 @@ __device__ __forceinline__ uint32_t resolve_symbol(const HuffTables &t, uint32_t
 
 // entry: bits 0..3 stream bits consumed, bit 5 single, bit 6 exact, bits 7..14 first exponent,
 // bits 16..19 length of the first symbol, bits 23..30 second exponent
+template <int kBits = kPairBits>
 __device__ __forceinline__ uint32_t pair_entry(const HuffTables &t, uint32_t v) {
     uint32_t s0, s1;
-    const uint32_t l0 = resolve_symbol(t, v, kPairBits, s0);
+    const uint32_t l0 = resolve_symbol(t, v, kBits, s0);
     if (!l0) return kEntExact;
-    const uint32_t l1 = resolve_symbol(t, v >> l0, kPairBits - l0, s1);
+    const uint32_t l1 = resolve_symbol(t, v >> l0, kBits - l0, s1);
     return l1 ? ((s0 << 7) | (s1 << 23) | (l0 << 16) | (l0 + l1)) : ((s0 << 7) | (l0 << 16) | l0 | kEntSingle);
 }
 
@@ -678,8 +688,8 @@ staged_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, Sink
         // Folded + exact tables were built once for this layer.  The blob holds ONE copy of the folded
         // table followed by the exact tables; it lands at the tail of the table region (so that the
         // exact tables fall into their place) and is fanned out into the interleaved copies below.
-        mbar_expect_tx(table_bar, kPreparedBytes);
-        bulk_copy_g2s(smem_base + kLutBytes - kPairEntries * 4, prepared, kPreparedBytes, table_bar);
+        mbar_expect_tx(table_bar, kPreparedSingle);
+        bulk_copy_g2s(smem_base + kLutBytes - kPairEntries * 4, prepared, kPreparedSingle, table_bar);
     }
 
     auto next_index = [&]() -> int {               // next row (or, with `split`, next record) of this CTA
@@ -868,14 +878,32 @@ static int staged_prepare(K kernel) {
 static bool staged_shape_ok(const Layer &L) { return aligned(L.rem, 16) && aligned(L.exp, 16); }
 
 
-// blob = folded pair table (one copy), exact tables, then one word: how many folded entries do not
-// resolve two symbols (0 lets the fused kernel run its loop without the per-step test)
+// number of flagged entries of the folded table (0 = every 12-bit window resolves two symbols)
+__device__ __forceinline__ uint32_t prepared_flagged(const uint8_t *exact_region) {
+    return *reinterpret_cast<const uint32_t *>(exact_region + sizeof(HuffTables));
+}
+
+// blob = folded pair table (one copy), exact tables with one word behind them (how many folded entries do not resolve two
+// symbols; 0 = no code is longer than 6 bits), single-symbol tables, wide pair tables.  The first block makes the first two,
+// the others share the rest.
 __global__ void __launch_bounds__(1024) huffman_prepare_kernel(HuffArgs targs, uint8_t *blob) {
     __shared__ HuffTables tab;
     __shared__ uint32_t flagged;
     if (threadIdx.x == 0) flagged = 0u;
     load_tables(tab, targs, threadIdx.x, blockDim.x);
     __syncthreads();
+    if (blockIdx.x > 0) {
+        const int first = (blockIdx.x - 1) * blockDim.x + threadIdx.x, step = (gridDim.x - 1) * blockDim.x;
+        for (int i = first; i < kSingleBytes / 4; i += step) {
+            const uint32_t s = tab.lut[0][(i >> 5) & 63], n = tab.len[s];
+            reinterpret_cast<uint32_t *>(blob + kPreparedSingle)[i] = (s << (i < kSingleBytes / 8 ? 7 : 23)) | (n & 31u);
+        }
+        for (int v = first; v < (1 << kWideBits); v += step)
+            reinterpret_cast<uint32_t *>(blob + kPreparedWide)[v] = pair_entry<kWideBits>(tab, v);
+        for (int v = first; v < (1 << kWidestBits); v += step)
+            reinterpret_cast<uint32_t *>(blob + kPreparedWidest)[v] = pair_entry<kWidestBits>(tab, v);
+        return;
+    }
     uint32_t mine = 0;
     for (int v = threadIdx.x; v < kPairEntries; v += blockDim.x) {
         const uint32_t e = pair_entry(tab, v);

@@ -74,9 +74,6 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 constexpr int kTileDecoders = 16;                 // decoder warps
 constexpr int kTileIssuer = kTileDecoders;        // warp index of the TMA + MMA issuer
@@ -287,8 +284,8 @@ tile_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (kHuff && prepared != nullptr && threadIdx.x == 0) {
-        mbar_expect_tx(table_bar, kPreparedBytes);
-        bulk_copy_g2s(smem_base + kLutBytes - kPairEntries * 4, prepared, kPreparedBytes, table_bar);
+        mbar_expect_tx(table_bar, kPreparedSingle);
+        bulk_copy_g2s(smem_base + kLutBytes - kPairEntries * 4, prepared, kPreparedSingle, table_bar);
     }
 
     auto request_x = [&](uint32_t u) {               // one thread; the stage must be free

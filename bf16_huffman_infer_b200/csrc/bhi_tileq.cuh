@@ -113,8 +113,8 @@ tileq_kernel(Layer L, typename Codec::Args targs, const uint8_t *prepared, const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (prepared != nullptr && tid == 0) {
-        mbar_expect_tx(table_bar, kPreparedBytes);
-        bulk_copy_g2s(smem_base + G.lut_bytes - kPairEntries * 4, prepared, kPreparedBytes, table_bar);
+        mbar_expect_tx(table_bar, kPreparedSingle);
+        bulk_copy_g2s(smem_base + G.lut_bytes - kPairEntries * 4, prepared, kPreparedSingle, table_bar);
     }
 
     // X stage u (counted over all sets of this CTA) holds the two blocks of W stage u: four atoms of 64 columns

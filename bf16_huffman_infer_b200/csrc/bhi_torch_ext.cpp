@@ -190,7 +190,7 @@ ForwardCall forward_of(StableIValue *stack, const Tensor &X, const Tensor &rem, 
     const int64_t K = static_cast<int64_t>(v.S) * v.Nc;
     STD_TORCH_CHECK(X.size(-1) == K, "X must have split_k*Nc columns");
     const int64_t B = X.numel() / K;
-    STD_TORCH_CHECK(B <= BHI_MAX_BATCH, "batch_size <= 8");
+    STD_TORCH_CHECK(B <= BHI_MAX_ROWS, "batch_size <= 32");
     std::optional<Tensor> bias = torch::stable::detail::to<std::optional<Tensor>>(stack[5]);
     const uint16_t *bias_ptr = nullptr;
     if (bias.has_value()) {
@@ -205,7 +205,14 @@ ForwardCall forward_of(StableIValue *stack, const Tensor &X, const Tensor &rem, 
     return {v, torch::stable::new_empty(X, shape), static_cast<int>(B), bias_ptr};
 }
 
-// forward_huffman(X, A_rem, A_exp, offsets, prepared, bias?) -> Y   (up to 8 rows of X, any leading dimensions)
+// The result of a forward call; an empty tensor where more than 8 rows need the dense matrix.
+StableIValue forward_result(int rc, const Tensor &Y) {
+    if (rc == BHI_ERR_LIMIT) return torch::stable::detail::from(torch::stable::new_empty(Y, {0}));
+    check(rc);
+    return torch::stable::detail::from(Y);
+}
+
+// forward_huffman(X, A_rem, A_exp, offsets, prepared, bias?) -> Y   (up to 32 rows of X, any leading dimensions)
 void boxed_forward_huffman(StableIValue *stack, uint64_t, uint64_t) {
     Tensor X = arg(stack, 0), rem = arg(stack, 1), exp = arg(stack, 2), off = arg(stack, 3), blob = arg(stack, 4);
     want(blob, ScalarType::Byte, "prepared");
@@ -213,10 +220,11 @@ void boxed_forward_huffman(StableIValue *stack, uint64_t, uint64_t) {
     STD_TORCH_CHECK(blob.numel() == bhi_huffman_prepared_bytes(), "prepared has the wrong size");
     torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
     ForwardCall f = forward_of(stack, X, rem, exp, off);
-    check(bhi_gemv_bf16_huffman_prepared_bias(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words,
-                                              ptr<const uint16_t>(X), f.bias, ptr<uint16_t>(f.Y), ptr<const int32_t>(off),
-                                              ptr<const uint8_t>(blob), f.v.S, f.v.M, f.v.Nc, f.B, stream_of(rem)));
-    stack[0] = torch::stable::detail::from(f.Y);
+    const auto launch = f.B <= BHI_MAX_BATCH ? bhi_gemv_bf16_huffman_prepared_bias : bhi_rows_bf16_huffman_prepared;
+    const int rc = launch(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X), f.bias,
+                          ptr<uint16_t>(f.Y), ptr<const int32_t>(off), ptr<const uint8_t>(blob), f.v.S, f.v.M, f.v.Nc, f.B,
+                          stream_of(rem));
+    stack[0] = forward_result(rc, f.Y);
 }
 
 // forward_ans(X, A_rem, A_exp, offsets, LUT, bias?) -> Y
@@ -227,10 +235,11 @@ void boxed_forward_ans(StableIValue *stack, uint64_t, uint64_t) {
     const int precision = ans_precision_of(lut);
     torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
     ForwardCall f = forward_of(stack, X, rem, exp, off);
-    check(bhi_gemv_bf16_ans_bias(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X),
-                                 f.bias, ptr<uint16_t>(f.Y), ptr<const int32_t>(off), ptr<const uint32_t>(lut), precision,
-                                 f.v.S, f.v.M, f.v.Nc, f.B, stream_of(rem)));
-    stack[0] = torch::stable::detail::from(f.Y);
+    const auto launch = f.B <= BHI_MAX_BATCH ? bhi_gemv_bf16_ans_bias : bhi_rows_bf16_ans;
+    const int rc = launch(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X), f.bias,
+                          ptr<uint16_t>(f.Y), ptr<const int32_t>(off), ptr<const uint32_t>(lut), precision, f.v.S, f.v.M,
+                          f.v.Nc, f.B, stream_of(rem));
+    stack[0] = forward_result(rc, f.Y);
 }
 
 // huffman_decode_prepared(A_rem, A_exp, Y(a!), offsets, prepared) -> ()

@@ -31,7 +31,9 @@ from .utils import get_block_size_n, split_bf16
 OP_PER_LANE = 1
 ANS_PRECISION = 8
 SLAB_ROWS = 4096          # rows encoded per slab; 64 padding words follow every slab
-FUSED_MAX_ROWS = 8        # up to here: fused decode + GEMV; beyond: decode, then a library GEMM (as the reference)
+FUSED_MAX_ROWS = 8        # up to here: fused decode + GEMV, as the reference
+FUSED_MORE_ROWS = 32      # up to here without gradients: the same kernel with more products per decoded word; beyond, or with
+                          # gradients: decode, then a library GEMM (as the reference)
 # Rows up to which the fused decode + tensor-core product (mm_huffman_prepared / mm_ans, at most 128) is used
 # instead of decode + GEMM.  Off by default: on B200 it is within 5 % of decode + library GEMM up to 32 rows and
 # behind it beyond (python -m bf16_huffman_infer_b200.examples.linear_bench), but needs no dense scratch.
@@ -568,6 +570,10 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
         output = weight._forward(input.contiguous(), None)
         output += bias
         return output
+    if FUSED_MAX_ROWS < rows <= FUSED_MORE_ROWS and rows > TENSOR_MAX_ROWS and _takes_more_rows(input, weight, bias):
+        output = weight._forward(input.contiguous(), bias)
+        if output.numel():
+            return output
     shape = input.shape
     input = input.flatten(0, -2)
     if rows <= max(FUSED_MAX_ROWS, min(TENSOR_MAX_ROWS, 128)):
@@ -579,9 +585,18 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
     return output.unflatten(0, shape[:-1])
 
 
+def _takes_more_rows(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> bool:
+    """Whether 9 to 32 rows can take the fused product, which has no backward and knows BF16 only."""
+    if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled():
+        return False
+    if bias is not None and not (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()):
+        return False
+    return not (torch.is_grad_enabled() and (input.requires_grad or (bias is not None and bias.requires_grad)))
+
+
 def linear_huffman(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor] = None) -> Tensor:
-    """``F.linear`` on a Huffman-coded weight: fused decode+GEMV up to 8 rows, decode then GEMM beyond
-    (reference ``functional.py:390-411``); optionally the fused tensor-core product up to ``TENSOR_MAX_ROWS``."""
+    """``F.linear`` on a Huffman-coded weight: fused decode+GEMV up to 8 rows (up to 32 without gradients), decode then
+    GEMM beyond (reference ``functional.py:390-411``); optionally the fused tensor-core product up to ``TENSOR_MAX_ROWS``."""
     return _linear_compressed(input, weight, bias)
 
 

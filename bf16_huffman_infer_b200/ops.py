@@ -63,7 +63,7 @@ def set_launch_overlap(on: bool) -> bool:
 
 
 # ---- prepared Huffman tables (folded once per layer instead of inside every launch) -------------------
-PREPARED_BYTES = 16384 + 2048
+PREPARED_BYTES = 16384 + 2048 + 16384 + 32768 + 65536
 
 
 def huffman_prepare(LUT1: Tensor, LUT2: Tensor, LUT3: Tensor, LUT4: Tensor, code_lengths: Tensor, prepared: Tensor) -> None:
@@ -81,7 +81,8 @@ def gemv_bf16_huffman_prepared(A_rem: Tensor, A_exp: Tensor, X: Tensor, Y: Tenso
 
 
 # A layer's forward call as one operator (output allocation, checks, launch, bias): (X, A_rem, A_exp, offsets, prepared or
-# LUT, bias or None) -> Y, up to 8 rows of X with any leading dimensions.  Bound here because a decode step calls them
+# LUT, bias or None) -> Y, up to 32 rows of X with any leading dimensions; more than 8 rows may yield an empty tensor, for
+# layers that the fused product does not take (very long records).  Bound here because a decode step calls them
 # once per layer and the way through Python is most of what a small layer costs.
 forward_huffman = _ops.forward_huffman.default
 forward_ans = _ops.forward_ans.default

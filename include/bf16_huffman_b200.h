@@ -122,6 +122,17 @@ int bhi_huffman_decode_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int
                                 uint16_t *Y, const int32_t *offsets, const uint8_t *prepared,
                                 int split_k, int M, int Nc, void *stream);
 
+/* 9..BHI_MAX_ROWS rows of X by the same kernel, X 4-byte aligned; bias BF16 [M] (may be null) is added to the 32-bit sum.
+ * BHI_ERR_LIMIT, with nothing launched, where the layer's records are too long or a buffer is not aligned: decode to a
+ * dense matrix then. */
+#define BHI_MAX_ROWS 32
+int bhi_rows_bf16_huffman_prepared(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                                   const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets,
+                                   const uint8_t *prepared, int split_k, int M, int Nc, int batch, void *stream);
+int bhi_rows_bf16_ans(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
+                      const uint16_t *X, const uint16_t *bias, uint16_t *Y, const int32_t *offsets, const uint32_t *LUT,
+                      int precision, int split_k, int M, int Nc, int batch, void *stream);
+
 /* Same two operations for the rANS-coded form; LUT is u32[2^precision] with
  * sym<<24 | freq<<12 | (slot - cum[sym]), BHI_ANS_PRECISION (8, the reference's constant) <= precision <=
  * BHI_ANS_MAX_PRECISION (12, what the 12-bit fields of the word allow; the reference's kernel asserts the
