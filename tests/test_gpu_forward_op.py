@@ -5,7 +5,7 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
-from _util import make_input, make_weight
+from _util import make_input, make_weight, rel_err
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -43,3 +43,42 @@ def test_forward_call(algo, tables, M, K, lead):
     trained = nn.Parameter(bias.clone())
     CompressedLinear(weight, trained)(x).float().sum().backward()
     assert trained.grad is not None and torch.equal(trained.grad, torch.full_like(bias, rows))
+
+
+@pytest.mark.parametrize("algo,tables", [("huffman", "limit6"), ("huffman", "escape"), ("huffman", "reference"), ("ans", None)])
+@pytest.mark.parametrize("M,K", [(3, 128), (130, 4736), (1021, 4096), (260, 12288), (64, 16384)])
+def test_nine_to_thirty_two_rows(algo, tables, M, K):
+    """More products per decoded word: counts around the groups of eight, X in segments that end mid-way, records too long
+    for shared memory, the bias inside the sum; gradients take the dense matrix."""
+    from bf16_huffman_infer_b200 import ANSWeight, CompressedLinear, HuffmanWeight, set_huffman_tables
+    W, bias = make_weight(M, K, 4), make_weight(1, M, 5)[0]
+    previous = set_huffman_tables(tables or "limit6")
+    try:
+        weight = (ANSWeight if algo == "ans" else HuffmanWeight).compress_split_n(W.to(DEV), n=3 if K == 12288 else 1, to_cpu=False)
+    finally:
+        set_huffman_tables(previous)
+    layer = CompressedLinear(weight, nn.Parameter(bias.to(DEV)))
+    for rows in (9, 16, 17, 24, 25, 32):
+        x = make_input(rows, K, rows)
+        with torch.no_grad():
+            y = layer(x.view(rows, 1, K).to(DEV))
+        assert y.shape == (rows, 1, M)
+        ref = x.double() @ W.double().T + bias.double()
+        assert rel_err(y.view(rows, M).float().cpu().numpy(), ref.numpy()) <= 1e-2, rows
+    xg = make_input(12, K, 1).to(DEV).requires_grad_()
+    layer(xg).float().sum().backward()
+    assert xg.grad is not None and layer.bias.grad is not None
+
+
+def test_unaligned_activations():
+    """Activations that start 4 bytes past a 16-byte boundary: X is staged by plain stores, whole and in segments."""
+    from bf16_huffman_infer_b200 import CompressedLinear, HuffmanWeight
+    for M, K, rows in ((260, 4096, 1), (260, 12288, 8), (260, 4096, 20)):
+        W = make_weight(M, K, 6)
+        layer = CompressedLinear(HuffmanWeight.compress(W.to(DEV), to_cpu=False), None)
+        x = make_input(rows, K, 7)
+        flat = torch.empty(rows * K + 8, dtype=torch.bfloat16, device=DEV)
+        shifted = flat[2:2 + rows * K].view(rows, K).copy_(x)
+        with torch.no_grad():
+            y = layer(shifted)
+        assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).numpy()) <= 1e-2
