@@ -175,6 +175,44 @@ void boxed_gemv_bf16_huffman_prepared(StableIValue *stack, uint64_t, uint64_t) {
                                          ptr<const uint8_t>(blob), v.S, v.M, v.Nc, static_cast<int>(B), stream_of(rem)));
 }
 
+// Uninitialised BF16 tensors on `like`'s device, without the way through the dispatcher that new_empty takes (1 us of a
+// 7 us call).
+Tensor empty_bf16(const Tensor &like, int64_t dims, const int64_t *sizes, const int64_t *strides) {
+    AtenTensorHandle out = nullptr;
+    TORCH_ERROR_CODE_CHECK(aoti_torch_empty_strided(dims, sizes, strides, aoti_torch_dtype_bfloat16(), aoti_torch_device_type_cuda(),
+                                                    like.get_device_index(), &out));
+    return Tensor(out);
+}
+
+// X's leading dimensions and `columns` columns
+Tensor output_like(const Tensor &X, int64_t columns) {
+    constexpr int64_t kDims = 16;
+    const int64_t dims = X.dim();
+    STD_TORCH_CHECK(dims >= 1 && dims <= kDims, "X has too many dimensions");
+    int64_t sizes[kDims], strides[kDims], step = 1;
+    for (int64_t d = dims - 1; d >= 0; d--) {
+        sizes[d] = d == dims - 1 ? columns : X.size(d);
+        strides[d] = step;
+        step *= sizes[d];
+    }
+    return empty_bf16(X, dims, sizes, strides);
+}
+
+Tensor dense_of(const Tensor &rem, const LayerView &v) {
+    const int64_t K = static_cast<int64_t>(v.S) * v.Nc;
+    const int64_t sizes[2] = {v.M, K}, strides[2] = {K, 1};
+    return empty_bf16(rem, 2, sizes, strides);
+}
+
+// Makes the tensor's device the current one for a scope; a device that is current already costs one query.
+struct OnDevice {
+    std::optional<torch::stable::accelerator::DeviceGuard> guard;
+    explicit OnDevice(const Tensor &t) {
+        const auto index = t.get_device_index();
+        if (torch::stable::accelerator::getCurrentDeviceIndex() != index) guard.emplace(index);
+    }
+};
+
 // What a layer's forward call needs, in one operator: output allocation, checks and launch.
 struct ForwardCall {
     LayerView v;
@@ -199,10 +237,7 @@ ForwardCall forward_of(StableIValue *stack, const Tensor &X, const Tensor &rem, 
         STD_TORCH_CHECK(bias->numel() == v.M, "bias must have M entries");
         bias_ptr = ptr<const uint16_t>(*bias);
     }
-    std::vector<int64_t> shape(X.dim());
-    for (int64_t d = 0; d + 1 < X.dim(); d++) shape[d] = X.size(d);
-    shape[X.dim() - 1] = v.M;
-    return {v, torch::stable::new_empty(X, shape), static_cast<int>(B), bias_ptr};
+    return {v, output_like(X, v.M), static_cast<int>(B), bias_ptr};
 }
 
 // The result of a forward call; an empty tensor where more than 8 rows need the dense matrix.
@@ -218,7 +253,7 @@ void boxed_forward_huffman(StableIValue *stack, uint64_t, uint64_t) {
     want(blob, ScalarType::Byte, "prepared");
     same_device(rem, blob, "prepared");
     STD_TORCH_CHECK(blob.numel() == bhi_huffman_prepared_bytes(), "prepared has the wrong size");
-    torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
+    OnDevice on(rem);
     ForwardCall f = forward_of(stack, X, rem, exp, off);
     const auto launch = f.B <= BHI_MAX_BATCH ? bhi_gemv_bf16_huffman_prepared_bias : bhi_rows_bf16_huffman_prepared;
     const int rc = launch(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X), f.bias,
@@ -233,13 +268,41 @@ void boxed_forward_ans(StableIValue *stack, uint64_t, uint64_t) {
     want(lut, ScalarType::Int, "LUT");
     same_device(rem, lut, "LUT");
     const int precision = ans_precision_of(lut);
-    torch::stable::accelerator::DeviceGuard guard(rem.get_device_index());
+    OnDevice on(rem);
     ForwardCall f = forward_of(stack, X, rem, exp, off);
     const auto launch = f.B <= BHI_MAX_BATCH ? bhi_gemv_bf16_ans_bias : bhi_rows_bf16_ans;
     const int rc = launch(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), f.v.exp_words, ptr<const uint16_t>(X), f.bias,
                           ptr<uint16_t>(f.Y), ptr<const int32_t>(off), ptr<const uint32_t>(lut), precision, f.v.S, f.v.M,
                           f.v.Nc, f.B, stream_of(rem));
     stack[0] = forward_result(rc, f.Y);
+}
+
+// dense_huffman(A_rem, A_exp, offsets, prepared) -> W [M, K]
+void boxed_dense_huffman(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor rem = arg(stack, 0), exp = arg(stack, 1), off = arg(stack, 2), blob = arg(stack, 3);
+    LayerView v = layer_of(rem, exp, off);
+    want(blob, ScalarType::Byte, "prepared");
+    same_device(rem, blob, "prepared");
+    STD_TORCH_CHECK(blob.numel() == bhi_huffman_prepared_bytes(), "prepared has the wrong size");
+    OnDevice on(rem);
+    Tensor W = dense_of(rem, v);
+    check(bhi_huffman_decode_prepared(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), v.exp_words, ptr<uint16_t>(W),
+                                      ptr<const int32_t>(off), ptr<const uint8_t>(blob), v.S, v.M, v.Nc, stream_of(rem)));
+    stack[0] = torch::stable::detail::from(W);
+}
+
+// dense_ans(A_rem, A_exp, offsets, LUT) -> W [M, K]
+void boxed_dense_ans(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor rem = arg(stack, 0), exp = arg(stack, 1), off = arg(stack, 2), lut = arg(stack, 3);
+    LayerView v = layer_of(rem, exp, off);
+    want(lut, ScalarType::Int, "LUT");
+    same_device(rem, lut, "LUT");
+    const int precision = ans_precision_of(lut);
+    OnDevice on(rem);
+    Tensor W = dense_of(rem, v);
+    check(bhi_ans_decode(ptr<const uint8_t>(rem), ptr<const uint32_t>(exp), v.exp_words, ptr<uint16_t>(W), ptr<const int32_t>(off),
+                         ptr<const uint32_t>(lut), precision, v.S, v.M, v.Nc, stream_of(rem)));
+    stack[0] = torch::stable::detail::from(W);
 }
 
 // huffman_decode_prepared(A_rem, A_exp, Y(a!), offsets, prepared) -> ()
@@ -592,6 +655,8 @@ STABLE_TORCH_LIBRARY(BHI_TORCH_NAMESPACE, m) {
     m.def("gemv_bf16_ans_exchange(Tensor A_rem, Tensor A_exp, Tensor X, Tensor offsets, Tensor LUT, Tensor peers, int rank, int row_base, int m_total) -> ()");
     m.def("forward_huffman(Tensor X, Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor prepared, Tensor? bias) -> Tensor");
     m.def("forward_ans(Tensor X, Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor LUT, Tensor? bias) -> Tensor");
+    m.def("dense_huffman(Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor prepared) -> Tensor");
+    m.def("dense_ans(Tensor A_rem, Tensor A_exp, Tensor offsets, Tensor LUT) -> Tensor");
     m.def("set_launch_overlap(int on) -> int");
     // whole-layer encoder
     m.def("split_histogram(Tensor W, int split_k, int row0, Tensor(a!) rem, Tensor(b!) histogram) -> ()");
@@ -618,6 +683,8 @@ STABLE_TORCH_LIBRARY_IMPL(BHI_TORCH_NAMESPACE, CUDA, m) {
     m.impl("gemv_bf16_huffman_prepared", &boxed_gemv_bf16_huffman_prepared);
     m.impl("forward_huffman", &boxed_forward_huffman);
     m.impl("forward_ans", &boxed_forward_ans);
+    m.impl("dense_huffman", &boxed_dense_huffman);
+    m.impl("dense_ans", &boxed_dense_ans);
     m.impl("huffman_decode_prepared", &boxed_huffman_decode_prepared);
     m.impl("linear_bf16_huffman_prepared", &boxed_linear_bf16_huffman_prepared);
     m.impl("linear_bf16_ans", &boxed_linear_bf16_ans);

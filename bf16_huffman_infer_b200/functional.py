@@ -149,13 +149,14 @@ class _Ingested:
     """A dense layer on the device with what its one pass over the weight yields: the sign/mantissa plane and the
     exponent counts.  A weight in host memory is passed over slab by slab while the rest is still on its way."""
 
-    def __init__(self, a: Tensor, split_k: int):
+    def __init__(self, a: Tensor, split_k: int, to_cpu: bool):
         assert a.dim() == 2 and a.dtype == torch.bfloat16
         assert a.size(1) % split_k == 0 and (a.size(1) // split_k) % 128 == 0, a.shape
         a = a.detach()
         dev = _work_device(a)
         M, K = a.shape
         self.split_k = split_k
+        self.host_rem: Optional[Tensor] = None
         self.rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8, device=dev)
         counts = torch.zeros(256, dtype=torch.int64, device=dev)
         if a.is_cuda:
@@ -163,7 +164,17 @@ class _Ingested:
             ops.split_histogram(self.w, split_k, 0, self.rem, counts)
         else:
             self.w = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
-            transfer.upload_rows(a, self.w, lambda lo, hi: ops.split_histogram(self.w[lo:hi], split_k, lo, self.rem, counts))
+            if to_cpu:
+                self.host_rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8)
+
+            def arrived(lo: int, hi: int) -> None:
+                ops.split_histogram(self.w[lo:hi], split_k, lo, self.rem, counts)
+                if to_cpu:
+                    # the pages that will take the plane on its way back are faulted in while the link is busy with the
+                    # next slab (the faults are half the time of a copy into new memory)
+                    self.host_rem[:, lo:hi].zero_()
+
+            transfer.upload_rows(a, self.w, arrived)
         self.histogram = counts.cpu()
 
 
@@ -183,7 +194,7 @@ class _Plan:
         exp = torch.zeros(_checked_total(total), dtype=torch.int32, device=dev)
         self.cls._emit_pass(layer, self.tables, self.offsets, exp)
         if to_cpu:
-            return self.cls(rem=transfer.download(layer.rem), exp=transfer.download(exp),
+            return self.cls(rem=transfer.download(layer.rem, layer.host_rem), exp=transfer.download(exp),
                             offsets=transfer.download(self.offsets), **self.luts)
         luts = _tables_to(self.luts, dev)
         # the buffers must be complete in memory before a fused kernel with launch overlap reads them
@@ -205,7 +216,7 @@ def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor
 def _compress(a: Tensor, split_k: int, coders: Sequence[type], to_cpu: bool) -> "HuffmanWeight":
     """``a`` by the coder that stores it in the fewest bytes (the first of those that tie).  The sizes are known after
     the size pass, so only the coder that is kept writes its records."""
-    layer = _Ingested(a, split_k)
+    layer = _Ingested(a, split_k, to_cpu)
     plans: List[_Plan] = [_Plan(c, layer, c._codec_of(layer.histogram)) for c in coders]
     totals = torch.cat([p.total for p in plans]).tolist() if len(plans) > 1 else [int(plans[0].total.item())]
     for t in totals:
@@ -344,28 +355,29 @@ class HuffmanWeight(nn.Module):
         """The decode tables folded for the fused kernels (built on first use on each device, so the
         first call has to happen outside CUDA-graph capture; warm-up iterations take care of that).
         Not a buffer: it is derived data and stays out of ``state_dict`` and size accounting."""
-        b = self._buffers
+        d = self.__dict__
+        b = d["_buffers"]
         t1, t2, t3, t4, cl = b["LUT1"], b["LUT2"], b["LUT3"], b["LUT4"], b["code_lengths"]
         # in-place loads (load_state_dict) bump the version; a tensor whose data was replaced has another address
         src = (t1.data_ptr(), t2.data_ptr(), t3.data_ptr(), t4.data_ptr(), cl.data_ptr(),
                t1._version, t2._version, t3._version, t4._version, cl._version)
-        if self.__dict__.get("_prepared_src") != src:
+        if d.get("_prepared_src") != src:
             blob = torch.empty(ops.PREPARED_BYTES, dtype=torch.uint8, device=self.rem.device)
             ops.huffman_prepare(t1, t2, t3, t4, cl, blob)
             # codes of at most 6 bits: every 12-bit window holds two whole codes (the kernels pick their warp layout by it)
             ops.huffman_table_hint(blob, int(cl.max().item()) <= 6)
-            self.__dict__["_prepared"] = blob
-            self.__dict__["_prepared_src"] = src
-        return self.__dict__["_prepared"]
+            d["_prepared"] = blob
+            d["_prepared_src"] = src
+        return d["_prepared"]
 
     def _plain(self) -> bool:
         """The buffers are as the operators take them (``compress`` makes no others)."""
-        b = self._buffers
+        b = self.__dict__["_buffers"]
         rem, exp, off = b["rem"], b["exp"], b["offsets"]
         return rem.dim() == 3 and off.dim() == 2 and rem.is_contiguous() and exp.is_contiguous() and off.is_contiguous()
 
     def _forward(self, x: Tensor, bias: Optional[Tensor]) -> Tensor:
-        b = self._buffers
+        b = self.__dict__["_buffers"]
         return ops.forward_huffman(x, b["rem"], b["exp"], b["offsets"], self.prepared(), bias)
 
     def _mv(self, x: Tensor) -> Tensor:
@@ -376,10 +388,9 @@ class HuffmanWeight(nn.Module):
 
     def get_weight(self) -> Tensor:
         """Dense BF16 ``[M, K]`` (reference ``functional.py:99-108``)."""
-        assert self.rem.device.type == "cuda"
-        weight = torch.empty(self.shape, dtype=torch.bfloat16, device=self.rem.device)
-        ops.huffman_decode_prepared(self.rem, self.exp, weight, self.offsets, self.prepared())
-        return weight
+        b = self._buffers
+        assert b["rem"].is_cuda
+        return ops.dense_huffman(b["rem"], b["exp"], b["offsets"], self.prepared())
 
     # -- encoding -----------------------------------------------------------------------------
     @classmethod
@@ -474,7 +485,7 @@ class ANSWeight(HuffmanWeight):
         return linear_ans(*args, **(kwargs or {}))
 
     def _forward(self, x: Tensor, bias: Optional[Tensor]) -> Tensor:
-        b = self._buffers
+        b = self.__dict__["_buffers"]
         return ops.forward_ans(x, b["rem"], b["exp"], b["offsets"], b["LUT"], bias)
 
     def _mv(self, x: Tensor) -> Tensor:
@@ -484,10 +495,9 @@ class ANSWeight(HuffmanWeight):
         return mm_ans(self.rem, self.exp, x, self.offsets, self.LUT)
 
     def get_weight(self) -> Tensor:
-        assert self.rem.device.type == "cuda"
-        weight = torch.empty(self.shape, dtype=torch.bfloat16, device=self.rem.device)
-        ops.ans_decode(self.rem, self.exp, weight, self.offsets, self.LUT)
-        return weight
+        b = self._buffers
+        assert b["rem"].is_cuda
+        return ops.dense_ans(b["rem"], b["exp"], b["offsets"], b["LUT"])
 
     @classmethod
     def get_codec(cls, a: Tensor) -> RANSEncoder:
@@ -551,7 +561,11 @@ class CompressedLinear(nn.Module):
         return self.weight.shape[1]
 
     def forward(self, input: Tensor) -> Tensor:
-        return _linear_compressed(input, self.weight, self.bias)
+        d = self.__dict__                       # nn.Module's own attribute lookup costs more than the checks below
+        bias = d["_parameters"].get("bias")
+        if bias is None:
+            bias = self.bias
+        return _linear_compressed(input, d["_modules"]["weight"], bias)
 
 
 def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> Tensor:
@@ -562,26 +576,27 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
         assert input.is_cuda and input.dtype == torch.bfloat16
         if input.requires_grad:
             input = input.detach()
+        if not input.is_contiguous():
+            input = input.contiguous()
         if bias is None:
-            return weight._forward(input.contiguous(), None)
+            return weight._forward(input, None)
         if (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
                 and not (bias.requires_grad and torch.is_grad_enabled())):
-            return weight._forward(input.contiguous(), bias)
-        output = weight._forward(input.contiguous(), None)
+            return weight._forward(input, bias)
+        output = weight._forward(input, None)
         output += bias
         return output
     if FUSED_MAX_ROWS < rows <= FUSED_MORE_ROWS and rows > TENSOR_MAX_ROWS and _takes_more_rows(input, weight, bias):
         output = weight._forward(input.contiguous(), bias)
         if output.numel():
             return output
+    if rows > max(FUSED_MAX_ROWS, min(TENSOR_MAX_ROWS, 128)):
+        return F.linear(input, weight.get_weight(), bias)
     shape = input.shape
     input = input.flatten(0, -2)
-    if rows <= max(FUSED_MAX_ROWS, min(TENSOR_MAX_ROWS, 128)):
-        output = weight._mv(input) if rows <= FUSED_MAX_ROWS else weight._mm(input)
-        if bias is not None:
-            output += bias[None, :]
-    else:
-        output = F.linear(input, weight.get_weight(), bias)
+    output = weight._mv(input) if rows <= FUSED_MAX_ROWS else weight._mm(input)
+    if bias is not None:
+        output += bias[None, :]
     return output.unflatten(0, shape[:-1])
 
 

@@ -86,6 +86,9 @@ def gemv_bf16_huffman_prepared(A_rem: Tensor, A_exp: Tensor, X: Tensor, Y: Tenso
 # once per layer and the way through Python is most of what a small layer costs.
 forward_huffman = _ops.forward_huffman.default
 forward_ans = _ops.forward_ans.default
+# a layer's dense BF16 matrix, allocated inside: (A_rem, A_exp, offsets, prepared or LUT) -> W
+dense_huffman = _ops.dense_huffman.default
+dense_ans = _ops.dense_ans.default
 
 
 def linear_bf16_huffman_prepared(A_rem: Tensor, A_exp: Tensor, X: Tensor, Y: Tensor, offsets: Tensor, prepared: Tensor) -> None:

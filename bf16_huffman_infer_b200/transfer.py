@@ -54,13 +54,14 @@ def upload_rows(src: Tensor, dst: Tensor, arrived: Optional[Callable[[int, int],
             arrived(lo, hi)
 
 
-def download(src: Tensor) -> Tensor:
-    """A device tensor as a new host tensor; complete when the call returns."""
+def download(src: Tensor, out: Optional[Tensor] = None) -> Tensor:
+    """A device tensor as a host tensor (``out``, contiguous and pageable, or a new one); complete when the call returns."""
     nbytes = src.numel() * src.element_size()
     if nbytes <= _SMALL:
-        return src.cpu()
+        return src.cpu() if out is None else out.copy_(src)
     stream = torch.cuda.current_stream(src.device)
-    out = torch.empty(src.shape, dtype=src.dtype)
+    if out is None:
+        out = torch.empty(src.shape, dtype=src.dtype)
     flat_src, flat_out = src.contiguous().view(-1).view(torch.uint8), out.view(-1).view(torch.uint8)
     slabs = _slabs(nbytes)
     here = [torch.cuda.Event() for _ in slabs]
