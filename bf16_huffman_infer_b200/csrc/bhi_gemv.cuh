@@ -47,6 +47,8 @@ struct GemvGeom {
     int x_slots;               // segments of the ring; 0 = all of X is resident
     int batch;
     int max_quads;             // of a unit: 2, or 1 when records are long
+    int split;                 // the groups of a CTA share its quads and divide the chunks among them
+    uint32_t acc_off;          // ... whose sums meet here
 };
 
 // Values the compiler must not see: multiply-adds by them stay on the FMA pipe.
@@ -281,13 +283,14 @@ struct GemvPair {
 // there) above the state's own 32 + bits bits, where the next step's funnel shift never looks.
 // As many copies of the table as fill its place; a 64-bit load is served in two halves of 16 lanes, so 16 copies are free
 // of conflicts.
-//   k8 = true   8 bits: 32 copies, so that the entry stride is 256 bytes and the address one byte permutation of the state
-//               and the lane's offset
-//   k8 = false  any precision, half the space
-template <bool k8>
+//   k8 = true   8 bits in 64 KB: 32 copies, so that the entry stride is 256 bytes and the address one byte permutation of
+//               the state and the lane's offset
+//   k8 = false  any precision, in 64 KB or, where X needs the room, 32
+template <bool k8, uint32_t kBytes>
 struct GemvAns {
     using Codec = AnsCodec;
-    static constexpr uint32_t kTableBytes = k8 ? 64 * 1024 : 32 * 1024;
+    static constexpr uint32_t kTableBytes = kBytes;
+    static_assert(!k8 || kBytes == 64 * 1024, "the address permutation needs a stride of 256 bytes");
     struct Stream {
         uint32_t lo, hi, nx;
     };
@@ -299,16 +302,28 @@ struct GemvAns {
             const uint32_t w = __ldg(a.lut + v);
             return make_uint2(w & 0xFFFu, (w & 0xFF000000u) | (((w >> 12) & 0xFFFu) << k.ans_bits));
         };
-        if (k8) {
-            // half an entry (16 copies) per thread, each lane starting at another 16 bytes of it: no bank conflicts
-            for (uint32_t i = tid; i < 512u; i += threads) {
-                const uint2 e = entry(i >> 1);
+        // 128 bytes of copies per thread and turn, written 16 bytes at a time, each lane starting at another 16 of them: no
+        // bank conflicts.  An entry that has fewer copies than that shares the 128 bytes with its neighbours.
+        const uint32_t copies_log2 = (kBytes == 64 * 1024 ? 13u : 12u) - k.ans_bits;
+#pragma unroll
+        for (uint32_t i = tid; i < kBytes / 128u; i += threads) {
+            if (copies_log2 >= 4u) {
+                const uint2 e = entry(i >> (copies_log2 - 4u));
 #pragma unroll
                 for (uint32_t j = 0; j < 8u; j++)
                     reinterpret_cast<uint4 *>(table)[8u * i + ((j + tid) & 7u)] = make_uint4(e.x, e.y, e.x, e.y);
+            } else {
+                uint2 lo[8], hi[8];
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; j++) {
+                    const uint32_t at = 16u * i + 2u * ((j + tid) & 7u);
+                    lo[j] = entry(at >> copies_log2);
+                    hi[j] = entry((at + 1u) >> copies_log2);
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; j++)
+                    reinterpret_cast<uint4 *>(table)[8u * i + ((j + tid) & 7u)] = make_uint4(lo[j].x, lo[j].y, hi[j].x, hi[j].y);
             }
-        } else {
-            for (uint32_t i = tid; i < kTableBytes / 8; i += threads) reinterpret_cast<uint2 *>(table)[i] = entry(i >> (12u - k.ans_bits));
         }
     }
     static __device__ __forceinline__ bool usable(const AnsTables &) { return true; }
@@ -500,9 +515,14 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     // Quads are dealt to the groups of the grid in equal contiguous ranges; a group takes them two at a time.
     const int nquads = (L.M + 3) >> 2;
     auto deal = [&](int g) { return static_cast<int>(static_cast<int64_t>(nquads) * g / (static_cast<int>(gridDim.x) * NG)); };
-    const int quad_lo = deal(blockIdx.x * NG + group), quad_hi = deal(blockIdx.x * NG + group + 1);
-    const int row_lo = 4 * deal(blockIdx.x * NG);                      // rows of the CTA
-    const int rows_cta = min(4 * deal(blockIdx.x * NG + NG), L.M) - row_lo;
+    const bool split = !kRing && NB <= 1 && G.split;
+    const int cta_lo = deal(blockIdx.x * NG), cta_hi = deal(blockIdx.x * NG + NG);
+    const int k_lo = split ? L.S * group / NG : 0, k_hi = split ? L.S * (group + 1) / NG : L.S;
+    const int quad_lo = !split ? deal(blockIdx.x * NG + group) : k_lo < k_hi ? cta_lo : cta_hi;
+    const int quad_hi = !split ? deal(blockIdx.x * NG + group + 1) : cta_hi;
+    const int row_lo = 4 * cta_lo;                                     // rows of the CTA
+    const int rows_cta = min(4 * cta_hi, L.M) - row_lo;
+    float *acc = reinterpret_cast<float *>(smem + G.acc_off);          // [quad of the CTA][group][lane]
     const int nblk = L.Nc >> 7;
     const int chunks = (nblk + kRG - 1) / kRG;                         // of a record
 
@@ -579,8 +599,8 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     auto quads_of = [&](const Place &u) { return min(G.max_quads, quad_hi - u.quad); };
     auto after = [&](const Place &u) {
         Place v{u.quad, u.k + 1};
-        if (v.k == L.S) {
-            v.k = 0;
+        if (v.k == k_hi) {
+            v.k = k_lo;
             v.quad += G.max_quads;
         }
         return v;
@@ -648,7 +668,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (n > 1) cp_async_16(dst + 512u, rem[1] + (bytes ? blk * 128 : -(lane >> 3) * 128), bytes);
     };
 
-    Place cur{quad_lo, 0}, nxt = after(cur);
+    Place cur{quad_lo, k_lo}, nxt = after(cur);
     request(cur);
     if (cur.quad < quad_hi) {
         rem_rows(cur);
@@ -850,7 +870,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (n == 2) dispatch(std::integral_constant<int, 2>{});
         else dispatch(std::integral_constant<int, 1>{});
 
-        const bool set_done = cur.k == L.S - 1;
+        const bool set_done = cur.k == k_hi - 1;
         if (NB > 0 && set_done) {
             gemv_group_barrier(group);        // the previous set's partial sums have been read
 #pragma unroll
@@ -869,7 +889,9 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
 #pragma unroll
                 for (int w = 1; w < kGemvWarps; w++) v += pp[w * 64 * kAcc];
                 const int row = 4 * (cur.quad + q) + t, b = 8 * g + gq;
-                if (b < B && row < L.M) {
+                if (split) {
+                    acc[((cur.quad + q - cta_lo) * NG + group) * 32 + lane] = v;
+                } else if (b < B && row < L.M) {
                     if (exchange) ys[b * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
                     else if (B <= BHI_MAX_BATCH) Y[static_cast<int64_t>(b) * L.M + row] = finish_value(v, bias, row);
                     else Y[static_cast<int64_t>(b) * L.M + row] =
@@ -882,6 +904,20 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         slot ^= 1;
     }
 
+    if (NB == 1 && split) {                   // the groups' sums, in the order of their chunks
+        asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
+        for (int i = warp; i < cta_hi - cta_lo; i += NG * kGemvWarps) {
+            float v = 0.f;
+#pragma unroll
+            for (int g = 0; g < NG; g++)
+                if (L.S * g / NG < L.S * (g + 1) / NG) v += acc[(i * NG + g) * 32 + lane];
+            const int row = 4 * (cta_lo + i) + t;
+            if (gq < B && row < L.M) {
+                if (exchange) ys[gq * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
+                else Y[static_cast<int64_t>(gq) * L.M + row] = finish_value(v, bias, row);
+            }
+        }
+    }
     if (kRing) {                              // groups with fewer units see the segments through, so that the others get theirs
         while (x_seg < x_total) {
             x_wait();
@@ -925,12 +961,20 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     const uint32_t cap = f.per_sm == 2 ? kSmemMax / 2 - 512 : kSmemMax;
     const int64_t per_row = 64 * static_cast<int64_t>(L.S) * L.M;
     const uint32_t rows = static_cast<uint32_t>((L.exp_words + per_row * 15 / 16) / per_row);
-    const int nq = ((L.M + 3) / 4 * f.groups + grid * f.groups - 1) / (grid * f.groups) + 1;       // most quads of a CTA
-    // table | exact tables, barriers | partial sums | staged results | sign/mantissa chunks | record rings | X (their slack)
+    const int nquads = (L.M + 3) / 4, nq = (nquads + grid - 1) / grid + 1;                         // most quads of a CTA
+    // Few quads and several chunks: a group would take the chunks of its quad or two one after the other while others have
+    // none.  The groups of a CTA share its quads instead and divide the chunks, where that shortens the longest group's
+    // work by a tenth (a unit of one quad takes six tenths of one of two).
+    auto sets = [&](int quads) { return f.quads == 2 ? quads / 2 * 10 + quads % 2 * 6 : quads * 6; };
+    const int group_quads = (nquads + grid * f.groups - 1) / (grid * f.groups), cta_quads = (nquads + grid - 1) / grid;
+    G.split = f.x != GemvX::ring && L.S > 1 && acc_groups <= 1 &&
+              10 * ((L.S + f.groups - 1) / f.groups) * sets(cta_quads) <= 9 * L.S * sets(group_quads);
+    // table | exact tables, barriers | partial sums | staged results | split sums | sign/mantissa chunks | record rings | X (their slack)
     G.exact_off = up(table_bytes);
     G.part_off = G.exact_off + kExactBytes + kGemvCtrlBytes;
     G.ys_off = G.part_off + up(static_cast<uint64_t>(f.groups) * kGemvWarps * 64 * 4 * acc_groups);
-    G.rem_off = G.ys_off + (exchange ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
+    G.acc_off = G.ys_off + (exchange ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
+    G.rem_off = G.acc_off + (G.split && acc_groups ? up(static_cast<uint64_t>(nq) * f.groups * 128) : 0u);
     G.ring_off = G.rem_off + f.groups * kGemvWarps * 2u * kRemChunk;
     G.ring_bytes = up(4ull * f.quads * (rows * 256ull + 32u) * f.quarters / 4u);
     const uint64_t x_off = static_cast<uint64_t>(G.ring_off) + static_cast<uint64_t>(f.groups) * G.ring_bytes;
@@ -1053,11 +1097,12 @@ static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const 
         if (rc != kStagedDeclined) return rc;
         return gemv_launch_rows<GemvPair<kWideBits>, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
     } else {
-        if (targs.bits == 8) {
-            const int rc = gemv_launch_rows<GemvAns<true>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
-            if (rc != kStagedDeclined) return rc;
-        }
-        return gemv_launch_rows<GemvAns<false>, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
+        // (a finer model on a layer of at most a quad per group: filling the larger table costs more than its conflicts)
+        int rc = kStagedDeclined;
+        if (targs.bits == 8) rc = gemv_launch_rows<GemvAns<true, 64 * 1024>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
+        else if (L.M > 16 * sm_count()) rc = gemv_launch_rows<GemvAns<false, 64 * 1024>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
+        if (rc != kStagedDeclined) return rc;
+        return gemv_launch_rows<GemvAns<false, 32 * 1024>, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
     }
 }
 
