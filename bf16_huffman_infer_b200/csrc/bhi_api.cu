@@ -81,12 +81,8 @@ static int run_gemv(const Layer &L, const typename Codec::Args &targs, const uin
     BHI_REQUIRE(aligned(X, 4) && aligned(Y, 2), "activation buffers must be 4-byte (X) / 2-byte (Y) aligned");
     const int path = g_path.load();
     const bool complete = pair_complete_hint(prepared);
-    if (path == 0) {
+    if (path != 1) {
         int rc = gemv_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, complete, st);
-        if (rc != kStagedDeclined) return rc;
-    }
-    if (path == 0 || path == 2) {
-        int rc = staged_gemv<Codec>(L, targs, prepared, X, bias, Y, B, st);
         if (rc != kStagedDeclined) return rc;
     }
     // one warp per row, enough blocks to give every row its own warp up to 8 waves of blocks per SM
@@ -110,12 +106,8 @@ static int run_decode(const Layer &L, const typename Codec::Args &targs, const u
                       cudaStream_t st) {
     BHI_REQUIRE(Y, "null output buffer");
     BHI_REQUIRE(aligned(Y, 4), "output must be 4-byte aligned");
-    if (g_path.load() == 0) {
-        int rc = gemv_launch<Codec>(L, targs, prepared, nullptr, nullptr, Y, nullptr, 0, pair_complete_hint(prepared), st);
-        if (rc != kStagedDeclined) return rc;
-    }
     if (g_path.load() != 1) {
-        int rc = staged_decode<Codec>(L, targs, prepared, Y, st);
+        int rc = gemv_launch<Codec>(L, targs, prepared, nullptr, nullptr, Y, nullptr, 0, pair_complete_hint(prepared), st);
         if (rc != kStagedDeclined) return rc;
     }
     const int64_t nrec = static_cast<int64_t>(L.S) * L.M;
@@ -177,10 +169,7 @@ static int run_exchange(const Layer &L, const typename Codec::Args &targs, const
     peers.rank = ex->rank;
     peers.row_base = ex->row_base;
     peers.m_total = ex->M_total;
-    int rc = kStagedDeclined;
-    const bool complete = pair_complete_hint(prepared);
-    if (g_path.load() == 0) rc = gemv_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, complete, st);
-    if (rc == kStagedDeclined) rc = staged_exchange<Codec>(L, targs, prepared, X, peers, B, st);
+    const int rc = gemv_launch<Codec>(L, targs, prepared, X, nullptr, nullptr, &peers, B, pair_complete_hint(prepared), st);
     return rc == kStagedDeclined ? fail(BHI_ERR_ARG, "shape not supported by the exchange kernel") : rc;
 }
 

@@ -23,7 +23,7 @@
 //
 // Results: the four warps of a group add their partial sums through shared memory in pass order (deterministic).
 // Row-sharded layers stage their results and store them into every rank's output with coalesced peer stores at the end
-// of the kernel (see ExchangeSink for the protocol).
+// of the kernel (see PeerSet for the protocol).
 #pragma once
 
 #include "bhi_staged.cuh"
@@ -1032,12 +1032,14 @@ static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, co
 //   one CTA of twice the groups (one copy of table and X for all), X resident   27.2 / 27.6; 1.25 units 28.1 / 28.7 / 28.9
 //   same, X through the ring   30.9 / 31.4 / 31.9
 //   units of four rows, for long records   35.7
+// The last form stages no record at all.
 template <class Dec, int NB, bool kLast>
 static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                            const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, cudaStream_t st) {
     constexpr GemvX kFew = NB == 0 ? GemvX::none : GemvX::resident, kMany = NB == 0 ? GemvX::none : GemvX::ring;
     const GemvForm forms[] = {{2, 2, 2, 8, kFew}, {2, 2, 2, 5, kFew}, {4, 1, 2, 8, kFew}, {4, 1, 2, 5, kFew}, {4, 1, 2, 8, kMany},
-                              {4, 1, 2, 5, kMany}, {4, 1, 1, 8, kMany}, {2, 1, 1, 8, kMany}, {2, 1, 1, 5, kMany}};
+                              {4, 1, 2, 5, kMany}, {4, 1, 1, 8, kMany}, {2, 1, 1, 8, kMany}, {2, 1, 1, 5, kMany},
+                              {2, 1, 1, 0, kMany}};
     const int nquads = (L.M + 3) / 4, only = gemv_groups();
     for (const GemvForm &f : forms) {
         if (only && f.groups != only) continue;

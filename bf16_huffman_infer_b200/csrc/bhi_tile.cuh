@@ -158,7 +158,7 @@ struct HuffReg {
     __device__ __forceinline__ uint32_t pair(const uint8_t *smem, const Consts &k, const HuffTables &t, const uint32_t *exp,
                                              uint32_t at, uint32_t lim, uint32_t copy_off) {
         uint32_t win = __funnelshift_r(w0, w1, c);
-        uint32_t e = HuffStaged::lookup(smem, k, win, copy_off);
+        uint32_t e = pair_lookup(smem, k, win, copy_off);
         if (!kChecked || !(e & (kEntSingle | kEntExact))) {
             advance(exp, at, lim, e & kEntBits);
             return e;
@@ -171,7 +171,7 @@ struct HuffReg {
             advance(exp, at, lim, e & kEntBits);
         }
         win = __funnelshift_r(w0, w1, c);
-        const uint32_t e2 = HuffStaged::lookup(smem, k, win, copy_off);
+        const uint32_t e2 = pair_lookup(smem, k, win, copy_off);
         uint32_t s1 = (e2 >> 7) & 0xFFu, l1 = (e2 >> 16) & 15u;
         if (e2 & kEntExact) {
             const uint2 f = huff_exact_symbol(win, &t);

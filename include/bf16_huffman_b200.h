@@ -45,20 +45,16 @@ const char *bhi_last_error(void);
 int bhi_abi_version(void);
 
 /* Which implementation the gemv / decode entry points use:
- *   0 = automatic (the four-rows-per-warp-group kernel when the shape allows it, else the
- *       one-row-per-warp staged kernel, else the generic path)
+ *   0, 2 = automatic (the fused kernel when the buffers are aligned, else the generic path)
  *   1 = generic path only (one warp per record, direct global loads)
- *   2 = skip the four-rows-per-warp-group kernel (one-row-per-warp staged kernel, else generic)
- * The linear entry points choose between their two kernels the same way: 0 = the one whose decoders stage records in
- * shared memory when the batch leaves room for them (up to about 48 rows), else the one that keeps its streams in
+ * The linear entry points: 0 = the fused kernel up to 32 rows, then the tensor-memory kernel whose decoders stage records in
+ * shared memory while the batch leaves room for them (up to about 48 rows), else the one that keeps its streams in
  * registers; 2 = the latter always.
  * Process-wide; meant for tests and A/B measurements.  Returns the previous value. */
 int bhi_set_kernel_path(int path);
 
-/* Warps per block of the four-rows-per-warp-group kernel: 32 (a lane decodes two streams), 16 (a lane
- * decodes four streams, twice the registers per thread) or 0 = chosen per call (16 for rANS and for Huffman
- * tables declared pair-complete, see bhi_huffman_table_hint; else 32).  Process-wide; returns the previous
- * value, -1 for any other argument.  For A/B measurements. */
+/* Warps per SM's block of the fused kernel: 32 = two blocks of eight warps, 16 = one block of sixteen, 0 = whichever fits
+ * the launch best.  Process-wide; returns the previous value, -1 for any other argument.  For A/B measurements. */
 int bhi_set_quad_warps(int warps);
 
 /* Launch overlap (programmatic dependent launch), process-wide, off by default.  When on, a fused
@@ -94,9 +90,9 @@ int bhi_huffman_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_
                        int split_k, int M, int Nc, void *stream);
 
 /* ---- prepared Huffman tables ---------------------------------------------------------------
- * The fused kernels do not decode with the four byte tables directly: they fold them into a
- * 4096-entry two-symbols-per-lookup table (kept in four bank-interleaved copies).  The two entry points above rebuild that table inside
- * every launch, which costs a few microseconds per call.  A caller that keeps a layer around can
+ * The fused kernels do not decode with the four byte tables directly: they fold them into single-symbol and
+ * two-symbols-per-lookup tables.  The two entry points above rebuild such a table inside every launch, which costs a few
+ * microseconds per call.  A caller that keeps a layer around can
  * fold the tables once into a blob of bhi_huffman_prepared_bytes() bytes (16-byte aligned device
  * memory owned by the caller) and pass the blob instead of the five tables; the kernels then
  * fetch it with a single bulk copy.  Results are identical.  No counterpart in the reference
