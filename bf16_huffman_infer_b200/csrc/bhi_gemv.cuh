@@ -953,8 +953,8 @@ struct GemvForm {
     GemvX x;
 };
 
-// Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record: the longest of
-// a unit is hardly longer, and a unit that is too long after all starts its copies late or is decoded from global memory.
+// Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record and takes a unit
+// whose longest is a word row and an eighth longer; one that is longer still is decoded from global memory.
 static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool exchange,
                       GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
@@ -976,7 +976,9 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     G.acc_off = G.ys_off + (exchange ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
     G.rem_off = G.acc_off + (G.split && acc_groups ? up(static_cast<uint64_t>(nq) * f.groups * 128) : 0u);
     G.ring_off = G.rem_off + f.groups * kGemvWarps * 2u * kRemChunk;
-    G.ring_bytes = up(4ull * f.quads * (rows * 256ull + 32u) * f.quarters / 4u);
+    auto unit = [&](uint64_t r) { return 4ull * f.quads * (r * 256u + 32u); };
+    const uint64_t wanted = unit(rows) * f.quarters / 4u, longest = f.quarters ? unit(rows + 1u + rows / 8u) : 0u;
+    G.ring_bytes = up(wanted > longest ? wanted : longest);
     const uint64_t x_off = static_cast<uint64_t>(G.ring_off) + static_cast<uint64_t>(f.groups) * G.ring_bytes;
     if (x_off + kSlackBytes > cap) return false;
     G.x_off = static_cast<uint32_t>(x_off);
@@ -1038,7 +1040,7 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
                            const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, cudaStream_t st) {
     constexpr GemvX kFew = NB == 0 ? GemvX::none : GemvX::resident, kMany = NB == 0 ? GemvX::none : GemvX::ring;
     const GemvForm forms[] = {{2, 2, 2, 8, kFew}, {2, 2, 2, 5, kFew}, {4, 1, 2, 8, kFew}, {4, 1, 2, 5, kFew}, {4, 1, 2, 8, kMany},
-                              {4, 1, 2, 5, kMany}, {4, 1, 1, 8, kMany}, {2, 1, 1, 8, kMany}, {2, 1, 1, 5, kMany},
+                              {4, 1, 2, 5, kMany}, {4, 1, 1, 5, kFew}, {4, 1, 1, 5, kMany}, {2, 1, 1, 5, kMany},
                               {2, 1, 1, 0, kMany}};
     const int nquads = (L.M + 3) / 4, only = gemv_groups();
     for (const GemvForm &f : forms) {
