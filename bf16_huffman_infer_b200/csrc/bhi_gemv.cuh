@@ -489,7 +489,10 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int group = warp / kGemvWarps, wig = warp % kGemvWarps;      // warp inside the group = its pass
     const int r = lane >> 3, t = lane & 3, gq = lane >> 2;
-    const uint32_t sigma4 = 4u * (8 * wig + (lane & 7));               // byte offset of the lane's stream inside a word row
+    // Dense: no product ties rows together, so a warp takes whole rows (two of the eight, or one of four) and lane l the
+    // streams l and l + 32: its stores are whole 128-byte lines.
+    const uint32_t sigma4 = NB > 0 ? 4u * (8 * wig + (lane & 7)) : 4u * lane;      // byte offset of the lane's stream inside a word row
+    auto row_of = [&](int q, int n, int row) { return NB > 0 ? 4 * q + row : n * wig + q; };       // row of a unit of n quads
     const bool exchange = NB == 1 && peers.world > 0;
     const int B = G.batch;
 
@@ -654,12 +657,13 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
 
     // A lane's share of the copies that bring a chunk of its warp's sign/mantissa rows: 16 bytes of block lane / 8 of the
-    // chunk, row (lane / 2) % 4 of each quad.
+    // chunk, row (lane / 2) % 4 of each quad (dense: of each of the warp's rows).
     const uint8_t *rem[2];
     auto rem_rows = [&](const Place &u) {
 #pragma unroll
         for (int q = 0; q < 2; q++)
-            rem[q] = L.rem + static_cast<int64_t>(record_of(u, 4 * q + ((lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 + wig * 32 + (lane & 1) * 16;
+            rem[q] = L.rem + static_cast<int64_t>(record_of(u, row_of(q, quads_of(u), (lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 +
+                     (NB > 0 ? wig * 32 + (lane & 1) * 16 : (lane & 7) * 16);
     };
     uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
     auto fetch = [&](int n, int blk, uint32_t to) {
@@ -766,7 +770,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             if (NB == 0) {
 #pragma unroll
                 for (int q = 0; q < n; q++) {
-                    const int m = 4 * (cur.quad + q) + r;
+                    const int m = 4 * cur.quad + row_of(q, n, r);
                     live[q] = m < L.M;
                     out[q] = reinterpret_cast<uint32_t *>(Y) + (((static_cast<int64_t>(m) * L.S + cur.k) * L.Nc) >> 1) + (sigma4 >> 2);
                 }
@@ -850,7 +854,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 if (!arrived && lane == 0) atomicExch(&g_staged_status, 1);
                 Dec dec[n];
 #pragma unroll
-                for (int q = 0; q < n; q++) dec[q].open(smem_base + ubase + (4 * q + r) * (rows * 256u + 32u) + sigma4, rows);
+                for (int q = 0; q < n; q++) dec[q].open(smem_base + ubase + row_of(q, n, r) * (rows * 256u + 32u) + sigma4, rows);
                 run(quads, dec);
             } else {
                 if (posted[4 * slot + 2] != 0u) {          // its copies were started all the same
@@ -860,7 +864,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 GemvDirect<Codec> dec[n];
 #pragma unroll
                 for (int q = 0; q < n; q++) {
-                    const uint32_t first = static_cast<uint32_t>(__ldg(L.offsets + record_of(cur, 4 * q + r)));
+                    const uint32_t first = static_cast<uint32_t>(__ldg(L.offsets + record_of(cur, row_of(q, n, r))));
                     dec[q].open(GlobalRecord{L.exp, exp_words, first + (sigma4 >> 2)}, &tab);
                 }
                 run(quads, dec);
