@@ -60,7 +60,7 @@ WORKLOADS = {
     "tiny": (2, 1024, 3072, 8, 2, 128, 8192),
 }
 # DRAM bytes read + written per launch / algorithmic bytes of the fused Huffman GEMV, from the ncu capture
-# summarised in profiles/quad_gemv_huffman_12288x4096_b1.md (dram__bytes_read.sum + dram__bytes_write.sum)
+# summarised in profiles/gemv_huffman_49152x4096_b1.md (dram__bytes_read.sum + dram__bytes_write.sum)
 TRAFFIC_OVER_ALGORITHMIC = 1.0046
 QWEN3_SHAPES = {"q_o": (4096, 4096), "k_v": (1024, 4096), "gate_up": (12288, 4096), "down": (4096, 12288)}
 
@@ -438,13 +438,12 @@ def ours(args, rank, world, dev, light=False):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": alg_bytes / launches_per_step * TRAFFIC_OVER_ALGORITHMIC,
                      "traffic_source": "algorithmic bytes x 1.0046, the ratio of dram__bytes_read.sum + dram__bytes_write.sum to "
-                                       "algorithmic bytes in profiles/quad_gemv_huffman_12288x4096_b1.md",
+                                       "algorithmic bytes in profiles/gemv_huffman_49152x4096_b1.md",
                      "algorithmic_bytes_per_launch": alg_bytes / launches_per_step,
                      "avg_launch_us": ms_step * 1e3 / launches_per_step,
                      "frac_of_nominal_8tbs": achieved / 8000.0,
-                     "kernel": ("quad_kernel<HuffCodec, B, 2> (four weight rows per warp group, one mma.sync tile per block for all rows of X)"
-                                if args.algo == "huffman" and args.tables.startswith("limit") and B > 0 else
-                                "quad_kernel / staged_kernel by table kind and batch")},
+                     "kernel": "gemv_kernel<GemvSingle | GemvPair | GemvAns by coder and table, ...> (eight weight rows per warp group, "
+                               "one mma.sync per block and four of them for eight rows of X)"},
         "clocks": clocks.summary(),
     }
     if ms_e2e is not None:
