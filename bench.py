@@ -60,8 +60,8 @@ WORKLOADS = {
     "tiny": (2, 1024, 3072, 8, 2, 128, 8192),
 }
 # DRAM bytes read + written per launch / algorithmic bytes of the fused Huffman GEMV, from the ncu capture
-# summarised in profiles/gemv_huffman_49152x4096_b1.md (dram__bytes_read.sum + dram__bytes_write.sum)
-TRAFFIC_OVER_ALGORITHMIC = 1.0046
+# summarised in profiles/gemv_huffman_49152x4096_b1.md (dram__bytes.sum.per_second x duration)
+TRAFFIC_OVER_ALGORITHMIC = 1.022
 QWEN3_SHAPES = {"q_o": (4096, 4096), "k_v": (1024, 4096), "gate_up": (12288, 4096), "down": (4096, 12288)}
 
 
@@ -437,7 +437,7 @@ def ours(args, rank, world, dev, light=False):
         "gpu_launches": launches_per_step * steps,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": alg_bytes / launches_per_step * TRAFFIC_OVER_ALGORITHMIC,
-                     "traffic_source": "algorithmic bytes x 1.0046, the ratio of dram__bytes_read.sum + dram__bytes_write.sum to "
+                     "traffic_source": "algorithmic bytes x 1.022, the ratio of dram__bytes.sum.per_second x duration to "
                                        "algorithmic bytes in profiles/gemv_huffman_49152x4096_b1.md",
                      "algorithmic_bytes_per_launch": alg_bytes / launches_per_step,
                      "avg_launch_us": ms_step * 1e3 / launches_per_step,
@@ -473,8 +473,9 @@ def side_run(args, rank, world, dev, **override):
 def per_shape_arm(dev, steps=5):
     """Every Qwen3-8B linear shape x both coders on its own: graph replay over more than L2 of distinct copies."""
     import math
-    from bf16_huffman_infer_b200 import ANSWeight, CompressedLinear, HuffmanWeight
+    from bf16_huffman_infer_b200 import ANSWeight, CompressedLinear, HuffmanWeight, set_ans_precision
     peak, _ = peaks()
+    set_ans_precision(8)                               # the default model, whatever the runs before this one asked for
     rows = []
     for name, (M, K) in QWEN3_SHAPES.items():
         g = torch.Generator(device=dev).manual_seed(0)
