@@ -958,7 +958,8 @@ struct GemvForm {
 };
 
 // Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record and takes a unit
-// whose longest is a word row and an eighth longer; one that is longer still is decoded from global memory.
+// whose longest is a word row and an eighth longer (a word row where it has room for one unit only); one that is longer
+// still is decoded from global memory.
 static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool exchange,
                       GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
@@ -981,7 +982,8 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     G.rem_off = G.acc_off + (G.split && acc_groups ? up(static_cast<uint64_t>(nq) * f.groups * 128) : 0u);
     G.ring_off = G.rem_off + f.groups * kGemvWarps * 2u * kRemChunk;
     auto unit = [&](uint64_t r) { return 4ull * f.quads * (r * 256u + 32u); };
-    const uint64_t wanted = unit(rows) * f.quarters / 4u, longest = f.quarters ? unit(rows + 1u + rows / 8u) : 0u;
+    const uint64_t spare = f.quarters > 4 ? 1u + rows / 8u : 1u;
+    const uint64_t wanted = unit(rows) * f.quarters / 4u, longest = f.quarters ? unit(rows + spare) : 0u;
     G.ring_bytes = up(wanted > longest ? wanted : longest);
     const uint64_t x_off = static_cast<uint64_t>(G.ring_off) + static_cast<uint64_t>(f.groups) * G.ring_bytes;
     if (x_off + kSlackBytes > cap) return false;
@@ -1036,6 +1038,8 @@ static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, co
 //   two CTAs per SM, X resident, two units in the ring   25.8
 //   same, 1.25 units (the next unit's copies wait for this one's space; the other groups work on)   26.2 / 26.7
 //   one CTA of twice the groups (one copy of table and X for all), X resident   27.2 / 27.6; 1.25 units 28.1 / 28.7 / 28.9
+//   same, room for one unit only, where X stays resident just so (3584 x 18944, two rows: rANS 70.5 against 79.9 with X
+//   through the ring, which also bars dividing the chunks; tables of the reference's builder 50.6 against 69.2)
 //   same, X through the ring   30.9 / 31.4 / 31.9
 //   units of four rows, for long records   35.7
 // The last form stages no record at all.
@@ -1043,8 +1047,8 @@ template <class Dec, int NB, bool kLast>
 static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                            const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, cudaStream_t st) {
     constexpr GemvX kFew = NB == 0 ? GemvX::none : GemvX::resident, kMany = NB == 0 ? GemvX::none : GemvX::ring;
-    const GemvForm forms[] = {{2, 2, 2, 8, kFew}, {2, 2, 2, 5, kFew}, {4, 1, 2, 8, kFew}, {4, 1, 2, 5, kFew}, {4, 1, 2, 8, kMany},
-                              {4, 1, 2, 5, kMany}, {4, 1, 1, 5, kFew}, {4, 1, 1, 5, kMany}, {2, 1, 1, 5, kMany},
+    const GemvForm forms[] = {{2, 2, 2, 8, kFew}, {2, 2, 2, 5, kFew}, {4, 1, 2, 8, kFew}, {4, 1, 2, 5, kFew}, {4, 1, 2, 4, kFew},
+                              {4, 1, 2, 8, kMany}, {4, 1, 2, 5, kMany}, {4, 1, 1, 5, kFew}, {4, 1, 1, 5, kMany}, {2, 1, 1, 5, kMany},
                               {2, 1, 1, 0, kMany}};
     const int nquads = (L.M + 3) / 4, only = gemv_groups();
     for (const GemvForm &f : forms) {

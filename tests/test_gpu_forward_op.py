@@ -82,3 +82,20 @@ def test_unaligned_activations():
         with torch.no_grad():
             y = layer(shifted)
         assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).numpy()) <= 1e-2
+
+
+@pytest.mark.parametrize("algo,tables", [("huffman", "reference"), ("ans", None)])
+@pytest.mark.parametrize("M", [1, 598, 1187])
+def test_one_unit_rings(algo, tables, M):
+    """Two rows over 18944 columns in four chunks: X stays resident beside record rings that take a single unit."""
+    from bf16_huffman_infer_b200 import ANSWeight, CompressedLinear, HuffmanWeight, set_huffman_tables
+    K, W = 18944, make_weight(M, 18944, 7)
+    previous = set_huffman_tables(tables or "limit6")
+    try:
+        weight = (ANSWeight if algo == "ans" else HuffmanWeight).compress(W.to(DEV), to_cpu=False)
+    finally:
+        set_huffman_tables(previous)
+    x = make_input(2, K, 8).to(DEV)
+    y = CompressedLinear(weight, None)(x)
+    want = x.float() @ W.to(DEV).float().T
+    assert ((y.float() - want).norm() / want.norm()).item() < 4e-3
