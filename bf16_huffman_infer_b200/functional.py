@@ -358,7 +358,8 @@ class HuffmanWeight(nn.Module):
         d = self.__dict__
         b = d["_buffers"]
         t1, t2, t3, t4, cl = b["LUT1"], b["LUT2"], b["LUT3"], b["LUT4"], b["code_lengths"]
-        # in-place loads (load_state_dict) bump the version; a tensor whose data was replaced has another address
+        # in-place loads (load_state_dict) bump the version; a tensor whose data was replaced has another address, because
+        # the memory of the tables that were folded is held as long as the blob is
         src = (t1.data_ptr(), t2.data_ptr(), t3.data_ptr(), t4.data_ptr(), cl.data_ptr(),
                t1._version, t2._version, t3._version, t4._version, cl._version)
         if d.get("_prepared_src") != src:
@@ -367,8 +368,26 @@ class HuffmanWeight(nn.Module):
             # codes of at most 6 bits: every 12-bit window holds two whole codes (the kernels pick their warp layout by it)
             ops.huffman_table_hint(blob, int(cl.max().item()) <= 6)
             d["_prepared"] = blob
+            d["_prepared_tables"] = tuple(t.detach() for t in (t1, t2, t3, t4, cl))
             d["_prepared_src"] = src
         return d["_prepared"]
+
+    @staticmethod
+    def _drop_prepared(state: Dict) -> Dict:
+        for name in ("_prepared_src", "_prepared", "_prepared_tables"):
+            state.pop(name, None)
+        return state
+
+    def _apply(self, *args, **kwargs):
+        super()._apply(*args, **kwargs)
+        blob = self.__dict__.get("_prepared")
+        if blob is not None and blob.device != self.rem.device:
+            self._drop_prepared(self.__dict__)
+        return self
+
+    def __getstate__(self):
+        """Copies and pickles fold their own tables."""
+        return self._drop_prepared(self.__dict__.copy())
 
     def _plain(self) -> bool:
         """The buffers are as the operators take them (``compress`` makes no others)."""
