@@ -59,7 +59,7 @@ def test_copies_and_pickles_fold_their_own(folds):
 @pytest.mark.gpu
 def test_move_load_move():
     from bf16_huffman_infer_b200 import HuffmanWeight, set_huffman_tables
-    W = make_weight(64, 256, 0)
+    W = make_weight(64, 384, 0)
     weights = []
     for method in ("limit6", "escape", "reference"):
         previous = set_huffman_tables(method)
