@@ -21,6 +21,7 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 from torch import Tensor, nn
+from torch.autograd import forward_ad
 from tqdm import tqdm
 
 from . import ops, transfer
@@ -619,9 +620,16 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
     return output.unflatten(0, shape[:-1])
 
 
+def _transformed() -> bool:
+    """A tangent, a batch dimension or a gradient of torch.func may ride on a tensor, or the call is being traced for
+    other inputs: what the fused operators do not carry on and F.linear over the dense matrix does."""
+    return (forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch._C._get_tracing_state() is not None)
+
+
 def _takes_more_rows(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> bool:
-    """Whether 9 to 32 rows can take the fused product, which has no backward and knows BF16 only."""
-    if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled():
+    """Whether 9 to 32 rows can take the fused product, which has no derivatives and knows BF16 only."""
+    if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled() or _transformed():
         return False
     if bias is not None and not (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()):
         return False

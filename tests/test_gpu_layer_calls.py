@@ -1,0 +1,55 @@
+"""Calls of a compressed layer that a layer over the dense matrix answers: derivatives other than by backward, batching,
+tracing, unusual biases and shapes."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwad
+import torch.nn.functional as F
+from torch import nn
+
+from _util import make_input, make_weight
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+M, K = 130, 512
+
+
+@pytest.fixture(scope="module", params=["huffman", "ans"])
+def coded(request):
+    """(dense matrix, compressed weight, bias)"""
+    from bf16_huffman_infer_b200 import ANSWeight, HuffmanWeight
+    W = make_weight(M, K, 0).to(DEV)
+    cls = HuffmanWeight if request.param == "huffman" else ANSWeight
+    return W, cls.compress(W, to_cpu=False), make_weight(1, M, 1)[0].to(DEV)
+
+
+def _layer(weight, bias):
+    from bf16_huffman_infer_b200 import CompressedLinear
+    return CompressedLinear(weight, None if bias is None else nn.Parameter(bias.clone(), requires_grad=False))
+
+
+def _close(y, want):
+    """BF16 roundings of FP32 sums in two orders: each output within one BF16 step (2^-8 of it) and the sums' own error."""
+    return bool(((y - want).double().norm() / want.double().norm()) < 2.0 ** -8)
+
+
+@pytest.mark.parametrize("rows", [9, 12, 32])
+def test_forward_mode_nine_to_thirty_two_rows(coded, rows):
+    W, weight, bias = coded
+    layer = _layer(weight, bias)
+    x, t = make_input(rows, K, 1).to(DEV), make_input(rows, K, 2).to(DEV)
+    with fwad.dual_level():
+        y = fwad.unpack_dual(layer(fwad.make_dual(x, t)))
+        assert y.tangent is not None
+        assert _close(y.primal, F.linear(x, W, bias)) and _close(y.tangent, F.linear(t, W))
+    y, tangent = torch.func.jvp(layer, (x,), (t,))
+    assert _close(y, F.linear(x, W, bias)) and _close(tangent, F.linear(t, W))
+    assert _close(torch.func.vmap(layer)(torch.stack([x, t])), F.linear(torch.stack([x, t]), W, bias))
+
+
+def test_trace_of_nine_rows_runs_with_more(coded):
+    W, weight, bias = coded
+    x = make_input(12, K, 1).to(DEV)
+    more = make_input(40, K, 2).to(DEV)
+    with torch.no_grad():
+        traced = torch.jit.trace(_layer(weight, bias), (x,), check_trace=False)
+        assert _close(traced(x), F.linear(x, W, bias)) and _close(traced(more), F.linear(more, W, bias))
