@@ -592,7 +592,7 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
     assert input.dim() >= 2, input
     rows = input.numel() // max(input.size(-1), 1)
     if rows <= FUSED_MAX_ROWS and weight._plain():
-        # one operator call; a bias that needs its gradient, or is not a BF16 vector on the layer's device, is added after it
+        # one operator call; a bias that needs a derivative, or is not a whole BF16 vector on the layer's device, is added after it
         assert input.is_cuda and input.dtype == torch.bfloat16
         if input.requires_grad:
             input = input.detach()
@@ -600,12 +600,11 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
             input = input.contiguous()
         if bias is None:
             return weight._forward(input, None)
-        if (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
-                and not (bias.requires_grad and torch.is_grad_enabled())):
+        if _takes_bias(weight, bias, input) and not (bias.requires_grad and torch.is_grad_enabled()) and not _transformed():
             return weight._forward(input, bias)
-        output = weight._forward(input, None)
-        output += bias
-        return output
+        output = weight._forward(input.flatten(0, -2), None)
+        output += bias[None, :]
+        return output.unflatten(0, input.shape[:-1])
     if FUSED_MAX_ROWS < rows <= FUSED_MORE_ROWS and rows > TENSOR_MAX_ROWS and _takes_more_rows(input, weight, bias):
         output = weight._forward(input.contiguous(), bias)
         if output.numel():
@@ -620,6 +619,12 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
     return output.unflatten(0, shape[:-1])
 
 
+def _takes_bias(weight: HuffmanWeight, bias: Tensor, input: Tensor) -> bool:
+    """Whether the operators take the bias as it is; others (one value for all outputs, another type) are torch's to add."""
+    return (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
+            and bias.shape == weight.__dict__["_buffers"]["rem"].shape[1:2])
+
+
 def _transformed() -> bool:
     """A tangent, a batch dimension or a gradient of torch.func may ride on a tensor, or the call is being traced for
     other inputs: what the fused operators do not carry on and F.linear over the dense matrix does."""
@@ -631,7 +636,7 @@ def _takes_more_rows(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor
     """Whether 9 to 32 rows can take the fused product, which has no derivatives and knows BF16 only."""
     if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled() or _transformed():
         return False
-    if bias is not None and not (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()):
+    if bias is not None and not _takes_bias(weight, bias, input):
         return False
     return not (torch.is_grad_enabled() and (input.requires_grad or (bias is not None and bias.requires_grad)))
 

@@ -53,3 +53,33 @@ def test_trace_of_nine_rows_runs_with_more(coded):
     with torch.no_grad():
         traced = torch.jit.trace(_layer(weight, bias), (x,), check_trace=False)
         assert _close(traced(x), F.linear(x, W, bias)) and _close(traced(more), F.linear(more, W, bias))
+
+
+@pytest.mark.parametrize("rows", [4, 12, 40])
+def test_biases_of_other_shapes(coded, rows):
+    """What an in-place addition (up to 8 rows) or F.linear (more) takes is taken, and what they refuse is refused."""
+    W, weight, bias = coded
+    x = make_input(rows, K, 1).to(DEV)
+    plain = F.linear(x, W)
+    takes = [bias, bias.float(), bias[:1], bias[:1].expand(M)] if rows <= 8 else [bias, bias[:1], bias[0], bias.expand(rows, M)]
+    refuses = [bias[0], bias[None], bias[1:], bias[None].float(), bias.expand(rows, M), bias.cpu()] if rows <= 8 else \
+        [bias[1:], bias.float(), bias.cpu()]
+    with torch.no_grad():
+        for b in takes:
+            layer = _layer(weight, None)
+            layer.bias = b
+            assert _close(layer(x), plain + b), (b.shape, b.dtype)
+        for b in refuses:
+            layer = _layer(weight, None)
+            layer.bias = b
+            with pytest.raises((RuntimeError, IndexError)):
+                layer(x)
+
+
+def test_tangent_of_the_bias(coded):
+    W, weight, bias = coded
+    x, t = make_input(4, K, 1).to(DEV), make_weight(1, M, 2)[0].to(DEV)
+    layer = _layer(weight, None)
+    with fwad.dual_level():
+        layer.bias = fwad.make_dual(bias, t)
+        assert torch.equal(fwad.unpack_dual(layer(x)).tangent, t.expand(4, M))
