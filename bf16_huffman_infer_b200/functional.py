@@ -581,11 +581,16 @@ class CompressedLinear(nn.Module):
         return self.weight.shape[1]
 
     def forward(self, input: Tensor) -> Tensor:
-        d = self.__dict__                       # nn.Module's own attribute lookup costs more than the checks below
+        # nn.Module's own attribute lookup and F.linear's dispatch cost more than the checks below; whoever watches or
+        # overrides F.linear (a function mode, a tensor subclass, a weight class of its own) still sees the call
+        d = self.__dict__
+        weight = d["_modules"]["weight"]
         bias = d["_parameters"].get("bias")
         if bias is None:
             bias = self.bias
-        return _linear_compressed(input, d["_modules"]["weight"], bias)
+        if type(input) is Tensor and type(weight) in (HuffmanWeight, ANSWeight) and not torch._C._is_torch_function_mode_enabled():
+            return _linear_compressed(input, weight, bias)
+        return F.linear(input, weight, bias)
 
 
 def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> Tensor:

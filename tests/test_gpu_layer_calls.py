@@ -83,3 +83,31 @@ def test_tangent_of_the_bias(coded):
     with fwad.dual_level():
         layer.bias = fwad.make_dual(bias, t)
         assert torch.equal(fwad.unpack_dual(layer(x)).tangent, t.expand(4, M))
+
+
+@pytest.mark.parametrize("rows", [4, 12, 40])
+def test_overrides_of_linear_see_the_call(coded, rows):
+    from torch.overrides import TorchFunctionMode
+    W, weight, bias = coded
+    layer, x = _layer(weight, bias), make_input(rows, K, 1).to(DEV)
+    seen = []
+
+    class Watch(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    class Own(type(weight)):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return super().__torch_function__(func, types, args, kwargs)
+
+    with torch.no_grad():
+        want = layer(x)
+        with Watch():
+            assert torch.equal(layer(x), want)
+        assert seen.count(F.linear) >= 1
+        seen.clear()
+        assert torch.equal(_layer(Own(**weight.kwargs()), bias)(x), want)
+        assert F.linear in seen
