@@ -186,7 +186,7 @@ Tensor empty_bf16(const Tensor &like, int64_t dims, const int64_t *sizes, const 
 
 // X's leading dimensions and `columns` columns
 Tensor output_like(const Tensor &X, int64_t columns) {
-    constexpr int64_t kDims = 16;
+    constexpr int64_t kDims = 64;         // torch's own limit for most operators
     const int64_t dims = X.dim();
     STD_TORCH_CHECK(dims >= 1 && dims <= kDims, "X has too many dimensions");
     int64_t sizes[kDims], strides[kDims], step = 1;

@@ -111,3 +111,12 @@ def test_overrides_of_linear_see_the_call(coded, rows):
         seen.clear()
         assert torch.equal(_layer(Own(**weight.kwargs()), bias)(x), want)
         assert F.linear in seen
+
+
+@pytest.mark.parametrize("rows", [4, 12])
+def test_many_leading_dimensions(coded, rows):
+    W, weight, bias = coded
+    x = make_input(rows, K, 1).to(DEV).view(*[1] * 22, rows, K)
+    with torch.no_grad():
+        y = _layer(weight, bias)(x)
+    assert y.shape == x.shape[:-1] + (M,) and _close(y, F.linear(x, W, bias))
