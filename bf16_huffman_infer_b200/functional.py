@@ -631,15 +631,16 @@ def _takes_bias(weight: HuffmanWeight, bias: Tensor, input: Tensor) -> bool:
 
 
 def _transformed() -> bool:
-    """A tangent, a batch dimension or a gradient of torch.func may ride on a tensor, or the call is being traced for
-    other inputs: what the fused operators do not carry on and F.linear over the dense matrix does."""
-    return (forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch._C._get_tracing_state() is not None)
+    """A tangent, a batch dimension or a gradient of torch.func may ride on a tensor, which the operators do not carry on."""
+    return forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
 
 
 def _takes_more_rows(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor]) -> bool:
-    """Whether 9 to 32 rows can take the fused product, which has no derivatives and knows BF16 only."""
-    if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled() or _transformed():
+    """Whether 9 to 32 rows can take the fused product, which has no derivatives, knows BF16 only and would bind a trace to
+    its row limit."""
+    if not (input.is_cuda and input.dtype == torch.bfloat16 and weight._plain()) or torch.is_autocast_enabled():
+        return False
+    if _transformed() or torch._C._get_tracing_state() is not None:
         return False
     if bias is not None and not _takes_bias(weight, bias, input):
         return False
