@@ -166,7 +166,7 @@ class _Ingested:
         else:
             self.w = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
             if to_cpu:
-                self.host_rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8)
+                self.host_rem = torch.empty(split_k, M, K // split_k, dtype=torch.uint8, device="cpu")
 
             def arrived(lo: int, hi: int) -> None:
                 ops.split_histogram(self.w[lo:hi], split_k, lo, self.rem, counts)
@@ -551,8 +551,8 @@ class ANSWeight(HuffmanWeight):
 
     @classmethod
     def _encoder_tables(cls, codec, dev) -> Dict[str, Tensor]:
-        return _tables_to({"freq": torch.tensor(codec.freq, dtype=torch.int32),
-                           "cum": torch.tensor(codec.cum, dtype=torch.int32)}, dev)
+        return _tables_to({"freq": torch.tensor(codec.freq, dtype=torch.int32, device="cpu"),
+                           "cum": torch.tensor(codec.cum, dtype=torch.int32, device="cpu")}, dev)
 
     @classmethod
     def _size_pass(cls, layer: _Ingested, t: Dict[str, Tensor], rows: Tensor) -> None:

@@ -23,7 +23,7 @@ _SMALL = 1 << 20             # below this one plain copy is as fast
 
 def _slabs(nbytes: int):
     count = min(SLABS, -(-nbytes // SLAB_BYTES))
-    return [torch.empty(SLAB_BYTES, dtype=torch.uint8, pin_memory=True) for _ in range(count)]
+    return [torch.empty(SLAB_BYTES, dtype=torch.uint8, device="cpu", pin_memory=True) for _ in range(count)]
 
 
 def upload_rows(src: Tensor, dst: Tensor, arrived: Optional[Callable[[int, int], None]] = None) -> None:
@@ -61,7 +61,7 @@ def download(src: Tensor, out: Optional[Tensor] = None) -> Tensor:
         return src.cpu() if out is None else out.copy_(src)
     stream = torch.cuda.current_stream(src.device)
     if out is None:
-        out = torch.empty(src.shape, dtype=src.dtype)
+        out = torch.empty(src.shape, dtype=src.dtype, device="cpu")
     flat_src, flat_out = src.contiguous().view(-1).view(torch.uint8), out.view(-1).view(torch.uint8)
     slabs = _slabs(nbytes)
     here = [torch.cuda.Event() for _ in slabs]
