@@ -99,9 +99,9 @@ def _work_device(a: Tensor) -> torch.device:
 
 
 def _exp_histogram(a: Tensor) -> Tensor:
-    """256 exponent counts of a BF16 tensor (int64, on the CPU)."""
+    """256 exponent counts of a BF16 tensor, or of the bits of one with 16-bit elements (int64, on the CPU)."""
     a = a.detach().contiguous()
-    if a.is_cuda and a.numel() % 128 == 0 and 0 < a.numel() < 2 ** 38 and a.data_ptr() % 4 == 0:
+    if a.is_cuda and a.dtype == torch.bfloat16 and a.numel() % 128 == 0 and 0 < a.numel() < 2 ** 38 and a.data_ptr() % 4 == 0:
         counts = torch.zeros(256, dtype=torch.int64, device=a.device)
         ops.split_histogram(a.view(-1, 128), 1, 0, torch.empty(0, dtype=torch.uint8, device=a.device), counts)
         return counts.cpu()

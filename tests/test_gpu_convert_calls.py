@@ -26,3 +26,12 @@ def test_default_device(default, home, to_cpu):
             weight = cls.compress(W.to(home), to_cpu=to_cpu)
         assert {b.device.type for b in weight.buffers()} == {"cpu" if to_cpu else "cuda"}
         assert torch.equal(weight.to(DEV).get_weight().cpu(), W)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int16])
+def test_codec_of_bits(dtype):
+    """The code of a tensor whose bits are BF16 values, whatever type they are declared as."""
+    W = make_weight(64, 256, 1).to(DEV)
+    for cls in _classes():
+        a, b = cls.get_lut_kwargs(cls.get_codec(W)), cls.get_lut_kwargs(cls.get_codec(W.view(dtype)))
+        assert all(torch.equal(a[k], b[k]) for k in a)
