@@ -705,6 +705,8 @@ def convert(linear: nn.Linear, name, disable_precision_check: bool = True, algo:
     if fallback:
         print("Fallback to regular nn.Linear")
         return linear
+    if home.type == "cuda" and module.weight.algo == "huffman":
+        module.weight.prepared()              # so that a layer converted on its device can be captured without a first call
     return module
 
 

@@ -35,3 +35,23 @@ def test_codec_of_bits(dtype):
     for cls in _classes():
         a, b = cls.get_lut_kwargs(cls.get_codec(W)), cls.get_lut_kwargs(cls.get_codec(W.view(dtype)))
         assert all(torch.equal(a[k], b[k]) for k in a)
+
+
+@pytest.mark.parametrize("algo", ["huffman", "ans", "smallest"])
+def test_capture_right_after_conversion(algo):
+    """A layer converted on the device is captured without a call before: its folded tables are there."""
+    from bf16_huffman_infer_b200 import CompressedLinear, convert
+    linear = nn.Linear(512, 256, dtype=torch.bfloat16, device=DEV).requires_grad_(False)
+    linear.weight.copy_(make_weight(256, 512, 2))
+    x = make_weight(1, 512, 3).to(DEV)
+    want = F.linear(x, linear.weight, linear.bias)
+    layer = convert(linear, "layer", algo=algo)
+    assert isinstance(layer, CompressedLinear)
+    if algo != "ans":
+        assert "_prepared" in layer.weight.__dict__ or layer.weight.algo == "ans"
+    graph = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(graph):
+        y = layer(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert ((y - want).double().norm() / want.double().norm()).item() < 2.0 ** -8
