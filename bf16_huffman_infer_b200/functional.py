@@ -496,7 +496,7 @@ class ANSWeight(HuffmanWeight):
         self.rem = nn.Buffer(rem)
         self.exp = nn.Buffer(exp)
         self.offsets = nn.Buffer(offsets)
-        self.LUT = nn.Buffer(torch.as_tensor(LUT))
+        self.LUT = nn.Buffer(LUT if isinstance(LUT, Tensor) else torch.as_tensor(LUT))      # as_tensor moves to a default device
 
     @classmethod
     def __torch_function__(cls, func, types, args=(), kwargs=None):

@@ -41,9 +41,9 @@ def test_codec_of_bits(dtype):
 def test_capture_right_after_conversion(algo):
     """A layer converted on the device is captured without a call before: its folded tables are there."""
     from bf16_huffman_infer_b200 import CompressedLinear, convert
-    linear = nn.Linear(512, 256, dtype=torch.bfloat16, device=DEV).requires_grad_(False)
-    linear.weight.copy_(make_weight(256, 512, 2))
-    x = make_weight(1, 512, 3).to(DEV)
+    linear = nn.Linear(1536, 512, dtype=torch.bfloat16, device=DEV).requires_grad_(False)
+    linear.weight.copy_(make_weight(512, 1536, 2))
+    x = make_weight(1, 1536, 3).to(DEV)
     want = F.linear(x, linear.weight, linear.bias)
     layer = convert(linear, "layer", algo=algo)
     assert isinstance(layer, CompressedLinear)
