@@ -42,11 +42,13 @@ constexpr uint32_t kTableAt = 1024;           // where dynamic shared memory sta
 struct GemvGeom {
     uint32_t exact_off, part_off, ys_off, rem_off, ring_off, x_off;
     uint32_t ring_bytes;       // per group
+    uint32_t ring_early;       // ... of which two units fill so much that the second's copies start before the first is read
+    uint32_t pair_rows;        // longest record, in word rows, of a unit of two quads that the ring takes
     uint32_t x_pitch;          // bytes between rows of X
     uint32_t x_slot;           // bytes of a segment of the X ring
     int x_slots;               // segments of the ring; 0 = all of X is resident
     int batch;
-    int max_quads;             // of a unit: 2, or 1 when records are long
+    int max_quads;             // of a unit: 2, or 1 when all records are long
     int split;                 // the groups of a CTA share its quads and divide the chunks among them
     uint32_t acc_off;          // ... whose sums meet here
 };
@@ -471,6 +473,31 @@ __device__ __forceinline__ void copy_x_row(uint32_t dst, const uint16_t *src, ui
     }
 }
 
+// Which of up to 32 pairs of quads, from quad `first` on, have in chunks [k_lo, k_hi) a record of more than `most` words:
+// bit i for pair i (window pairs).
+__device__ __forceinline__ uint32_t pairs_apart(const int32_t *offsets, int S, int M, uint32_t exp_words, int first, int quad_hi, int k_lo,
+                                             int k_hi, int window, uint32_t most) {
+    const int lane = threadIdx.x & 31, q = first + 2 * (lane & (window - 1));
+    bool longer = false;
+    if (q + 1 < quad_hi) {
+        for (int k = k_lo + lane / window; k < k_hi; k += 32 / window) {
+            const int rec = k * M + 4 * q, last = k * M + M;
+            uint32_t at[9];
+#pragma unroll
+            for (int i = 0; i < 9; i++) {
+                const int m = min(rec + i, last);
+                at[i] = m < S * M ? static_cast<uint32_t>(__ldg(offsets + m)) : exp_words;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) longer |= at[i + 1] > at[i] && at[i + 1] - at[i] > most;
+        }
+    }
+    uint32_t apart = __ballot_sync(0xFFFFFFFFu, longer);
+    if (window <= 16) apart |= apart >> 16;
+    if (window == 8) apart |= apart >> 8;
+    return apart;
+}
+
 // NB = groups of eight X rows (0: no product, the dense matrix is written instead).  NG = groups of four warps per CTA.
 // Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
 // X or tables two CTAs could not both hold.  kRing: X passes through a ring that one more warp fills and all groups read in
@@ -503,7 +530,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     const uint32_t bar0 = ctrl_at + 16u * group;                       // record copies: two slots per group
     const uint32_t table_bar = ctrl_at + 80u, x_bar = ctrl_at + 88u;
     const uint32_t x_full = ctrl_at + 96u, x_empty = x_full + 8u * kXSlotsMax;      // X ring: filled, read by all warps
-    volatile uint32_t *posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256) + 8 * group;     // [slot]{word rows, base, staged}
+    volatile uint32_t *posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256) + 8 * group;     // [slot]{word rows, base, staged}, [3] sets
     float *part = reinterpret_cast<float *>(smem + G.part_off) + group * (kGemvWarps * 64 * kAcc);
     uint16_t *ys = reinterpret_cast<uint16_t *>(smem + G.ys_off);
     const uint32_t xs = smem_base + G.x_off;
@@ -547,20 +574,21 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     }
     __syncthreads();
 
-    // Segments of X that pass through the ring: every unit reads those of its chunk, in order.
-    int x_total = 0;
-    if (kRing) {
-        for (int g = 0; g < NG; g++) {
-            const int quads = deal(blockIdx.x * NG + g + 1) - deal(blockIdx.x * NG + g);
-            x_total = max(x_total, (quads + G.max_quads - 1) / G.max_quads * L.S * chunks);
-        }
-    }
+    // Segments of X that pass through the ring: every unit reads those of its chunk, in order.  The groups post how many sets
+    // of quads they have.
+    volatile uint32_t *all_posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256);
+    auto x_segments = [&]() {
+        uint32_t sets = 0u;
+        for (int g = 0; g < NG; g++) sets = max(sets, all_posted[8 * g + 3]);
+        return static_cast<int>(sets) * L.S * chunks;
+    };
     // ---- the warp that fills the X ring.  (With the readers filling it between their chunks, the last reader of a segment
     // its next one, the refill lay on the slowest warp and cost half as much again as the decoding.)
     if (kRing && warp == NG * kGemvWarps) {
         __syncthreads();                                               // the readers' barrier before their loop
         pdl_wait();
         const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
+        const int x_total = x_segments();
         int slot = 0, k = 0, ch = 0;
         uint32_t phase = 1u;                                           // nobody has to have read the first lap's places
         for (int i = 0; i < x_total; i++) {
@@ -593,25 +621,40 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     }
 
     // ---- units ---------------------------------------------------------------------------------------------------------
-    // The quads of the group max_quads by max_quads; for each set, the chunks in order.  The group's first warp knows where
-    // the records of the next unit lie (its lanes 0..7 hold one row each), places them in the ring, starts their copies and
-    // posts {word rows, base, staged} for the others; the offsets it needs are requested one unit ahead of that.
+    // A set is a pair of quads, or one quad: the last of an odd number, and both of a pair that has, in any chunk, a record
+    // longer than the ring takes beside seven of that length.  For each set, the chunks in order.  The group's first warp
+    // knows where the records of the next unit lie (its lanes 0..7 hold one row each), places them in the ring, starts their
+    // copies and posts {word rows, base, staged} for the others; the offsets it needs are requested one unit ahead of that.
     struct Place {
-        int quad, k;
+        int quad, k, n;
     };
-    auto quads_of = [&](const Place &u) { return min(G.max_quads, quad_hi - u.quad); };
+    const uint32_t exp_words = static_cast<uint32_t>(L.exp_words);
+    const int window = L.S == 1 ? 32 : L.S == 2 ? 16 : 8;              // pairs looked at together, one chunk per lane
+    int seen = quad_lo;                                                // first quad of the window
+    uint32_t alone = 0u;                                               // bit i: the quads of its pair i are taken one by one
+    auto look = [&](int first) {
+        seen = first;
+        alone = G.max_quads == 2 ? pairs_apart(L.offsets, L.S, L.M, exp_words, first, quad_hi, k_lo, k_hi, window, 64u * G.pair_rows) : ~0u;
+    };
+    auto quads_seen = [&](int quad) {
+        const int i = quad - seen;
+        return (i & 1) || (alone >> (i >> 1) & 1u) ? 1 : min(2, quad_hi - quad);
+    };
     auto after = [&](const Place &u) {
-        Place v{u.quad, u.k + 1};
+        Place v{u.quad, u.k + 1, u.n};
         if (v.k == k_hi) {
             v.k = k_lo;
-            v.quad += G.max_quads;
+            v.quad += u.n;
+            if (v.quad < quad_hi) {
+                if (v.quad - seen >= 2 * window) look(v.quad);
+                v.n = quads_seen(v.quad);
+            }
         }
         return v;
     };
-    const uint32_t exp_words = static_cast<uint32_t>(L.exp_words);
     const bool leader = wig == 0;
     auto record_of = [&](const Place &u, int row) {                    // row 0..7 of the unit
-        return u.k * L.M + min(4 * u.quad + (row < 4 * quads_of(u) ? row : 0), L.M - 1);
+        return u.k * L.M + min(4 * u.quad + (row < 4 * u.n ? row : 0), L.M - 1);
     };
     uint32_t off = 0u, end = 0u;                                       // leader, lanes 0..7: first and last exponent word
     auto request = [&](const Place &u) {
@@ -630,7 +673,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         uint32_t rows = fits ? words >> 6 : 0u;
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
-        foot = (4u * quads_of(u) * (rows * 256u + 32u) + 255u) & ~255u;
+        foot = (4u * u.n * (rows * 256u + 32u) + 255u) & ~255u;
         staged = __all_sync(0xFFFFFFFFu, fits) && foot <= G.ring_bytes;
         base = slot == 0 ? ring : ring + G.ring_bytes - foot;
         if (lane == 0) {
@@ -641,7 +684,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     auto start_copies = [&](const Place &u, int slot) {
         const uint32_t bar = bar0 + 8u * slot;
-        const int n = quads_of(u);
+        const int n = u.n;
         uint32_t total = lane < 4 * n ? words * 4u : 0u, rows = words >> 6;
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
@@ -662,7 +705,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     auto rem_rows = [&](const Place &u) {
 #pragma unroll
         for (int q = 0; q < 2; q++)
-            rem[q] = L.rem + static_cast<int64_t>(record_of(u, row_of(q, quads_of(u), (lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 +
+            rem[q] = L.rem + static_cast<int64_t>(record_of(u, row_of(q, u.n, (lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 +
                      (NB > 0 ? wig * 32 + (lane & 1) * 16 : (lane & 7) * 16);
     };
     uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
@@ -672,17 +715,55 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (n > 1) cp_async_16(dst + 512u, rem[1] + (bytes ? blk * 128 : -(lane >> 3) * 128), bytes);
     };
 
-    Place cur{quad_lo, k_lo}, nxt = after(cur);
+    // The first pairs are taken for whole until the look at their records is back: what they need is on its way by then.
+    Place cur{quad_lo, k_lo, min(G.max_quads, quad_hi - quad_lo)};
     request(cur);
     if (cur.quad < quad_hi) {
         rem_rows(cur);
-        fetch(quads_of(cur), 0, 0u);
+        fetch(cur.n, 0, 0u);
         if (leader) {
             place(cur, 0);
             if (staged) start_copies(cur, 0);
         }
     }
+    Place nxt{cur.quad, k_lo + 1, cur.n};
+    if (nxt.k == k_hi) nxt = Place{cur.quad + cur.n, k_lo, min(G.max_quads, quad_hi - cur.quad - cur.n)};
     request(nxt);
+    if (cur.quad < quad_hi) {
+        look(quad_lo);
+        const int n = quads_seen(quad_lo);
+        if (n != cur.n) {                                              // records that came for two quads serve one
+            cur.n = n;
+            if (NB == 0) {                                             // the warps' rows are others
+                cp_async_wait();
+                rem_rows(cur);
+                fetch(n, 0, 0u);
+            }
+            if (leader && !staged) {
+                request(cur);
+                place(cur, 0);
+                if (staged) start_copies(cur, 0);
+            }
+        }
+        Place real{quad_lo, k_lo + 1, n};
+        if (real.k == k_hi) {
+            real = Place{quad_lo + n, k_lo, 1};
+            if (real.quad < quad_hi) real.n = quads_seen(real.quad);
+        }
+        if (real.quad != nxt.quad || real.n != nxt.n) {
+            nxt = real;
+            request(nxt);
+        }
+    }
+    if (kRing && leader) {                                             // all sets of the group, for the warp that fills the X ring
+        int sets = 0;
+        for (Place u{quad_lo, k_lo, 1}; u.quad < quad_hi; sets++) {
+            if (u.quad - seen >= 2 * window) look(u.quad);
+            u.quad += quads_seen(u.quad);
+        }
+        if (lane == 0) posted[3] = sets;
+        if (seen != quad_lo) look(quad_lo);
+    }
     uint32_t prev_foot = staged ? foot : 0u;                           // leader: ring bytes of the unit being decoded
 
     bool usable = smem_base == kTableAt;      // the table's place is a constant in the loads; else records are decoded directly
@@ -729,6 +810,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
 #pragma unroll
     for (int g = 0; g < kAcc; g++)
         x_row[g] = xs + min(8 * g + (lane & 7), max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 3) & 1) + 128u * (lane >> 4);
+    const int x_total = kRing ? x_segments() : 0;
     int x_slot = 0, x_seg = 0;
     uint32_t x_phase = 0u;
     auto x_wait = [&]() {
@@ -754,7 +836,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         bool late = false;                    // leader: the next unit's copies have to wait for this one's space
         if (leader && nxt.quad < quad_hi) {
             place(nxt, slot ^ 1);
-            late = staged && prev_foot + foot > G.ring_bytes;
+            late = staged && prev_foot + foot > G.ring_early;
             if (staged && !late) start_copies(nxt, slot ^ 1);
             prev_foot = staged ? foot : 0u;
         }
@@ -822,7 +904,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                     fetch(n, blk + kRG, half ^ kRemChunk);
                 } else if (nxt.quad < quad_hi) {
                     rem_rows(nxt);
-                    fetch(quads_of(nxt), 0, half ^ kRemChunk);
+                    fetch(nxt.n, 0, half ^ kRemChunk);
                 }
                 x_wait();
                 const uint32_t rw = rem_at + half + 4u * lane, xa = kRing ? x_slot * G.x_slot : xo;
@@ -870,7 +952,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 run(quads, dec);
             }
         };
-        const int n = quads_of(cur);
+        const int n = cur.n;
         if (n == 2) dispatch(std::integral_constant<int, 2>{});
         else dispatch(std::integral_constant<int, 1>{});
 
@@ -957,9 +1039,12 @@ struct GemvForm {
     GemvX x;
 };
 
-// Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record and takes a unit
-// whose longest is a word row and an eighth longer (a word row where it has room for one unit only); one that is longer
-// still is decoded from global memory.
+// Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record, so that it takes a
+// unit whose longest is a word row and an eighth longer (a word row where it has room for one unit only), and grows into what
+// the form leaves.  Rows of a layer whose scales differ have records of different lengths: a pair of quads that does not fit
+// together comes quad by quad, and a quad that does not fit alone is decoded from global memory, several times as slow.
+// (4096 x 12288, rANS, one row of X, row scales log-normal with sigma 0.35: 177 us without the growth and the quads, 42 with
+// them, as with equal rows; 12288 x 4096, limit6, four rows: 76 and 30.  Equal rows pay 0 to 0.7 us for the look.)
 static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool exchange,
                       GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
@@ -1004,7 +1089,13 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     }
     if (x_bytes < kSlackBytes) x_bytes = kSlackBytes;
     if (x_off + x_bytes > cap) return false;
-    smem_bytes = static_cast<uint32_t>(x_off + x_bytes);
+    // What is left goes to the rings, for units of longer records; copies start as early as in the ring that was asked for
+    // (two units of all the space in flight at once cost 2 to 4 % where the form means them to take turns).
+    G.ring_early = G.ring_bytes;
+    if (f.quarters) G.ring_bytes += ((cap - static_cast<uint32_t>(x_off + x_bytes)) / f.groups) & ~255u;
+    G.x_off += f.groups * (G.ring_bytes - G.ring_early);
+    G.pair_rows = G.ring_bytes < 256u ? 0u : (G.ring_bytes / 8u - 32u) / 256u;
+    smem_bytes = static_cast<uint32_t>(G.x_off + x_bytes);
     G.batch = B;
     G.max_quads = f.quads;
     return true;
