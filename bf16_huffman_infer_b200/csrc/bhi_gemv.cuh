@@ -132,7 +132,7 @@ struct GemvSingle {
     uint32_t p0, p1, plim, off;
     static __device__ __forceinline__ const uint8_t *source(const uint8_t *prepared) { return prepared + kPreparedSingle; }
     static __device__ __forceinline__ void fill(uint8_t *, const HuffTables &, const HuffArgs &, const GemvConsts &, int, int) {}
-    static __device__ __forceinline__ bool usable(const HuffTables &t) { return *reinterpret_cast<const uint32_t *>(&t + 1) == 0u; }
+    static __device__ __forceinline__ bool usable(const HuffTables &t) { return prepared_longest(reinterpret_cast<const uint8_t *>(&t)) <= 6u; }
     __device__ __forceinline__ void open(uint32_t base, uint32_t rows) {
         off = base & 255u;
         p0 = p1 = (base >> 8) * 32u - 7u;

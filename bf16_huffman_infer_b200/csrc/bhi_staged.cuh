@@ -51,7 +51,7 @@ constexpr int kPreparedWide = kPreparedSingle + kSingleBytes;
 constexpr int kPreparedWidest = kPreparedWide + (4 << kWideBits);
 constexpr int kPreparedBytes = kPreparedWidest + (4 << kWidestBits);
 
-static_assert(sizeof(HuffTables) <= kExactBytes && sizeof(AnsTables) <= kExactBytes, "exact tables do not fit");
+static_assert(sizeof(HuffTables) + 8 <= kExactBytes && sizeof(AnsTables) <= kExactBytes, "exact tables do not fit");
 static_assert((4 << kAnsBitsMax) * kCopies <= kLutBytes, "the largest rANS table does not fit the fast-table region");
 
 __device__ int g_staged_status = 0;            // 0 = fine; otherwise the last failure code
@@ -311,13 +311,18 @@ __device__ __forceinline__ uint32_t prepared_flagged(const uint8_t *exact_region
     return *reinterpret_cast<const uint32_t *>(exact_region + sizeof(HuffTables));
 }
 
-// blob = folded pair table (one copy), exact tables with one word behind them (how many folded entries do not resolve two
-// symbols; 0 = no code is longer than 6 bits), single-symbol tables, wide pair tables.  The first block makes the first two,
-// the others share the rest.
+// length of the longest code
+__device__ __forceinline__ uint32_t prepared_longest(const uint8_t *exact_region) {
+    return *reinterpret_cast<const uint32_t *>(exact_region + sizeof(HuffTables) + 4);
+}
+
+// blob = folded pair table (one copy), exact tables with two words behind them (how many folded entries do not resolve two
+// symbols, and the length of the longest code; a code of a single symbol is one bit long and leaves half the entries
+// unresolved), single-symbol tables, wide pair tables.  The first block makes the first two, the others share the rest.
 __global__ void __launch_bounds__(1024) huffman_prepare_kernel(HuffArgs targs, uint8_t *blob) {
     __shared__ HuffTables tab;
-    __shared__ uint32_t flagged;
-    if (threadIdx.x == 0) flagged = 0u;
+    __shared__ uint32_t flagged, longest;
+    if (threadIdx.x == 0) flagged = longest = 0u;
     load_tables(tab, targs, threadIdx.x, blockDim.x);
     __syncthreads();
     if (blockIdx.x > 0) {
@@ -339,12 +344,13 @@ __global__ void __launch_bounds__(1024) huffman_prepare_kernel(HuffArgs targs, u
         mine += (e & (kEntSingle | kEntExact)) ? 1u : 0u;
     }
     if (mine) atomicAdd(&flagged, mine);
+    if (threadIdx.x < 256) atomicMax(&longest, static_cast<uint32_t>(tab.len[threadIdx.x]));
     __syncthreads();
     uint32_t *dst = reinterpret_cast<uint32_t *>(blob + kPairEntries * 4);
     const uint32_t *src = reinterpret_cast<const uint32_t *>(&tab);
     constexpr int kTabWords = static_cast<int>(sizeof(HuffTables) / 4);
     for (int i = threadIdx.x; i < kExactBytes / 4; i += blockDim.x)
-        dst[i] = i < kTabWords ? src[i] : (i == kTabWords ? flagged : 0u);
+        dst[i] = i < kTabWords ? src[i] : (i == kTabWords ? flagged : i == kTabWords + 1 ? longest : 0u);
 }
 
 }  // namespace bhi
