@@ -23,7 +23,8 @@
 //
 // Results: the four warps of a group add their partial sums through shared memory in pass order (deterministic).
 // Row-sharded layers stage their results and store them into every rank's output with coalesced peer stores at the end
-// of the kernel (see PeerSet for the protocol).
+// of the kernel (see PeerSet for the protocol); where a CTA has too many rows for that, above a million rows per launch, the
+// lanes that hold the results store them.
 #pragma once
 
 #include "bhi_staged.cuh"
@@ -51,6 +52,7 @@ struct GemvGeom {
     int max_quads;             // of a unit: 2, or 1 when all records are long
     int split;                 // the groups of a CTA share its quads and divide the chunks among them
     uint32_t acc_off;          // ... whose sums meet here
+    int direct;                // row-sharded layers: results go to the peers one by one, there is no room to stage them
 };
 
 // Values the compiler must not see: multiply-adds by them stay on the FMA pipe.
@@ -782,6 +784,8 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     if (exchange) {
         launch_no = *reinterpret_cast<const volatile uint32_t *>(peers.launches) + 1u;
         if (blockIdx.x == 0 && tid < peers.world) red_release_sys_add(pick(peers.ready, tid), 1u);
+        // results that are not staged are stored from the first set on: see the end for those that are
+        if (G.direct && tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
     }
     if (NB > 0 && !kRing) {
         const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
@@ -825,6 +829,15 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 x_slot = 0;
                 x_phase ^= 1u;
             }
+        }
+    };
+
+    auto keep = [&](int b, int row, float v) {                          // a result of a row-sharded layer
+        if (!G.direct) {
+            ys[b * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
+        } else {
+#pragma unroll 1
+            for (int q = 0; q < peers.world; q++) pick(peers.y, q)[static_cast<int64_t>(b) * peers.m_total + peers.row_base + row] = f32_to_bf16_rn(v);
         }
     };
 
@@ -978,7 +991,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 if (split) {
                     acc[((cur.quad + q - cta_lo) * NG + group) * 32 + lane] = v;
                 } else if (b < B && row < L.M) {
-                    if (exchange) ys[b * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
+                    if (exchange) keep(b, row, v);
                     else if (B <= BHI_MAX_BATCH) Y[static_cast<int64_t>(b) * L.M + row] = finish_value(v, bias, row);
                     else Y[static_cast<int64_t>(b) * L.M + row] =
                         f32_to_bf16_rn(bias ? v + __uint_as_float(static_cast<uint32_t>(__ldg(bias + row)) << 16) : v);
@@ -999,7 +1012,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 if (L.S * g / NG < L.S * (g + 1) / NG) v += acc[(i * NG + g) * 32 + lane];
             const int row = 4 * (cta_lo + i) + t;
             if (gq < B && row < L.M) {
-                if (exchange) ys[gq * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
+                if (exchange) keep(gq, row, v);
                 else Y[static_cast<int64_t>(gq) * L.M + row] = finish_value(v, bias, row);
             }
         }
@@ -1013,15 +1026,17 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     if (exchange) {
         // one thread asks whether every peer's buffer may be overwritten (an acquire at system scope); the barrier that
         // makes the staged results visible hands its answer to the others
-        if (tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
-        asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
-        for (int i = tid; i < B * rows_cta; i += kThreads) {
-            const int b = i / rows_cta, rr = i - b * rows_cta;
-            const uint16_t v = ys[i];
-            const int64_t to = static_cast<int64_t>(b) * peers.m_total + peers.row_base + row_lo + rr;
+        if (!G.direct) {
+            if (tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
+            asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
+            for (int i = tid; i < B * rows_cta; i += kThreads) {
+                const int b = i / rows_cta, rr = i - b * rows_cta;
+                const uint16_t v = ys[i];
+                const int64_t to = static_cast<int64_t>(b) * peers.m_total + peers.row_base + row_lo + rr;
 #pragma unroll
-            for (int q = 0; q < kMaxPeers; q++)
-                if (q < peers.world) peers.y[q][to] = v;
+                for (int q = 0; q < kMaxPeers; q++)
+                    if (q < peers.world) peers.y[q][to] = v;
+            }
         }
         exchange_finish(peers, launch_no);
     }
@@ -1045,7 +1060,7 @@ struct GemvForm {
 // together comes quad by quad, and a quad that does not fit alone is decoded from global memory, several times as slow.
 // (4096 x 12288, rANS, one row of X, row scales log-normal with sigma 0.35: 177 us without the growth and the quads, 42 with
 // them, as with equal rows; 12288 x 4096, limit6, four rows: 76 and 30.  Equal rows pay 0 to 0.7 us for the look.)
-static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool exchange,
+static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool stage_results,
                       GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
     const uint32_t cap = f.per_sm == 2 ? kSmemMax / 2 - 512 : kSmemMax;
@@ -1063,7 +1078,7 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     G.exact_off = up(table_bytes);
     G.part_off = G.exact_off + kExactBytes + kGemvCtrlBytes;
     G.ys_off = G.part_off + up(static_cast<uint64_t>(f.groups) * kGemvWarps * 64 * 4 * acc_groups);
-    G.acc_off = G.ys_off + (exchange ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
+    G.acc_off = G.ys_off + (stage_results ? up(static_cast<uint64_t>(B) * 4 * nq * 2) : 0u);
     G.rem_off = G.acc_off + (G.split && acc_groups ? up(static_cast<uint64_t>(nq) * f.groups * 128) : 0u);
     G.ring_off = G.rem_off + f.groups * kGemvWarps * 2u * kRemChunk;
     auto unit = [&](uint64_t r) { return 4ull * f.quads * (r * 256u + 32u); };
@@ -1142,26 +1157,30 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
                               {4, 1, 2, 8, kMany}, {4, 1, 2, 5, kMany}, {4, 1, 1, 5, kFew}, {4, 1, 1, 5, kMany}, {2, 1, 1, 5, kMany},
                               {2, 1, 1, 0, kMany}};
     const int nquads = (L.M + 3) / 4, only = gemv_groups();
-    for (const GemvForm &f : forms) {
-        if (only && f.groups != only) continue;
-        if (!kLast && (f.quads < 2 || f.x == GemvX::ring)) break;
-        if (NB > 1 && (f.x == GemvX::resident || f.groups == 2)) continue;     // more than eight rows hardly ever fit
-        int grid = sm_count() * f.per_sm;
-        if (grid > nquads) grid = nquads;
-        GemvGeom G{};
-        uint32_t smem_bytes = 0;
-        if (!gemv_plan(L, B, Dec::kTableBytes, NB, f, grid, peers != nullptr, G, smem_bytes)) continue;
-        if (f.x == GemvX::ring) {
-            if constexpr (NB > 0 && kLast) {
-                if constexpr (NB == 1) {
-                    if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+    for (int direct = 0; direct <= (kLast && peers != nullptr ? 1 : 0); direct++) {
+        for (const GemvForm &f : forms) {
+            if (only && f.groups != only) continue;
+            if (!kLast && (f.quads < 2 || f.x == GemvX::ring)) break;
+            if (peers != nullptr && !direct && f.quarters == 0) continue;           // staged records before staged results
+            if (NB > 1 && (f.x == GemvX::resident || f.groups == 2)) continue;     // more than eight rows hardly ever fit
+            int grid = sm_count() * f.per_sm;
+            if (grid > nquads) grid = nquads;
+            GemvGeom G{};
+            uint32_t smem_bytes = 0;
+            if (!gemv_plan(L, B, Dec::kTableBytes, NB, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
+            G.direct = direct;
+            if (f.x == GemvX::ring) {
+                if constexpr (NB > 0 && kLast) {
+                    if constexpr (NB == 1) {
+                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                    }
+                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
                 }
-                return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
-            }
-        } else {
-            if constexpr (NB <= 1) {
-                if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
-                return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+            } else {
+                if constexpr (NB <= 1) {
+                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                }
             }
         }
     }

@@ -129,9 +129,8 @@ def test_single_rank_arena_matches_plain_layer(algo):
         assert torch.equal(peer(big), lin(big))                      # more than 8 rows: the ordinary path
 
 
-def test_results_too_large_to_stage_take_the_direct_stores(abi):
-    """Many rows per CTA at batch 8: the staged-result buffer would not fit, each row is stored by the lanes
-    that hold it; same results as the plain GEMV."""
+def test_many_rows_per_cta(abi):
+    """540 rows per CTA at batch 8, staged in shared memory; same results as the plain GEMV."""
     M, K, B = 80000, 128, 8
     Wb, shards = _shard("ans", M, K, 1, 4, 1)
     X = make_input(B, K, 6)
@@ -151,6 +150,34 @@ def test_results_too_large_to_stage_take_the_direct_stores(abi):
     plain = abi.gemv("ans", shards[0], x)
     assert torch.equal(plain, y[:B])
     assert rel_err(y[:B].float().cpu().numpy(), oracle.matvec(Wb, bits_of(X))) <= TOL
+
+
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+def test_results_too_large_to_stage_take_the_direct_stores(abi, algo):
+    """So many rows per CTA at batch 8 that their results have no room in shared memory in any form: each is stored by the
+    lane that holds it; same results as the plain GEMV."""
+    from bf16_huffman_infer_b200 import ANSWeight, HuffmanWeight
+    M, K, B = 2_000_003, 128, 8
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    W = (torch.randn(M, K, device=DEV, generator=gen) * 0.02).bfloat16()
+    weight = (HuffmanWeight if algo == "huffman" else ANSWeight).compress_split_n(W, n=1, to_cpu=False)
+    del W
+    w = weight.kwargs()
+    x = make_input(B, K, 6).to(DEV)
+    y = torch.zeros(8, M, dtype=torch.bfloat16, device=DEV)
+    counters = torch.zeros(2, 32, dtype=torch.int32, device=DEV)
+    launches = torch.zeros(2, dtype=torch.int32, device=DEV)
+    ex = Exchange(world=1, rank=0, row_base=0, M_total=M)
+    ex.y[0] = y.data_ptr()
+    ex.ready[0] = counters[0].data_ptr()
+    ex.done[0] = counters[1].data_ptr()
+    ex.launches = launches.data_ptr()
+    for _ in range(2):
+        _launch(abi, algo, w, x, ex)
+    torch.cuda.synchronize()
+    assert _status(abi) == 0
+    assert torch.equal(abi.gemv(algo, w, x, prepared=algo == "huffman"), y[:B])
+    assert launches.tolist() == [2, 0] and counters[:, 0].tolist() == [2, 2]
 
 
 def test_wait_on_a_missing_peer_runs_out(abi):
