@@ -141,7 +141,7 @@ static int run_rows(const Layer &L, const typename Codec::Args &targs, const uin
     BHI_REQUIRE(X && Y, "null activation buffer");
     BHI_REQUIRE(B > BHI_MAX_BATCH && B <= BHI_MAX_ROWS, "batch must be in [9, 32]");
     int rc = kStagedDeclined;
-    if (g_path.load() == 0 && aligned(X, 4) && aligned(Y, 2) && aligned(bias, 2))
+    if (g_path.load() != 1 && aligned(X, 4) && aligned(Y, 2) && aligned(bias, 2))
         rc = gemv_launch<Codec>(L, targs, prepared, X, bias, Y, nullptr, B, pair_complete_hint(prepared), st);
     return rc == kStagedDeclined ? fail(BHI_ERR_LIMIT, "layer or buffers not supported by the fused product of 9 to 32 rows") : rc;
 }

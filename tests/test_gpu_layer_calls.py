@@ -120,3 +120,17 @@ def test_many_leading_dimensions(coded, rows):
     with torch.no_grad():
         y = _layer(weight, bias)(x)
     assert y.shape == x.shape[:-1] + (M,) and _close(y, F.linear(x, W, bias))
+
+
+@pytest.mark.parametrize("path", [0, 2])
+def test_both_automatic_paths_take_more_rows(coded, path):
+    from _util import Abi
+    W, weight, bias = coded
+    abi = Abi()
+    previous = abi.set_path(path)
+    try:
+        x = make_input(12, K, 1).to(DEV)
+        y = weight._forward(x, bias)
+        assert y.shape == (12, M) and _close(y, F.linear(x, W, bias))
+    finally:
+        abi.set_path(previous)
