@@ -30,9 +30,9 @@ __global__ void huffman_encode_chars_kernel(const uint8_t *__restrict__ data, in
     out_len[t] = cnt;
 }
 
-// One entry of an rANS encoding model.  A state is below freq << 32 <= 2^44 when it is divided, so its quotient by freq
-// is the high half of (2 * state) * inv with inv = ceil(2^63 / freq): the excess inv * freq - 2^63 is below freq <= 2^12
-// and 2^44 * 2^12 < 2^63, so no quotient is off by one.  (A 64-bit division in its place lies on the serial
+// One entry of an rANS encoding model.  A state is below freq << 32 <= 2^47 when it is divided (models have at most 15 bits),
+// so its quotient by freq is the high half of (2 * state) * inv with inv = ceil(2^63 / freq): the excess
+// inv * freq - 2^63 is below freq <= 2^15 and 2^47 * 2^15 < 2^63, so no quotient is off by one.  (A 64-bit division in its place lies on the serial
 // chain of every stream: size and emit pass over a 12288 x 4096 layer took 279 and 287 us with it, 81 and 95 us now.)
 struct AnsModel {
     uint64_t inv[256];
@@ -60,7 +60,7 @@ template <class Put>
 __device__ __forceinline__ void ans_push(uint64_t &state, const AnsModel &t, uint32_t sym, uint32_t bits, Put &&put) {
     const uint32_t f = t.freq[sym];
     if (f == 0u) return;
-    if ((state >> 32) >= f) {                      // once is enough: the state is below 2^(32 + bits) and bits <= 12
+    if ((state >> 32) >= f) {                      // once is enough: the state is below 2^(32 + bits) and f >= 1
         put(static_cast<uint32_t>(state));
         state >>= 32;
     }

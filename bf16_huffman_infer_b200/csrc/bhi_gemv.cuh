@@ -768,7 +768,10 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     }
     uint32_t prev_foot = staged ? foot : 0u;                           // leader: ring bytes of the unit being decoded
 
-    bool usable = smem_base == kTableAt;      // the table's place is a constant in the loads; else records are decoded directly
+    // The table's place is a constant in the loads.  Where shared memory starts elsewhere records are decoded directly: right,
+    // but several times as slow, so the status says so.
+    bool usable = smem_base == kTableAt;
+    if (!usable && tid == 0) atomicExch(&g_staged_status, 10);
     if (kHuff && prepared != nullptr) {
         if (!mbar_wait_bounded(table_bar, 0u) && tid == 0) atomicExch(&g_staged_status, 2);
         usable = usable && Dec::usable(*reinterpret_cast<const Tables *>(&tab));

@@ -68,8 +68,9 @@ int bhi_set_launch_overlap(int on);
 /* Reads and clears the device-side status word of the current device.  0 = no incident; otherwise
  * the last bounded wait that ran out inside a kernel: 1 a record's bulk copy (the record was
  * skipped), 2 the prepared-table copy, 3-7 the tensor-core path's stage / accumulator barriers,
- * 8 peers not ready and 9 peers not done in an exchange kernel.  The kernels always run to their
- * end.  Synchronises the device; meant for tests and post-mortems, not for the launch path. */
+ * 8 peers not ready and 9 peers not done in an exchange kernel; or 10, no wait: shared memory does
+ * not start where the fused kernel's tables are read, and all records were decoded from global
+ * memory, rightly but several times as slowly.  The kernels always run to their end.  Synchronises the device; meant for tests and post-mortems, not for the launch path. */
 int bhi_debug_status(int *status_out);
 
 /* Y[b, m] = sum_c X[b, c] * W[m, c] computed straight from the Huffman-coded weight.
