@@ -35,15 +35,14 @@ SLAB_ROWS = 4096          # rows encoded per slab; 64 padding words follow every
 FUSED_MAX_ROWS = 8        # up to here: fused decode + GEMV, as the reference
 FUSED_MORE_ROWS = 32      # up to here without gradients: the same kernel with more products per decoded word; beyond, or with
                           # gradients: decode, then a library GEMM (as the reference)
-# Rows up to which the fused decode + tensor-core product (mm_huffman_prepared / mm_ans, at most 128) is used
-# instead of decode + GEMM.  Off by default: on B200 it is within 5 % of decode + library GEMM up to 32 rows and
-# behind it beyond (python -m bf16_huffman_infer_b200.examples.linear_bench), but needs no dense scratch.
-# BHI_TENSOR_ROWS=32 (or up to 128) turns it on.
+# Rows up to which mm_huffman_prepared / mm_ans (at most 128) are used instead: up to 32 the same kernel again, beyond, the
+# products that keep their sums in tensor memory.  Off by default: beyond 32 rows those are slower than decode + library GEMM
+# (python -m bf16_huffman_infer_b200.examples.linear_bench), but need no dense scratch.  BHI_TENSOR_ROWS=128 turns them on.
 TENSOR_MAX_ROWS = int(os.environ.get("BHI_TENSOR_ROWS", "0"))
 # Which prefix code HuffmanWeight.compress builds (huffman.py; every choice yields tables of the reference's
 # format, readable by any decoder of it, the reference's included):
-#   "limit6"    (default) optimal code with no length above 6 bits: any two codes fit the 12-bit index of the fused
-#               kernels' folded table, so they never leave their two-symbols-per-lookup loop (fastest; about 4 %
+#   "limit6"    (default) optimal code with no length above 6 bits: the fused kernel decodes it symbol by symbol in
+#               tables that hold a copy per lane, free of bank conflicts and of exceptions (fastest; about 4 %
 #               larger than "escape" on N(0, s) weights; falls back to "escape" beyond 64 distinct exponents);
 #   "escape"    escape-byte code, near-entropy on every histogram (smallest);
 #   "reference" the reference's own builder, bit for bit (and so its compressed bytes); on some histograms its
@@ -373,9 +372,11 @@ class HuffmanWeight(nn.Module):
             d["_prepared_src"] = src
         return d["_prepared"]
 
-    @staticmethod
-    def _drop_prepared(state: Dict) -> Dict:
-        for name in ("_prepared_src", "_prepared", "_prepared_tables"):
+    derived = ("_prepared_src", "_prepared", "_prepared_tables")        # what prepared() keeps
+
+    @classmethod
+    def _drop_prepared(cls, state: Dict) -> Dict:
+        for name in cls.derived:
             state.pop(name, None)
         return state
 
@@ -387,7 +388,7 @@ class HuffmanWeight(nn.Module):
         return self
 
     def __getstate__(self):
-        """Copies and pickles fold their own tables."""
+        """Copies and pickles fold their own tables (shallow_copy_model's, which share the buffers, share the fold too)."""
         return self._drop_prepared(self.__dict__.copy())
 
     def _plain(self) -> bool:

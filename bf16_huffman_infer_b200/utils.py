@@ -98,4 +98,9 @@ def shallow_copy_model(model: nn.Module) -> nn.Module:
         for v in vars(m).values():
             if torch.is_tensor(v):
                 memo[id(v)] = v
-    return copy.deepcopy(model, memo=memo)
+    copied = copy.deepcopy(model, memo=memo)
+    for m, c in zip(model.modules(), copied.modules()):
+        for name in getattr(m, "derived", ()):           # left out of other copies, whose buffers are their own
+            if name in vars(m):
+                vars(c)[name] = vars(m)[name]
+    return copied

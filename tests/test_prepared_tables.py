@@ -56,6 +56,16 @@ def test_copies_and_pickles_fold_their_own(folds):
     assert int(w.prepared()[0]) == 3
 
 
+def test_copies_that_share_the_buffers_share_the_fold(folds):
+    from bf16_huffman_infer_b200.utils import shallow_copy_model
+    model = torch.nn.Sequential(_weight(3), _weight(4))
+    model[0].prepared()
+    copied = shallow_copy_model(model)
+    assert copied[0] is not model[0] and copied[0].LUT1 is model[0].LUT1
+    assert copied[0].prepared() is model[0].prepared()
+    assert "_prepared" not in vars(copied[1]) and int(copied[1].prepared()[0]) == 4
+
+
 @pytest.mark.gpu
 def test_move_load_move():
     from bf16_huffman_infer_b200 import HuffmanWeight, set_huffman_tables
