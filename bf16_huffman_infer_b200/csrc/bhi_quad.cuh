@@ -14,20 +14,15 @@ namespace bhi {
 
 constexpr int kQuadGroups = 8;                                 // warp groups per CTA, one quad each at a time
 constexpr int kQuadCtrlBytes = 1024;                           // mbarriers
-constexpr int kQuadPartBytes = kQuadGroups * 2 * 4 * 32 * 4;   // [group][parity][warp of the group][lane] partial sums
 constexpr uint32_t kQuadRingWant = 59u * 256u;                 // per group: two units of four 7-row records
-constexpr uint32_t kQuadRingLeast = 8u * 1024u;                // below this the shape is declined
 constexpr uint32_t kEntFlags = kEntSingle | kEntExact;
 
 struct QuadGeom {
     uint32_t lut_bytes;        // fast table region (copies * one table)
     uint32_t copy_shift;       // log2(bytes between consecutive table entries) = 2 + log2(copies)
     uint32_t index_mask;       // table index bits, already at their place in a biased window
-    uint32_t part_off, acc_off, ys_off, x_off, ring_off;
-    uint32_t x_bytes;          // one stage of X
+    uint32_t ring_off;
     uint32_t ring_bytes;       // per group
-    int chunks_per_stage;
-    int stages;
 };
 
 __device__ __forceinline__ uint32_t lds32(const uint8_t *smem, uint32_t a) { return *reinterpret_cast<const uint32_t *>(smem + a); }

@@ -38,8 +38,7 @@ constexpr uint32_t kRemMask = 0x807F807Fu;     // sign + mantissa bits of a bf16
 // values it has to keep the multiply-add form.
 struct Consts {
     uint32_t ans_bits, ans_mask;             // rANS: probability precision of the layer's table and 2^bits - 1
-    uint32_t one, eight, entry, shift16;     // entry = bytes between consecutive fast-table entries (4 * copies);
-                                             // shift16 = 65536 (a left shift by 16 as a multiply)
+    uint32_t eight, entry;                   // entry = bytes between consecutive fast-table entries (4 * copies)
 };
 
 // A prepared-table blob (Huffman): one copy of the folded pair table, the exact tables, the single-symbol tables with one
@@ -106,8 +105,8 @@ __device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uin
 
 // ---- row-sharded GEMV whose epilogue is the all-gather ------------------------------------------------
 // Every rank computes the rows [row_base, row_base + M) of Y [B, M_total] and needs all of it.  Instead
-// of a collective after the kernel, the lanes that hold a finished dot product store it straight into
-// the Y buffer of every rank (plain stores to peer-mapped pointers over NVLink; lane r serves rank r).
+// of a collective after the kernel, the CTA stores its finished dot products straight into the Y buffer
+// of every rank (plain stores to peer-mapped pointers over NVLink, every thread to all ranks in turn).
 // Four counter words per layer and rank make that safe without any other kernel:
 //   ready  - each rank adds 1 on every peer when its launch may be written to (its earlier consumers of
 //            Y are done: the add comes after the wait for the previous kernel in the stream); a warp

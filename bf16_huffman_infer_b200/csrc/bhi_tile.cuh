@@ -28,8 +28,8 @@
 //   * with both out of the way the kernel runs at the speed of its decoders: about 86 warp instructions per row and block
 //     (the GEMV kernel's four-row layout needs 36) at a third of the issue slots, the rest being global-load latency.
 //     That is 0.8 to 1.0 us per block of 32 to 64 rows, against 0.45 us for the same rows in the decode-to-dense kernel,
-//     so decode + library GEMM stays ahead (23 / 61 / 63 us against 31 / 62 / 83 us on 4096x4096, 12288x4096, 4096x12288 at
-//     16 rows) and remains the default above 8 rows; this path is an option (BHI_TENSOR_ROWS in the host layer).
+//     so decode + library GEMM stays ahead (57 us against 80 on 12288x4096 at 128 rows) and is the default above the 32 rows
+//     of the fused kernel (bhi_gemv.cuh); this path is an option (BHI_TENSOR_ROWS in the host layer).
 //
 // Barriers (all waits bounded, failures reported through bhi_debug_status):
 //   full[s]    16 decoder warps                          -> issuer may multiply W stage s
@@ -540,7 +540,7 @@ static int tile_launch_r(const Layer &L, const typename Codec::Args &targs, cons
     cfg.attrs = attr;
     cfg.numAttrs = overlap_launches() ? 1 : 0;
     const uint32_t ans_bits = ans_bits_of(targs);
-    const Consts k{ans_bits, (1u << ans_bits) - 1u, 1u, 8u, 4u * kCopies, 65536u};
+    const Consts k{ans_bits, (1u << ans_bits) - 1u, 8u, 4u * kCopies};
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, xmap, Y, B, plan, k);
     return e == cudaSuccess ? BHI_OK : cuda_fail(e, "fused tensor-core kernel launch");
 }

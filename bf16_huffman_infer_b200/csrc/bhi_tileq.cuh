@@ -1,5 +1,6 @@
-// Fused decode + tensor-core product with the four-row decoders of the GEMV kernel (sm_100a: tcgen05 + TMEM), for up to
-// 32 activation rows.
+// Fused decode + tensor-core product with decoders of four rows at a time (sm_100a: tcgen05 + TMEM).  Up to 32 activation
+// rows the kernel of bhi_gemv.cuh serves every prepared or rANS layer faster (12288 x 4096, escape tables, 17 rows: 51 us
+// against 104); left for this one are 33 to about 48 rows, and 9 to 32 of a layer whose tables are not prepared.
 //
 // Same product and same roles as tile_kernel (bhi_tile.cuh): decoder warps fill K-major W stages in shared memory, one
 // warp issues the MMAs, one requests the X blocks by TMA, four read the accumulators back.  What differs is where the
@@ -46,7 +47,7 @@ constexpr int kTqWStages = 2;
 constexpr int kTqXStagesMax = 8;
 
 struct TqPlan {
-    QuadGeom G;            // table region, ring geometry (part / acc / ys / x fields unused)
+    QuadGeom G;            // table region, ring geometry
     uint32_t x_rows, x_atom, x_stage, x_stages;
     uint32_t x_off, w_off, total;
     int sets_per_cta;
@@ -539,7 +540,7 @@ static int tileq_launch(const Layer &L, const typename Codec::Args &targs, const
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap_launches() ? 1 : 0;
-    const Consts k{ans_bits, (1u << ans_bits) - 1u, 1u, 8u, 4u * kCopies, 65536u};
+    const Consts k{ans_bits, (1u << ans_bits) - 1u, 8u, 4u * kCopies};
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, xmap, Y, B, plan, k);
     return e == cudaSuccess ? BHI_OK : cuda_fail(e, "fused tensor-core kernel launch");
 }

@@ -365,7 +365,7 @@ class HuffmanWeight(nn.Module):
         if d.get("_prepared_src") != src:
             blob = torch.empty(ops.PREPARED_BYTES, dtype=torch.uint8, device=self.rem.device)
             ops.huffman_prepare(t1, t2, t3, t4, cl, blob)
-            # codes of at most 6 bits: every 12-bit window holds two whole codes (the kernels pick their warp layout by it)
+            # codes of at most 6 bits go through the tables of single symbols
             ops.huffman_table_hint(blob, int(cl.max().item()) <= 6)
             d["_prepared"] = blob
             d["_prepared_tables"] = tuple(t.detach() for t in (t1, t2, t3, t4, cl))

@@ -239,8 +239,8 @@ def length_limited_code(freqs: Dict[int, float], limit: int) -> Dict[int, Tuple[
     """``{symbol: (length, value)}`` of the optimal prefix code whose lengths do not exceed ``limit`` (<= 8).
 
     Every code fits the first byte table, so the byte-decomposed format holds it as it is.  With
-    ``limit = 6`` any two consecutive codes fit a 12-bit window: the fused kernels then resolve two
-    symbols with every table lookup and never take their symbol-by-symbol path.  Falls back to the
+    ``limit = 6`` a table of 64 symbols resolves every code, small enough for a copy per lane: the fused
+    kernel looks symbols up without bank conflicts and without exceptions.  Falls back to the
     escape-byte code when there are more symbols than ``2**limit``.  No counterpart in the reference.
     """
     assert 1 <= limit <= 8

@@ -94,15 +94,14 @@ int bhi_huffman_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_
  * The fused kernels do not decode with the four byte tables directly: they fold them into single-symbol and
  * two-symbols-per-lookup tables.  The two entry points above rebuild such a table inside every launch, which costs a few
  * microseconds per call.  A caller that keeps a layer around can
- * fold the tables once into a blob of bhi_huffman_prepared_bytes() bytes (16-byte aligned device
- * memory owned by the caller) and pass the blob instead of the five tables; the kernels then
+ * fold the tables once into a blob of bhi_huffman_prepared_bytes() bytes (130 KB: every table that a launch may
+ * fetch, 18 to 66 KB of it; 16-byte aligned device memory owned by the caller) and pass the blob instead of the five tables; the kernels then
  * fetch it with a single bulk copy.  Results are identical.  No counterpart in the reference
  * (its kernels index the byte tables directly, src/kernel.cu:370-377). */
 int bhi_huffman_prepared_bytes(void);
 /* Tuning hint for a prepared blob (host-side bookkeeping, no device work): pair_complete != 0 declares that
- * no code of the table is longer than 6 bits, so that any two consecutive codes fit the 12-bit index of the
- * folded table.  The fused kernels pick their warp layout by it; results never depend on it (whether the
- * per-step test can be skipped is read from the blob itself).  bhi_huffman_prepare clears the hint of the
+ * no code of the table is longer than 6 bits.  The fused kernel then takes its tables of single symbols; results
+ * never depend on it (the longest length is read from the blob itself).  bhi_huffman_prepare clears the hint of the
  * blob it writes; give the hint after preparing.  Thread-safe. */
 int bhi_huffman_table_hint(const uint8_t *prepared, int pair_complete);
 int bhi_huffman_prepare(const uint8_t *LUT1, const uint8_t *LUT2, const uint8_t *LUT3, const uint8_t *LUT4,
@@ -152,11 +151,12 @@ int bhi_ans_decode(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_word
  * GEMV entry points are faster up to 8).  The reference has no operator for this range: it decodes
  * the weight to a dense scratch with huffman_decode / ans_decode and calls a library GEMM
  * (bf16_huffman_infer/functional.py:398-407, 469-478).  These entry points replace that pair of
- * calls: a set of weight rows is decoded into shared memory and multiplied there by tcgen05.mma
- * with the accumulator in tensor memory, so the dense weight never reaches HBM and no scratch is
+ * calls: above 32 rows a set of weight rows is decoded into shared memory and multiplied there by
+ * tcgen05.mma with the accumulator in tensor memory, so the dense weight never reaches HBM and no scratch is
  * needed.  Accumulation is FP32 over the whole row, one rounding to BF16 at the end.  X must be
- * 16-byte aligned.  Measured on B200: within 5 % of decode + library GEMM up to 32 rows, behind it
- * beyond. */
+ * 16-byte aligned.  Up to 32 rows of a prepared or rANS layer the fused GEMV's kernel runs instead.
+ * Measured on B200, 12288 x 4096, limit6, decode + library GEMM in brackets: 36 us (54) at 16 rows,
+ * 50 (54) at 32; beyond that behind the pair, 80 (57) at 128. */
 int bhi_linear_bf16_huffman(const uint8_t *A_rem, const uint32_t *A_exp, int64_t exp_words,
                             const uint16_t *X, uint16_t *Y, const int32_t *offsets,
                             const uint8_t *LUT1, const uint8_t *LUT2, const uint8_t *LUT3,

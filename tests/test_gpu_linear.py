@@ -53,8 +53,9 @@ SHAPES = [
 ]
 
 
-# the two fused tensor-core kernels: path 0 = records staged in shared memory while the batch leaves room for them (up to
-# about 48 rows), streams in registers beyond; path 2 = streams in registers at every batch
+# path 0 = the fused kernel up to 32 rows (prepared or rANS), then the tensor-memory kernel that stages records in shared
+# memory while the batch leaves room for them (up to about 48 rows), then the one that keeps its streams in registers;
+# path 2 = the latter at every batch
 @pytest.mark.parametrize("path", [0, 2], ids=["staged", "registers"])
 @pytest.mark.parametrize("prepared", [False, True], ids=["tables", "prepared"])
 @pytest.mark.parametrize("algo", ["huffman", "ans"])
@@ -65,7 +66,7 @@ def test_linear_matches_oracle(abi, path, prepared, algo, M, K, S, seed):
     Wb, w = _device_layer(algo, M, K, S, seed)
     previous = abi.set_path(path)
     try:
-        for B in (9, 16, 24, 33, 48, 64, 100, 128, 1):
+        for B in (9, 16, 24, 33, 40, 48, 64, 100, 128, 1):
             X = make_input(B, K, seed + B)
             y = abi.linear(algo, w, X.to(DEV), prepared=prepared).float().cpu().numpy()
             ref = oracle.matvec(Wb, bits_of(X))
@@ -79,7 +80,8 @@ def test_linear_matches_oracle(abi, path, prepared, algo, M, K, S, seed):
 @pytest.mark.parametrize("method", ["limit6", "escape"])
 @pytest.mark.parametrize("M,K,S", [(200, 4736, 1), (96, 4736 * 4, 4), (4224, 384, 3)])
 def test_linear_other_tables_and_odd_block_counts(abi, path, method, M, K, S):
-    """Tables without unresolved windows take the branch-free loops; 37 blocks per chunk end on half a stage pair."""
+    """Tables without unresolved windows take the branch-free loops; 37 blocks per chunk end on half a stage pair.  33 to 48
+    rows, and 12 and 32 without prepared tables, are staged for the tensor-memory kernel."""
     W = make_weight(M, K, 21, 0.02)
     Wb = bits_of(W)
     tabs = tables_for("huffman", oracle.histogram(Wb), method)
@@ -87,10 +89,11 @@ def test_linear_other_tables_and_odd_block_counts(abi, path, method, M, K, S):
     w = to_device(dict(rem=rem, exp=exp, offsets=offsets, **{k: v for k, v in tabs.items() if k != "code_values"}), DEV)
     previous = abi.set_path(path)
     try:
-        for B in (12, 32, 72):
+        for B in (12, 32, 33, 40, 48, 72):
             X = make_input(B, K, B)
-            y = abi.linear("huffman", w, X.to(DEV), prepared=True).float().cpu().numpy()
-            assert rel_err(y, oracle.matvec(Wb, bits_of(X))) <= TOL, B
+            for prepared in (True, False):
+                y = abi.linear("huffman", w, X.to(DEV), prepared=prepared).float().cpu().numpy()
+                assert rel_err(y, oracle.matvec(Wb, bits_of(X))) <= TOL, (B, prepared)
         assert _status(abi) == 0
     finally:
         abi.set_path(previous)

@@ -43,15 +43,15 @@ SHAPES = [
 ]
 
 
-# kernel variants of the fused product: (kernel path, warps of the four-row kernel, prepared tables)
+# forms of the fused product: (kernel path, 0 and 2 being automatic; warps per block; prepared tables)
 VARIANTS = {"auto": (0, 0, False), "auto-prepared": (0, 0, True), "generic": (1, 0, False),
-            "rowwarp": (2, 0, False), "rowwarp-prepared": (2, 0, True),
-            "quad32": (0, 32, False), "quad32-prepared": (0, 32, True), "quad16": (0, 16, False), "quad16-prepared": (0, 16, True)}
+            "auto2": (2, 0, False), "auto2-prepared": (2, 0, True),
+            "warps32": (0, 32, False), "warps32-prepared": (0, 32, True), "warps16": (0, 16, False), "warps16-prepared": (0, 16, True)}
 PATHS = [(0, 0), (0, 32), (0, 16), (2, 0), (1, 0)]
 
 
 class use_path:
-    """Selects a kernel path (and the warp count of the four-row kernel) for the duration of a block."""
+    """Selects a kernel path (and the fused kernel's warps per block) for the duration of a block."""
 
     def __init__(self, abi, path, warps=0):
         self.abi, self.path, self.warps = abi, path, warps
