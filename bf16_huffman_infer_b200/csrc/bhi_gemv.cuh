@@ -52,7 +52,6 @@ struct GemvGeom {
     int max_quads;             // of a unit: 2, or 1 when all records are long
     int split;                 // the groups of a CTA share its quads and divide the chunks among them
     uint32_t acc_off;          // ... whose sums meet here
-    int direct;                // row-sharded layers: results go to the peers one by one, there is no room to stage them
 };
 
 // Values the compiler must not see: multiply-adds by them stay on the FMA pipe.
@@ -475,14 +474,14 @@ __device__ __forceinline__ void copy_x_row(uint32_t dst, const uint16_t *src, ui
     }
 }
 
-// Which of up to 32 pairs of quads, from quad `first` on, have in chunks [k_lo, k_hi) a record of more than `most` words:
-// bit i for pair i (window pairs).
-__device__ __forceinline__ uint32_t pairs_apart(const int32_t *offsets, int S, int M, uint32_t exp_words, int first, int quad_hi, int k_lo,
-                                             int k_hi, int window, uint32_t most) {
-    const int lane = threadIdx.x & 31, q = first + 2 * (lane & (window - 1));
-    bool longer = false;
-    if (q + 1 < quad_hi) {
-        for (int k = k_lo + lane / window; k < k_hi; k += 32 / window) {
+// How many sets the quads [quad_lo, quad_hi) make (whole warp): pairs, but two of a pair that has, in any chunk, a record of
+// more than `most` words.
+__device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, uint32_t exp_words, int quad_lo, int quad_hi, uint32_t most) {
+    int sets = (quad_hi - quad_lo + 1) >> 1;
+    for (int q0 = quad_lo; q0 + 1 < quad_hi; q0 += 64) {
+        const int q = q0 + 2 * static_cast<int>(threadIdx.x & 31);
+        bool longer = false;
+        for (int k = 0; k < S && q + 1 < quad_hi; k++) {
             const int rec = k * M + 4 * q, last = k * M + M;
             uint32_t at[9];
 #pragma unroll
@@ -493,18 +492,19 @@ __device__ __forceinline__ uint32_t pairs_apart(const int32_t *offsets, int S, i
 #pragma unroll
             for (int i = 0; i < 8; i++) longer |= at[i + 1] > at[i] && at[i + 1] - at[i] > most;
         }
+        sets += __popc(__ballot_sync(0xFFFFFFFFu, longer));
     }
-    uint32_t apart = __ballot_sync(0xFFFFFFFFu, longer);
-    if (window <= 16) apart |= apart >> 16;
-    if (window == 8) apart |= apart >> 8;
-    return apart;
+    return sets;
 }
 
 // NB = groups of eight X rows (0: no product, the dense matrix is written instead).  NG = groups of four warps per CTA.
 // Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
 // X or tables two CTAs could not both hold.  kRing: X passes through a ring that one more warp fills and all groups read in
 // step.  (20 warps of 96 registers instead of 16 gain nothing: it is pipes that are short, not warps.)
-template <class Dec, int NB, int NG, bool kRing>
+// kShard: a layer whose rows are shared among ranks (1: results staged, 2: stored one by one).  An argument of the template,
+// because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
+// layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
+template <class Dec, int NB, int NG, bool kRing, int kShard>
 __global__ void __launch_bounds__(NG * kGemvWarps * 32 + (kRing ? 32 : 0), NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
             PeerSet peers, GemvGeom G, GemvConsts kc) {
@@ -522,7 +522,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     // streams l and l + 32: its stores are whole 128-byte lines.
     const uint32_t sigma4 = NB > 0 ? 4u * (8 * wig + (lane & 7)) : 4u * lane;      // byte offset of the lane's stream inside a word row
     auto row_of = [&](int q, int n, int row) { return NB > 0 ? 4 * q + row : n * wig + q; };       // row of a unit of n quads
-    const bool exchange = NB == 1 && peers.world > 0;
+    constexpr bool exchange = NB == 1 && kShard > 0;
     const int B = G.batch;
 
     Tables &tab = *reinterpret_cast<Tables *>(smem + G.exact_off);
@@ -532,7 +532,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     const uint32_t bar0 = ctrl_at + 16u * group;                       // record copies: two slots per group
     const uint32_t table_bar = ctrl_at + 80u, x_bar = ctrl_at + 88u;
     const uint32_t x_full = ctrl_at + 96u, x_empty = x_full + 8u * kXSlotsMax;      // X ring: filled, read by all warps
-    volatile uint32_t *posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256) + 8 * group;     // [slot]{word rows, base, staged}, [3] sets
+    volatile uint32_t *posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256) + 8 * group;     // [slot]{word rows, base, staged, quads}
     float *part = reinterpret_cast<float *>(smem + G.part_off) + group * (kGemvWarps * 64 * kAcc);
     uint16_t *ys = reinterpret_cast<uint16_t *>(smem + G.ys_off);
     const uint32_t xs = smem_base + G.x_off;
@@ -578,10 +578,10 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
 
     // Segments of X that pass through the ring: every unit reads those of its chunk, in order.  The groups post how many sets
     // of quads they have.
-    volatile uint32_t *all_posted = reinterpret_cast<volatile uint32_t *>(ctrl + 256);
+    volatile uint32_t *all_sets = reinterpret_cast<volatile uint32_t *>(ctrl + 384);
     auto x_segments = [&]() {
         uint32_t sets = 0u;
-        for (int g = 0; g < NG; g++) sets = max(sets, all_posted[8 * g + 3]);
+        for (int g = 0; g < NG; g++) sets = max(sets, all_sets[g]);
         return static_cast<int>(sets) * L.S * chunks;
     };
     // ---- the warp that fills the X ring.  (With the readers filling it between their chunks, the last reader of a segment
@@ -625,69 +625,66 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     // ---- units ---------------------------------------------------------------------------------------------------------
     // A set is a pair of quads, or one quad: the last of an odd number, and both of a pair that has, in any chunk, a record
     // longer than the ring takes beside seven of that length.  For each set, the chunks in order.  The group's first warp
-    // knows where the records of the next unit lie (its lanes 0..7 hold one row each), places them in the ring, starts their
-    // copies and posts {word rows, base, staged} for the others; the offsets it needs are requested one unit ahead of that.
+    // knows where the records of the next unit lie (its lanes 0..7 hold one row each; of a set's first unit the others hold
+    // the same rows in the three chunks after), decides how many quads the set has, places the records in the ring, starts
+    // their copies and posts {word rows, base, staged, quads} for the others; the offsets it needs are requested one unit
+    // ahead of that.  Until then a pair counts as whole.
     struct Place {
         int quad, k, n;
     };
     const uint32_t exp_words = static_cast<uint32_t>(L.exp_words);
-    const int window = L.S == 1 ? 32 : L.S == 2 ? 16 : 8;              // pairs looked at together, one chunk per lane
-    int seen = quad_lo;                                                // first quad of the window
-    uint32_t alone = 0u;                                               // bit i: the quads of its pair i are taken one by one
-    auto look = [&](int first) {
-        seen = first;
-        alone = G.max_quads == 2 ? pairs_apart(L.offsets, L.S, L.M, exp_words, first, quad_hi, k_lo, k_hi, window, 64u * G.pair_rows) : ~0u;
-    };
-    auto quads_seen = [&](int quad) {
-        const int i = quad - seen;
-        return (i & 1) || (alone >> (i >> 1) & 1u) ? 1 : min(2, quad_hi - quad);
-    };
     auto after = [&](const Place &u) {
         Place v{u.quad, u.k + 1, u.n};
         if (v.k == k_hi) {
             v.k = k_lo;
             v.quad += u.n;
-            if (v.quad < quad_hi) {
-                if (v.quad - seen >= 2 * window) look(v.quad);
-                v.n = quads_seen(v.quad);
-            }
+            v.n = G.max_quads == 1 || ((v.quad - quad_lo) & 1) ? 1 : min(2, quad_hi - v.quad);
         }
         return v;
     };
     const bool leader = wig == 0;
-    auto record_of = [&](const Place &u, int row) {                    // row 0..7 of the unit
-        return u.k * L.M + min(4 * u.quad + (row < 4 * u.n ? row : 0), L.M - 1);
+    auto row_in_layer = [&](const Place &u, int row) { return min(4 * u.quad + (row < 4 * u.n ? row : 0), L.M - 1); };      // row 0..7 of the unit
+    auto record_of = [&](const Place &u, int row) { return u.k * L.M + row_in_layer(u, row); };
+    uint32_t off = 0u, end = 0u;                                       // leader: first and last exponent word
+    auto load_span = [&](int rec) {
+        off = static_cast<uint32_t>(__ldg(L.offsets + rec));
+        end = rec + 1 < L.S * L.M ? static_cast<uint32_t>(__ldg(L.offsets + rec + 1)) : exp_words;
     };
-    uint32_t off = 0u, end = 0u;                                       // leader, lanes 0..7: first and last exponent word
     auto request = [&](const Place &u) {
-        if (leader && u.quad < quad_hi) {
-            const int rec = record_of(u, lane & 7);
-            off = static_cast<uint32_t>(__ldg(L.offsets + rec));
-            end = rec + 1 < L.S * L.M ? static_cast<uint32_t>(__ldg(L.offsets + rec + 1)) : exp_words;
-        }
+        if (leader && u.quad < quad_hi) load_span(min(u.k + (u.k == k_lo ? lane >> 3 : 0), k_hi - 1) * L.M + row_in_layer(u, lane & 7));
     };
     uint32_t words = 0u, at = 0u, foot = 0u, base = 0u;                // leader: the unit being placed
     bool staged = false;
-    auto place = [&](const Place &u, int slot) {
+    auto place = [&](Place &u, int slot) {
         at = off;
         words = end - off;                                             // in storage order, whole word rows, inside the buffer
         const bool fits = words - 1u < (1u << 16) && ((words & 63u) | (off & 3u)) == 0u && off < end && end <= exp_words;
-        uint32_t rows = fits ? words >> 6 : 0u;
+        if (u.n == 2 && u.k == k_lo) {
+            bool longer = off < end && words > 64u * G.pair_rows;
+            for (int k = k_lo + 4 + (lane >> 3); k < k_hi; k += 4) {   // a layer of more than four chunks
+                load_span(k * L.M + row_in_layer(u, lane & 7));
+                longer |= off < end && end - off > 64u * G.pair_rows;
+            }
+            if (__any_sync(0xFFFFFFFFu, longer)) u.n = 1;
+        }
+        uint32_t rows = fits && lane < 4 * u.n ? words >> 6 : 0u;
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
+        rows = __shfl_sync(0xFFFFFFFFu, rows, 0);
         foot = (4u * u.n * (rows * 256u + 32u) + 255u) & ~255u;
-        staged = __all_sync(0xFFFFFFFFu, fits) && foot <= G.ring_bytes;
+        staged = __all_sync(0xFFFFFFFFu, fits || lane >= 4 * u.n) && foot <= G.ring_bytes;
         base = slot == 0 ? ring : ring + G.ring_bytes - foot;
         if (lane == 0) {
             posted[4 * slot] = rows;
             posted[4 * slot + 1] = base;
             posted[4 * slot + 2] = staged ? 1u : 0u;
+            posted[4 * slot + 3] = u.n;
         }
     };
     auto start_copies = [&](const Place &u, int slot) {
         const uint32_t bar = bar0 + 8u * slot;
         const int n = u.n;
-        uint32_t total = lane < 4 * n ? words * 4u : 0u, rows = words >> 6;
+        uint32_t total = lane < 4 * n ? words * 4u : 0u, rows = lane < 4 * n ? words >> 6 : 0u;
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
             total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
@@ -717,54 +714,35 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (n > 1) cp_async_16(dst + 512u, rem[1] + (bytes ? blk * 128 : -(lane >> 3) * 128), bytes);
     };
 
-    // The first pairs are taken for whole until the look at their records is back: what they need is on its way by then.
+    // How many quads the set of unit u has, now that it is known.  Dense, a warp's rows depend on it: those of the first chunk
+    // are fetched once more if it was taken for a pair.
+    auto settle = [&](Place &u, int n) {
+        if (NB == 0 && n != u.n) {
+            u.n = n;
+            cp_async_wait();
+            rem_rows(u);
+            fetch(n, 0, half);
+        }
+        u.n = n;
+    };
+
     Place cur{quad_lo, k_lo, min(G.max_quads, quad_hi - quad_lo)};
     request(cur);
     if (cur.quad < quad_hi) {
         rem_rows(cur);
         fetch(cur.n, 0, 0u);
         if (leader) {
-            place(cur, 0);
-            if (staged) start_copies(cur, 0);
+            Place placed = cur;
+            place(placed, 0);
+            if (staged) start_copies(placed, 0);
+            settle(cur, placed.n);
         }
     }
-    Place nxt{cur.quad, k_lo + 1, cur.n};
-    if (nxt.k == k_hi) nxt = Place{cur.quad + cur.n, k_lo, min(G.max_quads, quad_hi - cur.quad - cur.n)};
+    Place nxt = after(cur);
     request(nxt);
-    if (cur.quad < quad_hi) {
-        look(quad_lo);
-        const int n = quads_seen(quad_lo);
-        if (n != cur.n) {                                              // records that came for two quads serve one
-            cur.n = n;
-            if (NB == 0) {                                             // the warps' rows are others
-                cp_async_wait();
-                rem_rows(cur);
-                fetch(n, 0, 0u);
-            }
-            if (leader && !staged) {
-                request(cur);
-                place(cur, 0);
-                if (staged) start_copies(cur, 0);
-            }
-        }
-        Place real{quad_lo, k_lo + 1, n};
-        if (real.k == k_hi) {
-            real = Place{quad_lo + n, k_lo, 1};
-            if (real.quad < quad_hi) real.n = quads_seen(real.quad);
-        }
-        if (real.quad != nxt.quad || real.n != nxt.n) {
-            nxt = real;
-            request(nxt);
-        }
-    }
-    if (kRing && leader) {                                             // all sets of the group, for the warp that fills the X ring
-        int sets = 0;
-        for (Place u{quad_lo, k_lo, 1}; u.quad < quad_hi; sets++) {
-            if (u.quad - seen >= 2 * window) look(u.quad);
-            u.quad += quads_seen(u.quad);
-        }
-        if (lane == 0) posted[3] = sets;
-        if (seen != quad_lo) look(quad_lo);
+    if (kRing && leader) {                                             // for the warp that fills the X ring
+        const int sets = G.max_quads == 2 ? count_sets(L.offsets, L.S, L.M, exp_words, quad_lo, quad_hi, 64u * G.pair_rows) : max(quad_hi - quad_lo, 0);
+        if (lane == 0) all_sets[group] = sets;
     }
     uint32_t prev_foot = staged ? foot : 0u;                           // leader: ring bytes of the unit being decoded
 
@@ -788,7 +766,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         launch_no = *reinterpret_cast<const volatile uint32_t *>(peers.launches) + 1u;
         if (blockIdx.x == 0 && tid < peers.world) red_release_sys_add(pick(peers.ready, tid), 1u);
         // results that are not staged are stored from the first set on: see the end for those that are
-        if (G.direct && tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
+        if (kShard == 2 && tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
     }
     if (NB > 0 && !kRing) {
         const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
@@ -836,7 +814,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
 
     auto keep = [&](int b, int row, float v) {                          // a result of a row-sharded layer
-        if (!G.direct) {
+        if (kShard != 2) {
             ys[b * rows_cta + (row - row_lo)] = f32_to_bf16_rn(v);
         } else {
 #pragma unroll 1
@@ -846,6 +824,10 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
 
     uint32_t phases = 0u;
     int slot = 0;
+    if (cur.quad < quad_hi && !leader) {
+        settle(cur, posted[3]);
+        nxt = after(cur);
+    }
     while (cur.quad < quad_hi) {
         const uint32_t rows = posted[4 * slot], ubase = posted[4 * slot + 1];
         const bool is_staged = posted[4 * slot + 2] != 0u && usable;
@@ -856,8 +838,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             if (staged && !late) start_copies(nxt, slot ^ 1);
             prev_foot = staged ? foot : 0u;
         }
-        const Place nn = after(nxt);
-        request(nn);
+        request(after(nxt));
 
         // the unit with n quads, by decoders of type D
         auto run = [&](auto quads, auto &dec) {
@@ -1001,8 +982,9 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                 }
             }
         }
+        if (nxt.quad < quad_hi && !leader) settle(nxt, posted[4 * (slot ^ 1) + 3]);
         cur = nxt;
-        nxt = nn;
+        nxt = after(nxt);
         slot ^= 1;
     }
 
@@ -1029,7 +1011,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     if (exchange) {
         // one thread asks whether every peer's buffer may be overwritten (an acquire at system scope); the barrier that
         // makes the staged results visible hands its answer to the others
-        if (!G.direct) {
+        if (kShard != 2) {
             if (tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
             asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
             for (int i = tid; i < B * rows_cta; i += kThreads) {
@@ -1062,7 +1044,7 @@ struct GemvForm {
 // the form leaves.  Rows of a layer whose scales differ have records of different lengths: a pair of quads that does not fit
 // together comes quad by quad, and a quad that does not fit alone is decoded from global memory, several times as slow.
 // (4096 x 12288, rANS, one row of X, row scales log-normal with sigma 0.35: 177 us without the growth and the quads, 42 with
-// them, as with equal rows; 12288 x 4096, limit6, four rows: 76 and 30.  Equal rows pay 0 to 0.7 us for the look.)
+// them, as with equal rows; 12288 x 4096, limit6, four rows: 76 and 30.)
 static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool stage_results,
                       GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
@@ -1119,11 +1101,11 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     return true;
 }
 
-template <class Dec, int NB, int NG, bool kRing>
-static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+template <class Dec, int NB, int NG, bool kRing, int kShard>
+static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
                       cudaStream_t st) {
-    auto kernel = gemv_kernel<Dec, NB, NG, kRing>;
+    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard>;
     if (int rc = staged_prepare(kernel)) return rc;
     PeerSet ps{};
     if (peers) ps = *peers;
@@ -1141,6 +1123,19 @@ static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, co
     const GemvConsts k{bits, (1u << bits) - 1u, bits == 12u ? 0xFFFu : (2u << bits) - 1u, 8u, Dec::kTableBytes >> bits};
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, L, targs, prepared, X, bias, Y, ps, G, k);
     return e == cudaSuccess ? BHI_OK : cuda_fail(e, "gemv kernel launch");
+}
+
+template <class Dec, int NB, int NG, bool kRing>
+static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, bool direct, int grid, const GemvGeom &G,
+                      uint32_t smem_bytes, cudaStream_t st) {
+    if constexpr (NB == 1) {
+        if constexpr (kRing) {
+            if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+        }
+        if (peers) return gemv_start_as<Dec, NB, NG, kRing, 1>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+    }
+    return gemv_start_as<Dec, NB, NG, kRing, 0>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
 }
 
 // The first form that fits, best first.  Measured on 12288 x 4096, limit6, in us where each fits with one, four, eight rows:
@@ -1165,24 +1160,24 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
             if (only && f.groups != only) continue;
             if (!kLast && (f.quads < 2 || f.x == GemvX::ring)) break;
             if (peers != nullptr && !direct && f.quarters == 0) continue;           // staged records before staged results
+            if (direct && f.x != GemvX::ring) continue;                            // so many rows that X hardly counts
             if (NB > 1 && (f.x == GemvX::resident || f.groups == 2)) continue;     // more than eight rows hardly ever fit
             int grid = sm_count() * f.per_sm;
             if (grid > nquads) grid = nquads;
             GemvGeom G{};
             uint32_t smem_bytes = 0;
             if (!gemv_plan(L, B, Dec::kTableBytes, NB, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
-            G.direct = direct;
             if (f.x == GemvX::ring) {
                 if constexpr (NB > 0 && kLast) {
                     if constexpr (NB == 1) {
-                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
                     }
-                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
                 }
             } else {
                 if constexpr (NB <= 1) {
-                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
-                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
                 }
             }
         }

@@ -10,7 +10,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("algo,tables", [("huffman", "limit6"), ("huffman", "escape"), ("huffman", "reference"), ("ans", None)])
-@pytest.mark.parametrize("M,K", [(1021, 4096), (302, 12288), (2045, 5120), (262, 18944)])
+@pytest.mark.parametrize("M,K", [(1021, 4096), (302, 12288), (2045, 5120), (262, 18944), (150, 28672), (9001, 1536)])
 @pytest.mark.parametrize("sigma", [0.35, 0.8, 2.5])
 def test_rows_of_different_scale(algo, tables, M, K, sigma):
     from bf16_huffman_infer_b200 import ANSWeight, CompressedLinear, HuffmanWeight, set_huffman_tables
