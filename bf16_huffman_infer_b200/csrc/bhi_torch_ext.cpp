@@ -234,7 +234,7 @@ ForwardCall forward_of(StableIValue *stack, const Tensor &X, const Tensor &rem, 
     if (bias.has_value()) {
         want(*bias, ScalarType::BFloat16, "bias");
         same_device(rem, *bias, "bias");
-        STD_TORCH_CHECK(bias->numel() == v.M, "bias must have M entries");
+        STD_TORCH_CHECK(bias->dim() == 1 && bias->numel() == v.M, "bias must be a vector of M entries");
         bias_ptr = ptr<const uint16_t>(*bias);
     }
     return {v, output_like(X, v.M), static_cast<int>(B), bias_ptr};

@@ -606,8 +606,12 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
             input = input.contiguous()
         if bias is None:
             return weight._forward(input, None)
-        if _takes_bias(weight, bias, input) and not (bias.requires_grad and torch.is_grad_enabled()) and not _transformed():
-            return weight._forward(input, bias)
+        if _takes_bias(bias, input) and not (bias.requires_grad and torch.is_grad_enabled()) and not _transformed():
+            try:
+                return weight._forward(input, bias)
+            except RuntimeError:                     # nothing was launched; asked afterwards, the shape costs nothing here
+                if _is_row(weight, bias):
+                    raise
         output = weight._forward(input.flatten(0, -2), None)
         output += bias[None, :]
         return output.unflatten(0, input.shape[:-1])
@@ -625,10 +629,14 @@ def _linear_compressed(input: Tensor, weight: HuffmanWeight, bias: Optional[Tens
     return output.unflatten(0, shape[:-1])
 
 
-def _takes_bias(weight: HuffmanWeight, bias: Tensor, input: Tensor) -> bool:
-    """Whether the operators take the bias as it is; others (one value for all outputs, another type) are torch's to add."""
-    return (bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
-            and bias.shape == weight.__dict__["_buffers"]["rem"].shape[1:2])
+def _takes_bias(bias: Tensor, input: Tensor) -> bool:
+    """Whether the operators take the bias as it is, its shape aside; others are torch's to add."""
+    return bias.dtype == torch.bfloat16 and bias.device == input.device and bias.is_contiguous()
+
+
+def _is_row(weight: HuffmanWeight, bias: Tensor) -> bool:
+    """A value for each output, which the operators want; torch's addition also takes one for all."""
+    return bias.shape == weight.__dict__["_buffers"]["rem"].shape[1:2]
 
 
 def _transformed() -> bool:
@@ -643,7 +651,7 @@ def _takes_more_rows(input: Tensor, weight: HuffmanWeight, bias: Optional[Tensor
         return False
     if _transformed() or torch._C._get_tracing_state() is not None:
         return False
-    if bias is not None and not _takes_bias(weight, bias, input):
+    if bias is not None and not (_takes_bias(bias, input) and _is_row(weight, bias)):
         return False
     return not (torch.is_grad_enabled() and (input.requires_grad or (bias is not None and bias.requires_grad)))
 
