@@ -1215,6 +1215,11 @@ constexpr int kGemvMaxRows = 32;
 
 // B rows of X (0: the dense matrix into Y).  pair_complete: the caller knows that no code of the prepared table is longer
 // than 6 bits; only a tuning hint, the kernel reads from the table header whether it is so.
+// The larger table first, where it leaves room for the favourable forms, although its CTAs then have an SM to themselves; one
+// row of X, in us, with the larger / only the smaller table:
+//                           1024 x 4096   4096 x 4096   12288 x 4096   4096 x 12288   5120 x 5120
+//   pair table, 14 / 13 bits    8.4 / 8.8   14.7 / 16.1    34.9 / 37.1    35.5 / 37.7   25.4 / 23.5   (escape)
+//   rANS, 8 bits, 64 / 32 KB    9.4 / 9.2   17.1 / 19.4    43.3 / 50.0    42.5 / 52.5   30.0 / 30.9
 template <class Codec>
 static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                        const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {

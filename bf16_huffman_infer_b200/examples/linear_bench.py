@@ -1,8 +1,8 @@
 """The two branches for more than 8 activation rows, one layer at a time.
 
-For each layer shape and row count: the fused decode + tensor-core product (``mm_huffman_prepared`` / ``mm_ans``,
-what ``BHI_TENSOR_ROWS`` turns on) against decode-to-dense followed by ``torch.matmul`` (the default branch, as in
-the reference, ``functional.py:405-407``).  Timed on the device over enough distinct copies of the layer to exceed
+For each layer shape and row count: the fused decode + product (``mm_huffman_prepared`` / ``mm_ans``: up to 32 rows the
+kernel that layers take by default, beyond, what ``BHI_TENSOR_ROWS`` turns on) against decode-to-dense followed by
+``torch.matmul`` (the default branch beyond 32 rows, as in the reference, ``functional.py:405-407``).  Timed on the device over enough distinct copies of the layer to exceed
 L2, replayed from a CUDA graph::
 
     python -m bf16_huffman_infer_b200.examples.linear_bench [--shapes 4096x4096,12288x4096,4096x12288]
