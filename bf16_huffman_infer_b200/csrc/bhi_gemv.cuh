@@ -126,6 +126,18 @@ struct Cursor {
         bit = next;
     }
 };
+// A cursor that is moved by whole table entries: the address of the word row it stands in, and the bit.  Only the low seven bits
+// of `bit` count, the symbols of the entries may stand above them.  No step is longer than a row, so the row changes when bit 5
+// does.  Two integer instructions per four symbols less than a cursor in bits alone (49152 x 4096: 93.6 us with that, 92.7 so);
+// pair tables, whose flagged entries move a cursor in parts, gained nothing (6144 x 2048, reference tables: 16.9 and 17.1 us).
+struct Cursor {
+    uint32_t at, bit;
+    __device__ __forceinline__ uint32_t window() const { return __funnelshift_r(lds_table<0>(at), lds_table<256>(at), bit); }
+    __device__ __forceinline__ void step(const GemvCtx &c, uint32_t next) {
+        at = umad((next ^ bit) & 32u, c.k.eight, at);
+        bit = next;
+    }
+};
 // Ring words change between records.  Their loads are free to move among each other, but what they depend on passes
 // through here, after the wait for the record's copies, so they cannot move before it.
 __device__ __forceinline__ void keep_order(uint32_t &a, uint32_t &b) { asm volatile("" : "+r"(a), "+r"(b)::"memory"); }
@@ -514,10 +526,12 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
 // X or tables two CTAs could not both hold.  kRing: X passes through a ring that one more warp fills and all groups read in
 // step.  (20 warps of 96 registers instead of 16 gain nothing: it is pipes that are short, not warps.)
+// kHalf: two groups, and no more CTAs than SMs, so that half of each SM is the next kernel's: it has its tables and records by
+// the time this one ends.  For launches so small that latencies, not the pipes, set their time (see kHalfUnits).
 // kShard: a layer whose rows are shared among ranks (1: results staged, 2: stored one by one).  An argument of the template,
 // because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
 // layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
-template <class Dec, int NB, int NG, bool kRing, int kShard>
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf>
 __global__ void __launch_bounds__(NG * kGemvWarps * 32 + (kRing ? 32 : 0), NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
             PeerSet peers, GemvGeom G, GemvConsts kc) {
@@ -575,7 +589,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     if (tid == 0) {
         for (uint32_t i = 0; i < 2u * NG; i++) mbar_init(ctrl_at + 8u * i, 1);
         mbar_init(table_bar, 1);
-        mbar_init(x_bar, 1);
+        mbar_init(x_bar, kHalf ? NG * kGemvWarps : 1);
         for (uint32_t i = 0; kRing && i < kXSlotsMax; i++) {
             mbar_init(x_full + 8u * i, 1);
             mbar_init(x_empty + 8u * i, NG * kGemvWarps);
@@ -773,7 +787,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     }
 
     // Everything above read weights only.  X (and Y) belong to the previous kernel in the stream.
-    pdl_wait();
+    if (!kHalf) pdl_wait();
     uint32_t launch_no = 0;
     if (exchange) {
         launch_no = *reinterpret_cast<const volatile uint32_t *>(peers.launches) + 1u;
@@ -781,7 +795,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         // results that are not staged are stored from the first set on: see the end for those that are
         if (kShard == 2 && tid == 0 && !counter_wait_bounded(pick(peers.ready, peers.rank), launch_no * peers.world)) atomicExch(&g_staged_status, 8);
     }
-    if (NB > 0 && !kRing) {
+    if (NB > 0 && !kRing && !kHalf) {
         const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
         const uint32_t bytes = static_cast<uint32_t>(L.S) * L.Nc * 2u;
         if (tid == 0 && bulk) mbar_expect_tx(x_bar, bytes * B);
@@ -791,7 +805,24 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (!bulk && tid == 0) mbar_arrive(x_bar);
     }
     __syncthreads();
-    if (NB > 0 && !kRing && !mbar_wait_bounded(x_bar, 0u) && tid == 0) atomicExch(&g_staged_status, 3);
+    if (NB > 0 && !kRing && !kHalf && !mbar_wait_bounded(x_bar, 0u) && tid == 0) atomicExch(&g_staged_status, 3);
+
+    // Beside the previous kernel: its end is waited for, and X fetched, when the records of the first unit are here and those
+    // of the second on their way.
+    bool x_asked = false;
+    auto ask_for_x = [&]() {
+        x_asked = true;
+        pdl_wait();
+        const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
+        const uint32_t bytes = static_cast<uint32_t>(L.S) * L.Nc * 2u;
+        if (bulk && tid == 0) mbar_expect_tx_only(x_bar, bytes * B);
+        __syncwarp();
+        if (!bulk || warp == 0)
+            for (int b = bulk ? lane : warp; b < B; b += bulk ? 32 : NG * kGemvWarps)
+                copy_x_row(xs + b * G.x_pitch, X + static_cast<int64_t>(b) * L.S * L.Nc, bytes, x_bar, bulk, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(x_bar);
+    };
 
     // ---- decode and multiply -------------------------------------------------------------------------------------------
     float c[2][kAcc][4];
@@ -852,6 +883,11 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             prev_foot = staged ? foot : 0u;
         }
         request(after(nxt));
+        if (kHalf && !x_asked) {
+            if (is_staged && !mbar_wait_bounded(bar0 + 8u * slot, (phases >> slot) & 1u) && lane == 0) atomicExch(&g_staged_status, 1);
+            ask_for_x();
+            if (!mbar_wait_bounded(x_bar, 0u) && lane == 0) atomicExch(&g_staged_status, 3);
+        }
 
         // the unit with n quads, by decoders of type D
         auto run = [&](auto quads, auto &dec) {
@@ -1001,6 +1037,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         slot ^= 1;
     }
 
+    if (kHalf && !x_asked) ask_for_x();       // a group without units copies its share of an unaligned X
     if (NB == 1 && split) {                   // the groups' sums, in the order of their chunks
         asm volatile("bar.sync 5, %0;" ::"n"(kThreads) : "memory");
         for (int i = warp; i < cta_hi - cta_lo; i += NG * kGemvWarps) {
@@ -1114,11 +1151,11 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     return true;
 }
 
-template <class Dec, int NB, int NG, bool kRing, int kShard>
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf>
 static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
                       cudaStream_t st) {
-    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard>;
+    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf>;
     if (int rc = staged_prepare(kernel)) return rc;
     PeerSet ps{};
     if (peers) ps = *peers;
@@ -1144,11 +1181,11 @@ static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, co
                       uint32_t smem_bytes, cudaStream_t st) {
     if constexpr (NB == 1) {
         if constexpr (kRing) {
-            if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+            if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
         }
-        if (peers) return gemv_start_as<Dec, NB, NG, kRing, 1>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+        if (peers) return gemv_start_as<Dec, NB, NG, kRing, 1, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
     }
-    return gemv_start_as<Dec, NB, NG, kRing, 0>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+    return gemv_start_as<Dec, NB, NG, kRing, 0, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
 }
 
 // The first form that fits, best first.  Measured on 12288 x 4096, limit6, in us where each fits with one, four, eight rows:
@@ -1198,6 +1235,30 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
     return kStagedDeclined;
 }
 
+// The kHalf launch of a small layer, in half an SM's shared memory.
+template <class Dec>
+static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+                            const uint16_t *bias, uint16_t *Y, int B, cudaStream_t st) {
+    const int nquads = (L.M + 3) / 4, grid = nquads < sm_count() ? nquads : sm_count();
+    for (int quarters = 8; quarters >= 4; quarters -= 4) {             // two units in the ring, or the one that most groups have
+        GemvGeom G{};
+        uint32_t smem_bytes = 0;
+        if (gemv_plan(L, B, Dec::kTableBytes, 1, GemvForm{2, 2, 2, quarters, GemvX::resident}, grid, false, G, smem_bytes))
+            return gemv_start_as<Dec, 1, 2, false, 0, true>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st);
+    }
+    return kStagedDeclined;
+}
+
+// Layers of up to this many quads per SM, counting each of their chunks, take half of each SM: a unit of two quads, or two of
+// one, for each of an SM's two groups.  One row of X, back to back in a graph, in us, the other forms / half an SM:
+//   limit6   512 x 2048  4.1/3.7   1024 x 4096  6.3/5.5   2048 x 2048  5.7/4.4   2368 x 2048  5.9/4.5   2368 x 4096  8.3/7.0
+//            1024 x 6144 (two chunks)  6.5/5.8; beyond the line  4096 x 2048  7.3/7.7   2048 x 6144  9.1/10.3   4096 x 4096  11.2/12.7
+//   rANS     512 x 3584  7.6/6.8   1024 x 4096  9.2/8.0   2048 x 2048  7.6/6.2   2048 x 4096  11.5/11.1
+// More than two chunks are divided among four groups instead (512 x 18944: 9.1/12.9, 512 x 12288: 11.1/10.5).  Pair tables of
+// 14 bits leave no room beside themselves and of 13 gain only where a group has one quad at most and often not then
+// (1024 x 1024 escape 4.2/3.8, 1024 x 4096 8.2/8.1, 512 x 2048 reference 6.0/6.3, 2048 x 2048 8.4/9.7), so they stay out.
+constexpr int kHalfUnits = 4, kHalfChunks = 2;
+
 // kLast: no other decoder is tried after this one, so it takes the less favourable forms too.  kMore: more than eight rows.
 template <class Dec, bool kLast, bool kMore>
 static int gemv_launch_rows(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
@@ -1238,7 +1299,13 @@ static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const 
                        const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16) || B > kGemvMaxRows) return kStagedDeclined;
     if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31) || L.exp_words >= (1ll << 32)) return kStagedDeclined;
+    const bool half = B >= 1 && B <= 8 && peers == nullptr && gemv_groups() == 0 && L.S <= kHalfChunks &&
+                      L.S * ((L.M + 3ll) / 4) <= static_cast<int64_t>(kHalfUnits) * sm_count();
     if constexpr (std::is_same<Codec, HuffCodec>::value) {
+        if (half && pair_complete) {
+            const int rc = gemv_launch_half<GemvSingle>(L, targs, prepared, X, bias, Y, B, st);
+            if (rc != kStagedDeclined) return rc;
+        }
         if (prepared == nullptr) return gemv_launch_rows<GemvPair<kPairBits>, true, false>(L, targs, prepared, X, bias, Y, peers, B, st);
         if (pair_complete) return gemv_launch_rows<GemvSingle, true, true>(L, targs, prepared, X, bias, Y, peers, B, st);
         const int rc = gemv_launch_rows<GemvPair<kWidestBits>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
@@ -1247,6 +1314,9 @@ static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const 
     } else {
         // (a finer model on a layer of at most a quad per group: filling the larger table costs more than its conflicts)
         int rc = kStagedDeclined;
+        if (half && targs.bits == 8) rc = gemv_launch_half<GemvAns<true, 64 * 1024>>(L, targs, prepared, X, bias, Y, B, st);
+        if (half && rc == kStagedDeclined) rc = gemv_launch_half<GemvAns<false, 32 * 1024>>(L, targs, prepared, X, bias, Y, B, st);
+        if (rc != kStagedDeclined) return rc;
         if (targs.bits == 8) rc = gemv_launch_rows<GemvAns<true, 64 * 1024>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
         else if (L.M > 16 * sm_count()) rc = gemv_launch_rows<GemvAns<false, 64 * 1024>, false, false>(L, targs, prepared, X, bias, Y, peers, B, st);
         if (rc != kStagedDeclined) return rc;

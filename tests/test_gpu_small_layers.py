@@ -1,0 +1,99 @@
+"""Layers at the edges of the launch forms for small layers (half of each SM, one or two chunks) and of the product forms (up to
+four rows of X, up to eight), against a double-precision product of the decoded weights."""
+import ctypes
+
+import pytest
+import torch
+
+from _util import Abi, make_input, make_weight, rel_err
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _weight(algo, W, bits=8):
+    from bf16_huffman_infer_b200 import ANSWeight, HuffmanWeight, set_ans_precision
+    previous = set_ans_precision(bits)
+    try:
+        return (ANSWeight if algo == "ans" else HuffmanWeight).compress(W.to(DEV), to_cpu=False)
+    finally:
+        set_ans_precision(previous)
+
+
+@pytest.mark.parametrize("algo,bits", [("huffman", 8), ("ans", 8), ("ans", 12)])
+@pytest.mark.parametrize("M,K", [(1, 1024), (5, 1152), (593, 1024), (1184, 2048), (1185, 2048), (2365, 1024), (2368, 4096), (2372, 1024),
+                                 (591, 6144), (1184, 6144), (1185, 6144), (300, 12288)])
+def test_edges_of_small_layers(algo, bits, M, K):
+    abi, status = Abi(), ctypes.c_int(-1)
+    abi.check(abi.lib.bhi_debug_status(ctypes.byref(status)))            # what earlier calls left
+    W = make_weight(M, K, M).to(DEV)
+    weight = _weight(algo, W, bits)
+    bias = make_input(1, M, 3).flatten().to(DEV)
+    for rows in (1, 2, 3, 4, 5, 8):
+        x = make_input(rows, K, rows).to(DEV)
+        ref = (x.double() @ W.double().T).cpu().numpy()
+        aside = torch.cat([x.flatten()[:2], x.flatten()])[2:].view(rows, K)          # 4-byte aligned only: X is copied by loads
+        for given in (x, aside):
+            y = weight._forward(given, None)
+            assert rel_err(y.float().cpu().numpy(), ref) <= 1e-2, rows
+            assert torch.equal(y, weight._forward(given, None))
+        # a bias is added to the rounded product and rounded again, as torch adds it
+        assert torch.equal(weight._forward(x, bias), y + bias)
+    abi.check(abi.lib.bhi_debug_status(ctypes.byref(status)))
+    assert status.value == 0
+
+
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+def test_chains_of_small_layers(algo):
+    """Each layer reads what the one before it wrote, while its own tables and records arrive beside that one: eagerly, in a
+    graph, and with the launches of another stream in between."""
+    from bf16_huffman_infer_b200 import CompressedLinear
+    K, depth = 1024, 12
+    layers = []
+    for i in range(depth):
+        layers.append(CompressedLinear(_weight(algo, make_weight(K, K, i, 1.0 / 32).to(DEV)), None))
+    x = make_input(2, K, 9).to(DEV)
+
+    def chain():
+        out = [x]
+        for layer in layers:
+            out.append(layer(out[-1]))
+        return out
+
+    with torch.no_grad():
+        want = chain()
+        torch.cuda.synchronize()
+        for got, layer, y in zip(want, layers, want[1:]):
+            ref = got.double() @ layer.weight.get_weight().double().T
+            assert rel_err(y.float().cpu().numpy(), ref.cpu().numpy()) <= 1e-2
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            again = chain()
+        again_here = chain()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            replayed = chain()
+        for y in replayed[1:]:
+            y.zero_()
+        for _ in range(5):
+            graph.replay()
+        torch.cuda.synchronize()
+    for a, b, c, d in zip(want, again, again_here, replayed):
+        assert torch.equal(a, b) and torch.equal(a, c) and torch.equal(a, d)
+
+
+@pytest.mark.parametrize("sigma", [0.8, 2.5])
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+def test_small_layers_of_uneven_rows(algo, sigma):
+    """Records too long for the ring of half an SM come quad by quad or from global memory."""
+    for M, K in ((700, 4096), (2300, 3584)):
+        W = (make_weight(M, K, 1).float() * torch.exp(sigma * torch.randn(M, 1, generator=torch.Generator().manual_seed(M)))).bfloat16().to(DEV)
+        weight = _weight(algo, W)
+        for rows in (1, 4, 8):
+            x = make_input(rows, K, rows).to(DEV)
+            ref = x.double() @ W.double().T
+            scale = ref.abs().amax(0, keepdim=True).clamp(min=1e-30)               # row by row, so that small rows count as much
+            y = weight._forward(x, None).double()
+            assert rel_err((y / scale).cpu().numpy(), (ref / scale).cpu().numpy()) <= 1e-2, rows
