@@ -126,18 +126,6 @@ struct Cursor {
         bit = next;
     }
 };
-// A cursor that is moved by whole table entries: the address of the word row it stands in, and the bit.  Only the low seven bits
-// of `bit` count, the symbols of the entries may stand above them.  No step is longer than a row, so the row changes when bit 5
-// does.  Two integer instructions per four symbols less than a cursor in bits alone (49152 x 4096: 93.6 us with that, 92.7 so);
-// pair tables, whose flagged entries move a cursor in parts, gained nothing (6144 x 2048, reference tables: 16.9 and 17.1 us).
-struct Cursor {
-    uint32_t at, bit;
-    __device__ __forceinline__ uint32_t window() const { return __funnelshift_r(lds_table<0>(at), lds_table<256>(at), bit); }
-    __device__ __forceinline__ void step(const GemvCtx &c, uint32_t next) {
-        at = umad((next ^ bit) & 32u, c.k.eight, at);
-        bit = next;
-    }
-};
 // Ring words change between records.  Their loads are free to move among each other, but what they depend on passes
 // through here, after the wait for the record's copies, so they cannot move before it.
 __device__ __forceinline__ void keep_order(uint32_t &a, uint32_t &b) { asm volatile("" : "+r"(a), "+r"(b)::"memory"); }
