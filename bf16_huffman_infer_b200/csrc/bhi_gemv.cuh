@@ -35,7 +35,8 @@ constexpr int kGemvWarps = 4;                 // warps of a group
 constexpr int kRG = 4;                        // blocks per chunk of the sign/mantissa rows, and per segment of the X ring
 constexpr uint32_t kRemChunk = 1024;          // bytes of a chunk: four blocks, eight rows, 32 bytes of a pass
 constexpr uint32_t kXSegCols = 128 * kRG;
-constexpr uint32_t kXPad = 16;                // bytes between rows of X: eight rows of a fragment lie on different banks
+constexpr int kFewRows = 4;                    // most rows of X that can be the eight B columns of a product, twice
+constexpr uint32_t kXPad = 16;                // bytes between rows of X (twice that for few rows): what one wavefront reads lies on different banks
 constexpr int kXSlotsMax = 4;                 // most segments of the X ring
 constexpr int kGemvCtrlBytes = 512;           // mbarriers, unit descriptors
 constexpr uint32_t kTableAt = 1024;           // where dynamic shared memory starts in the CTA's window (the system's share lies below)
@@ -78,6 +79,10 @@ template <uint32_t kOffset>
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&v)[4], uint32_t a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4+%5];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a), "n"(kOffset) : "memory");
+}
+template <uint32_t kOffset>
+__device__ __forceinline__ void ldmatrix_x2(uint32_t (&v)[2], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2+%3];" : "=r"(v[0]), "=r"(v[1]) : "r"(a), "n"(kOffset) : "memory");
 }
 // 16 bytes, or (bytes = 0) zeros without reading the source
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint32_t bytes) {
@@ -516,10 +521,14 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // step.  (20 warps of 96 registers instead of 16 gain nothing: it is pipes that are short, not warps.)
 // kHalf: two groups, and no more CTAs than SMs, so that half of each SM is the next kernel's: it has its tables and records by
 // the time this one ends.  For launches so small that latencies, not the pipes, set their time (see kHalfUnits).
+// kFew: at most four rows of X.  The weights are then the sixteen A rows (row r and half s of either quad) and X the eight B
+// columns (half s, X row b): one product instead of two serves both quads of a block, and a fragment of X takes two wavefronts
+// of shared memory instead of four.  Of the products those of equal halves count, (r, s) x (s, b); their sum over s is the
+// result.  (One row: 49152 x 4096 limit6 92.9 us, so 90.4, rANS 151.0, 146.8; 12288 x 4096 escape 34.5, 33.8.)
 // kShard: a layer whose rows are shared among ranks (1: results staged, 2: stored one by one).  An argument of the template,
 // because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
 // layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
-template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf>
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew>
 __global__ void __launch_bounds__(NG * kGemvWarps * 32 + (kRing ? 32 : 0), NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
             PeerSet peers, GemvGeom G, GemvConsts kc) {
@@ -557,7 +566,9 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     GemvCtx ctx;
     ctx.exact = reinterpret_cast<const HuffTables *>(&tab);
     ctx.k = kc;
-    ctx.lane_table = kHuff ? 4u * lane : (8u * lane) & (kc.entry - 1u);
+    // (through a shuffle, which cannot be computed anew: without it the compiler put that into every lookup of the limit6 form
+    // for few rows, 4 instructions more per 128 weights)
+    ctx.lane_table = __shfl_sync(0xFFFFFFFFu, kHuff ? 4u * lane : (8u * lane) & (kc.entry - 1u), lane);
 
     // Quads are dealt to the groups of the grid in equal contiguous ranges; a group takes them two at a time.
     const int nquads = (L.M + 3) >> 2;
@@ -822,11 +833,13 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     clear();
     // ldmatrix: lane i supplies the address of row i % 8 of matrix i / 8: pairs 8j.., 8j + 4.., 32 + 8j.., 32 + 8j + 4.. of a
-    // block.  Rows past the batch repeat the last one; their products are never read.
+    // block.  Rows past the batch repeat the last one; their products are never read.  Few rows: two matrices, rows 0..3 of pairs
+    // 8j.. and 0..3 of pairs 8j + 4.., and the same of pairs 32 + 8j.. .
     uint32_t x_row[kAcc];
 #pragma unroll
     for (int g = 0; g < kAcc; g++)
-        x_row[g] = xs + min(8 * g + (lane & 7), max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 3) & 1) + 128u * (lane >> 4);
+        x_row[g] = kFew ? xs + min(lane & 3, max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 2) & 1) + 128u * ((lane >> 3) & 1)
+                        : xs + min(8 * g + (lane & 7), max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 3) & 1) + 128u * (lane >> 4);
     const int x_total = kRing ? x_segments() : 0;
     int x_slot = 0, x_seg = 0;
     uint32_t x_phase = 0u;
@@ -907,7 +920,12 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                             w0[q] = bitselect(prmt(w, 0u, 0x1100u), e[q][i][0], kRemMask);
                             w1[q] = bitselect(prmt(w, 0u, 0x3322u), e[q][i][1], kRemMask);
                         }
-                        if (NB > 0) {
+                        if constexpr (kFew) {
+                            uint32_t f[2];
+                            if (i == 0) ldmatrix_x2<j * 256u>(f, x_row[0] + xa);
+                            else ldmatrix_x2<j * 256u + 256u>(f, x_row[0] + xa);
+                            mma_bf16_16x8x16(c[0][0], w0[0], n > 1 ? w0[n - 1] : 0u, w1[0], n > 1 ? w1[n - 1] : 0u, f[0], f[1]);
+                        } else if constexpr (NB > 0) {
 #pragma unroll
                             for (int g = 0; g < kAcc; g++) {
                                 uint32_t f[4];
@@ -994,9 +1012,18 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (NB > 0 && set_done) {
             gemv_group_barrier(group);        // the previous set's partial sums have been read
 #pragma unroll
-            for (int q = 0; q < 2; q++)
+            for (int q = 0; q < 2; q++) {
+                if constexpr (kFew) {         // row r of the quad and X rows 2 (t % 2) and the next, of half s where the columns are that half's
+                    if ((t >> 1) == (gq & 1)) {
+                        float *pp = part + (wig * 2 + q) * 32 + 16 * (gq & 1) + 8 * (t & 1) + r;
+                        pp[0] = c[0][0][2 * q];
+                        pp[4] = c[0][0][2 * q + 1];
+                    }
+                } else {
 #pragma unroll
-                for (int g = 0; g < kAcc; g++) part[((wig * 2 + q) * kAcc + g) * 32 + lane] = c[q][g][0] + c[q][g][3];
+                    for (int g = 0; g < kAcc; g++) part[((wig * 2 + q) * kAcc + g) * 32 + lane] = c[q][g][0] + c[q][g][3];
+                }
+            }
             clear();
         }
         gemv_group_barrier(group);            // the unit's ring space is free; partial sums and the next unit's place are visible
@@ -1004,10 +1031,10 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         if (NB > 0 && set_done) {
             for (int z = wig; z < n * kAcc; z += kGemvWarps) {          // warp z % 4 finishes (quad, eight X rows) z
                 const int q = z / kAcc, g = z % kAcc;
-                const float *pp = part + (q * kAcc + g) * 32 + lane;
-                float v = pp[0];
+                const float *pp = part + (q * kAcc + g) * 32 + (kFew ? lane & 15 : lane);
+                float v = kFew ? pp[0] + pp[16] : pp[0];
 #pragma unroll
-                for (int w = 1; w < kGemvWarps; w++) v += pp[w * 64 * kAcc];
+                for (int w = 1; w < kGemvWarps; w++) v += kFew ? pp[w * 64 * kAcc] + pp[w * 64 * kAcc + 16] : pp[w * 64 * kAcc];
                 const int row = 4 * (cur.quad + q) + t, b = 8 * g + gq;
                 if (split) {
                     acc[((cur.quad + q - cta_lo) * NG + group) * 32 + lane] = v;
@@ -1083,8 +1110,8 @@ struct GemvForm {
 // together comes quad by quad, and a quad that does not fit alone is decoded from global memory, several times as slow.
 // (4096 x 12288, rANS, one row of X, row scales log-normal with sigma 0.35: 177 us without the growth and the quads, 42 with
 // them, as with equal rows; 12288 x 4096, limit6, four rows: 76 and 30.)
-static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, const GemvForm &f, int grid, bool stage_results,
-                      GemvGeom &G, uint32_t &smem_bytes) {
+static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_groups, bool few, const GemvForm &f, int grid,
+                      bool stage_results, GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
     const uint32_t cap = f.per_sm == 2 ? kSmemMax / 2 - 512 : kSmemMax;
     const int64_t per_row = 64 * static_cast<int64_t>(L.S) * L.M;
@@ -1115,7 +1142,7 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     G.x_slots = 0;
     G.x_pitch = G.x_slot = 0;
     if (f.x == GemvX::resident) {
-        const uint64_t pitch = static_cast<uint64_t>(L.S) * L.Nc * 2u + kXPad;
+        const uint64_t pitch = static_cast<uint64_t>(L.S) * L.Nc * 2u + (few ? 2u : 1u) * kXPad;
         x_bytes = pitch * B;
         G.x_pitch = static_cast<uint32_t>(pitch);
     } else if (f.x == GemvX::ring) {
@@ -1139,11 +1166,11 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     return true;
 }
 
-template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf>
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew>
 static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
                       cudaStream_t st) {
-    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf>;
+    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf, kFew>;
     if (int rc = staged_prepare(kernel)) return rc;
     PeerSet ps{};
     if (peers) ps = *peers;
@@ -1165,15 +1192,18 @@ static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs,
 
 template <class Dec, int NB, int NG, bool kRing>
 static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
-                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, bool direct, int grid, const GemvGeom &G,
+                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, bool direct, bool few, int grid, const GemvGeom &G,
                       uint32_t smem_bytes, cudaStream_t st) {
     if constexpr (NB == 1) {
         if constexpr (kRing) {
-            if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+            if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2, false, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
         }
-        if (peers) return gemv_start_as<Dec, NB, NG, kRing, 1, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+        if (peers) return gemv_start_as<Dec, NB, NG, kRing, 1, false, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+        if constexpr (!kRing) {
+            if (few) return gemv_start_as<Dec, NB, NG, kRing, 0, false, true>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+        }
     }
-    return gemv_start_as<Dec, NB, NG, kRing, 0, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
+    return gemv_start_as<Dec, NB, NG, kRing, 0, false, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
 }
 
 // The first form that fits, best first.  Measured on 12288 x 4096, limit6, in us where each fits with one, four, eight rows:
@@ -1204,18 +1234,19 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
             if (grid > nquads) grid = nquads;
             GemvGeom G{};
             uint32_t smem_bytes = 0;
-            if (!gemv_plan(L, B, Dec::kTableBytes, NB, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
+            const bool few = NB == 1 && B <= kFewRows && peers == nullptr && f.x == GemvX::resident;
+            if (!gemv_plan(L, B, Dec::kTableBytes, NB, few, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
             if (f.x == GemvX::ring) {
                 if constexpr (NB > 0 && kLast) {
                     if constexpr (NB == 1) {
-                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
+                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
                     }
-                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
                 }
             } else {
                 if constexpr (NB <= 1) {
-                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
-                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, direct, grid, G, smem_bytes, st);
+                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
                 }
             }
         }
@@ -1231,8 +1262,9 @@ static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &tar
     for (int quarters = 8; quarters >= 4; quarters -= 4) {             // two units in the ring, or the one that most groups have
         GemvGeom G{};
         uint32_t smem_bytes = 0;
-        if (gemv_plan(L, B, Dec::kTableBytes, 1, GemvForm{2, 2, 2, quarters, GemvX::resident}, grid, false, G, smem_bytes))
-            return gemv_start_as<Dec, 1, 2, false, 0, true>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st);
+        if (gemv_plan(L, B, Dec::kTableBytes, 1, B <= kFewRows, GemvForm{2, 2, 2, quarters, GemvX::resident}, grid, false, G, smem_bytes))
+            return B <= kFewRows ? gemv_start_as<Dec, 1, 2, false, 0, true, true>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st)
+                                 : gemv_start_as<Dec, 1, 2, false, 0, true, false>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st);
     }
     return kStagedDeclined;
 }
