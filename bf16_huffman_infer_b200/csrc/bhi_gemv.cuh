@@ -694,9 +694,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             if (__any_sync(0xFFFFFFFFu, longer)) u.n = 1;
         }
         uint32_t rows = fits && lane < 4 * u.n ? words >> 6 : 0u;
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
-        rows = __shfl_sync(0xFFFFFFFFu, rows, 0);
+        rows = __reduce_max_sync(0xFFFFFFFFu, rows);
         foot = (4u * u.n * (rows * 256u + 32u) + 255u) & ~255u;
         staged = __all_sync(0xFFFFFFFFu, fits || lane >= 4 * u.n) && foot <= G.ring_bytes;
         base = slot == 0 ? ring : ring + G.ring_bytes - foot;
@@ -710,12 +708,8 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     auto start_copies = [&](const Place &u, int slot) {
         const uint32_t bar = bar0 + 8u * slot;
         const int n = u.n;
-        uint32_t total = lane < 4 * n ? words * 4u : 0u, rows = lane < 4 * n ? words >> 6 : 0u;
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
-            rows = max(rows, __shfl_xor_sync(0xFFFFFFFFu, rows, o));
-        }
+        const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, lane < 4 * n ? words * 4u : 0u);
+        const uint32_t rows = __reduce_max_sync(0xFFFFFFFFu, lane < 4 * n ? words >> 6 : 0u);
         if (lane == 0) mbar_expect_tx(bar, total);
         __syncwarp();
         if (lane < 4 * n) {
@@ -1029,7 +1023,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         gemv_group_barrier(group);            // the unit's ring space is free; partial sums and the next unit's place are visible
         if (late) start_copies(nxt, slot ^ 1);
         if (NB > 0 && set_done) {
-            for (int z = wig; z < n * kAcc; z += kGemvWarps) {          // warp z % 4 finishes (quad, eight X rows) z
+            for (int z = wig ^ 2; z < n * kAcc; z += kGemvWarps) {      // warp z % 4 ^ 2, the leader last, finishes (quad, eight X rows) z
                 const int q = z / kAcc, g = z % kAcc;
                 const float *pp = part + (q * kAcc + g) * 32 + (kFew ? lane & 15 : lane);
                 float v = kFew ? pp[0] + pp[16] : pp[0];
