@@ -488,6 +488,25 @@ int bhi_split_histogram(const uint16_t *W, int rows, int K, int split_k, uint8_t
     return launch_status("split pass launch");
 }
 
+int bhi_huffman_limit_tables(const int64_t *histogram, int limit, uint8_t *LUT1, uint8_t *LUT2, uint8_t *LUT3, uint8_t *LUT4,
+                             uint8_t *code_lengths, uint32_t *code_values, int64_t *status, void *stream) {
+    BHI_REQUIRE(histogram && LUT1 && LUT2 && LUT3 && LUT4 && code_lengths && code_values && status, "null buffer");
+    BHI_REQUIRE(limit >= 1 && limit <= kLimitMax, "code lengths can be limited to 1..8 bits");
+    BHI_REQUIRE(aligned(histogram, 8) && aligned(code_values, 4) && aligned(status, 8), "unaligned buffer");
+    huffman_limit_tables_kernel<<<1, kTableThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const long long *>(histogram), limit, LUT1, LUT2, LUT3, LUT4, code_lengths, code_values, status);
+    return launch_status("huffman tables launch");
+}
+
+int bhi_ans_tables(const int64_t *histogram, int precision, uint32_t *freq, uint32_t *cum, uint32_t *LUT, int64_t *status, void *stream) {
+    BHI_REQUIRE(histogram && freq && cum && LUT && status, "null buffer");
+    BHI_REQUIRE(precision >= BHI_ANS_PRECISION && precision <= BHI_ANS_MAX_PRECISION, "rANS precision must be in [8, 12]");
+    BHI_REQUIRE(aligned(histogram, 8) && aligned(freq, 4) && aligned(cum, 4) && aligned(LUT, 4) && aligned(status, 8), "unaligned buffer");
+    ans_tables_kernel<<<1, kTableThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const long long *>(histogram), precision, freq, cum, LUT, status);
+    return launch_status("rANS tables launch");
+}
+
 int bhi_record_offsets(const int32_t *words_per_row, int split_k, int M, int slab_rows, int32_t *offsets, int64_t *total,
                        void *stream) {
     BHI_REQUIRE(words_per_row && offsets && total, "null buffer");

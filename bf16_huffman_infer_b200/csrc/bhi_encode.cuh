@@ -306,6 +306,208 @@ split_histogram_kernel(const uint32_t *__restrict__ W, int rows, int row0, int M
     }
 }
 
+// ---- code tables of a layer, from its histogram --------------------------------------------------------------------------
+// The same tables as the host's builders make, on the device: the host would have to wait for the histogram, build, and send
+// the tables back before the size pass can start (two codes: 0.45 ms of a conversion of 0.9 ms).  One block each; what bounds
+// it is a chain of a few hundred dependent steps.  Histograms that these kernels do not serve (more symbols than the limit
+// allows, a frequency that its field cannot hold) set `status`, and the host builds the tables after all.
+constexpr int kTableThreads = 256;
+constexpr int kLimitMax = 8;
+
+// exclusive sum over the block's 256 values
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *scratch /*[8]*/) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t run = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, run, o);
+        if (lane >= o) run += up;
+    }
+    __syncthreads();
+    if (lane == 31) scratch[warp] = run;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) run += scratch[w];
+    return run - v;
+}
+
+// Optimal prefix code with no length above `limit` (package-merge) in canonical order.  A level's list is the leaves merged
+// with the packages (pairs) of the level before, leaves first where weights are equal.  Every level holds the leaves in their
+// own order, so a leaf's length is the number of levels whose chosen prefix reaches it: 2 n - 2 items of the last level, and
+// of each level before, two for each package chosen after it.
+__global__ void __launch_bounds__(kTableThreads)
+huffman_limit_tables_kernel(const long long *__restrict__ hist, int limit, uint8_t *lut1, uint8_t *lut2, uint8_t *lut3, uint8_t *lut4,
+                            uint8_t *code_lengths, uint32_t *code_values, int64_t *status) {
+    constexpr int kMax = 1 << kLimitMax;
+    __shared__ long long weight[kMax], list[2 * kMax], packages[kMax];
+    __shared__ uint8_t sym[kMax], isleaf[2 * kMax], len_of[256];
+    __shared__ uint16_t leaves_before[kLimitMax][2 * kMax + 1];        // of each level, among its first i items
+    __shared__ uint32_t scratch[8], value_of[256];
+    const int tid = threadIdx.x;
+    const long long mine = hist[tid];
+    const uint32_t at = block_scan(mine > 0 ? 1u : 0u, scratch);
+    __syncthreads();
+    const int n = __syncthreads_count(mine > 0);
+    if (tid == 0) *status = n > (1 << limit) || n == 0;
+    if (n > (1 << limit) || n == 0) return;
+    len_of[tid] = 0;
+    value_of[tid] = 0u;
+    list[tid] = mine;                                                  // (the counts, for the ranks below)
+    __syncthreads();
+    // leaves by (weight, symbol)
+    if (mine > 0) {
+        int rank = 0;
+        for (int s = 0; s < 256; s++) rank += list[s] > 0 && (list[s] < mine || (list[s] == mine && s < tid));
+        weight[rank] = mine;
+        sym[rank] = static_cast<uint8_t>(tid);
+    }
+    __syncthreads();
+    // levels
+    int items = n;
+    if (tid < n) {
+        list[tid] = weight[tid];
+        leaves_before[0][tid + 1] = static_cast<uint16_t>(tid + 1);
+    }
+    if (tid < limit) leaves_before[tid][0] = 0;
+    __syncthreads();
+    for (int level = 1; level < limit; level++) {
+        const int pairs = items / 2;
+        if (tid < pairs) packages[tid] = list[2 * tid] + list[2 * tid + 1];
+        __syncthreads();
+        if (tid < n) {
+            int lo = 0, hi = pairs;                                    // packages lighter than this leaf
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (packages[mid] < weight[tid]) lo = mid + 1;
+                else hi = mid;
+            }
+            list[tid + lo] = weight[tid];
+            isleaf[tid + lo] = 1;
+        }
+        if (tid < pairs) {
+            int lo = 0, hi = n;                                        // leaves no heavier than this package
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (weight[mid] <= packages[tid]) lo = mid + 1;
+                else hi = mid;
+            }
+            list[tid + lo] = packages[tid];
+            isleaf[tid + lo] = 0;
+        }
+        items = n + pairs;
+        __syncthreads();
+        const uint32_t a = 2 * tid < items ? isleaf[2 * tid] : 0u, b = 2 * tid + 1 < items ? isleaf[2 * tid + 1] : 0u;
+        const uint32_t before = block_scan(a + b, scratch);
+        if (2 * tid < items) leaves_before[level][2 * tid + 1] = static_cast<uint16_t>(before + a);
+        if (2 * tid + 1 < items) leaves_before[level][2 * tid + 2] = static_cast<uint16_t>(before + a + b);
+        __syncthreads();
+    }
+    if (tid < n) {
+        int chosen = 2 * n - 2, length = n == 1 ? 1 : 0;
+        for (int level = limit - 1; level >= 0; level--) {
+            const int leaves = leaves_before[level][chosen];
+            length += tid < leaves;
+            chosen = 2 * (chosen - leaves);
+        }
+        len_of[sym[tid]] = static_cast<uint8_t>(length);
+    }
+    __syncthreads();
+    // canonical codes: by (length, symbol); a code is the number of leaves of the full tree to its left
+    const int length = len_of[tid];
+    if (length > 0) {
+        uint32_t code = 0;
+        for (int s = 0; s < 256; s++) {
+            const int l = len_of[s];
+            if (l > 0 && (l < length || (l == length && s < tid))) code += 1u << (kLimitMax - l);
+        }
+        value_of[tid] = __brev(code >> (kLimitMax - length)) >> (32 - length);
+    }
+    __syncthreads();
+    int found = 255;
+    for (int s = 0; s < 256; s++) {
+        const int l = len_of[s];
+        if (l > 0 && (tid & ((1 << l) - 1)) == static_cast<int>(value_of[s])) found = s;
+    }
+    lut1[tid] = static_cast<uint8_t>(found);
+    lut2[tid] = lut3[tid] = lut4[tid] = 255;
+    code_lengths[tid] = static_cast<uint8_t>(length);
+    code_values[tid] = value_of[tid];
+}
+
+// rANS model: counts scaled to a sum of 2^bits (rounded half to even, at least 1), the difference handed out or taken back unit
+// by unit over the symbols in the order of their rounding errors.
+__global__ void __launch_bounds__(kTableThreads)
+ans_tables_kernel(const long long *__restrict__ hist, int bits, uint32_t *freq, uint32_t *cum, uint32_t *lut, int64_t *status) {
+    __shared__ double err[256];
+    __shared__ int scaled[256], order[256];
+    __shared__ uint32_t scratch[8];
+    __shared__ unsigned long long total;
+    __shared__ int have;
+    const int tid = threadIdx.x, target = 1 << bits;
+    const long long mine = hist[tid];
+    if (tid == 0) {
+        total = 0ull;
+        have = 0;
+    }
+    __syncthreads();
+    atomicAdd(&total, static_cast<unsigned long long>(mine));
+    __syncthreads();
+    const int n = __syncthreads_count(mine > 0);
+    int q = 0;
+    double e = 0.0;
+    if (mine > 0) {
+        const double exact = static_cast<double>(mine * target) / static_cast<double>(total);
+        q = max(static_cast<int>(rint(exact)), 1);
+        e = exact - q;
+    }
+    err[tid] = e;
+    scaled[tid] = q;
+    atomicAdd(&have, q);
+    __syncthreads();
+    const bool small = have < target;
+    if (mine > 0) {                                                    // largest underestimate first, or largest overestimate
+        int rank = 0;
+        for (int s = 0; s < 256; s++)
+            if (scaled[s] > 0 && s != tid) rank += small ? err[s] > e || (err[s] == e && s > tid) : err[s] < e || (err[s] == e && s < tid);
+        order[rank] = tid;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int rest = target - have;
+        if (n > 0 && n <= target) {
+            for (int i = 0; rest > 0; i = i + 1 == n ? 0 : i + 1) {
+                scaled[order[i]]++;
+                rest--;
+            }
+            for (int i = 0; rest < 0; i = i + 1 == n ? 0 : i + 1) {
+                if (scaled[order[i]] > 1) {
+                    scaled[order[i]]--;
+                    rest++;
+                }
+            }
+        }
+        have = target - rest;
+    }
+    __syncthreads();
+    const uint32_t f = scaled[tid];
+    const int wide = __syncthreads_count(f > 0xFFFu);
+    if (tid == 0) *status = wide > 0 || have != target;
+    if (have != target) return;
+    const uint32_t c = block_scan(f, scratch);
+    freq[tid] = f;
+    cum[tid] = c;
+    order[tid] = static_cast<int>(c);
+    __syncthreads();
+    for (int slot = tid; slot < target; slot += kTableThreads) {
+        int lo = 0, hi = 256;                                          // the last symbol whose slots start here or before
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (order[mid] <= slot) lo = mid;
+            else hi = mid;
+        }
+        lut[slot] = (static_cast<uint32_t>(lo) << 24) | ((static_cast<uint32_t>(scaled[lo]) & 0xFFFu) << 12) | static_cast<uint32_t>(slot - order[lo]);
+    }
+}
+
 // ---- record offsets --------------------------------------------------------------------------------------------------
 // Exclusive sum of the record sizes (64 words per record row; 64 more after every slab of `slab` rows and after the last
 // row of a chunk), in storage order.  One block: a layer has some thousand records, and the launch waits for the size

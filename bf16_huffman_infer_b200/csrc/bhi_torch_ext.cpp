@@ -561,6 +561,43 @@ void boxed_record_offsets(StableIValue *stack, uint64_t, uint64_t) {
                              static_cast<int>(iarg(stack, 1)), ptr<int32_t>(off), ptr<int64_t>(total), stream_of(rows)));
 }
 
+// huffman_limit_tables(histogram, limit, LUT1(a!), LUT2(b!), LUT3(c!), LUT4(d!), code_lengths(e!), code_values(f!), status(g!)) -> ()
+void boxed_huffman_limit_tables(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor hist = arg(stack, 0), values = arg(stack, 7), status = arg(stack, 8);
+    want(hist, ScalarType::Long, "histogram");
+    want(values, ScalarType::Int, "code_values");
+    want(status, ScalarType::Long, "status");
+    uint8_t *t[5];
+    for (int i = 0; i < 5; i++) {
+        Tensor lut = arg(stack, 2 + i);
+        want(lut, ScalarType::Byte, "a code table");
+        same_device(hist, lut, "a code table");
+        STD_TORCH_CHECK(lut.numel() == 256, "code tables must have 256 entries");
+        t[i] = ptr<uint8_t>(lut);
+    }
+    for (const Tensor *x : {&values, &status}) same_device(hist, *x, "a code table");
+    STD_TORCH_CHECK(hist.numel() == 256 && values.numel() == 256 && status.numel() == 1, "histogram and code_values must have 256 entries, status one");
+    torch::stable::accelerator::DeviceGuard guard(hist.get_device_index());
+    check(bhi_huffman_limit_tables(ptr<const int64_t>(hist), static_cast<int>(iarg(stack, 1)), t[0], t[1], t[2], t[3], t[4],
+                                   ptr<uint32_t>(values), ptr<int64_t>(status), stream_of(hist)));
+}
+
+// ans_tables(histogram, freq(a!), cum(b!), LUT(c!), status(d!)) -> ()
+void boxed_ans_tables(StableIValue *stack, uint64_t, uint64_t) {
+    Tensor hist = arg(stack, 0), freq = arg(stack, 1), cum = arg(stack, 2), lut = arg(stack, 3), status = arg(stack, 4);
+    want(hist, ScalarType::Long, "histogram");
+    want(freq, ScalarType::Int, "freq");
+    want(cum, ScalarType::Int, "cum");
+    want(lut, ScalarType::Int, "LUT");
+    want(status, ScalarType::Long, "status");
+    for (const Tensor *x : {&freq, &cum, &lut, &status}) same_device(hist, *x, "an rANS table");
+    STD_TORCH_CHECK(hist.numel() == 256 && freq.numel() == 256 && cum.numel() == 256 && status.numel() == 1,
+                    "histogram, freq and cum must have 256 entries, status one");
+    torch::stable::accelerator::DeviceGuard guard(hist.get_device_index());
+    check(bhi_ans_tables(ptr<const int64_t>(hist), ans_precision_of(lut), ptr<uint32_t>(freq), ptr<uint32_t>(cum),
+                         ptr<uint32_t>(lut), ptr<int64_t>(status), stream_of(hist)));
+}
+
 // huffman_size_pass(W, split_k, code_lengths, words_per_row(a!)) -> ()
 void boxed_huffman_size_pass(StableIValue *stack, uint64_t, uint64_t) {
     Tensor W = arg(stack, 0), len = arg(stack, 2), rows = arg(stack, 3);
@@ -661,6 +698,8 @@ STABLE_TORCH_LIBRARY(BHI_TORCH_NAMESPACE, m) {
     // whole-layer encoder
     m.def("split_histogram(Tensor W, int split_k, int row0, Tensor(a!) rem, Tensor(b!) histogram) -> ()");
     m.def("record_offsets(Tensor words_per_row, int slab_rows, Tensor(a!) offsets, Tensor(b!) total) -> ()");
+    m.def("huffman_limit_tables(Tensor histogram, int limit, Tensor(a!) LUT1, Tensor(b!) LUT2, Tensor(c!) LUT3, Tensor(d!) LUT4, Tensor(e!) code_lengths, Tensor(f!) code_values, Tensor(g!) status) -> ()");
+    m.def("ans_tables(Tensor histogram, Tensor(a!) freq, Tensor(b!) cum, Tensor(c!) LUT, Tensor(d!) status) -> ()");
     m.def("huffman_size_pass(Tensor W, int split_k, Tensor code_lengths, Tensor(a!) words_per_row) -> ()");
     m.def("huffman_emit_pass(Tensor W, int split_k, Tensor code_lengths, Tensor code_values, Tensor offsets, Tensor(a!) rem, Tensor(b!) exp) -> ()");
     m.def("ans_size_pass(Tensor W, int split_k, Tensor freq, Tensor cum, Tensor(a!) words_per_row, Tensor(b!) stream_words) -> ()");
@@ -692,6 +731,8 @@ STABLE_TORCH_LIBRARY_IMPL(BHI_TORCH_NAMESPACE, CUDA, m) {
     m.impl("gemv_bf16_ans_exchange", &boxed_gemv_bf16_ans_exchange);
     m.impl("split_histogram", &boxed_split_histogram);
     m.impl("record_offsets", &boxed_record_offsets);
+    m.impl("huffman_limit_tables", &boxed_huffman_limit_tables);
+    m.impl("ans_tables", &boxed_ans_tables);
     m.impl("huffman_size_pass", &boxed_huffman_size_pass);
     m.impl("huffman_emit_pass", &boxed_huffman_emit_pass);
     m.impl("ans_size_pass", &boxed_ans_size_pass);

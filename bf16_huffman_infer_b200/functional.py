@@ -175,19 +175,28 @@ class _Ingested:
                     self.host_rem[:, lo:hi].zero_()
 
             transfer.upload_rows(a, self.w, arrived)
-        self.histogram = counts.cpu()
+        self.counts = counts
+
+    @property
+    def histogram(self) -> Tensor:
+        return self.counts.cpu()
 
 
 class _Plan:
-    """One coder's measure of a layer: its tables on the device and where every record will lie."""
+    """One coder's measure of a layer: its tables and where every record will lie.  ``result`` (i64 ``[2]``, on the device) gets
+    the words of the exponent plane and, from tables that were made on the device, whether they serve the layer."""
 
-    def __init__(self, cls, layer: _Ingested, codec):
-        self.cls, self.layer, self.codec = cls, layer, codec
-        self.luts = cls.get_lut_kwargs(codec)
-        self.tables = cls._encoder_tables(codec, layer.w.device)
+    def __init__(self, cls, layer: _Ingested, result: Tensor, on_device: bool = True):
+        self.cls, self.layer = cls, layer
+        made = cls._device_tables(layer.counts, result[1:]) if on_device else None
+        if made is None:
+            codec = cls._codec_of(layer.histogram)
+            made = _tables_to(cls.get_lut_kwargs(codec), layer.w.device), cls._encoder_tables(codec, layer.w.device)
+        self.luts, self.tables = made
         rows = torch.empty(layer.rem.shape[:2], dtype=torch.int32, device=layer.w.device)
         cls._size_pass(layer, self.tables, rows)
-        self.offsets, self.total = _record_offsets_async(rows)
+        self.offsets = torch.empty_like(rows)
+        ops.record_offsets(rows, SLAB_ROWS, self.offsets, result[:1])
 
     def finish(self, total: int, to_cpu: bool) -> "HuffmanWeight":
         layer, dev = self.layer, self.layer.w.device
@@ -195,11 +204,10 @@ class _Plan:
         self.cls._emit_pass(layer, self.tables, self.offsets, exp)
         if to_cpu:
             return self.cls(rem=transfer.download(layer.rem, layer.host_rem), exp=transfer.download(exp),
-                            offsets=transfer.download(self.offsets), **self.luts)
-        luts = _tables_to(self.luts, dev)
+                            offsets=transfer.download(self.offsets), **_tables_home(self.luts))
         # the buffers must be complete in memory before a fused kernel with launch overlap reads them
         torch.cuda.current_stream(dev).synchronize()
-        return self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **luts)
+        return self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **self.luts)
 
 
 def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor]:
@@ -213,12 +221,23 @@ def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor
     return out
 
 
+def _tables_home(tables: Dict[str, Tensor]) -> Dict[str, Tensor]:
+    """The way back."""
+    packed = torch.cat([t.view(torch.uint8) for t in tables.values()]).cpu()
+    parts = packed.split([t.numel() * t.element_size() for t in tables.values()])
+    return {name: part.clone().view(t.dtype) for (name, t), part in zip(tables.items(), parts)}
+
+
 def _compress(a: Tensor, split_k: int, coders: Sequence[type], to_cpu: bool) -> "HuffmanWeight":
     """``a`` by the coder that stores it in the fewest bytes (the first of those that tie).  The sizes are known after
     the size pass, so only the coder that is kept writes its records."""
     layer = _Ingested(a, split_k, to_cpu)
-    plans: List[_Plan] = [_Plan(c, layer, c._codec_of(layer.histogram)) for c in coders]
-    totals = torch.cat([p.total for p in plans]).tolist() if len(plans) > 1 else [int(plans[0].total.item())]
+    results = torch.zeros(len(coders), 2, dtype=torch.int64, device=layer.w.device)
+    plans: List[_Plan] = [_Plan(c, layer, r) for c, r in zip(coders, results)]
+    totals, unserved = zip(*results.tolist())
+    if any(unserved):
+        plans = [_Plan(p.cls, layer, r, on_device=False) if bad else p for p, r, bad in zip(plans, results, unserved)]
+        totals, _ = zip(*results.tolist())
     for t in totals:
         _checked_total(t)
     sizes = [4 * t + sum(v.nelement() * v.element_size() for v in p.luts.values()) for p, t in zip(plans, totals)]
@@ -460,6 +479,16 @@ class HuffmanWeight(nn.Module):
         return packed.view(torch.int32), row_words.to(torch.int32)
 
     @classmethod
+    def _device_tables(cls, counts: Tensor, status: Tensor) -> Optional[Tuple[Dict[str, Tensor], Dict[str, Tensor]]]:
+        """The layer's tables and the encoder's, made from the histogram on its device; None where only the host builds them."""
+        if not HUFFMAN_TABLES.startswith("limit") or not 1 <= int(HUFFMAN_TABLES[5:]) <= 8:
+            return None
+        luts = {k: torch.empty(256, dtype=torch.uint8, device=counts.device) for k in ("LUT1", "LUT2", "LUT3", "LUT4", "code_lengths")}
+        values = torch.empty(256, dtype=torch.int32, device=counts.device)
+        ops.huffman_limit_tables(counts, int(HUFFMAN_TABLES[5:]), *luts.values(), values, status)
+        return luts, {"code_values": values, "code_lengths": luts["code_lengths"]}
+
+    @classmethod
     def _encoder_tables(cls, codec, dev) -> Dict[str, Tensor]:
         return _tables_to({"code_values": torch.from_numpy(codec.code_values.view("int32")),
                            "code_lengths": torch.from_numpy(codec.code_lengths)}, dev)
@@ -549,6 +578,13 @@ class ANSWeight(HuffmanWeight):
         cum = torch.tensor(codec.cum, dtype=torch.int32, device=dev)
         ops.ans_encode(flat, freq, cum, words, counts)
         return words, counts.view(rows, groups).amax(dim=1)
+
+    @classmethod
+    def _device_tables(cls, counts: Tensor, status: Tensor) -> Optional[Tuple[Dict[str, Tensor], Dict[str, Tensor]]]:
+        freq, cum = (torch.empty(256, dtype=torch.int32, device=counts.device) for _ in range(2))
+        lut = torch.empty(1 << ANS_PRECISION, dtype=torch.int32, device=counts.device)
+        ops.ans_tables(counts, freq, cum, lut, status)
+        return {"LUT": lut}, {"freq": freq, "cum": cum}
 
     @classmethod
     def _encoder_tables(cls, codec, dev) -> Dict[str, Tensor]:

@@ -130,6 +130,12 @@ def record_offsets(words_per_row: Tensor, slab_rows: int, offsets: Tensor, total
     _ops.record_offsets.default(words_per_row, slab_rows, offsets, total)
 
 
+# a layer's code tables from its histogram, on the device; `status` (i64 [1]) becomes nonzero where the host has to build them:
+# (histogram, limit, LUT1..4, code_lengths, code_values, status) and (histogram, freq, cum, LUT, status)
+huffman_limit_tables = _ops.huffman_limit_tables.default
+ans_tables = _ops.ans_tables.default
+
+
 def huffman_size_pass(W: Tensor, split_k: int, code_lengths: Tensor, words_per_row: Tensor) -> None:
     _ops.huffman_size_pass.default(W, split_k, code_lengths, words_per_row)
 

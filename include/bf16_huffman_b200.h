@@ -258,6 +258,14 @@ int bhi_split_histogram(const uint16_t *W, int rows, int K, int split_k, uint8_t
 int bhi_record_offsets(const int32_t *words_per_row, int split_k, int M, int slab_rows, int32_t *offsets, int64_t *total,
                        void *stream);
 
+/* Code tables from a histogram (i64 [256]) on the device: those of the optimal code with no length above `limit` (1..8) bits,
+ * and an rANS model of `precision` probability bits with its decode table (2^precision words).  *status (device) becomes 0, or
+ * nonzero where the histogram cannot be served: more symbols than 2^limit, or a frequency that the table word cannot hold. */
+int bhi_huffman_limit_tables(const int64_t *histogram, int limit, uint8_t *LUT1, uint8_t *LUT2, uint8_t *LUT3, uint8_t *LUT4,
+                             uint8_t *code_lengths, uint32_t *code_values, int64_t *status, void *stream);
+int bhi_ans_tables(const int64_t *histogram, int precision, uint32_t *freq, uint32_t *cum, uint32_t *LUT, int64_t *status,
+                   void *stream);
+
 /* Emit pass: writes A_rem (permuted bytes; null when bhi_split_histogram has written it) and the coded words of every
  * record at its offset.  A_exp must be zero-filled by the caller (padding words are never written).
  * code_values u32 [256]: code bits with the first path bit in bit 0. */
