@@ -210,8 +210,10 @@ static int check_enc(const void *W, int M, int K, int S) {
     return BHI_OK;
 }
 
-static int enc_blocks(int M, int S) {
-    return static_cast<int>((static_cast<int64_t>(S) * M + kEncRecords - 1) / kEncRecords);
+// blocks for all records, at `per_block` each, or as many as fit the device at `per_sm` (0: no such limit)
+static int enc_blocks(int M, int S, int per_block = kEncRecords, int per_sm = 0) {
+    const int64_t need = (static_cast<int64_t>(S) * M + per_block - 1) / per_block, cap = static_cast<int64_t>(sm_count()) * per_sm;
+    return static_cast<int>(per_sm && need > cap ? cap : need);
 }
 
 }  // namespace bhi
@@ -532,7 +534,8 @@ int bhi_ans_size_pass(const uint16_t *W, int M, int K, int split_k, const uint32
     if (int rc = check_enc(W, M, K, split_k)) return rc;
     BHI_REQUIRE(freq && cum && words_per_row && stream_words, "null buffer");
     EncGeom g{W, M, K, split_k, K / split_k};
-    ans_size_kernel<<<enc_blocks(M, split_k), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    if (int rc = staged_prepare(ans_size_kernel, kAnsEncBytes)) return rc;
+    ans_size_kernel<<<enc_blocks(M, split_k, kAnsEncRecords, 2), kAnsEncThreads, kAnsEncBytes, static_cast<cudaStream_t>(stream)>>>(
         g, freq, cum, words_per_row, stream_words);
     return launch_status("rANS size pass launch");
 }
@@ -544,7 +547,7 @@ int bhi_huffman_emit_pass(const uint16_t *W, int M, int K, int split_k, const ui
     BHI_REQUIRE(code_lengths && code_values && offsets && A_exp, "null buffer");
     BHI_REQUIRE(aligned(A_rem, 2) && aligned(A_exp, 4), "unaligned output");
     EncGeom g{W, M, K, split_k, K / split_k};
-    huffman_emit_kernel<<<enc_blocks(M, split_k), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    huffman_emit_kernel<<<enc_blocks(M, split_k, kEncRecords, kEncBlocksPerSm), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         g, code_lengths, code_values, offsets, A_rem, A_exp);
     return launch_status("huffman emit pass launch");
 }
@@ -556,7 +559,8 @@ int bhi_ans_emit_pass(const uint16_t *W, int M, int K, int split_k, const uint32
     BHI_REQUIRE(freq && cum && offsets && stream_words && A_exp, "null buffer");
     BHI_REQUIRE(aligned(A_rem, 2) && aligned(A_exp, 4), "unaligned output");
     EncGeom g{W, M, K, split_k, K / split_k};
-    ans_emit_kernel<<<enc_blocks(M, split_k), kEncThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    if (int rc = staged_prepare(ans_emit_kernel, kAnsEncBytes)) return rc;
+    ans_emit_kernel<<<enc_blocks(M, split_k, kAnsEncRecords, 2), kAnsEncThreads, kAnsEncBytes, static_cast<cudaStream_t>(stream)>>>(
         g, freq, cum, offsets, stream_words, A_rem, A_exp);
     return launch_status("rANS emit pass launch");
 }

@@ -96,6 +96,7 @@ __global__ void ans_encode_words_kernel(const uint8_t *__restrict__ data, int st
 // ---- whole-layer encoder ---------------------------------------------------------------------------
 constexpr int kEncThreads = 256;                 // 4 records per block
 constexpr int kEncRecords = kEncThreads / 64;
+constexpr int kEncAhead = 4;                     // blocks of a record that are loaded together
 
 struct EncGeom {
     const uint16_t *W;     // [M, K]
@@ -155,90 +156,179 @@ __device__ __forceinline__ void store_rem(uint8_t *rem_row, int st, int blk, uin
     *reinterpret_cast<uint16_t *>(rem_row + blk * 128 + (st & 31) * 4 + (st >> 5) * 2) = static_cast<uint16_t>(lo | (hi << 8));
 }
 
-__global__ void __launch_bounds__(kEncThreads)
+// The coded words of every record.  What bounds it is the work per symbol (12288 x 4096: 43 us, of which HBM 19; with one table of
+// codes and one of lengths 62), so the table has a copy for each lane: the
+// 32 lookups of a warp always hit 32 different banks, and their address is the exponent where it stands in the weight (128 bytes
+// per entry).  Codes of at most 16 bits, which all but the reference's own builder make, stand with their lengths in one word and
+// are joined in pairs.  Blocks stay for several records, as the copies take a while to write.
+constexpr int kEncBlocksPerSm = 6;               // 33 KB of shared memory each
+
+__global__ void __launch_bounds__(kEncThreads, kEncBlocksPerSm)
 huffman_emit_kernel(EncGeom g, const uint8_t *__restrict__ code_len, const uint32_t *__restrict__ code_val,
                     const int32_t *__restrict__ offsets, uint8_t *rem, uint32_t *__restrict__ exp) {
+    __shared__ uint32_t table[256 * 32];
     __shared__ uint8_t len[256];
-    __shared__ uint32_t val[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) { len[i] = code_len[i]; val[i] = code_val[i]; }
+    static_assert(kEncThreads == 256, "a thread writes one symbol's copies");
+    const uint32_t my_len = code_len[threadIdx.x], my_val = code_val[threadIdx.x];
+    len[threadIdx.x] = static_cast<uint8_t>(my_len);
+    const bool pairs = !__syncthreads_or(my_len > 16u);
+    for (int i = 0; i < 32; i++) table[threadIdx.x * 32 + ((i + threadIdx.x) & 31)] = pairs ? my_val | my_len << 16 : my_val;
     __syncthreads();
-    int64_t rec; int k, m, st;
-    if (!enc_locate(g, rec, k, m, st)) return;
-    uint8_t *rem_row = rem ? rem + rec * g.Nc : nullptr;
-    uint32_t *out = exp + static_cast<uint32_t>(offsets[rec]) + st;
-    uint64_t acc = 0;
-    uint32_t have = 0;
-    for (int blk = 0; blk < (g.Nc >> 7); blk++) {
-        const uint32_t p = enc_pair(g, k, m, st, blk);
-        if (rem_row) store_rem(rem_row, st, blk, p);
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            const uint32_t e = t ? exp_hi(p) : exp_lo(p);
-            acc |= static_cast<uint64_t>(val[e]) << have;
-            have += len[e];
-            if (have >= 32) {
+    const uint8_t *mine = reinterpret_cast<const uint8_t *>(table) + 4 * (threadIdx.x & 31);
+    auto entry = [&](uint32_t at) { return *reinterpret_cast<const uint32_t *>(mine + at); };
+    const int nblk = g.Nc >> 7, st = threadIdx.x & 63;
+    const int64_t records = static_cast<int64_t>(g.S) * g.M;
+    for (int64_t rec = static_cast<int64_t>(blockIdx.x) * kEncRecords + (threadIdx.x >> 6); rec < records; rec += static_cast<int64_t>(gridDim.x) * kEncRecords) {
+        const int k = static_cast<int>(rec / g.M), m = static_cast<int>(rec - static_cast<int64_t>(k) * g.M);
+        uint8_t *rem_row = rem ? rem + rec * g.Nc : nullptr;
+        uint32_t *out = exp + static_cast<uint32_t>(offsets[rec]) + st;
+        uint64_t acc = 0;
+        uint32_t have = 0;
+        auto append = [&](uint32_t bits, uint32_t n) {                 // n <= 32
+            acc |= static_cast<uint64_t>(bits) << have;
+            have += n;
+            if (have >= 32u) {
                 *out = static_cast<uint32_t>(acc);
                 out += kStreamsPerRecord;
                 acc >>= 32;
-                have -= 32;
+                have -= 32u;
+            }
+        };
+        for (int blk = 0; blk < nblk; blk += kEncAhead) {
+            uint32_t p[kEncAhead];
+#pragma unroll
+            for (int i = 0; i < kEncAhead; i++) p[i] = blk + i < nblk ? enc_pair(g, k, m, st, blk + i) : 0u;
+#pragma unroll
+            for (int i = 0; i < kEncAhead; i++) {
+                if (blk + i < nblk) {
+                    if (rem_row) store_rem(rem_row, st, blk + i, p[i]);
+                    const uint32_t e0 = entry(p[i] & 0x7F80u), e1 = entry((p[i] >> 16) & 0x7F80u);
+                    if (pairs) {
+                        append((e0 & 0xFFFFu) | (e1 & 0xFFFFu) << (e0 >> 16), (e0 >> 16) + (e1 >> 16));
+                    } else {
+                        append(e0, len[exp_lo(p[i])]);
+                        append(e1, len[exp_hi(p[i])]);
+                    }
+                }
+            }
+        }
+        if (have > 0) *out = static_cast<uint32_t>(acc);
+    }
+}
+
+// rANS over one stream of a record, symbols last to first; `put` sees words in emission order.  Bound by the integer work of a
+// step and its chain: 12288 x 4096 73 us in the size pass and 86 in the emit pass (79 and 92 with one model for all lanes and a
+// 64-bit product).  The model has a copy for each lane (96 KB, two blocks of 512 threads per SM, which stay for several records):
+// the lookups of a warp hit 32 different banks.
+constexpr int kAnsEncThreads = 512;
+constexpr int kAnsEncRecords = kAnsEncThreads / 64;
+constexpr int kAnsEncBytes = 256 * 32 * 12;
+
+struct AnsLaneModel {
+    const uint2 *inv;          // [256][32], this lane's column
+    const uint32_t *fc;        // freq | cum << 16, the same
+    uint32_t bits;
+};
+
+__device__ __forceinline__ AnsLaneModel load_lane_model(uint8_t *smem, const uint32_t *freq, const uint32_t *cum) {
+    uint2 *inv = reinterpret_cast<uint2 *>(smem);
+    uint32_t *fc = reinterpret_cast<uint32_t *>(smem + 256 * 32 * 8);
+    const uint32_t s = threadIdx.x & 255u, first = (threadIdx.x >> 8) * 16u;       // two threads per symbol
+    const uint32_t f = freq[s], c = cum[s];
+    const uint64_t v = f ? ((1ull << 63) + f - 1u) / f : 0ull;                     // see AnsModel
+    for (uint32_t i = 0; i < 16u; i++) {
+        const uint32_t at = 32u * s + ((first + i + s) & 31u);
+        inv[at] = make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
+        fc[at] = f | c << 16;
+    }
+    const uint32_t total = cum[255] + freq[255];
+    __syncthreads();
+    return {inv + (threadIdx.x & 31), fc + (threadIdx.x & 31), total ? 31u - static_cast<uint32_t>(__clz(total)) : kAnsBitsMin};
+}
+
+template <class Put>
+__device__ __forceinline__ void ans_encode_record_stream(const EncGeom &g, int k, int m, int st, const AnsLaneModel &t, Put &&put) {
+    // As ans_push, word by word: the state's high word is below f <= 2^15 once it is renormalised, which leaves four products of
+    // the quotient's long multiplication and no carries; r + cum fills the bits below q << bits.
+    uint32_t lo = 1u << t.bits, hi = 0u;
+    auto push = [&](uint32_t sym) {
+        const uint32_t w = t.fc[32u * sym], f = w & 0xFFFFu;
+        if (f == 0u) return;
+        const uint2 v = t.inv[32u * sym];
+        if (hi >= f) {
+            put(lo);
+            lo = hi;
+            hi = 0u;
+        }
+        const uint64_t mid = static_cast<uint64_t>(hi) * v.x + (static_cast<uint64_t>(lo) * v.y + __umulhi(lo, v.x));
+        const uint32_t top = hi * v.y + static_cast<uint32_t>(mid >> 32);
+        const uint32_t q = __funnelshift_l(static_cast<uint32_t>(mid), top, 1);
+        lo = q * ((1u << t.bits) - f) + (lo + (w >> 16));              // q 2^bits + (lo - q f) + cum
+        hi = q >> (32u - t.bits);
+    };
+    for (int last = (g.Nc >> 7) - 1; last >= 0; last -= kEncAhead) {
+        uint32_t p[kEncAhead];
+#pragma unroll
+        for (int i = 0; i < kEncAhead; i++) p[i] = last >= i ? enc_pair(g, k, m, st, last - i) : 0u;
+#pragma unroll
+        for (int i = 0; i < kEncAhead; i++) {
+            if (last >= i) {
+                push(exp_hi(p[i]));
+                push(exp_lo(p[i]));
             }
         }
     }
-    if (have > 0) *out = static_cast<uint32_t>(acc);
+    if (lo | hi) put(lo);
+    if (hi) put(hi);
 }
 
-// rANS over one stream of a record, symbols last to first; `put` sees words in emission order.
-template <class Put>
-__device__ __forceinline__ void ans_encode_record_stream(const EncGeom &g, int k, int m, int st, const AnsModel &model,
-                                                         Put &&put) {
-    const uint32_t bits = ans_model_bits(model);
-    uint64_t state = 1ull << bits;
-    for (int blk = (g.Nc >> 7) - 1; blk >= 0; blk--) {
-        const uint32_t p = enc_pair(g, k, m, st, blk);
-        ans_push(state, model, exp_hi(p), bits, put);
-        ans_push(state, model, exp_lo(p), bits, put);
-    }
-    while (state > 0) { put(static_cast<uint32_t>(state)); state >>= 32; }
-}
-
-__global__ void __launch_bounds__(kEncThreads)
+__global__ void __launch_bounds__(kAnsEncThreads, 2)
 ans_size_kernel(EncGeom g, const uint32_t *__restrict__ freq, const uint32_t *__restrict__ cum,
                 int32_t *__restrict__ words_per_row, uint8_t *__restrict__ stream_words) {
-    __shared__ AnsModel model;
-    __shared__ uint32_t scratch[kEncThreads / 32];
-    load_model(model, freq, cum);
-    __syncthreads();
-    int64_t rec; int k, m, st;
-    const bool live = enc_locate(g, rec, k, m, st);
-    uint32_t cnt = 0;
-    if (live) {
-        ans_encode_record_stream(g, k, m, st, model, [&](uint32_t) { cnt++; });
-        stream_words[rec * 64 + st] = static_cast<uint8_t>(cnt);
+    extern __shared__ __align__(16) uint8_t enc_smem[];
+    __shared__ uint32_t worst_of[kAnsEncThreads / 32];
+    const AnsLaneModel model = load_lane_model(enc_smem, freq, cum);
+    const int st = threadIdx.x & 63, warp = threadIdx.x >> 5;
+    const int64_t records = static_cast<int64_t>(g.S) * g.M;
+    for (int64_t first = static_cast<int64_t>(blockIdx.x) * kAnsEncRecords; first < records; first += static_cast<int64_t>(gridDim.x) * kAnsEncRecords) {
+        const int64_t rec = first + (threadIdx.x >> 6);
+        uint32_t cnt = 0;
+        if (rec < records) {
+            const int k = static_cast<int>(rec / g.M), m = static_cast<int>(rec - static_cast<int64_t>(k) * g.M);
+            ans_encode_record_stream(g, k, m, st, model, [&](uint32_t) { cnt++; });
+            stream_words[rec * 64 + st] = static_cast<uint8_t>(cnt);
+        }
+        const uint32_t worst = __reduce_max_sync(0xFFFFFFFFu, cnt);
+        if ((threadIdx.x & 31) == 0) worst_of[warp] = worst;
+        __syncthreads();
+        if (rec < records && st == 0) words_per_row[rec] = static_cast<int32_t>(max(worst_of[warp], worst_of[warp + 1]));
+        __syncthreads();
     }
-    const uint32_t worst = record_max(cnt, scratch);
-    if (live && st == 0) words_per_row[rec] = static_cast<int32_t>(worst);
 }
 
-__global__ void __launch_bounds__(kEncThreads)
+__global__ void __launch_bounds__(kAnsEncThreads, 2)
 ans_emit_kernel(EncGeom g, const uint32_t *__restrict__ freq, const uint32_t *__restrict__ cum,
                 const int32_t *__restrict__ offsets, const uint8_t *__restrict__ stream_words,
                 uint8_t *rem, uint32_t *__restrict__ exp) {
-    __shared__ AnsModel model;
-    load_model(model, freq, cum);
-    __syncthreads();
-    int64_t rec; int k, m, st;
-    if (!enc_locate(g, rec, k, m, st)) return;
-    if (rem) {
-        uint8_t *rem_row = rem + rec * g.Nc;
-        for (int blk = 0; blk < (g.Nc >> 7); blk++) store_rem(rem_row, st, blk, enc_pair(g, k, m, st, blk));
+    extern __shared__ __align__(16) uint8_t enc_smem[];
+    const AnsLaneModel model = load_lane_model(enc_smem, freq, cum);
+    const int st = threadIdx.x & 63;
+    const int64_t records = static_cast<int64_t>(g.S) * g.M;
+    for (int64_t rec = static_cast<int64_t>(blockIdx.x) * kAnsEncRecords + (threadIdx.x >> 6); rec < records;
+         rec += static_cast<int64_t>(gridDim.x) * kAnsEncRecords) {
+        const int k = static_cast<int>(rec / g.M), m = static_cast<int>(rec - static_cast<int64_t>(k) * g.M);
+        if (rem) {
+            uint8_t *rem_row = rem + rec * g.Nc;
+            for (int blk = 0; blk < (g.Nc >> 7); blk++) store_rem(rem_row, st, blk, enc_pair(g, k, m, st, blk));
+        }
+        // the j-th emitted word is the (cnt-1-j)-th word the decoder reads
+        uint32_t *out = exp + static_cast<uint32_t>(offsets[rec]) + st;
+        int at = static_cast<int>(stream_words[rec * 64 + st]) - 1;
+        ans_encode_record_stream(g, k, m, st, model, [&](uint32_t w) {
+            if (at >= 0) out[static_cast<int64_t>(at) * kStreamsPerRecord] = w;
+            at--;
+        });
     }
-    // the j-th emitted word is the (cnt-1-j)-th word the decoder reads
-    uint32_t *out = exp + static_cast<uint32_t>(offsets[rec]) + st;
-    int at = static_cast<int>(stream_words[rec * 64 + st]) - 1;
-    ans_encode_record_stream(g, k, m, st, model, [&](uint32_t w) {
-        if (at >= 0) out[static_cast<int64_t>(at) * kStreamsPerRecord] = w;
-        at--;
-    });
 }
 
 // ---- sign/mantissa plane and exponent histogram ----------------------------------------------------------------------
@@ -339,24 +429,26 @@ huffman_limit_tables_kernel(const long long *__restrict__ hist, int limit, uint8
                             uint8_t *code_lengths, uint32_t *code_values, int64_t *status) {
     constexpr int kMax = 1 << kLimitMax;
     __shared__ long long weight[kMax], list[2 * kMax], packages[kMax];
-    __shared__ uint8_t sym[kMax], isleaf[2 * kMax], len_of[256];
+    __shared__ uint8_t sym[kMax], used[256], isleaf[2 * kMax], len_of[256];          // sym: by rank, used: in order
     __shared__ uint16_t leaves_before[kLimitMax][2 * kMax + 1];        // of each level, among its first i items
     __shared__ uint32_t scratch[8], value_of[256];
     const int tid = threadIdx.x;
     const long long mine = hist[tid];
     const uint32_t at = block_scan(mine > 0 ? 1u : 0u, scratch);
-    __syncthreads();
     const int n = __syncthreads_count(mine > 0);
     if (tid == 0) *status = n > (1 << limit) || n == 0;
     if (n > (1 << limit) || n == 0) return;
     len_of[tid] = 0;
     value_of[tid] = 0u;
-    list[tid] = mine;                                                  // (the counts, for the ranks below)
+    if (mine > 0) {
+        used[at] = static_cast<uint8_t>(tid);
+        list[at] = mine;                                               // (the counts, for the ranks below)
+    }
     __syncthreads();
     // leaves by (weight, symbol)
     if (mine > 0) {
         int rank = 0;
-        for (int s = 0; s < 256; s++) rank += list[s] > 0 && (list[s] < mine || (list[s] == mine && s < tid));
+        for (int i = 0; i < n; i++) rank += list[i] < mine || (list[i] == mine && i < static_cast<int>(at));
         weight[rank] = mine;
         sym[rank] = static_cast<uint8_t>(tid);
     }
@@ -415,17 +507,17 @@ huffman_limit_tables_kernel(const long long *__restrict__ hist, int limit, uint8
     const int length = len_of[tid];
     if (length > 0) {
         uint32_t code = 0;
-        for (int s = 0; s < 256; s++) {
-            const int l = len_of[s];
-            if (l > 0 && (l < length || (l == length && s < tid))) code += 1u << (kLimitMax - l);
+        for (int i = 0; i < n; i++) {
+            const int s = used[i], l = len_of[s];
+            if (l < length || (l == length && s < tid)) code += 1u << (kLimitMax - l);
         }
         value_of[tid] = __brev(code >> (kLimitMax - length)) >> (32 - length);
     }
     __syncthreads();
     int found = 255;
-    for (int s = 0; s < 256; s++) {
-        const int l = len_of[s];
-        if (l > 0 && (tid & ((1 << l) - 1)) == static_cast<int>(value_of[s])) found = s;
+    for (int i = 0; i < n; i++) {
+        const int s = used[i];
+        if ((tid & ((1 << len_of[s]) - 1)) == static_cast<int>(value_of[s])) found = s;
     }
     lut1[tid] = static_cast<uint8_t>(found);
     lut2[tid] = lut3[tid] = lut4[tid] = 255;
@@ -451,6 +543,7 @@ ans_tables_kernel(const long long *__restrict__ hist, int bits, uint32_t *freq, 
     __syncthreads();
     atomicAdd(&total, static_cast<unsigned long long>(mine));
     __syncthreads();
+    const int at = static_cast<int>(block_scan(mine > 0 ? 1u : 0u, scratch));
     const int n = __syncthreads_count(mine > 0);
     int q = 0;
     double e = 0.0;
@@ -459,15 +552,17 @@ ans_tables_kernel(const long long *__restrict__ hist, int bits, uint32_t *freq, 
         q = max(static_cast<int>(rint(exact)), 1);
         e = exact - q;
     }
-    err[tid] = e;
+    if (mine > 0) {
+        err[at] = e;
+        atomicAdd(&have, q);
+    }
     scaled[tid] = q;
-    atomicAdd(&have, q);
     __syncthreads();
     const bool small = have < target;
     if (mine > 0) {                                                    // largest underestimate first, or largest overestimate
         int rank = 0;
-        for (int s = 0; s < 256; s++)
-            if (scaled[s] > 0 && s != tid) rank += small ? err[s] > e || (err[s] == e && s > tid) : err[s] < e || (err[s] == e && s < tid);
+        for (int i = 0; i < n; i++)
+            if (i != at) rank += small ? err[i] > e || (err[i] == e && i > at) : err[i] < e || (err[i] == e && i < at);
         order[rank] = tid;
     }
     __syncthreads();

@@ -288,7 +288,7 @@ __device__ __forceinline__ void build_fast_table(uint32_t *fast, const AnsTables
 bool overlap_launches();     // process-wide switch, see bhi_set_launch_overlap
 
 template <class K>
-static int staged_prepare(K kernel) {
+static int staged_prepare(K kernel, int bytes = kSmemMax) {
     // Opt in to the large dynamic shared-memory carve-out once per device and kernel.  Keyed by the
     // kernel's address: instantiations that differ only in a non-type argument share their pointer type.
     static std::mutex mu;
@@ -299,7 +299,7 @@ static int staged_prepare(K kernel) {
     std::lock_guard<std::mutex> lock(mu);
     uint64_t &bits = done[key];
     if (!(bits >> dev & 1u)) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
         bits |= 1ull << dev;
     }
