@@ -14,16 +14,19 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libbf16_huffman_b200.so")
 EXT_PATH = os.path.join(PKG_DIR, "_C.abi3.so")
 
+ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+    *ARCH_FLAGS, "-lineinfo", "-O3", "-std=c++17",
     "--use_fast_math", "-Xptxas", "-v", "-Xptxas", "--warn-on-spills",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-Xcompiler", "-fPIC",
 ]
 
 
@@ -56,7 +59,11 @@ def build_library(force: bool = False) -> str:
     if not force and _newer(LIB_PATH, sources):
         return LIB_PATH
     units = [s for s in sources if s.endswith(".cu")]
-    _run([_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH, *units], "build_lib.log")
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor(len(units)) as pool:      # the files take minutes each
+        objects = [os.path.join(tmp, os.path.basename(u)[:-3] + ".o") for u in units]
+        logs = [os.path.basename(u)[:-3] + ".log" for u in units]
+        list(pool.map(lambda u, o, log: _run([_nvcc(), *NVCC_FLAGS, "-c", "-o", o, u], log), units, objects, logs))
+        _run([_nvcc(), *ARCH_FLAGS, "-shared", "-o", LIB_PATH, *objects], "build_lib.log")
     return LIB_PATH
 
 

@@ -9,9 +9,7 @@
 #include "bhi_encode.cuh"
 #include "bhi_generic.cuh"
 #include "bhi_staged.cuh"
-#include "bhi_gemv.cuh"
-#include "bhi_tile.cuh"
-#include "bhi_tileq.cuh"
+#include "bhi_launch.cuh"
 
 namespace bhi {
 
@@ -241,10 +239,13 @@ int bhi_huffman_table_hint(const uint8_t *prepared, int pair_complete) {
 
 int bhi_debug_status(int *status_out) {
     BHI_REQUIRE(status_out, "null output");
-    int v = 0, zero = 0;
+    int v = 0;
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&v, g_staged_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_staged_status, &zero, sizeof(int));
+    for (auto take : {take_gemv_huffman_status, take_gemv_ans_status, take_tiles_status}) {
+        int one = 0;
+        if (e == cudaSuccess) e = take(&one);
+        if (one) v = one;
+    }
     if (e != cudaSuccess) return cuda_fail(e, "status read");
     *status_out = v;
     return BHI_OK;

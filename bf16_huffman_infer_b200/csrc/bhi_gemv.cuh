@@ -27,6 +27,7 @@
 // lanes that hold the results store them.
 #pragma once
 
+#include "bhi_launch.cuh"
 #include "bhi_staged.cuh"
 
 namespace bhi {
@@ -515,6 +516,15 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
     return sets;
 }
 
+// Sixteen warps and one more have 96 registers each (five warps share a quarter of the register file).  Where that spills, the
+// one more is a warpgroup, of which one warp works: it gives registers back, so that the sixteen can have 112 (640 x 96 at the
+// launch = 512 x 112 + 128 x 32).  12288 x 4096, 16 / 24 / 32 rows, in us, without and with it: escape 47.2 / 49.3 / 61.5,
+// 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6 36.5 (stays as it was) / 41.6 / 50.9, - / 40.6 / 48.5.
+template <class Dec, int NB, int NG, bool kRing>
+constexpr bool kShiftsRegisters = kRing && NG == 4 && (NB > 2 || !std::is_same<Dec, GemvSingle>::value);
+template <class Dec, int NB, int NG, bool kRing>
+constexpr int kRingThreads = !kRing ? 0 : kShiftsRegisters<Dec, NB, NG, kRing> ? 128 : 32;
+
 // NB = groups of eight X rows (0: no product, the dense matrix is written instead).  NG = groups of four warps per CTA.
 // Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
 // X or tables two CTAs could not both hold.  kRing: X passes through a ring that one more warp fills and all groups read in
@@ -529,7 +539,7 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
 // layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
 template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew>
-__global__ void __launch_bounds__(NG * kGemvWarps * 32 + (kRing ? 32 : 0), NG == 2 ? 2 : 1)
+__global__ void __launch_bounds__(NG * kGemvWarps * 32 + kRingThreads<Dec, NB, NG, kRing>, NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
             PeerSet peers, GemvGeom G, GemvConsts kc) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -612,8 +622,14 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     // ---- the warp that fills the X ring.  (With the readers filling it between their chunks, the last reader of a segment
     // its next one, the refill lay on the slowest warp and cost half as much again as the decoding.)
-    if (kRing && warp == NG * kGemvWarps) {
+    constexpr bool kShift = kShiftsRegisters<Dec, NB, NG, kRing>;
+    if (kRing && warp >= NG * kGemvWarps) {
+        if constexpr (kShift) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         __syncthreads();                                               // the readers' barrier before their loop
+        if (warp > NG * kGemvWarps) {
+            if (exchange) __syncthreads();                             // exchange_finish's
+            return;
+        }
         pdl_wait();
         const bool bulk = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
         const int x_total = x_segments();
@@ -648,6 +664,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         return;
     }
 
+    if constexpr (kShift) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     // ---- units ---------------------------------------------------------------------------------------------------------
     // A set is a pair of quads, or one quad: the last of an odd number, and both of a pair that has, in any chunk, a record
     // longer than the ring takes beside seven of that length.  For each set, the chunks in order.  The group's first warp
@@ -1170,7 +1187,7 @@ static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs,
     if (peers) ps = *peers;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NG * kGemvWarps * 32 + (kRing ? 32 : 0));
+    cfg.blockDim = dim3(NG * kGemvWarps * 32 + kRingThreads<Dec, NB, NG, kRing>);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1309,7 +1326,7 @@ constexpr int kGemvMaxRows = 32;
 //   pair table, 14 / 13 bits    8.4 / 8.8   14.7 / 16.1    34.9 / 37.1    35.5 / 37.7   25.4 / 23.5   (escape)
 //   rANS, 8 bits, 64 / 32 KB    9.4 / 9.2   17.1 / 19.4    43.3 / 50.0    42.5 / 52.5   30.0 / 30.9
 template <class Codec>
-static int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
+int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                        const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16) || B > kGemvMaxRows) return kStagedDeclined;
     if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31) || L.exp_words >= (1ll << 32)) return kStagedDeclined;

@@ -53,7 +53,14 @@ constexpr int kPreparedBytes = kPreparedWidest + (4 << kWidestBits);
 static_assert(sizeof(HuffTables) + 8 <= kExactBytes && sizeof(AnsTables) <= kExactBytes, "exact tables do not fit");
 static_assert((4 << kAnsBitsMax) * kCopies <= kLutBytes, "the largest rANS table does not fit the fast-table region");
 
-__device__ int g_staged_status = 0;            // 0 = fine; otherwise the last failure code
+static __device__ int g_staged_status = 0;     // 0 = fine; otherwise the last failure code.  One for each source file of kernels:
+
+// reads and clears this source file's
+static cudaError_t take_status(int *out) {
+    const int zero = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(out, g_staged_status, sizeof(int));
+    return e == cudaSuccess ? cudaMemcpyToSymbol(g_staged_status, &zero, sizeof(int)) : e;
+}
 
 // ---- PTX wrappers ----------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -271,7 +278,7 @@ __device__ __forceinline__ uint32_t pair_lookup(const uint8_t *smem, const Const
 
 // A code longer than the table index: resolve one symbol with the exact four-table cascade.
 // Returns {symbol, length}.  Out of line on purpose: it is rare and must not bloat the loop.
-__device__ __noinline__ uint2 huff_exact_symbol(uint32_t win, const HuffTables *t) {
+static __device__ __noinline__ uint2 huff_exact_symbol(uint32_t win, const HuffTables *t) {
     const uint32_t s = huff_cascade(*t, win);
     return make_uint2(s, t->len[s]);
 }
@@ -322,7 +329,7 @@ __device__ __forceinline__ uint32_t prepared_longest(const uint8_t *exact_region
 // blob = folded pair table (one copy), exact tables with two words behind them (how many folded entries do not resolve two
 // symbols, and the length of the longest code; a code of a single symbol is one bit long and leaves half the entries
 // unresolved), single-symbol tables, wide pair tables.  The first block makes the first two, the others share the rest.
-__global__ void __launch_bounds__(1024) huffman_prepare_kernel(HuffArgs targs, uint8_t *blob) {
+static __global__ void __launch_bounds__(1024) huffman_prepare_kernel(HuffArgs targs, uint8_t *blob) {
     __shared__ HuffTables tab;
     __shared__ uint32_t flagged, longest;
     if (threadIdx.x == 0) flagged = longest = 0u;

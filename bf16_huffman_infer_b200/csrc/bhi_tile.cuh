@@ -546,7 +546,7 @@ static int tile_launch_r(const Layer &L, const typename Codec::Args &targs, cons
 }
 
 template <class Codec>
-static int tile_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
+int tile_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
                        int B, cudaStream_t st) {
     const int r = tile_rows_per_warp(L, sm_count());
     TilePlan plan{};

@@ -504,7 +504,7 @@ static bool tileq_plan(const Layer &L, int B, uint32_t ans_bits, TqPlan &P) {
 }
 
 template <class Codec>
-static int tileq_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
+int tileq_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t *prepared, const uint16_t *X, uint16_t *Y,
                         int B, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16)) return kStagedDeclined;
     if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31)) return kStagedDeclined;
