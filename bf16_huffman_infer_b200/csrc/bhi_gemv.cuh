@@ -744,6 +744,11 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             rem[q] = L.rem + static_cast<int64_t>(record_of(u, row_of(q, u.n, (lane >> 1) & 3))) * L.Nc + (lane >> 3) * 128 +
                      (NB > 0 ? wig * 32 + (lane & 1) * 16 : (lane & 7) * 16);
     };
+    // A row's 32 bytes of a block are two rows of an 8 x 8 matrix, whose words the lanes want as ldmatrix deals them: one
+    // instruction for two blocks of both quads instead of four loads.  Lane i supplies row i % 8 of matrix i / 8.
+    // (49152 x 4096, limit6, one row 89.1 us, so 87.2; 12288 x 4096, eight rows 29.9, 29.1; rANS 144.2, 145.3, so not there.)
+    constexpr bool kRemMatrix = kHuff;
+    const uint32_t rem_lane = kRemMatrix ? 16u * (lane & 7) + 128u * ((lane >> 3) & 1) + 512u * (lane >> 4) : 4u * lane;
     uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
     auto fetch = [&](int n, int blk, uint32_t to) {
         const uint32_t bytes = blk + (lane >> 3) < nblk ? 16u : 0u, dst = rem_at + to + 16u * lane;
@@ -918,7 +923,13 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
             uint32_t xo = kRing ? 0u : static_cast<uint32_t>(cur.k * nblk) * 256u;
             auto pair = [&](auto which, uint32_t rw, uint32_t xa, bool both) {
                 constexpr uint32_t j = decltype(which)::value;          // 0 or 2: block of the chunk
-                uint32_t e[n][2][2];
+                uint32_t e[n][2][2], rems[4];                           // sign/mantissa words: [quad][block]
+                if constexpr (!kRemMatrix) {
+                } else if constexpr (n > 1) {
+                    ldmatrix_x4<j * 128u>(rems, rw);
+                } else {
+                    ldmatrix_x2<j * 128u>(*reinterpret_cast<uint32_t (*)[2]>(rems), rw);
+                }
                 D::step(ctx, dec, e);
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
@@ -926,7 +937,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                         uint32_t w0[n], w1[n];
 #pragma unroll
                         for (int q = 0; q < n; q++) {
-                            const uint32_t w = q == 0 ? (i == 0 ? lds_now<j * 128u>(rw) : lds_now<j * 128u + 128u>(rw))
+                            const uint32_t w = kRemMatrix ? rems[2 * q + i] : q == 0 ? (i == 0 ? lds_now<j * 128u>(rw) : lds_now<j * 128u + 128u>(rw))
                                                       : (i == 0 ? lds_now<j * 128u + 512u>(rw) : lds_now<j * 128u + 640u>(rw));
                             w0[q] = bitselect(prmt(w, 0u, 0x1100u), e[q][i][0], kRemMask);
                             w1[q] = bitselect(prmt(w, 0u, 0x3322u), e[q][i][1], kRemMask);
@@ -970,7 +981,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                     fetch(nxt.n, 0, half ^ kRemChunk);
                 }
                 x_wait();
-                const uint32_t rw = rem_at + half + 4u * lane, xa = kRing ? x_slot * G.x_slot : xo;
+                const uint32_t rw = rem_at + half + rem_lane, xa = kRing ? x_slot * G.x_slot : xo;
                 const int left = nblk - blk;
                 using J0 = std::integral_constant<uint32_t, 0>;
                 using J2 = std::integral_constant<uint32_t, 2>;
