@@ -747,7 +747,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     // A row's 32 bytes of a block are two rows of an 8 x 8 matrix, whose words the lanes want as ldmatrix deals them: one
     // instruction for two blocks of both quads instead of four loads.  Lane i supplies row i % 8 of matrix i / 8.
     // (49152 x 4096, limit6, one row 89.1 us, so 87.2; 12288 x 4096, eight rows 29.9, 29.1; rANS 144.2, 145.3, so not there.)
-    constexpr bool kRemMatrix = kHuff;
+    constexpr bool kRemMatrix = kHuff, kFewPairs = kFew && !kHuff;
     const uint32_t rem_lane = kRemMatrix ? 16u * (lane & 7) + 128u * ((lane >> 3) & 1) + 512u * (lane >> 4) : 4u * lane;
     uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
     auto fetch = [&](int n, int blk, uint32_t to) {
@@ -849,12 +849,13 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     clear();
     // ldmatrix: lane i supplies the address of row i % 8 of matrix i / 8: pairs 8j.., 8j + 4.., 32 + 8j.., 32 + 8j + 4.. of a
-    // block.  Rows past the batch repeat the last one; their products are never read.  Few rows: two matrices, rows 0..3 of pairs
-    // 8j.. and 0..3 of pairs 8j + 4.., and the same of pairs 32 + 8j.. .
+    // block.  Rows past the batch repeat the last one; their products are never read.  Few rows: rows 0..3 of pairs 8j.. and 0..3 of
+    // pairs 8j + 4.., the same of pairs 32 + 8j.., and for rANS both again of the next block (49152 x 4096 144.2 us, so
+    // 142.7; limit6 86.9, 87.8, so not there).
     uint32_t x_row[kAcc];
 #pragma unroll
     for (int g = 0; g < kAcc; g++)
-        x_row[g] = kFew ? xs + min(lane & 3, max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 2) & 1) + 128u * ((lane >> 3) & 1)
+        x_row[g] = kFew ? xs + min(lane & 3, max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 2) & 1) + 128u * (kFewPairs ? lane >> 3 : (lane >> 3) & 1)
                         : xs + min(8 * g + (lane & 7), max(B, 1) - 1) * G.x_pitch + 32u * wig + 16u * ((lane >> 3) & 1) + 128u * (lane >> 4);
     const int x_total = kRing ? x_segments() : 0;
     int x_slot = 0, x_seg = 0;
@@ -931,6 +932,8 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                     ldmatrix_x2<j * 128u>(*reinterpret_cast<uint32_t (*)[2]>(rems), rw);
                 }
                 D::step(ctx, dec, e);
+                uint32_t few[4];
+                if constexpr (kFewPairs) ldmatrix_x4<j * 256u>(few, x_row[0] + xa);
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
                     if (i == 0 || both) {
@@ -944,8 +947,14 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                         }
                         if constexpr (kFew) {
                             uint32_t f[2];
-                            if (i == 0) ldmatrix_x2<j * 256u>(f, x_row[0] + xa);
-                            else ldmatrix_x2<j * 256u + 256u>(f, x_row[0] + xa);
+                            if constexpr (kFewPairs) {
+                                f[0] = few[2 * i];
+                                f[1] = few[2 * i + 1];
+                            } else if (i == 0) {
+                                ldmatrix_x2<j * 256u>(f, x_row[0] + xa);
+                            } else {
+                                ldmatrix_x2<j * 256u + 256u>(f, x_row[0] + xa);
+                            }
                             mma_bf16_16x8x16(c[0][0], w0[0], n > 1 ? w0[n - 1] : 0u, w1[0], n > 1 ? w1[n - 1] : 0u, f[0], f[1]);
                         } else if constexpr (NB > 0) {
 #pragma unroll
@@ -1165,7 +1174,7 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     G.x_pitch = G.x_slot = 0;
     if (f.x == GemvX::resident) {
         const uint64_t pitch = static_cast<uint64_t>(L.S) * L.Nc * 2u + (few ? 2u : 1u) * kXPad;
-        x_bytes = pitch * B;
+        x_bytes = pitch * B + (few ? 256u : 0u);                       // two blocks are read together, the last one's neighbour too
         G.x_pitch = static_cast<uint32_t>(pitch);
     } else if (f.x == GemvX::ring) {
         G.x_pitch = 2u * kXSegCols + kXPad;

@@ -13,7 +13,7 @@ uses for that are still available (``compress_groups``) and produce the same wor
 """
 from __future__ import annotations
 
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import os
 
@@ -203,8 +203,9 @@ class _Plan:
         exp = torch.zeros(_checked_total(total), dtype=torch.int32, device=dev)
         self.cls._emit_pass(layer, self.tables, self.offsets, exp)
         if to_cpu:
-            return self.cls(rem=transfer.download(layer.rem, layer.host_rem), exp=transfer.download(exp),
-                            offsets=transfer.download(self.offsets), **_tables_home(self.luts))
+            home = _tables_home(self.luts)                             # under way before the downloads, which wait for the stream
+            rem, exp, offsets = transfer.download(layer.rem, layer.host_rem), transfer.download(exp), transfer.download(self.offsets)
+            return self.cls(rem=rem, exp=exp, offsets=offsets, **home())
         # the buffers must be complete in memory before a fused kernel with launch overlap reads them
         torch.cuda.current_stream(dev).synchronize()
         return self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **self.luts)
@@ -221,11 +222,17 @@ def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor
     return out
 
 
-def _tables_home(tables: Dict[str, Tensor]) -> Dict[str, Tensor]:
-    """The way back."""
-    packed = torch.cat([t.view(torch.uint8) for t in tables.values()]).cpu()
-    parts = packed.split([t.numel() * t.element_size() for t in tables.values()])
-    return {name: part.clone().view(t.dtype) for (name, t), part in zip(tables.items(), parts)}
+def _tables_home(tables: Dict[str, Tensor]) -> Callable[[], Dict[str, Tensor]]:
+    """The way back: the copy is enqueued here, and the tables are taken from it once the stream has been waited for."""
+    packed = torch.cat([t.view(torch.uint8) for t in tables.values()])
+    here = torch.empty(packed.shape, dtype=torch.uint8, device="cpu", pin_memory=True)
+    here.copy_(packed, non_blocking=True)
+
+    def taken() -> Dict[str, Tensor]:
+        parts = here.split([t.numel() * t.element_size() for t in tables.values()])
+        return {name: part.clone().view(t.dtype) for (name, t), part in zip(tables.items(), parts)}
+
+    return taken
 
 
 def _compress(a: Tensor, split_k: int, coders: Sequence[type], to_cpu: bool) -> "HuffmanWeight":
