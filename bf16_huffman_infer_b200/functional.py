@@ -189,10 +189,11 @@ class _Plan:
     def __init__(self, cls, layer: _Ingested, result: Tensor, on_device: bool = True):
         self.cls, self.layer = cls, layer
         made = cls._device_tables(layer.counts, result[1:]) if on_device else None
+        self.on_device = made is not None
         if made is None:
             codec = cls._codec_of(layer.histogram)
-            made = _tables_to(cls.get_lut_kwargs(codec), layer.w.device), cls._encoder_tables(codec, layer.w.device)
-        self.luts, self.tables = made
+            made = cls.get_lut_kwargs(codec), cls._encoder_tables(codec, layer.w.device)
+        self.luts, self.tables = made                                  # luts: where they were made
         rows = torch.empty(layer.rem.shape[:2], dtype=torch.int32, device=layer.w.device)
         cls._size_pass(layer, self.tables, rows)
         self.offsets = torch.empty_like(rows)
@@ -203,12 +204,14 @@ class _Plan:
         exp = torch.zeros(_checked_total(total), dtype=torch.int32, device=dev)
         self.cls._emit_pass(layer, self.tables, self.offsets, exp)
         if to_cpu:
-            home = _tables_home(self.luts)                             # under way before the downloads, which wait for the stream
+            home = _tables_home(self.luts) if self.on_device else lambda: self.luts          # under way before the downloads, which wait for the stream
             rem, exp, offsets = transfer.download(layer.rem, layer.host_rem), transfer.download(exp), transfer.download(self.offsets)
             return self.cls(rem=rem, exp=exp, offsets=offsets, **home())
+        luts = self.luts if self.on_device else _tables_to(self.luts, dev)
+        weight = self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **luts)          # while the records are being written
         # the buffers must be complete in memory before a fused kernel with launch overlap reads them
         torch.cuda.current_stream(dev).synchronize()
-        return self.cls(rem=layer.rem, exp=exp, offsets=self.offsets, **self.luts)
+        return weight
 
 
 def _tables_to(tables: Dict[str, Tensor], dev: torch.device) -> Dict[str, Tensor]:
