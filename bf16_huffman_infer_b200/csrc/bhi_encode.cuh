@@ -32,8 +32,9 @@ __global__ void huffman_encode_chars_kernel(const uint8_t *__restrict__ data, in
 
 // One entry of an rANS encoding model.  A state is below freq << 32 <= 2^47 when it is divided (models have at most 15 bits),
 // so its quotient by freq is the high half of (2 * state) * inv with inv = ceil(2^63 / freq): the excess
-// inv * freq - 2^63 is below freq <= 2^15 and 2^47 * 2^15 < 2^63, so no quotient is off by one.  (A 64-bit division in its place lies on the serial
-// chain of every stream: size and emit pass over a 12288 x 4096 layer took 279 and 287 us with it, 81 and 95 us now.)
+// inv * freq - 2^63 is below freq <= 2^15 and 2^47 * 2^15 < 2^63, so no quotient is off by one.  (A 64-bit division in its place lies on the
+// serial chain of every stream: size and emit pass over a 12288 x 4096 layer took 279 and 287 us with it, 81 and 95 us with the
+// product; the whole-layer encoder's form of it is below.)
 struct AnsModel {
     uint64_t inv[256];
     uint32_t freq[256], cum[256];

@@ -1,8 +1,9 @@
 // Fused decode + product for 1..32 rows of X, and decode to a dense matrix (sm_100a).
 //
-// What bounds it.  Not HBM: an SM runs out of issue slots (half of them on the half-rate integer pipe) and shared-memory
-// wavefronts before the compressed bytes run out.  The layout spends both sparingly: table lookups without bank conflicts,
-// one X fragment for eight weight rows, no staging work in registers.
+// What bounds it.  Not HBM: an SM runs out of integer work (the half-rate pipe takes half of the issue slots) and of shared-memory
+// wavefronts before the compressed bytes run out; with all sixteen warps in the loop both are four fifths full and more, so that
+// work taken out of either counts and waits taken out do not.  The layout spends both sparingly: table lookups without bank
+// conflicts, one X fragment for eight weight rows, no staging work in registers.
 //
 // Work mapping.  A *unit* is up to eight consecutive weight rows (two quads) of one K-chunk; a group of four warps works on
 // a unit.  Warp j of the group (its *pass*) decodes streams 8j..8j+7 and 32+8j..32+8j+7 of all eight rows: lane
@@ -1324,18 +1325,15 @@ static int gemv_launch_rows(const Layer &L, const typename Dec::Codec::Args &tar
     return kStagedDeclined;
 }
 
-// Each eight rows more cost one product per decoded word, and their accumulators registers (96 per thread: 16 rows of limit6
-// fit, with pair tables and rANS 92 and 44 bytes are spilled, at 32 rows 180 to 512).  Here / by way of the dense matrix
-// and a library GEMM, in us, graph-replayed from HBM, at 16, 24 and 32 rows:
+// Each eight rows more cost one product per decoded word, and their accumulators registers (see kShiftsRegisters).  Here / by way
+// of the dense matrix and a library GEMM, in us, graph-replayed from HBM, at 16, 24 and 32 rows:
 //                12288 x 4096                        4096 x 12288                       50000 x 2560
-//   limit6       36.3/54.1  43.1/54.4  50.3/54.4     35.4/57.5  41.2/57.9  47.7/58.1    86.4/128  101/129  127/129
-//   escape       47.9/57.3  51.3/57.3  62.3/57.5     47.8/61.5  50.9/61.6  60.2/61.7    110/133   129/133  161/133
-//   reference    54.1/61.9  63.5/62.2  77.2/62.3     54.1/65.5  62.6/65.9  74.0/65.7    134/145   150/146  183/146
-//   rANS, 8 bit  59.0/62.9  65.7/63.0  75.3/63.0     57.5/67.3  62.4/67.4  72.0/67.5    143/151   166/152  194/151
-// (1024 x 4096: escape 11.8/18.5, 13.5/16.1, 15.8/16.3; rANS 11.6/18.7, 15.5/16.4, 17.8/16.7.)  Longer codes than limit6's
-// would be served faster by the dense matrix from 25 rows on, rANS from 17.  They are not: with so few rows the library
-// divides the columns among its blocks and adds their sums as BF16, up to 1.5 % of the results' rms off, where the sums here
-// stay in 32 bits (0.2 %, the rounding of the result).
+//   limit6       36.0/54.1  41.1/54.4  48.3/54.4     35.9/57.5  40.3/57.9  47.5/58.1    82.9/128  95.9/129  115/129
+//   escape       44.9/57.3  47.9/57.3  56.7/57.5     45.4/61.5  49.6/61.6  59.3/61.7    102/133   120/133  135/133
+//   rANS, 8 bit  55.5/62.9  61.2/62.7  67.2/62.7     54.8/67.3  60.9/67.4  66.0/67.5    136/151   149/152  166/151
+// (1024 x 4096: escape 10.9/18.5, 12.4/16.1, 14.6/16.3; rANS 11.7/18.7, 13.2/16.4, 15.6/16.7.)  Only rANS would be served faster by
+// the dense matrix, from 25 rows on.  It is not: with so few rows the library divides the columns among its blocks and adds their
+// sums as BF16, up to 1.5 % of the results' rms off, where the sums here stay in 32 bits (0.2 %, the rounding of the result).
 constexpr int kGemvMaxRows = 32;
 
 // B rows of X (0: the dense matrix into Y).  pair_complete: the caller knows that no code of the prepared table is longer
