@@ -216,15 +216,21 @@ struct GemvPair {
     static __device__ __forceinline__ uint32_t lookup(uint32_t w) { return lds_table<kTableAt>(w & kMask); }
     // A flagged entry `e` at cursor p: the second symbol takes a lookup of its own, a code longer than the index the exact
     // tables.  Advances p; the entry returned has the two symbols and no bits.
-    static __device__ __forceinline__ uint32_t resolve(const GemvCtx &c, uint32_t e, uint32_t &p, uint32_t o, uint32_t limit) {
+    // With the window (`whole`: all of its 32 bits count), which still holds the second code where the first was resolved.
+    template <bool whole>
+    static __device__ __forceinline__ uint32_t resolve(const GemvCtx &c, uint32_t e, uint32_t window, uint32_t &p, uint32_t o, uint32_t limit) {
         uint32_t bits = e & 15u;
         if (e & kEntExact) {
             const uint2 f = huff_exact_symbol(ring_window(c, p + 2u, o), c.exact);
             e = f.x << 7;
             bits = f.y;
+            p = min(p + bits, limit);
+            window = ring_window(c, p, o);
+        } else {
+            p = min(p + bits, limit);
+            window = whole ? __funnelshift_r(window, 0u, bits) : ring_window(c, p, o);
         }
-        p = min(p + bits, limit);
-        const uint32_t f = lookup(ring_window(c, p, o));
+        const uint32_t f = lookup(window);
         uint32_t s = f >> 7;
         bits = (f >> 16) & 15u;
         if (f & kEntExact) {
@@ -236,21 +242,23 @@ struct GemvPair {
         return (e & 0x7F80u) | (s << 23);
     }
     // The flagged entries of one block, stream by stream, in one piece of code for all streams of a lane: copies of it for
-    // each would not fit the instruction cache.  blk = 0: w gets the window of the next block.
+    // each would not fit the instruction cache.  blk = 0: w gets the window of the next block.  Every instruction here counts: a
+    // quarter to a half of the blocks have a flagged entry in some lane (flags gathered by bytes, the first block's second code
+    // taken from the window that is here: 12288 x 4096 escape 33.4 us, so 32.9; reference tables 32.3, 31.9).
     template <int blk, int n>
     static __device__ __forceinline__ void resolve_block(const GemvCtx &c, GemvPair (&d)[n], uint32_t (&e)[n][2][2], uint32_t (&w)[n][2]) {
         uint32_t flags = 0u;
 #pragma unroll
         for (int q = 0; q < n; q++) flags |= e[q][blk][0] | e[q][blk][1];
         if (flags & kFlags) {
-            uint32_t todo = 0u;
-#pragma unroll
-            for (int z = 0; z < 2 * n; z++) todo |= (e[z >> 1][blk][z & 1] & kFlags) ? 1u << z : 0u;
+            // one byte per stream, with one flag at most
+            uint32_t todo = prmt(e[0][blk][0], e[0][blk][1], 0x0040u) & (kFlags | kFlags << 8);
+            if (n > 1) todo |= prmt(e[n - 1][blk][0], e[n - 1][blk][1], 0x4000u) & (kFlags << 16 | kFlags << 24);
 #pragma unroll 1
             do {
-                const int z = __ffs(todo) - 1;
+                const int z = (__ffs(todo) - 1) >> 3;
                 todo &= todo - 1u;
-                uint32_t p = 0u, o = 0u, limit = 0u, entry = 0u;
+                uint32_t p = 0u, o = 0u, limit = 0u, entry = 0u, window = 0u;
 #pragma unroll
                 for (int y = 0; y < 2 * n; y++)
                     if (y == z) {
@@ -258,8 +266,9 @@ struct GemvPair {
                         o = d[y >> 1].off + ((y & 1) ? 128u : 0u);
                         limit = d[y >> 1].plim;
                         entry = e[y >> 1][blk][y & 1];
+                        if (blk == 0) window = w[y >> 1][y & 1];
                     }
-                entry = resolve(c, entry, p, o, limit);
+                entry = resolve<blk == 0>(c, entry, window, p, o, limit);
                 const uint32_t next = blk == 0 ? ring_window(c, p, o) : 0u;
 #pragma unroll
                 for (int y = 0; y < 2 * n; y++)
