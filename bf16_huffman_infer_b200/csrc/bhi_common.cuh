@@ -52,12 +52,25 @@ __device__ __forceinline__ uint16_t f32_to_bf16_rn(float f) {
     return h;
 }
 
+// X and a bias may be what the previous kernel in the stream writes while this one has already started (launch overlap): they
+// are read after the wait for it, and not by way of the read-only path (__ldg), whose data has to stand for a kernel's whole life.
+__device__ __forceinline__ uint32_t load_written(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint16_t load_written(const uint16_t *p) {
+    uint16_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // An output value: the 32-bit sum rounded to BF16, then the layer's bias (if it has one) added to that value and the
 // result rounded again - what a separate addition of BF16 tensors gives.
 __device__ __forceinline__ uint16_t finish_value(float v, const uint16_t *bias, int m) {
     const uint16_t h = f32_to_bf16_rn(v);
     if (bias == nullptr) return h;
-    return f32_to_bf16_rn(__uint_as_float(static_cast<uint32_t>(h) << 16) + __uint_as_float(static_cast<uint32_t>(__ldg(bias + m)) << 16));
+    return f32_to_bf16_rn(__uint_as_float(static_cast<uint32_t>(h) << 16) + __uint_as_float(static_cast<uint32_t>(load_written(bias + m)) << 16));
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -496,9 +496,11 @@ __device__ __forceinline__ void copy_x_row(uint32_t dst, const uint16_t *src, ui
     if (bulk) {
         bulk_copy_g2s(dst, src, bytes, bar);
     } else {
-        for (uint32_t i = 4u * lane; i < bytes; i += 128u) {
-            const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(src) + (i >> 2));
+        for (uint32_t i = 4u * lane; i < bytes; i += 256u) {           // (two at a time; a block of columns is 256 bytes)
+            const uint32_t *p = reinterpret_cast<const uint32_t *>(src) + (i >> 2);
+            const uint32_t v = load_written(p), w = load_written(p + 32);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + i), "r"(v) : "memory");
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + i + 128u), "r"(w) : "memory");
         }
     }
 }
@@ -1083,7 +1085,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
                     if (exchange) keep(b, row, v);
                     else if (B <= BHI_MAX_BATCH) Y[static_cast<int64_t>(b) * L.M + row] = finish_value(v, bias, row);
                     else Y[static_cast<int64_t>(b) * L.M + row] =
-                        f32_to_bf16_rn(bias ? v + __uint_as_float(static_cast<uint32_t>(__ldg(bias + row)) << 16) : v);
+                        f32_to_bf16_rn(bias ? v + __uint_as_float(static_cast<uint32_t>(load_written(bias + row)) << 16) : v);
                 }
             }
         }

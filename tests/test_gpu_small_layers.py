@@ -84,6 +84,42 @@ def test_chains_of_small_layers(algo):
         assert torch.equal(a, b) and torch.equal(a, c) and torch.equal(a, d)
 
 
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+@pytest.mark.parametrize("K,depth", [(1024, 12), (4096, 6)])
+def test_chains_of_unaligned_inputs(algo, K, depth):
+    """X is what the layer before wrote, 4 bytes past an aligned address, so it comes by plain loads; the bias is a layer's
+    output too.  (4096 rows are past the launch form of small layers.)"""
+    layers = [_weight(algo, make_weight(K + 2, K, i, K ** -0.5).to(DEV)) for i in range(depth)]
+    x = make_input(1, K, 9).to(DEV)
+
+    def chain():
+        out = [x]
+        for i, w in enumerate(layers):
+            y = w._forward(out[-1], out[-1].flatten().new_zeros(K + 2) if i == 0 else last.flatten())
+            last = y
+            out.append(y.flatten()[2:].view(1, K))
+        return out
+
+    want = chain()
+    torch.cuda.synchronize()
+    bias = torch.zeros(K + 2, dtype=torch.bfloat16, device=DEV)
+    for i, w in enumerate(layers):
+        assert want[i].data_ptr() % 16 == (4 if i else 0)
+        y = w._forward(want[i].clone(), None)[0] + bias
+        assert torch.equal(y[2:], want[i + 1][0])
+        bias = y
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = chain()
+    for _ in range(20):
+        for y in replayed[1:]:
+            y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(want, replayed))
+
+
 @pytest.mark.parametrize("sigma", [0.8, 2.5])
 @pytest.mark.parametrize("algo", ["huffman", "ans"])
 def test_small_layers_of_uneven_rows(algo, sigma):
