@@ -534,8 +534,12 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6 36.5 (stays as it was) / 41.6 / 50.9, - / 40.6 / 48.5.
 template <class Dec, int NB, int NG, bool kRing>
 constexpr bool kShiftsRegisters = kRing && NG == 4 && (NB > 2 || !std::is_same<Dec, GemvSingle>::value);
-template <class Dec, int NB, int NG, bool kRing>
-constexpr int kRingThreads = !kRing ? 0 : kShiftsRegisters<Dec, NB, NG, kRing> ? 128 : 32;
+// The launch has to hold what both sides have in the end: setmaxnreg waits without limit for registers that are not there.  The
+// compiler's count may be below the launch bounds', so each such kernel's is looked at before its first launch.
+constexpr int kShiftAtLaunch = 96, kShiftUp = 112, kShiftDown = 32;
+static_assert(kShiftAtLaunch * (512 + 128) >= kShiftUp * 512 + kShiftDown * 128, "more registers than the launch brings");
+template <bool kRing, bool kShift>
+constexpr int kRingThreads = !kRing ? 0 : kShift ? 128 : 32;
 
 // NB = groups of eight X rows (0: no product, the dense matrix is written instead).  NG = groups of four warps per CTA.
 // Two: two CTAs share an SM, so the next kernel's CTAs start as this one's leave.  Four: one CTA per SM, for launches whose
@@ -550,8 +554,8 @@ constexpr int kRingThreads = !kRing ? 0 : kShiftsRegisters<Dec, NB, NG, kRing> ?
 // kShard: a layer whose rows are shared among ranks (1: results staged, 2: stored one by one).  An argument of the template,
 // because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
 // layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
-template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew>
-__global__ void __launch_bounds__(NG * kGemvWarps * 32 + kRingThreads<Dec, NB, NG, kRing>, NG == 2 ? 2 : 1)
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew, bool kShift>
+__global__ void __launch_bounds__(NG * kGemvWarps * 32 + kRingThreads<kRing, kShift>, NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
             PeerSet peers, GemvGeom G, GemvConsts kc) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -634,9 +638,8 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     // ---- the warp that fills the X ring.  (With the readers filling it between their chunks, the last reader of a segment
     // its next one, the refill lay on the slowest warp and cost half as much again as the decoding.)
-    constexpr bool kShift = kShiftsRegisters<Dec, NB, NG, kRing>;
     if (kRing && warp >= NG * kGemvWarps) {
-        if constexpr (kShift) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if constexpr (kShift) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kShiftDown));
         __syncthreads();                                               // the readers' barrier before their loop
         if (warp > NG * kGemvWarps) {
             if (exchange) __syncthreads();                             // exchange_finish's
@@ -676,7 +679,7 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
         return;
     }
 
-    if constexpr (kShift) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    if constexpr (kShift) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kShiftUp));
     // ---- units ---------------------------------------------------------------------------------------------------------
     // A set is a pair of quads, or one quad: the last of an odd number, and both of a pair that has, in any chunk, a record
     // longer than the ring takes beside seven of that length.  For each set, the chunks in order.  The group's first warp
@@ -1213,13 +1216,14 @@ template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kF
 static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
                       cudaStream_t st) {
-    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf, kFew>;
-    if (int rc = staged_prepare(kernel)) return rc;
+    constexpr bool kShift = kShiftsRegisters<Dec, NB, NG, kRing>;
+    auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf, kFew, kShift>;
+    if (int rc = staged_prepare(kernel, kSmemMax, kShift ? kShiftAtLaunch : 0)) return rc;
     PeerSet ps{};
     if (peers) ps = *peers;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NG * kGemvWarps * 32 + kRingThreads<Dec, NB, NG, kRing>);
+    cfg.blockDim = dim3(NG * kGemvWarps * 32 + kRingThreads<kRing, kShift>);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

@@ -295,7 +295,7 @@ __device__ __forceinline__ void build_fast_table(uint32_t *fast, const AnsTables
 bool overlap_launches();     // process-wide switch, see bhi_set_launch_overlap
 
 template <class K>
-static int staged_prepare(K kernel, int bytes = kSmemMax) {
+static int staged_prepare(K kernel, int bytes = kSmemMax, int registers = 0) {
     // Opt in to the large dynamic shared-memory carve-out once per device and kernel.  Keyed by the
     // kernel's address: instantiations that differ only in a non-type argument share their pointer type.
     static std::mutex mu;
@@ -308,6 +308,12 @@ static int staged_prepare(K kernel, int bytes = kSmemMax) {
     if (!(bits >> dev & 1u)) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
+        if (registers) {                           // as many per thread as the kernel's register shift counts on
+            cudaFuncAttributes a;
+            e = cudaFuncGetAttributes(&a, kernel);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncGetAttributes");
+            if (a.numRegs < registers) return fail(BHI_ERR_CUDA, "kernel was compiled with fewer registers than it shifts between its warps");
+        }
         bits |= 1ull << dev;
     }
     return BHI_OK;
