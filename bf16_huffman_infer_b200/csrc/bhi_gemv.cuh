@@ -1321,6 +1321,8 @@ static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &tar
 //   limit6   512 x 2048  4.1/3.7   1024 x 4096  6.3/5.5   2048 x 2048  5.7/4.4   2368 x 2048  5.9/4.5   2368 x 4096  8.3/7.0
 //            1024 x 6144 (two chunks)  6.5/5.8; beyond the line  4096 x 2048  7.3/7.7   2048 x 6144  9.1/10.3   4096 x 4096  11.2/12.7
 //   rANS     512 x 3584  7.6/6.8   1024 x 4096  9.2/8.0   2048 x 2048  7.6/6.2   2048 x 4096  11.5/11.1
+// Without launch overlap no next kernel comes early, half of each SM would stand empty and the form is not taken (one row: 1024 x 4096
+// limit6 7.9/8.3, 2368 x 4096 limit6 9.4/10.2, rANS 13.4/14.7).
 // More than two chunks are divided among four groups instead (512 x 18944: 9.1/12.9, 512 x 12288: 11.1/10.5).  Pair tables of
 // 14 bits leave no room beside themselves and of 13 gain only where a group has one quad at most and often not then
 // (1024 x 1024 escape 4.2/3.8, 1024 x 4096 8.2/8.1, 512 x 2048 reference 6.0/6.3, 2048 x 2048 8.4/9.7), so they stay out.
@@ -1363,7 +1365,7 @@ int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t
                        const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int B, bool pair_complete, cudaStream_t st) {
     if (!staged_shape_ok(L) || !aligned(prepared, 16) || B > kGemvMaxRows) return kStagedDeclined;
     if (static_cast<int64_t>(L.S) * L.M >= (1ll << 31) || L.exp_words >= (1ll << 32)) return kStagedDeclined;
-    const bool half = B >= 1 && B <= 8 && peers == nullptr && gemv_groups() == 0 && L.S <= kHalfChunks &&
+    const bool half = overlap_launches() && B >= 1 && B <= 8 && peers == nullptr && gemv_groups() == 0 && L.S <= kHalfChunks &&
                       L.S * ((L.M + 3ll) / 4) <= static_cast<int64_t>(kHalfUnits) * sm_count();
     if constexpr (std::is_same<Codec, HuffCodec>::value) {
         if (half && pair_complete) {

@@ -224,6 +224,22 @@ class Abi:
         return rem, exp, offsets, rows
 
 
+def launched(call):
+    """Names of the kernels that ``call`` launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as seen:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in seen.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+
+def gemv_arguments(call):
+    """Template arguments of the one fused kernel that ``call`` launches: decoder, NB, NG, kRing, kShard, kHalf, kFew, kShift."""
+    found = [re.search(r"gemv_kernel<(?:bhi::)?(.*), (\d), (\d), (\w+), (\d), (\w+), (\w+), (\w+)>", n) for n in launched(call)]
+    (match,) = [m for m in found if m]
+    return [{"true": 1, "false": 0}.get(a, a) if i == 0 or not a.isdigit() else int(a) for i, a in enumerate(match.groups())]
+
+
 def to_device(arrs, dev):
     out = {}
     for k, v in arrs.items():

@@ -5,7 +5,7 @@ import ctypes
 import pytest
 import torch
 
-from _util import Abi, make_input, make_weight, rel_err
+from _util import Abi, gemv_arguments, make_input, make_weight, rel_err
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -41,6 +41,30 @@ def test_edges_of_small_layers(algo, bits, M, K):
         assert torch.equal(weight._forward(x, bias), y + bias)
     abi.check(abi.lib.bhi_debug_status(ctypes.byref(status)))
     assert status.value == 0
+
+
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+@pytest.mark.parametrize("M,K", [(512, 2048), (1024, 4096)])
+def test_without_launch_overlap(algo, M, K):
+    """Half of each SM is left to the next kernel only where that one may come early; the results are the same either way."""
+    from bf16_huffman_infer_b200 import ops
+    W = make_weight(M, K, M).to(DEV)
+    weight = _weight(algo, W)
+    for rows in (1, 2, 8):
+        x = make_input(rows, K, rows).to(DEV)
+        ref = (x.double() @ W.double().T).cpu().numpy()
+        previous = ops.set_launch_overlap(True)
+        try:
+            beside = weight._forward(x, None)
+            if rows == 1:
+                assert gemv_arguments(lambda: weight._forward(x, None))[5] == 1
+            ops.set_launch_overlap(False)
+            alone = weight._forward(x, None)
+            assert gemv_arguments(lambda: weight._forward(x, None))[5] == 0
+        finally:
+            ops.set_launch_overlap(previous)
+        for y in (beside, alone):
+            assert rel_err(y.float().cpu().numpy(), ref) <= 1e-2
 
 
 @pytest.mark.parametrize("algo", ["huffman", "ans"])
