@@ -157,3 +157,17 @@ def test_small_layers_of_uneven_rows(algo, sigma):
             scale = ref.abs().amax(0, keepdim=True).clamp(min=1e-30)               # row by row, so that small rows count as much
             y = weight._forward(x, None).double()
             assert rel_err((y / scale).cpu().numpy(), (ref / scale).cpu().numpy()) <= 1e-2, rows
+
+
+@pytest.mark.parametrize("algo,bits,M,K,half", [("ans", 8, 2368, 2048, 1), ("ans", 8, 1024, 4096, 1), ("ans", 8, 2372, 2048, 0), ("ans", 8, 1536, 4096, 0),
+                                                ("ans", 8, 1024, 6144, 0), ("ans", 12, 1536, 4096, 1), ("huffman", 8, 2368, 4096, 1)])
+def test_which_layers_are_small(algo, bits, M, K, half):
+    """The line is drawn by the quads of an SM, for 8-bit rANS by their columns too; on either side the results are right."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are for 148 SMs")
+    W = make_weight(M, K, M).to(DEV)
+    weight = _weight(algo, W, bits)
+    x = make_input(2, K, 5).to(DEV)
+    y = weight._forward(x, None)
+    assert gemv_arguments(lambda: weight._forward(x, None))[5] == half
+    assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).cpu().numpy()) <= 1e-2
