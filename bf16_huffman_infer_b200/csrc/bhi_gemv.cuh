@@ -531,9 +531,11 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // Sixteen warps and one more have 96 registers each (five warps share a quarter of the register file).  Where that spills, the
 // one more is a warpgroup, of which one warp works: it gives registers back, so that the sixteen can have 112 (640 x 96 at the
 // launch = 512 x 112 + 128 x 32).  12288 x 4096, 16 / 24 / 32 rows, in us, without and with it: escape 47.2 / 49.3 / 61.5,
-// 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6 36.5 (stays as it was) / 41.6 / 50.9, - / 40.6 / 48.5.
+// 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6, 32 rows, 50.5, 47.4.  limit6 of 24 rows has 40 bytes of
+// spills and stays as it is: 3584 x 4096 15.4, with the shift 16.0; 4096 x 12288 40.4, 41.6; 3584 x 18944 58.9, 60.6 (50000 x 2560
+// 98.4, 95.1).
 template <class Dec, int NB, int NG, bool kRing>
-constexpr bool kShiftsRegisters = kRing && NG == 4 && (NB > 2 || !std::is_same<Dec, GemvSingle>::value);
+constexpr bool kShiftsRegisters = kRing && NG == 4 && (NB > 3 || !std::is_same<Dec, GemvSingle>::value);
 // The launch has to hold what both sides have in the end: setmaxnreg waits without limit for registers that are not there.  The
 // compiler's count may be below the launch bounds', so each such kernel's is looked at before its first launch.
 constexpr int kShiftAtLaunch = 96, kShiftUp = 112, kShiftDown = 32;
@@ -761,8 +763,9 @@ gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, c
     };
     // A row's 32 bytes of a block are two rows of an 8 x 8 matrix, whose words the lanes want as ldmatrix deals them: one
     // instruction for two blocks of both quads instead of four loads.  Lane i supplies row i % 8 of matrix i / 8.
-    // (49152 x 4096, limit6, one row 89.1 us, so 87.2; 12288 x 4096, eight rows 29.9, 29.1; rANS 144.2, 145.3, so not there.)
-    constexpr bool kRemMatrix = kHuff, kFewPairs = kFew && !kHuff;
+    // (49152 x 4096, limit6, one row 89.1 us, so 87.2; 12288 x 4096, eight rows 29.9, 29.1; rANS 144.2, 145.3, so not there, nor
+    // for limit6 of 24 rows, whose registers are short: 4096 x 4096 16.0, so 16.3.)
+    constexpr bool kRemMatrix = kHuff && !(NB == 3 && std::is_same<Dec, GemvSingle>::value), kFewPairs = kFew && !kHuff;
     const uint32_t rem_lane = kRemMatrix ? 16u * (lane & 7) + 128u * ((lane >> 3) & 1) + 512u * (lane >> 4) : 4u * lane;
     uint32_t half = 0u;                                                // half of the warp's buffer that holds the current chunk
     auto fetch = [&](int n, int blk, uint32_t to) {

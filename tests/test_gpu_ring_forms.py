@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from _util import Abi, make_input, make_weight, rel_err
+from _util import Abi, gemv_arguments, make_input, make_weight, rel_err
 from test_gpu_exchange import Exchange, _launch, _status
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +42,24 @@ def test_rows_through_the_ring(algo, tables, M, K):
     torch.cuda.synchronize()
     assert _status(abi) == 0 and launches.tolist() == [2, 0]
     assert torch.equal(abi.gemv(algo, w, x, prepared=algo == "huffman"), y)
+
+
+@pytest.mark.parametrize("algo,tables,M,K,rows,shift", [
+    ("huffman", "limit6", 3584, 4096, 17, 0), ("huffman", "limit6", 520, 8576, 24, 0), ("huffman", "limit6", 520, 8576, 25, 1),
+])
+def test_which_launches_shift_registers(algo, tables, M, K, rows, shift):
+    """Some forms decode slower with the shift's registers than without them; on either side the results are right."""
+    from bf16_huffman_infer_b200 import ANSWeight, HuffmanWeight, set_huffman_tables
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are for 148 SMs")
+    W = make_weight(M, K, 4).to(DEV)
+    previous = set_huffman_tables(tables or "limit6")
+    try:
+        weight = (HuffmanWeight if algo == "huffman" else ANSWeight).compress(W, to_cpu=False)
+    finally:
+        set_huffman_tables(previous)
+    x = make_input(rows, K, rows).to(DEV)
+    y = weight._forward(x, None)
+    assert gemv_arguments(lambda: weight._forward(x, None))[-1] == shift
+    assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).cpu().numpy()) <= 1e-2
+    assert torch.equal(y, weight._forward(x, None))
