@@ -146,6 +146,7 @@ __device__ __forceinline__ void keep_order(uint32_t &a, uint32_t &b) { asm volat
 // wavefront each instead of about 3.5 (151936 x 4096, four rows: 276 us, with a 12-bit pair table 320).
 struct GemvSingle {
     using Codec = HuffCodec;
+    static constexpr bool kRans = false;
     static constexpr uint32_t kSecond = 64 * 128;          // byte offset of the second symbol's table
     static constexpr uint32_t kTableBytes = kSingleBytes;
     static constexpr uint32_t kMask = 63u << 7;
@@ -196,6 +197,7 @@ struct GemvSingle {
 template <int kBits>
 struct GemvPair {
     using Codec = HuffCodec;
+    static constexpr bool kRans = false;
     static constexpr uint32_t kTableBytes = 4u << kBits;
     static constexpr uint32_t kMask = ((1u << kBits) - 1u) << 2;
     static constexpr uint32_t kFlags = kEntSingle | kEntExact;
@@ -321,6 +323,7 @@ struct GemvPair {
 template <bool k8, uint32_t kBytes>
 struct GemvAns {
     using Codec = AnsCodec;
+    static constexpr bool kRans = true;
     static constexpr uint32_t kTableBytes = kBytes;
     static_assert(!k8 || kBytes == 64 * 1024, "the address permutation needs a stride of 256 bytes");
     struct Stream {
@@ -533,9 +536,14 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // launch = 512 x 112 + 128 x 32).  12288 x 4096, 16 / 24 / 32 rows, in us, without and with it: escape 47.2 / 49.3 / 61.5,
 // 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6, 32 rows, 50.5, 47.4.  limit6 of 24 rows has 40 bytes of
 // spills and stays as it is: 3584 x 4096 15.4, with the shift 16.0; 4096 x 12288 40.4, 41.6; 3584 x 18944 58.9, 60.6 (50000 x 2560
-// 98.4, 95.1).
+// 98.4, 95.1).  rANS decodes single quads slower with the shift's registers and pairs of them faster: up to eight rows it stays
+// without (512 x 16256 27.6, with the shift 28.9; 4096 x 12288 50.5, 50.4), and of 9 to 16 rows only launches that have pairs shift
+// (2300 x 4096, a quad for each group, 14.9, 15.0; 2400 x 4096, 18.5, 16.9; 2600 x 8576, units of one quad, 41.2, 43.0).
 template <class Dec, int NB, int NG, bool kRing>
-constexpr bool kShiftsRegisters = kRing && NG == 4 && (NB > 3 || !std::is_same<Dec, GemvSingle>::value);
+constexpr bool kShiftsRegisters = kRing && NG == 4 && (std::is_same<Dec, GemvSingle>::value ? NB > 3 : !Dec::kRans || NB > 1);
+// ... and whether there is a kernel without the shift beside it
+template <class Dec, int NB>
+constexpr bool kShiftsOrNot = Dec::kRans && NB == 2;
 // The launch has to hold what both sides have in the end: setmaxnreg waits without limit for registers that are not there.  The
 // compiler's count may be below the launch bounds', so each such kernel's is looked at before its first launch.
 constexpr int kShiftAtLaunch = 96, kShiftUp = 112, kShiftDown = 32;
@@ -1215,11 +1223,10 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
     return true;
 }
 
-template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew>
+template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew, bool kShift = kShiftsRegisters<Dec, NB, NG, kRing>>
 static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                       const uint16_t *bias, uint16_t *Y, const PeerSet *peers, int grid, const GemvGeom &G, uint32_t smem_bytes,
                       cudaStream_t st) {
-    constexpr bool kShift = kShiftsRegisters<Dec, NB, NG, kRing>;
     auto kernel = gemv_kernel<Dec, NB, NG, kRing, kShard, kHalf, kFew, kShift>;
     if (int rc = staged_prepare(kernel, kSmemMax, kShift ? kShiftAtLaunch : 0)) return rc;
     PeerSet ps{};
@@ -1242,8 +1249,10 @@ static int gemv_start_as(const Layer &L, const typename Dec::Codec::Args &targs,
 
 template <class Dec, int NB, int NG, bool kRing>
 static int gemv_start(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
-                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, bool direct, bool few, int grid, const GemvGeom &G,
+                      const uint16_t *bias, uint16_t *Y, const PeerSet *peers, bool direct, bool few, bool shift, int grid, const GemvGeom &G,
                       uint32_t smem_bytes, cudaStream_t st) {
+    if constexpr (kRing && NG == 4 && kShiftsOrNot<Dec, NB>)
+        if (!shift) return gemv_start_as<Dec, NB, NG, kRing, 0, false, false, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
     if constexpr (NB == 1) {
         if constexpr (kRing) {
             if (direct) return gemv_start_as<Dec, NB, NG, kRing, 2, false, false>(L, targs, prepared, X, bias, Y, peers, grid, G, smem_bytes, st);
@@ -1284,19 +1293,20 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
             if (grid > nquads) grid = nquads;
             GemvGeom G{};
             uint32_t smem_bytes = 0;
+            const bool shift = !kShiftsOrNot<Dec, NB> || (f.quads == 2 && nquads > 4 * grid);
             const bool few = NB == 1 && B <= kFewRows && peers == nullptr && f.x == GemvX::resident;
             if (!gemv_plan(L, B, Dec::kTableBytes, NB, few, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
             if (f.x == GemvX::ring) {
                 if constexpr (NB > 0 && kLast) {
                     if constexpr (NB == 1) {
-                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
+                        if (f.groups == 2) return gemv_start<Dec, NB, 2, true>(L, targs, prepared, X, bias, Y, peers, direct, few, shift, grid, G, smem_bytes, st);
                     }
-                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, true>(L, targs, prepared, X, bias, Y, peers, direct, few, shift, grid, G, smem_bytes, st);
                 }
             } else {
                 if constexpr (NB <= 1) {
-                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
-                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, direct, few, grid, G, smem_bytes, st);
+                    if (f.groups == 2) return gemv_start<Dec, NB, 2, false>(L, targs, prepared, X, bias, Y, peers, direct, few, shift, grid, G, smem_bytes, st);
+                    return gemv_start<Dec, NB, 4, false>(L, targs, prepared, X, bias, Y, peers, direct, few, shift, grid, G, smem_bytes, st);
                 }
             }
         }

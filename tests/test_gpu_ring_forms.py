@@ -46,6 +46,8 @@ def test_rows_through_the_ring(algo, tables, M, K):
 
 @pytest.mark.parametrize("algo,tables,M,K,rows,shift", [
     ("huffman", "limit6", 3584, 4096, 17, 0), ("huffman", "limit6", 520, 8576, 24, 0), ("huffman", "limit6", 520, 8576, 25, 1),
+    ("ans", None, 520, 16256, 5, 0), ("ans", None, 4096, 12288, 8, 0), ("ans", None, 2368, 4096, 9, 0), ("ans", None, 2372, 4096, 9, 1),
+    ("ans", None, 2600, 8576, 16, 0), ("ans", None, 2600, 8576, 9, 1), ("ans", None, 520, 4096, 17, 1),
 ])
 def test_which_launches_shift_registers(algo, tables, M, K, rows, shift):
     """Some forms decode slower with the shift's registers than without them; on either side the results are right."""
