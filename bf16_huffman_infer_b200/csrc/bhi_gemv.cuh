@@ -539,11 +539,15 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // 98.4, 95.1).  rANS decodes single quads slower with the shift's registers and pairs of them faster: up to eight rows it stays
 // without (512 x 16256 27.6, with the shift 28.9; 4096 x 12288 50.5, 50.4), and of 9 to 16 rows only launches that have pairs shift
 // (2300 x 4096, a quad for each group, 14.9, 15.0; 2400 x 4096, 18.5, 16.9; 2600 x 8576, units of one quad, 41.2, 43.0).
+// Pair tables of 25 to 32 rows gain but where a CTA has six quads of three and more chunks, that is two groups with a pair of quads and two with
+// one in step (25 rows, 3000 x 14336 64.1, 69.2; 3584 x 18944 88.2, 97.8; 4096 x 14336 68.5, 72.5; with at most five quads or with seven
+// and more of them 2600 x 14336 61.9, 59.7; 4300 x 14336 68.9, 69.9, of 32 rows 73.2, 68.3; of one chunk 3584 x 4096 22.1, 21.4, of two,
+// 32 rows, 4096 x 6144 34.0, 31.9).
 template <class Dec, int NB, int NG, bool kRing>
 constexpr bool kShiftsRegisters = kRing && NG == 4 && (std::is_same<Dec, GemvSingle>::value ? NB > 3 : !Dec::kRans || NB > 1);
 // ... and whether there is a kernel without the shift beside it
 template <class Dec, int NB>
-constexpr bool kShiftsOrNot = Dec::kRans && NB == 2;
+constexpr bool kShiftsOrNot = Dec::kRans ? NB == 2 : NB == 4 && !std::is_same<Dec, GemvSingle>::value;
 // The launch has to hold what both sides have in the end: setmaxnreg waits without limit for registers that are not there.  The
 // compiler's count may be below the launch bounds', so each such kernel's is looked at before its first launch.
 constexpr int kShiftAtLaunch = 96, kShiftUp = 112, kShiftDown = 32;
@@ -1293,7 +1297,8 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
             if (grid > nquads) grid = nquads;
             GemvGeom G{};
             uint32_t smem_bytes = 0;
-            const bool shift = !kShiftsOrNot<Dec, NB> || (f.quads == 2 && nquads > 4 * grid);
+            const bool shift = !kShiftsOrNot<Dec, NB> || (Dec::kRans ? f.quads == 2 && nquads > 4 * grid
+                                                                     : f.quads < 2 || L.S < 3 || nquads <= 5 * grid || nquads >= 7 * grid);
             const bool few = NB == 1 && B <= kFewRows && peers == nullptr && f.x == GemvX::resident;
             if (!gemv_plan(L, B, Dec::kTableBytes, NB, few, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
             if (f.x == GemvX::ring) {

@@ -48,6 +48,9 @@ def test_rows_through_the_ring(algo, tables, M, K):
     ("huffman", "limit6", 3584, 4096, 17, 0), ("huffman", "limit6", 520, 8576, 24, 0), ("huffman", "limit6", 520, 8576, 25, 1),
     ("ans", None, 520, 16256, 5, 0), ("ans", None, 4096, 12288, 8, 0), ("ans", None, 2368, 4096, 9, 0), ("ans", None, 2372, 4096, 9, 1),
     ("ans", None, 2600, 8576, 16, 0), ("ans", None, 2600, 8576, 9, 1), ("ans", None, 520, 4096, 17, 1),
+    ("huffman", "escape", 2960, 12288, 25, 1), ("huffman", "escape", 2964, 12288, 25, 0), ("huffman", "escape", 4143, 12288, 32, 1),
+    ("huffman", "escape", 4140, 12288, 32, 0), ("huffman", "escape", 3584, 6144, 32, 1), ("huffman", "escape", 3584, 18944, 32, 0),
+    ("huffman", "escape", 3584, 12288, 24, 1), ("huffman", "limit6", 3584, 12288, 32, 1),
 ])
 def test_which_launches_shift_registers(algo, tables, M, K, rows, shift):
     """Some forms decode slower with the shift's registers than without them; on either side the results are right."""
