@@ -188,7 +188,8 @@ class _Plan:
 
     def __init__(self, cls, layer: _Ingested, result: Tensor, on_device: bool = True):
         self.cls, self.layer = cls, layer
-        made = cls._device_tables(layer.counts, result[1:]) if on_device else None
+        # (a class derived from these may have its own get_lut_kwargs, which the host's way asks)
+        made = cls._device_tables(layer.counts, result[1:]) if on_device and cls in (HuffmanWeight, ANSWeight) else None
         self.on_device = made is not None
         if made is None:
             codec = cls._codec_of(layer.histogram)

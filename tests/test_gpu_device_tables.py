@@ -80,3 +80,32 @@ def test_layers_that_the_device_cannot_serve(home):
             ANSWeight.compress(ones, to_cpu=home == "cpu")
     finally:
         set_ans_precision(previous)
+
+
+@pytest.mark.parametrize("home", ["cpu", DEV])
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+def test_weight_classes_with_tables_of_their_own(algo, home):
+    """compress() of a derived class takes the tables that its get_lut_kwargs returns."""
+    from _util import make_weight
+    from bf16_huffman_infer_b200 import ANSWeight, HuffmanWeight
+    base = ANSWeight if algo == "ans" else HuffmanWeight
+    asked = []
+
+    class Mine(base):
+        @classmethod
+        def get_lut_kwargs(cls, codec):
+            tables = super().get_lut_kwargs(codec)
+            if algo == "huffman":
+                tables["LUT4"][:] = 9                                    # which codes of at most 8 bits do not reach
+            asked.append({k: v.clone() for k, v in tables.items()})
+            return tables
+
+    W = make_weight(64, 1024, 3).to(home)
+    weight = Mine.compress(W, to_cpu=home == "cpu")
+    assert type(weight) is Mine and len(asked) == 1
+    for name, table in asked[0].items():
+        assert torch.equal(getattr(weight, name).cpu(), table), name
+    assert torch.equal(weight.to(DEV).get_weight().cpu(), W.cpu())
+    for name, table in base.compress(W, to_cpu=False).kwargs().items():
+        if name != "LUT4":
+            assert torch.equal(getattr(weight, name), table), name
