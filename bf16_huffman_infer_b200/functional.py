@@ -131,10 +131,11 @@ def _record_offsets(words_per_row: Tensor) -> Tuple[Tensor, int]:
     return (ends - sizes).to(torch.int32).view(S, M), total
 
 
-def _record_offsets_async(words_per_row: Tensor) -> Tuple[Tensor, Tensor]:
-    """Same on the device, without waiting for it: offsets, and the total as an i64 tensor of one value."""
+def _record_offsets_async(words_per_row: Tensor, total: Optional[Tensor] = None) -> Tuple[Tensor, Tensor]:
+    """Same on the device, without waiting for it: offsets, and the total as an i64 tensor of one value (``total``, if given)."""
     offsets = torch.empty_like(words_per_row)
-    total = torch.empty(1, dtype=torch.int64, device=words_per_row.device)
+    if total is None:
+        total = torch.empty(1, dtype=torch.int64, device=words_per_row.device)
     ops.record_offsets(words_per_row, SLAB_ROWS, offsets, total)
     return offsets, total
 
@@ -197,8 +198,7 @@ class _Plan:
         self.luts, self.tables = made                                  # luts: where they were made
         rows = torch.empty(layer.rem.shape[:2], dtype=torch.int32, device=layer.w.device)
         cls._size_pass(layer, self.tables, rows)
-        self.offsets = torch.empty_like(rows)
-        ops.record_offsets(rows, SLAB_ROWS, self.offsets, result[:1])
+        self.offsets, _ = _record_offsets_async(rows, result[:1])
 
     def finish(self, total: int, to_cpu: bool) -> "HuffmanWeight":
         layer, dev = self.layer, self.layer.w.device
