@@ -25,9 +25,7 @@ def test_rows_through_the_ring(algo, tables, M, K):
     for rows in (8, 9, 16, 17, 24, 25, 32):
         x = make_input(rows, K, rows).to(DEV)
         y = weight._forward(x, None)
-        if y.numel() == 0:                                               # left to the dense matrix
-            assert rows > 8
-            continue
+        assert y.shape == (rows, M)                                      # empty: left to the dense matrix, which none of these is
         assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).cpu().numpy()) <= 1e-2, rows
         assert torch.equal(y, weight._forward(x, None))
     w, x = weight.kwargs(), make_input(8, K, 8).to(DEV)

@@ -171,3 +171,30 @@ def test_which_layers_are_small(algo, bits, M, K, half):
     y = weight._forward(x, None)
     assert gemv_arguments(lambda: weight._forward(x, None))[5] == half
     assert rel_err(y.float().cpu().numpy(), (x.double() @ W.double().T).cpu().numpy()) <= 1e-2
+
+
+@pytest.mark.parametrize("algo", ["huffman", "ans"])
+@pytest.mark.parametrize("M,K", [(1, 1152), (9, 1152), (1030, 4096), (5, 6144), (3000, 2176)])
+def test_infinities_and_nans(algo, M, K):
+    """Products with rows past the batch, absent quads, the other half and, for an odd number of blocks, what lies behind a row are
+    discarded: an infinity or a NaN of X shows in its own row only, one of the weight in its own column only."""
+    W = make_weight(M, K, 7)
+    if M > 4:
+        W[2, 7], W[3, K - 1], W[4, 130] = float("inf"), float("nan"), float("-inf")
+    W = W.to(DEV)
+    weight = _weight(algo, W)
+    for rows in (1, 2, 3, 4, 5, 8):
+        x = make_input(rows, K, rows).to(DEV)
+        clean = weight._forward(x, None)
+        odd = [r for r in (0, 1, 3, 7) if r < rows][-2:] if rows > 1 else []
+        for i, r in enumerate(odd):
+            x[r, 0 if i else K - 1] = float("nan") if i else float("inf")
+        y = weight._forward(x, None)
+        kept = [r for r in range(rows) if r not in odd]
+        assert torch.equal(y[kept].view(torch.int16), clean[kept].view(torch.int16))
+        ref = x.double() @ W.double().T
+        assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+        assert torch.equal(y[y.isinf()].sign().double(), ref[ref.isinf()].sign())
+        ok = torch.where(ref.isfinite(), ref, torch.zeros_like(ref))
+        got = torch.where(ref.isfinite(), y.double(), torch.zeros_like(ref))
+        assert rel_err(got.cpu().numpy(), ok.cpu().numpy()) <= 1e-2
