@@ -1165,6 +1165,11 @@ struct GemvForm {
     GemvX x;
 };
 
+static uint32_t mean_rows(const Layer &L) {      // word rows of a record
+    const int64_t per_row = 64 * static_cast<int64_t>(L.S) * L.M;
+    return static_cast<uint32_t>((L.exp_words + per_row * 15 / 16) / per_row);
+}
+
 // Shared-memory plan of a form; false when it does not fit.  The record ring is sized by the average record, so that it takes a
 // unit whose longest is a word row and an eighth longer (a word row where it has room for one unit only), and grows into what
 // the form leaves.  Rows of a layer whose scales differ have records of different lengths: a pair of quads that does not fit
@@ -1175,8 +1180,7 @@ static bool gemv_plan(const Layer &L, int B, uint32_t table_bytes, int acc_group
                       bool stage_results, GemvGeom &G, uint32_t &smem_bytes) {
     auto up = [](uint64_t v) { return static_cast<uint32_t>((v + 255u) & ~static_cast<uint64_t>(255u)); };
     const uint32_t cap = f.per_sm == 2 ? kSmemMax / 2 - 512 : kSmemMax;
-    const int64_t per_row = 64 * static_cast<int64_t>(L.S) * L.M;
-    const uint32_t rows = static_cast<uint32_t>((L.exp_words + per_row * 15 / 16) / per_row);
+    const uint32_t rows = mean_rows(L);
     const int nquads = (L.M + 3) / 4, nq = (nquads + grid - 1) / grid + 1;                         // most quads of a CTA
     // Few quads and several chunks: a group would take the chunks of its quad or two one after the other while others have
     // none.  The groups of a CTA share its quads instead and divide the chunks, where that shortens the longest group's
@@ -1319,7 +1323,10 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
     return kStagedDeclined;
 }
 
-// The kHalf launch of a small layer, in half an SM's shared memory.
+// The kHalf launch of a small layer, in half an SM's shared memory.  Where a group has pairs of quads, their ring has to have room for
+// rows that differ in scale, as the other forms' have: pairs that do not fit come quad by quad, each waiting for its records.  (Rows
+// log-normal with sigma 0.6, other forms / half an SM with less room than this: limit6, four rows, 1200 x 4096  7.3/9.6, 2300 x 4096
+// 8.4/10.1; sigma 0.35, rANS of 12 bits, two rows, 1200 x 4096  12.1/14.7.)  rANS has no longest code, so its rows differ more.
 template <class Dec>
 static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &targs, const uint8_t *prepared, const uint16_t *X,
                             const uint16_t *bias, uint16_t *Y, int B, cudaStream_t st) {
@@ -1327,7 +1334,10 @@ static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &tar
     for (int quarters = 8; quarters >= 4; quarters -= 4) {             // two units in the ring, or the one that most groups have
         GemvGeom G{};
         uint32_t smem_bytes = 0;
-        if (gemv_plan(L, B, Dec::kTableBytes, 1, B <= kFewRows, GemvForm{2, 2, 2, quarters, GemvX::resident}, grid, false, G, smem_bytes))
+        if (!gemv_plan(L, B, Dec::kTableBytes, 1, B <= kFewRows, GemvForm{2, 2, 2, quarters, GemvX::resident}, grid, false, G, smem_bytes)) continue;
+        const int cta_quads = (nquads + grid - 1) / grid;
+        const uint32_t rows = mean_rows(L), room = Dec::kRans ? 2u * rows - 1u : rows + rows / 2u + 1u;
+        if ((G.split ? cta_quads : (cta_quads + 1) / 2) < 2 || G.pair_rows >= room)
             return B <= kFewRows ? gemv_start_as<Dec, 1, 2, false, 0, true, true>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st)
                                  : gemv_start_as<Dec, 1, 2, false, 0, true, false>(L, targs, prepared, X, bias, Y, nullptr, grid, G, smem_bytes, st);
     }
