@@ -1354,7 +1354,9 @@ static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &tar
 // More than two chunks are divided among four groups instead (512 x 18944: 9.1/12.9, 512 x 12288: 11.1/10.5).  Pair tables of
 // 14 bits leave no room beside themselves and of 13 gain only where a group has one quad at most and often not then
 // (1024 x 1024 escape 4.2/3.8, 1024 x 4096 8.2/8.1, 512 x 2048 reference 6.0/6.3, 2048 x 2048 8.4/9.7), so they stay out.
-// 8-bit rANS fills half an SM's pipes sooner than it fills an SM's: there the form is taken up to kHalfAnsCols columns of quads per SM.
+// 8-bit rANS has the larger table in the other forms and fills half an SM's pipes sooner than an SM's: it takes the form for layers of one
+// chunk with more quads than half the SMs (one row: 300 x 3584  6.7/6.3   256 x 3584  6.1/6.3   128 x 4096  6.5/6.9; two chunks 425 x 7168
+// 7.9/8.8) and up to kHalfAnsCols columns of quads per SM.
 // Two rows, other forms / half an SM, back to back and with an elementwise kernel before each launch: 1024 x 4096  9.3/8.1, 11.6/11.9;
 // 2368 x 2048  8.1/6.7, 10.3/10.9; beyond the line  1536 x 4096  10.2/9.7, 12.7/13.8   2368 x 4096  11.9/11.1, 14.3/15.6   1024 x 6144
 // 9.7/8.9, 12.0/12.9.  (limit6, one row: 1024 x 4096  6.2/5.4, 8.7/9.1   2368 x 4096  8.2/6.7, 10.4/11.0; rANS, 12 bits 2368 x 4096
@@ -1413,7 +1415,8 @@ int gemv_launch(const Layer &L, const typename Codec::Args &targs, const uint8_t
     } else {
         // (a finer model on a layer of at most a quad per group: filling the larger table costs more than its conflicts)
         int rc = kStagedDeclined;
-        const bool half_ans = half && (targs.bits > 8 || L.S * ((L.M + 3ll) / 4) * L.Nc <= static_cast<int64_t>(kHalfAnsCols) * sm_count());
+        const int64_t nquads = (L.M + 3ll) / 4;
+        const bool half_ans = half && (targs.bits > 8 || (L.S == 1 && 2 * nquads > sm_count() && nquads * L.Nc <= static_cast<int64_t>(kHalfAnsCols) * sm_count()));
         if (half_ans && targs.bits == 8) rc = gemv_launch_half<GemvAns<true, 64 * 1024>>(L, targs, prepared, X, bias, Y, B, st);
         if (half_ans && rc == kStagedDeclined) rc = gemv_launch_half<GemvAns<false, 32 * 1024>>(L, targs, prepared, X, bias, Y, B, st);
         if (rc != kStagedDeclined) return rc;

@@ -160,7 +160,9 @@ def test_small_layers_of_uneven_rows(algo, sigma):
 
 
 @pytest.mark.parametrize("algo,bits,M,K,half", [("ans", 8, 2368, 2048, 1), ("ans", 8, 1024, 4096, 1), ("ans", 8, 2372, 2048, 0), ("ans", 8, 1536, 4096, 0),
-                                                ("ans", 8, 1024, 6144, 0), ("ans", 12, 2368, 2048, 1), ("ans", 12, 1024, 4096, 1), ("ans", 12, 1536, 4096, 0),
+                                                ("ans", 8, 1024, 6144, 0), ("ans", 8, 600, 5120, 0),
+                                                ("ans", 8, 296, 3584, 0), ("ans", 8, 297, 3584, 1), ("ans", 12, 296, 3584, 1), ("ans", 12, 600, 5120, 1),
+                                                ("ans", 12, 2368, 2048, 1), ("ans", 12, 1024, 4096, 1), ("ans", 12, 1536, 4096, 0),
                                                 ("huffman", 8, 2368, 4096, 1), ("huffman", 8, 2368, 4864, 0)])
 def test_which_layers_are_small(algo, bits, M, K, half):
     """The line is drawn by the quads of an SM, for 8-bit rANS by their columns too; on either side the results are right."""
