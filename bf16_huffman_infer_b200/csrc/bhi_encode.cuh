@@ -32,9 +32,9 @@ __global__ void huffman_encode_chars_kernel(const uint8_t *__restrict__ data, in
 
 // One entry of an rANS encoding model.  A state is below freq << 32 <= 2^47 when it is divided (models have at most 15 bits),
 // so its quotient by freq is the high half of (2 * state) * inv with inv = ceil(2^63 / freq): the excess
-// inv * freq - 2^63 is below freq <= 2^15 and 2^47 * 2^15 < 2^63, so no quotient is off by one.  (A 64-bit division in its place lies on the
-// serial chain of every stream: size and emit pass over a 12288 x 4096 layer took 279 and 287 us with it, 81 and 95 us with the
-// product; the whole-layer encoder's form of it is below.)
+// inv * freq - 2^63 is below freq <= 2^15 and 2^47 * 2^15 < 2^63, so no quotient is off by one.  (A 64-bit division in its place
+// lies on the serial chain of every stream: size and emit pass over a 12288 x 4096 layer took 279 and 287 us with it, 81 and 95 us
+// with the product; the whole-layer encoder's form of it is below.)
 struct AnsModel {
     uint64_t inv[256];
     uint32_t freq[256], cum[256];
@@ -158,10 +158,10 @@ __device__ __forceinline__ void store_rem(uint8_t *rem_row, int st, int blk, uin
 }
 
 // The coded words of every record.  What bounds it is the work per symbol (12288 x 4096: 43 us, of which HBM 19; with one table of
-// codes and one of lengths 62), so the table has a copy for each lane: the
-// 32 lookups of a warp always hit 32 different banks, and their address is the exponent where it stands in the weight (128 bytes
-// per entry).  Codes of at most 16 bits, which all but the reference's own builder make, stand with their lengths in one word and
-// are joined in pairs.  Blocks stay for several records, as the copies take a while to write.
+// codes and one of lengths 62), so the table has a copy for each lane: the 32 lookups of a warp always hit 32 different banks, and
+// their address is the exponent where it stands in the weight (128 bytes per entry).  Codes of at most 16 bits, which all but the
+// reference's own builder make, stand with their lengths in one word and are joined in pairs.  Blocks stay for several records, as
+// the copies take a while to write.
 constexpr int kEncBlocksPerSm = 6;               // 33 KB of shared memory each
 
 __global__ void __launch_bounds__(kEncThreads, kEncBlocksPerSm)
@@ -335,9 +335,10 @@ ans_emit_kernel(EncGeom g, const uint32_t *__restrict__ freq, const uint32_t *__
 // ---- sign/mantissa plane and exponent histogram ----------------------------------------------------------------------
 // One pass over a slab of rows: both results need every weight and neither needs a code table, so the weight is read
 // once for both, and slabs of a weight that is still on its way from the host are taken as they arrive.  Bound by HBM
-// (3 bytes per weight) and the shared-memory adds: 49 us at 12288 x 4096, 24 us without the plane.  A warp takes four consecutive 128-column blocks at a time: two 128-byte loads and one 128-byte
-// store per block, eight loads in flight per lane.  Counts go to a column of the block's table that belongs to the
-// lane: the 32 adds of a warp always hit 32 different banks, however few exponents occur.
+// (3 bytes per weight) and the shared-memory adds: 49 us at 12288 x 4096, 24 us without the plane.  A warp takes four consecutive
+// 128-column blocks at a time: two 128-byte loads and one 128-byte store per block, eight loads in flight per lane.  Counts go to
+// a column of the block's table that belongs to the lane: the 32 adds of a warp always hit 32 different banks, however few
+// exponents occur.
 constexpr int kSplitThreads = 256;
 constexpr int kSplitUnroll = 4;
 
@@ -401,9 +402,9 @@ split_histogram_kernel(const uint32_t *__restrict__ W, int rows, int row0, int M
 // The same tables as the host's builders make, on the device: the host would have to wait for the histogram, build, and send
 // the tables back before the size pass can start (two codes: 0.45 ms of a conversion of 0.9 ms).  One block each; what bounds
 // it is a chain of a few hundred dependent steps.  Histograms that these kernels do not serve (more symbols than the limit
-// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, which the size pass reads before anybody has
-// looked at the status; the host builds the tables after all (for more than 64 exponents in 13 ms, beside which that pass does not show:
-// 4096 x 4096 14.8 ms with and without it).
+// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, which the size pass reads before anybody
+// has looked at the status; the host builds the tables after all (for more than 64 exponents in 13 ms, beside which that pass does
+// not show: 4096 x 4096 14.8 ms with and without it).
 constexpr int kTableThreads = 256;
 constexpr int kLimitMax = 8;
 

@@ -8,18 +8,19 @@
 // Work mapping.  A *unit* is up to eight consecutive weight rows (two quads) of one K-chunk; a group of four warps works on
 // a unit.  Warp j of the group (its *pass*) decodes streams 8j..8j+7 and 32+8j..32+8j+7 of all eight rows: lane
 // (r = lane/8, s = (lane/4)%2, t = lane%4) runs streams sigma = 8j + 4s + t and sigma + 32 of row r of either quad, four
-// streams in all.  Per 128-column block a lane rebuilds two bf16x2 words per quad, exactly the B fragment of one
-// mma.sync.m16n8k16 whose eight columns n = lane/4 are (row r, half s); the sixteen A rows are (half s, batch row b),
-// b = 0..7, the same for both quads.  The products of mismatched halves (c1, c2) are discarded and c0 + c3 of lane (b, t)
-// is the dot product of batch row b with weight row t of the quad.  The cost of a launch hardly depends on the batch up to
-// eight rows; every eight more cost one more product per block and quad, none of the decoding.
+// streams in all.  Per 128-column block a lane rebuilds two bf16x2 words per quad.  Up to four rows of X (kFew) they are the A
+// fragment of one mma.sync.m16n8k16 for both quads: sixteen rows (row r and half s of either quad), X the eight columns (half s,
+// X row b).  More rows: a quad's two words are the B fragment of a product of its own, eight columns n = lane/4 that are (row r,
+// half s); the sixteen A rows are (half s, X row b), b = 0..7, the same for both quads.  Either way the products of unequal
+// halves are discarded, and the sum over s of the others is the dot product of X row b with row r of the quad.  Every eight
+// rows of X more cost one more product per block and quad, none of the decoding.
 //
 // Memory.  The records of a unit are brought into the group's ring by bulk async copies on one mbarrier, one unit ahead,
 // each record shifted by 32 bytes against the previous one, so that the 32 lanes of a warp (4 rows x 8 streams) read 32
 // different banks.  Sign/mantissa rows pass through shared memory too, in chunks of four blocks copied asynchronously by
 // the warp that reads them: as loads into registers they took a quarter of the register file and stalled every warp
-// (151936 x 4096, four rows: 312 us, as copies 276 us).  X lies in shared memory row by row, padded by 16 bytes, where one
-// ldmatrix yields a fragment; it comes by bulk copy, whole if it fits, else through a ring of four-block segments that all
+// (151936 x 4096, four rows: 312 us, as copies 276 us).  X lies in shared memory row by row, padded by 16 bytes (few rows: 32),
+// where one ldmatrix yields a fragment; it comes by bulk copy, whole if it fits, else through a ring of four-block segments that all
 // groups read in step.
 //
 // Results: the four warps of a group add their partial sums through shared memory in pass order (deterministic).
@@ -531,18 +532,23 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
     return sets;
 }
 
-// Sixteen warps and one more have 96 registers each (five warps share a quarter of the register file).  Where that spills, the
-// one more is a warpgroup, of which one warp works: it gives registers back, so that the sixteen can have 112 (640 x 96 at the
-// launch = 512 x 112 + 128 x 32).  12288 x 4096, 16 / 24 / 32 rows, in us, without and with it: escape 47.2 / 49.3 / 61.5,
-// 45.0 / 46.2 / 55.5; rANS 58.8 / 64.6 / 73.5, 55.4 / 61.6 / 67.2; limit6, 32 rows, 50.5, 47.4.  limit6 of 24 rows has 40 bytes of
-// spills and stays as it is: 3584 x 4096 15.4, with the shift 16.0; 4096 x 12288 40.4, 41.6; 3584 x 18944 58.9, 60.6 (50000 x 2560
-// 98.4, 95.1).  rANS decodes single quads slower with the shift's registers and pairs of them faster: up to eight rows it stays
-// without (512 x 16256 27.6, with the shift 28.9; 4096 x 12288 50.5, 50.4), and of 9 to 16 rows only launches that have pairs shift
-// (2300 x 4096, a quad for each group, 14.9, 15.0; 2400 x 4096, 18.5, 16.9; 2600 x 8576, units of one quad, 41.2, 43.0).
-// Pair tables of 25 to 32 rows gain but where a CTA has six quads of three and more chunks, that is two groups with a pair of quads and two with
-// one in step (25 rows, 3000 x 14336 64.1, 69.2; 3584 x 18944 88.2, 97.8; 4096 x 14336 68.5, 72.5; with at most five quads or with seven
-// and more of them 2600 x 14336 61.9, 59.7; 4300 x 14336 68.9, 69.9, of 32 rows 73.2, 68.3; of one chunk 3584 x 4096 22.1, 21.4, of two,
-// 32 rows, 4096 x 6144 34.0, 31.9).
+// Sixteen warps and one more have 96 registers each (five warps share a quarter of the register file).  With the register shift the
+// one more is a warpgroup, of which one warp works: it gives registers back, so that the sixteen can have 112 (640 x 96 at the launch
+// = 512 x 112 + 128 x 32).  Without it / with it, in us:
+//   pair tables, up to eight rows        4096 x 12288 39.9/39.1   12288 x 8192 73.2/71.6   8192 x 28672 167.9/164.0   (escape, 8 rows)
+//   ... 16, 24, 32 rows                  12288 x 4096  47.2/45.0   49.3/46.2   61.5/55.5
+//   ... 25 rows, some CTA with six       3000 x 14336  64.1/69.2   3584 x 18944  88.2/97.8   4096 x 14336  68.5/72.5: two groups have a pair
+//       quads of three and more chunks   of quads and two a single one, in step.  These do without, but with at most five quads or from seven
+//                                        on 2600 x 14336  61.9/59.7   4300 x 14336, 32 rows, 73.2/68.3, and with fewer chunks 3584 x 4096
+//                                        22.1/21.4   4096 x 6144, 32 rows, 34.0/31.9
+//   rANS, up to eight rows               512 x 16256  27.6/28.9   1024 x 8192  18.6/19.3   4096 x 12288  50.7/50.5: without.  Single quads
+//                                        are decoded slower with the shift's registers, pairs of them faster
+//   ... 9 to 16 rows                     2300 x 4096 (a quad for each group)  14.9/15.0   2600 x 8576 (units of one quad)  41.2/43.0: without;
+//                                        2400 x 4096  18.5/16.9   12288 x 4096  58.2/54.9
+//   ... 24, 32 rows                      12288 x 4096  64.6/61.6   73.5/67.2   (but 4096 x 12288, 32 rows, of such different scales, log-normal with
+//                                        sigma 0.8, that records are decoded from global memory, 234/248)
+//   limit6, 24 rows                      3584 x 4096  15.4/16.0   4096 x 12288  40.4/41.6   50000 x 2560  98.4/95.1: without
+//   ... 32 rows                          12288 x 4096  50.9/48.5
 template <class Dec, int NB, int NG, bool kRing>
 constexpr bool kShiftsRegisters = kRing && NG == 4 && (std::is_same<Dec, GemvSingle>::value ? NB > 3 : !Dec::kRans || NB > 1);
 // ... and whether there is a kernel without the shift beside it
@@ -564,10 +570,13 @@ constexpr int kRingThreads = !kRing ? 0 : kShift ? 128 : 32;
 // kFew: at most four rows of X.  The weights are then the sixteen A rows (row r and half s of either quad) and X the eight B
 // columns (half s, X row b): one product instead of two serves both quads of a block, and a fragment of X takes two wavefronts
 // of shared memory instead of four.  Of the products those of equal halves count, (r, s) x (s, b); their sum over s is the
-// result.  (One row: 49152 x 4096 limit6 92.9 us, so 90.4, rANS 151.0, 146.8; 12288 x 4096 escape 34.5, 33.8.)
+// result.  (One row: 49152 x 4096 limit6 92.9 us, so 90.1, rANS 150.4, 146.2; 12288 x 4096 escape 34.6, 34.0.)
 // kShard: a layer whose rows are shared among ranks (1: results staged, 2: stored one by one).  An argument of the template,
 // because code that a launch does not run costs it time all the same: each part taken out of the kernel made launches of small
 // layers 0.1 to 0.2 us shorter (2048 x 2048, limit6: 6.0 us with all three in one kernel, 5.8 so).
+// kShift: see kShiftsRegisters.
+// (The ring forms of two groups have an SM to themselves, but bounds for one CTA, and up to 168 registers, made them slower:
+// 8192 x 16256 of 120 exponents, escape, 417.4 us, so 419.1; row-sharded, whose 96 registers spill 16 to 40 bytes, 427.5, 430.1.)
 template <class Dec, int NB, int NG, bool kRing, int kShard, bool kHalf, bool kFew, bool kShift>
 __global__ void __launch_bounds__(NG * kGemvWarps * 32 + kRingThreads<kRing, kShift>, NG == 2 ? 2 : 1)
 gemv_kernel(Layer L, typename Dec::Codec::Args targs, const uint8_t *prepared, const uint16_t *X, const uint16_t *bias, uint16_t *Y,
@@ -1345,22 +1354,21 @@ static int gemv_launch_half(const Layer &L, const typename Dec::Codec::Args &tar
 }
 
 // Layers of up to this many quads per SM, counting each of their chunks, take half of each SM: a unit of two quads, or two of
-// one, for each of an SM's two groups.  One row of X, back to back in a graph, in us, the other forms / half an SM:
-//   limit6   512 x 2048  4.1/3.7   1024 x 4096  6.3/5.5   2048 x 2048  5.7/4.4   2368 x 2048  5.9/4.5   2368 x 4096  8.3/7.0
-//            1024 x 6144 (two chunks)  6.5/5.8; beyond the line  4096 x 2048  7.3/7.7   2048 x 6144  9.1/10.3   4096 x 4096  11.2/12.7
-//   rANS     512 x 3584  7.6/6.8   1024 x 4096  9.2/8.0   2048 x 2048  7.6/6.2   2048 x 4096  11.5/11.1
-// Without launch overlap no next kernel comes early, half of each SM would stand empty and the form is not taken (one row: 1024 x 4096
-// limit6 7.9/8.3, 2368 x 4096 limit6 9.4/10.2, rANS 13.4/14.7).
+// one, for each of an SM's two groups.  Other forms / half an SM, in us, one row of X but where a count stands: back to back in a graph, and
+// with an elementwise kernel before each launch (after which nothing can start early; what comes before a launch is not known here):
+//   limit6         512 x 2048  3.9/3.5, 6.6/6.7   1024 x 4096  6.3/5.4, 8.8/9.2   2048 x 2048  5.6/4.2, 8.0/8.0   eight rows  6.0/4.5, 8.4/8.4
+//                  2368 x 4096  8.2/6.7, 10.5/11.0   1024 x 6144 (two chunks)  6.4/5.5, 8.9/9.2
+//                  beyond the line  4096 x 2048  7.3/7.7   2048 x 6144  9.1/10.3   4096 x 4096  11.2/12.7
+//   rANS, 8 bits   512 x 3584  7.5/6.7, 10.2/10.1   1024 x 4096  9.2/8.0, 11.5/11.9   2048 x 2048  7.6/6.7, 10.5/10.7   four rows  7.9/6.8, 10.3/10.8
+//   rANS, 12 bits  1024 x 4096  10.3/8.9, 13.5/13.1   2048 x 2048  9.1/8.0, 12.1/12.1   1180 x 6144  11.6/10.6   700 x 6144  10.1/10.4
+// 8-bit rANS has the larger table in the other forms and fills half an SM's pipes sooner than an SM's.  It takes the form for one chunk
+// (425 x 7168  7.9/8.8) with more quads than half the SMs (300 x 3584  6.7/6.3; 256 x 3584  6.1/6.3, 128 x 4096  6.5/6.9) and up to
+// kHalfAnsCols columns of quads per SM (two rows, beyond it, 1536 x 4096  10.2/9.7, 12.7/13.8   2368 x 4096  11.9/11.1, 14.3/15.6).
+// Without launch overlap no next kernel comes early, half of each SM would stand empty and the form is not taken (1024 x 4096 limit6
+// 7.9/8.3, 2368 x 4096 limit6 9.4/10.2, rANS 13.4/14.7).
 // More than two chunks are divided among four groups instead (512 x 18944: 9.1/12.9, 512 x 12288: 11.1/10.5).  Pair tables of
 // 14 bits leave no room beside themselves and of 13 gain only where a group has one quad at most and often not then
 // (1024 x 1024 escape 4.2/3.8, 1024 x 4096 8.2/8.1, 512 x 2048 reference 6.0/6.3, 2048 x 2048 8.4/9.7), so they stay out.
-// 8-bit rANS has the larger table in the other forms and fills half an SM's pipes sooner than an SM's: it takes the form for layers of one
-// chunk with more quads than half the SMs (one row: 300 x 3584  6.7/6.3   256 x 3584  6.1/6.3   128 x 4096  6.5/6.9; two chunks 425 x 7168
-// 7.9/8.8) and up to kHalfAnsCols columns of quads per SM.
-// Two rows, other forms / half an SM, back to back and with an elementwise kernel before each launch: 1024 x 4096  9.3/8.1, 11.6/11.9;
-// 2368 x 2048  8.1/6.7, 10.3/10.9; beyond the line  1536 x 4096  10.2/9.7, 12.7/13.8   2368 x 4096  11.9/11.1, 14.3/15.6   1024 x 6144
-// 9.7/8.9, 12.0/12.9.  (limit6, one row: 1024 x 4096  6.2/5.4, 8.7/9.1   2368 x 4096  8.2/6.7, 10.4/11.0; rANS, 12 bits 2368 x 4096
-// 14.3/13.2, 17.8/17.9.  What comes next is not known at a launch; the line is where the loss is half of the gain.)
 constexpr int kHalfUnits = 4, kHalfChunks = 2, kHalfAnsCols = 4 * 2048;
 
 // kLast: no other decoder is tried after this one, so it takes the less favourable forms too.  kMore: more than eight rows.
@@ -1380,12 +1388,13 @@ static int gemv_launch_rows(const Layer &L, const typename Dec::Codec::Args &tar
 // Each eight rows more cost one product per decoded word, and their accumulators registers (see kShiftsRegisters).  Here / by way
 // of the dense matrix and a library GEMM, in us, graph-replayed from HBM, at 16, 24 and 32 rows:
 //                12288 x 4096                        4096 x 12288                       50000 x 2560
-//   limit6       36.0/54.1  41.1/54.4  48.3/54.4     35.9/57.5  40.3/57.9  47.5/58.1    82.9/128  95.9/129  115/129
-//   escape       44.9/57.3  47.9/57.3  56.7/57.5     45.4/61.5  49.6/61.6  59.3/61.7    102/133   120/133  135/133
-//   rANS, 8 bit  55.5/62.9  61.2/62.7  67.2/62.7     54.8/67.3  60.9/67.4  66.0/67.5    136/151   149/152  166/151
-// (1024 x 4096: escape 10.9/18.5, 12.4/16.1, 14.6/16.3; rANS 11.7/18.7, 13.2/16.4, 15.6/16.7.)  Only rANS would be served faster by
-// the dense matrix, from 25 rows on.  It is not: with so few rows the library divides the columns among its blocks and adds their
-// sums as BF16, up to 1.5 % of the results' rms off, where the sums here stay in 32 bits (0.2 %, the rounding of the result).
+//   limit6       33.9/53.0  41.7/53.2  47.5/53.1     33.5/57.1  40.7/57.3  46.8/57.3    82.3/129  97.2/130  115/130
+//   escape       43.4/56.3  47.2/56.5  56.2/56.6     44.3/60.6  48.8/61.0  61.4/60.9    101/133   114/133  133/133
+//   rANS, 8 bit  55.1/61.8  60.8/62.1  66.9/62.1     54.4/66.6  60.1/66.8  65.6/66.9    136/151   149/152  165/152
+// (1024 x 4096: limit6 9.8/16.8, 11.8/15.2, 13.7/15.3; escape 10.7/18.7, 12.5/17.1, 14.4/17.2; rANS 11.5/19.2, 13.2/17.6, 15.5/17.8.)
+// Only rANS would be served faster by the dense matrix, from 25 rows on (pair tables alike there).  It is not: with so few rows the
+// library divides the columns among its blocks and adds their sums as BF16, up to 1.5 % of the results' rms off, where the sums here
+// stay in 32 bits (0.2 %, the rounding of the result).
 constexpr int kGemvMaxRows = 32;
 
 // B rows of X (0: the dense matrix into Y).  pair_complete: the caller knows that no code of the prepared table is longer

@@ -53,7 +53,8 @@ constexpr int kPreparedBytes = kPreparedWidest + (4 << kWidestBits);
 static_assert(sizeof(HuffTables) + 8 <= kExactBytes && sizeof(AnsTables) <= kExactBytes, "exact tables do not fit");
 static_assert((4 << kAnsBitsMax) * kCopies <= kLutBytes, "the largest rANS table does not fit the fast-table region");
 
-static __device__ int g_staged_status = 0;     // 0 = fine; otherwise the last failure code.  One for each source file of kernels:
+// 0 = fine; otherwise the last failure code.  Each source file of kernels has one of its own, which its take_status is for.
+static __device__ int g_staged_status = 0;
 
 // reads and clears this source file's
 static cudaError_t take_status(int *out) {
