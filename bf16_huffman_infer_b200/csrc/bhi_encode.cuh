@@ -402,8 +402,8 @@ split_histogram_kernel(const uint32_t *__restrict__ W, int rows, int row0, int M
 // The same tables as the host's builders make, on the device: the host would have to wait for the histogram, build, and send
 // the tables back before the size pass can start (two codes: 0.45 ms of a conversion of 0.9 ms).  One block each; what bounds
 // it is a chain of a few hundred dependent steps.  Histograms that these kernels do not serve (more symbols than the limit
-// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, which the size pass reads before anybody
-// has looked at the status; the host builds the tables after all (for more than 64 exponents in 13 ms, beside which that pass does
+// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, or with that frequency cut off in the decode
+// table: the size pass reads them before anybody has looked at the status; the host builds the tables after all (for more than 64 exponents in 13 ms, beside which that pass does
 // not show: 4096 x 4096 14.8 ms with and without it).
 constexpr int kTableThreads = 256;
 constexpr int kLimitMax = 8;
@@ -594,7 +594,7 @@ ans_tables_kernel(const long long *__restrict__ hist, int bits, uint32_t *freq, 
     const uint32_t f = scaled[tid];
     const int wide = __syncthreads_count(f > 0xFFFu);
     if (tid == 0) *status = wide > 0 || have != target;
-    if (wide > 0 || have != target) {
+    if (have != target) {
         freq[tid] = cum[tid] = 0u;
         for (int slot = tid; slot < target; slot += kTableThreads) lut[slot] = 0u;
         return;

@@ -260,7 +260,7 @@ int bhi_record_offsets(const int32_t *words_per_row, int split_k, int M, int sla
 
 /* Code tables from a histogram (i64 [256]) on the device: those of the optimal code with no length above `limit` (1..8) bits,
  * and an rANS model of `precision` probability bits with its decode table (2^precision words).  *status (device) becomes 0, or
- * nonzero, with tables of zeros, where the histogram cannot be served: more symbols than 2^limit, or a frequency that the table
+ * nonzero where the histogram cannot be served: more symbols than 2^limit (the tables are zeros), or a frequency that the table
  * word cannot hold. */
 int bhi_huffman_limit_tables(const int64_t *histogram, int limit, uint8_t *LUT1, uint8_t *LUT2, uint8_t *LUT3, uint8_t *LUT4,
                              uint8_t *code_lengths, uint32_t *code_values, int64_t *status, void *stream);

@@ -52,11 +52,9 @@ def test_rans_models(bits):
         codec = RANSEncoder(hist.tolist(), precision=bits)
         wide = max(codec.freq) > 0xFFF
         assert status.item() == wide
-        if wide:
-            assert not any(x.any() for x in (freq, cum, lut))
-            continue
         assert freq.tolist() == codec.freq and cum.tolist() == codec.cum, (n, hist)
-        assert torch.equal(lut.cpu(), ANSWeight.get_lut_kwargs(codec)["LUT"])
+        if not wide:
+            assert torch.equal(lut.cpu(), ANSWeight.get_lut_kwargs(codec)["LUT"])
 
 
 @pytest.mark.parametrize("home", ["cpu", DEV])
