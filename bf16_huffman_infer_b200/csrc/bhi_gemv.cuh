@@ -537,10 +537,10 @@ __device__ __forceinline__ int count_sets(const int32_t *offsets, int S, int M, 
 // = 512 x 112 + 128 x 32).  Without it / with it, in us:
 //   pair tables, up to eight rows        4096 x 12288 39.9/39.1   12288 x 8192 73.2/71.6   8192 x 28672 167.9/164.0   (escape, 8 rows)
 //   ... 16, 24, 32 rows                  12288 x 4096  47.2/45.0   49.3/46.2   61.5/55.5
-//   ... 25 rows, some CTA with six       3000 x 14336  64.1/69.2   3584 x 18944  88.2/97.8   4096 x 14336  68.5/72.5: two groups have a pair
-//       quads of three and more chunks   of quads and two a single one, in step.  These do without, but with at most five quads or from seven
-//                                        on 2600 x 14336  61.9/59.7   4300 x 14336, 32 rows, 73.2/68.3, and with fewer chunks 3584 x 4096
-//                                        22.1/21.4   4096 x 6144, 32 rows, 34.0/31.9
+//   ... 25 rows, some CTA with six       3000 x 14336  64.1/69.2   3584 x 18944  88.2/97.8   3630 x 7680  38.8/41.8: two groups have a pair of
+//       quads of several long chunks     quads and two a single one, in step.  These do without, but with at most five quads or from seven on
+//                                        2600 x 14336  61.9/59.7   4300 x 14336, 32 rows, 73.2/68.3, with one chunk 3584 x 4096  22.1/21.4,
+//                                        with short ones or rows 3630 x 9856 (11 blocks)  89.4/81.4   4096 x 6144, 32 rows, 34.0/31.9
 //   rANS, up to eight rows               512 x 16256  27.6/28.9   1024 x 8192  18.6/19.3   4096 x 12288  50.7/50.5: without.  Single quads
 //                                        are decoded slower with the shift's registers, pairs of them faster
 //   ... 9 to 16 rows                     2300 x 4096 (a quad for each group)  14.9/15.0   2600 x 8576 (units of one quad)  41.2/43.0: without;
@@ -1310,8 +1310,9 @@ static int gemv_launch_dec(const Layer &L, const typename Dec::Codec::Args &targ
             if (grid > nquads) grid = nquads;
             GemvGeom G{};
             uint32_t smem_bytes = 0;
-            const bool shift = !kShiftsOrNot<Dec, NB> || (Dec::kRans ? f.quads == 2 && nquads > 4 * grid
-                                                                     : f.quads < 2 || L.S < 3 || nquads <= 5 * grid || nquads >= 7 * grid);
+            const bool sixes = f.quads == 2 && nquads > 5 * grid && nquads < 7 * grid;       // some CTA has six quads
+            const bool long_chunks = L.S > 1 && L.Nc >= 12 * 128 && L.S * L.Nc >= 54 * 128;
+            const bool shift = !kShiftsOrNot<Dec, NB> || (Dec::kRans ? f.quads == 2 && nquads > 4 * grid : !(sixes && long_chunks));
             const bool few = NB == 1 && B <= kFewRows && peers == nullptr && f.x == GemvX::resident;
             if (!gemv_plan(L, B, Dec::kTableBytes, NB, few, f, grid, peers != nullptr && !direct, G, smem_bytes)) continue;
             if (f.x == GemvX::ring) {

@@ -48,7 +48,8 @@ def test_rows_through_the_ring(algo, tables, M, K):
     ("ans", None, 2600, 8576, 16, 0), ("ans", None, 2600, 8576, 9, 1), ("ans", None, 520, 4096, 17, 1),
     ("huffman", "escape", 2960, 12288, 25, 1), ("huffman", "escape", 2964, 12288, 25, 0), ("huffman", "escape", 4143, 12288, 32, 1),
     ("huffman", "escape", 4140, 12288, 32, 0), ("huffman", "escape", 3584, 6144, 32, 1), ("huffman", "escape", 3584, 18944, 32, 0),
-    ("huffman", "escape", 3584, 12288, 24, 1), ("huffman", "limit6", 3584, 12288, 32, 1),
+    ("huffman", "escape", 3584, 12288, 24, 1),
+    ("huffman", "escape", 3630, 9856, 25, 1), ("huffman", "escape", 3630, 7680, 25, 0), ("huffman", "escape", 3630, 6656, 25, 1), ("huffman", "limit6", 3584, 12288, 32, 1),
 ])
 def test_which_launches_shift_registers(algo, tables, M, K, rows, shift):
     """Some forms decode slower with the shift's registers than without them; on either side the results are right."""
