@@ -402,9 +402,9 @@ split_histogram_kernel(const uint32_t *__restrict__ W, int rows, int row0, int M
 // The same tables as the host's builders make, on the device: the host would have to wait for the histogram, build, and send
 // the tables back before the size pass can start (two codes: 0.45 ms of a conversion of 0.9 ms).  One block each; what bounds
 // it is a chain of a few hundred dependent steps.  Histograms that these kernels do not serve (more symbols than the limit
-// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, or with that frequency cut off in the decode
-// table: the size pass reads them before anybody has looked at the status; the host builds the tables after all (for more than 64 exponents in 13 ms, beside which that pass does
-// not show: 4096 x 4096 14.8 ms with and without it).
+// allows, a frequency that its field cannot hold) set `status` and leave tables of zeros, or with that frequency cut off in the
+// decode table: the size pass reads them before anybody has looked at the status.  The host builds the tables after all (for more
+// than 64 exponents in 13 ms, beside which that pass does not show: 4096 x 4096 14.8 ms with and without it).
 constexpr int kTableThreads = 256;
 constexpr int kLimitMax = 8;
 
